@@ -522,151 +522,6 @@ __device__ __forceinline__ float f16_at(const unsigned *w, int byte_off) {  // f
     return (byte_off & 2) ? f16hi(w[byte_off >> 2]) : f16lo(w[byte_off >> 2]);
 }
 
-template <int TYPE, int C>
-struct DequantR;
-
-template <int C>
-struct DequantR<B200_TYPE_Q4_0, C> {
-    static __device__ __forceinline__ void run(const unsigned (&w)[36], unsigned (&o)[32]) {
-#pragma unroll
-        for (int b = 0; b < 2; b++) {
-            constexpr int dummy = 0; (void)dummy;
-            const int base = 36 * C + 18 * b;  // byte offset of the block
-            const float d = f16_at(w, base), m8 = d * 8.0f;
-#pragma unroll
-            for (int j = 0; j < 16; j += 2) {
-                const unsigned q0 = BYTE_OF(w, base + 2 + j), q1 = BYTE_OF(w, base + 3 + j);
-                o[16 * b + j / 2]     = pack_bf16(d * byte_f<0>(q0 & 15) - m8, d * byte_f<0>(q1 & 15) - m8);
-                o[16 * b + 8 + j / 2] = pack_bf16(d * byte_f<0>(q0 >> 4) - m8, d * byte_f<0>(q1 >> 4) - m8);
-            }
-        }
-    }
-};
-
-template <int TYPE, int C>
-struct DequantRLegacy {
-    static __device__ __forceinline__ void run(const unsigned (&w)[group256_words(TYPE)], unsigned (&o)[32]) {
-        using L = LegacyLayout<TYPE>;
-#pragma unroll
-        for (int b = 0; b < 2; b++) {
-            const int base = 2 * L::BB * C + L::BB * b;  // byte offset of the block inside the 256-value group
-            const float d = f16_at(w, base);
-            float m = 0.f;
-            if constexpr (L::HAS_M) m = f16_at(w, base + 2);
-            if constexpr (TYPE == B200_TYPE_Q5_0) m = d * -16.0f;
-            unsigned qh = 0;
-            if constexpr (L::HAS_H) qh = BYTE_OF(w, base + L::QH) | (BYTE_OF(w, base + L::QH + 1) << 8) | (BYTE_OF(w, base + L::QH + 2) << 16) | (BYTE_OF(w, base + L::QH + 3) << 24);
-#pragma unroll
-            for (int j = 0; j < 16; j += 2) {
-                const unsigned q0 = BYTE_OF(w, base + L::QS + j), q1 = BYTE_OF(w, base + L::QS + 1 + j);
-                const unsigned l0 = (q0 & 15) | (((qh >> j) & 1u) << 4), l1 = (q1 & 15) | (((qh >> (j + 1)) & 1u) << 4);
-                const unsigned h0 = (q0 >> 4) | (((qh >> (16 + j)) & 1u) << 4), h1 = (q1 >> 4) | (((qh >> (17 + j)) & 1u) << 4);
-                o[16 * b + j / 2]     = pack_bf16(d * byte_f<0>(l0) + m, d * byte_f<0>(l1) + m);
-                o[16 * b + 8 + j / 2] = pack_bf16(d * byte_f<0>(h0) + m, d * byte_f<0>(h1) + m);
-            }
-        }
-    }
-};
-template <int C> struct DequantR<B200_TYPE_Q4_1, C> : DequantRLegacy<B200_TYPE_Q4_1, C> {};
-template <int C> struct DequantR<B200_TYPE_Q5_0, C> : DequantRLegacy<B200_TYPE_Q5_0, C> {};
-template <int C> struct DequantR<B200_TYPE_Q5_1, C> : DequantRLegacy<B200_TYPE_Q5_1, C> {};
-
-template <int C>
-struct DequantR<B200_TYPE_IQ4_NL, C> {
-    static __device__ __forceinline__ void run(const unsigned (&w)[36], unsigned (&o)[32]) {
-#pragma unroll
-        for (int b = 0; b < 2; b++) {
-            const int base = 2 * IQ4_NL_BYTES * C + IQ4_NL_BYTES * b;
-            iq4_unpack32([&](int k) { return BYTE_OF(w, base + 2 + k); }, f16_at(w, base), o + 16 * b);
-        }
-    }
-};
-template <int C>
-struct DequantR<B200_TYPE_IQ4_XS, C> {
-    static __device__ __forceinline__ void run(const unsigned (&w)[34], unsigned (&o)[32]) {
-        const float d = f16lo(w[0]);
-#pragma unroll
-        for (int b = 0; b < 2; b++)
-            iq4_unpack32([&](int k) { return BYTE_OF(w, 8 + 32 * C + 16 * b + k); }, d * iq4xs_scale(w[1], w[0] >> 16, 2 * C + b), o + 16 * b);
-    }
-};
-
-template <int C>
-struct DequantR<B200_TYPE_Q8_0, C> {
-    static __device__ __forceinline__ void run(const unsigned (&w)[68], unsigned (&o)[32]) {
-#pragma unroll
-        for (int b = 0; b < 2; b++) {
-            const int base = 68 * C + 34 * b;
-            const float d = f16_at(w, base), m128 = d * 128.0f;
-#pragma unroll
-            for (int j = 0; j < 32; j += 2) {
-                // int8 -> biased uint8 (x ^ 0x80 = x + 128), unbias after the multiply
-                const unsigned q0 = BYTE_OF(w, base + 2 + j) ^ 0x80u, q1 = BYTE_OF(w, base + 3 + j) ^ 0x80u;
-                o[16 * b + j / 2] = pack_bf16(d * byte_f<0>(q0) - m128, d * byte_f<0>(q1) - m128);
-            }
-        }
-    }
-};
-
-template <int TYPE, int C>
-struct DequantRK45 {
-    static constexpr int NW = TYPE == B200_TYPE_Q4_K ? 36 : 44;
-    static __device__ __forceinline__ void run(const unsigned (&w)[NW], unsigned (&o)[32]) {
-        constexpr int QS = (TYPE == B200_TYPE_Q4_K ? 4 : 12) + 8 * C;  // first word of this chunk's 32 qs bytes
-        const float d = f16lo(w[0]), dmin = f16hi(w[0]);
-        const unsigned sw[3] = {w[1], w[2], w[3]};
-#pragma unroll
-        for (int hf = 0; hf < 2; hf++) {
-            constexpr int dummy = 0; (void)dummy;
-            const int sb = 2 * C + hf;
-            int sc, mn;
-            k4_scale_min(sw, sb, sc, mn);
-            const float d1 = d * (float)sc, m1 = dmin * (float)mn;
-#pragma unroll
-            for (int i = 0; i < 8; i++) {  // word i holds bytes l = 4i .. 4i+3
-                unsigned x = (w[QS + i] >> (4 * hf)) & 0x0F0F0F0Fu;
-                if constexpr (TYPE == B200_TYPE_Q5_K) x |= ((w[4 + i] >> sb) & 0x01010101u) << 4;
-                o[16 * hf + 2 * i]     = pack_bf16(d1 * byte_f<0>(x) - m1, d1 * byte_f<1>(x) - m1);
-                o[16 * hf + 2 * i + 1] = pack_bf16(d1 * byte_f<2>(x) - m1, d1 * byte_f<3>(x) - m1);
-            }
-        }
-    }
-};
-template <int C> struct DequantR<B200_TYPE_Q4_K, C> : DequantRK45<B200_TYPE_Q4_K, C> {};
-template <int C> struct DequantR<B200_TYPE_Q5_K, C> : DequantRK45<B200_TYPE_Q5_K, C> {};
-
-template <int TYPE, int C>
-struct DequantRK23 {
-    static __device__ __forceinline__ void run(const unsigned (&w)[group256_words(TYPE)], unsigned (&o)[32]) {
-        dequant64_k23<TYPE>([&](int i) { return BYTE_OF(w, i); }, C, o);
-    }
-};
-template <int C> struct DequantR<B200_TYPE_Q2_K, C> : DequantRK23<B200_TYPE_Q2_K, C> {};
-template <int C> struct DequantR<B200_TYPE_Q3_K, C> : DequantRK23<B200_TYPE_Q3_K, C> {};
-
-template <int C>
-struct DequantR<B200_TYPE_Q6_K, C> {
-    static __device__ __forceinline__ void run(const unsigned (&w)[53], unsigned (&o)[32]) {
-        constexpr int half = C >> 1, hi = C & 1;
-        const float d = f16lo(w[52]);
-        const unsigned scw = w[48 + 2 * half + hi];  // 4 int8 scales of this chunk
-#pragma unroll
-        for (int g = 0; g < 4; g++) {
-            const int rlow = g >> 1, r = 2 * hi + rlow;
-            const float ds = d * (float)(int)(signed char)((scw >> (8 * g)) & 0xff), m32 = ds * 32.0f;
-#pragma unroll
-            for (int i = 0; i < 4; i++) {  // 4 values per word: l = 16*(g&1) + 4i ..
-                const int lw = 4 * (g & 1) + i;  // word index inside the 32-byte row
-                const unsigned lo = (w[16 * half + 8 * rlow + lw] >> (4 * hi)) & 0x0F0F0F0Fu;
-                const unsigned h2 = ((w[32 + 8 * half + lw] >> (2 * r)) & 0x03030303u) << 4;
-                const unsigned x = lo | h2;
-                o[8 * g + 2 * i]     = pack_bf16(ds * byte_f<0>(x) - m32, ds * byte_f<1>(x) - m32);
-                o[8 * g + 2 * i + 1] = pack_bf16(ds * byte_f<2>(x) - m32, ds * byte_f<3>(x) - m32);
-            }
-        }
-    }
-};
-
 // ================================================================ v2: asynchronous operand supply
 // Same tensor-core pipeline, but neither operand waits on a global load inside the producers:
 //   * B (bf16 activations) arrives by TMA (cp.async.bulk.tensor.2d, 128-byte swizzle applied by the copy engine) issued by
@@ -747,7 +602,7 @@ __global__ void __launch_bounds__(MQ2_THREADS, 1) mmq_tc2_kernel(const __grid_co
             fence_proxy_async_smem();
             mbar_arrive(&full_bar[s]);
         };
-        if constexpr (TYPE == B200_TYPE_BF16) {
+        {
             // dense bf16 rows: a K step is 128 bytes of the thread's row, stored as it is; the next step's bytes are in flight meanwhile
             const uint4 *q4 = reinterpret_cast<const uint4 *>(wrow) + (size_t)sb0 * 8;
             uint4 cur[8], nxt[8];
@@ -765,57 +620,6 @@ __global__ void __launch_bounds__(MQ2_THREADS, 1) mmq_tc2_kernel(const __grid_co
                 publish(kb, o);
 #pragma unroll
                 for (int i = 0; i < 8; i++) cur[i] = nxt[i];
-            }
-        } else {
-            // software pipeline: the raw bytes of group sb+1 are in flight (registers) while group sb is unpacked
-            constexpr int NW = group256_words(TYPE);
-            unsigned cur[NW], nxt[NW];
-            auto fetch = [&](unsigned (&w)[NW], int sb) {
-                if (row_ok) {
-                    if constexpr (TYPE == B200_TYPE_Q4_K || TYPE == B200_TYPE_Q5_K) {  // 16-byte aligned rows: LDG.128
-                        const uint4 *q4 = reinterpret_cast<const uint4 *>(wrow + (size_t)sb * G256);
-    #pragma unroll
-                        for (int i = 0; i < NW / 4; i++) {
-                            const uint4 v = __ldg(q4 + i);
-                            w[4 * i] = v.x; w[4 * i + 1] = v.y; w[4 * i + 2] = v.z; w[4 * i + 3] = v.w;
-                        }
-                    } else {
-                        // 2-byte aligned rows: 16-byte loads from the aligned-down address (a quarter of the LSU sector traffic of
-                        // 4-byte loads), then a word select (offset 0..3 words) and a funnel shift (0 or 2 bytes) per word
-                        const uintptr_t a = (uintptr_t)(wrow + (size_t)sb * G256);
-                        const uint4 *q4 = reinterpret_cast<const uint4 *>(a & ~(uintptr_t)15);
-                        const unsigned off = (unsigned)(a & 15) >> 2, sh = (unsigned)(a & 3) * 8;
-                        constexpr int NV = (NW + 1 + 3 + 3) / 4;
-                        unsigned t[NV * 4];
-    #pragma unroll
-                        for (int i = 0; i < NV; i++) {
-                            const uint4 v = __ldg(q4 + i);
-                            t[4 * i] = v.x; t[4 * i + 1] = v.y; t[4 * i + 2] = v.z; t[4 * i + 3] = v.w;
-                        }
-                        unsigned prev = (off & 2) ? ((off & 1) ? t[3] : t[2]) : ((off & 1) ? t[1] : t[0]);
-    #pragma unroll
-                        for (int i = 0; i < NW; i++) {
-                            const unsigned nx = (off & 2) ? ((off & 1) ? t[i + 4] : t[i + 3]) : ((off & 1) ? t[i + 2] : t[i + 1]);
-                            w[i] = __funnelshift_r(prev, nx, sh);
-                            prev = nx;
-                        }
-                    }
-                } else {
-    #pragma unroll
-                    for (int i = 0; i < NW; i++) w[i] = 0u;
-                }
-            };
-            fetch(cur, sb0);
-    #pragma unroll 1
-            for (int sb = 0; sb < nsb; sb++) {
-                if (sb + 1 < nsb) fetch(nxt, sb0 + sb + 1);
-                unsigned o[32];
-                DequantR<TYPE, 0>::run(cur, o); publish(sb * 4 + 0, o);
-                DequantR<TYPE, 1>::run(cur, o); publish(sb * 4 + 1, o);
-                DequantR<TYPE, 2>::run(cur, o); publish(sb * 4 + 2, o);
-                DequantR<TYPE, 3>::run(cur, o); publish(sb * 4 + 3, o);
-    #pragma unroll
-                for (int i = 0; i < NW; i++) cur[i] = nxt[i];
             }
         }
         mbar_wait(&tmem_full_bar, 0u);
@@ -1044,6 +848,10 @@ static int encode_rows(TmapBytes &tm, const void *base, int64_t K, int64_t rows,
     return B200_OK;
 }
 
+}  // namespace b200
+#include "mmq_pair.cuh"
+namespace b200 {
+
 template <int BN, bool GROUPED>
 static int bf16_gemm_launch(const MmqParams &p, int64_t n_pad, int64_t w_rows_per_product, cudaStream_t st, unsigned grid_y) {
     constexpr size_t smem = (size_t)bg_stages<BN>() * (MQ_BM * MQ_BK * 2 + BN * MQ_BK * 2) + 1024;
@@ -1139,15 +947,7 @@ static int mmq_dispatch_bn(const MmqParams &p, cudaStream_t st) {
             default: return mmq2_launch<TYPE, 256>(p, n_pad, st);
         }
     } else
-    if (p.K % 256 == 0 && !getenv("B200_MMQ_V1")) {
-        const int64_t n_pad = mmq_n_pad(p.N);
-        switch (mmq_bn(p.N)) {
-            case 32: return mmq2_launch<TYPE, 32>(p, n_pad, st);
-            case 64: return mmq2_launch<TYPE, 64>(p, n_pad, st);
-            case 128: return mmq2_launch<TYPE, 128>(p, n_pad, st);
-            default: return mmq2_launch<TYPE, 256>(p, n_pad, st);
-        }
-    }
+    if (p.K % 256 == 0) return mmq_pair_launch<TYPE, false>(p, mmq_n_pad(p.N), 0, 0, 0, st);
     if constexpr (TYPE != B200_TYPE_BF16) {
         switch (mmq_bn(p.N)) {
             case 32: return mmq_launch<TYPE, 32>(p, st);
@@ -1225,11 +1025,18 @@ __global__ void mid_gather_bf16_kernel(const float *__restrict__ b, const int *_
 }
 
 static int64_t mid_bn(int64_t n_rows, int n_expert) { return mmq_bn((n_rows + n_expert - 1) / n_expert); }
-static int64_t mid_max_tiles(int64_t n_rows, int n_expert) { return (n_rows + mid_bn(n_rows, n_expert) - 1) / mid_bn(n_rows, n_expert) + n_expert; }
+static int64_t mid_max_tiles(int64_t bn, int64_t n_rows, int n_expert) { return (n_rows + bn - 1) / bn + n_expert; }
+// quantised experts: the tile's width follows its rows, so the table's tiles are as wide as the accumulators allow unless experts are small
+static int64_t mid_tile(int type, int64_t n_rows, int n_expert) {
+    const int64_t bn = mid_bn(n_rows, n_expert);
+    return type == B200_TYPE_BF16 ? bn : bn < 128 ? 2 * bn : 256;
+}
 static size_t mid_xb_bytes(int64_t n_rows, int64_t K) { return ((size_t)n_rows * (size_t)K * 2 + 255) / 256 * 256; }
 
 template <int TYPE>
 static int mid_dispatch_bn(const MmqParams &p, int64_t bn, int64_t n_rows, unsigned grid_y, cudaStream_t st) {
+    if constexpr (TYPE != B200_TYPE_BF16) return mmq_pair_launch<TYPE, true>(p, n_rows, 0, grid_y, bn, st);
+    else
     switch (bn) {
         case 32: return mmq2_launch<TYPE, 32, true>(p, n_rows, st, grid_y);
         case 64: return mmq2_launch<TYPE, 64, true>(p, n_rows, st, grid_y);
@@ -1336,7 +1143,7 @@ extern "C" size_t b200_mul_mat_id_q_workspace_bytes(int type, int64_t K, int64_t
     (void)type; (void)M;
     const int64_t n_rows = n_used * T;
     if (K <= 0 || n_rows <= 0 || n_expert <= 0) return 0;
-    return mid_xb_bytes(n_rows, K) + sizeof(int) * (size_t)(1 + 3 * mid_max_tiles(n_rows, n_expert) + 2 * n_rows) + 256;
+    return mid_xb_bytes(n_rows, K) + sizeof(int) * (size_t)(1 + 3 * mid_max_tiles(mid_bn(n_rows, n_expert), n_rows, n_expert) + 2 * n_rows) + 256;
 }
 
 extern "C" int b200_mul_mat_id_q(int type, const void *as, size_t w_row_bytes, size_t expert_bytes, int32_t n_expert, const int32_t *ids,
@@ -1374,7 +1181,7 @@ extern "C" int b200_mul_mat_id_q(int type, const void *as, size_t w_row_bytes, s
         return B200_ERR_INVALID;
     }
     const cudaStream_t st = (cudaStream_t)stream;
-    const int64_t bn = mid_bn(n_rows, n_expert), max_tiles = mid_max_tiles(n_rows, n_expert);
+    const int64_t bn = mid_tile(type, n_rows, n_expert), max_tiles = mid_max_tiles(bn, n_rows, n_expert);
     __nv_bfloat16 *xb = (__nv_bfloat16 *)workspace;
     MidTables t;
     t.tile_tab = (int *)((unsigned char *)workspace + mid_xb_bytes(n_rows, K));

@@ -1,0 +1,725 @@
+// mmq_pair.cuh -- the prompt GEMM on pairs of SMs (tcgen05 cta_group::2), persistent over its tiles.  Included by mmq.cu, which holds the
+// block formats and the entry points.
+//
+//   dst[n][m] = sum_k W[m][k] * X[n][k]     W quantised (or dense bf16), X bf16 rows in the workspace, dst f32
+//
+// What bounds it: the tensor pipe once the weights are unpacked fast enough, and before that the L2.  One CTA with a 128 x 256 tile
+// fetches 32 KB of activations per K step of 64 (512 tensor cycles): 64 B per cycle and SM, more than the L2 gives 148 SMs.  So two CTAs
+// share a 256 x BN tile: each unpacks its own 128 weight rows into its shared memory and fetches HALF of the activation rows, and the
+// pair's one MMA reads both halves.
+//   * 16 producer warps a CTA, 8 weight rows each: a warp copies the raw blocks of its rows (256 values of each, contiguous 16-byte cp.async) into
+//     a ring of its own, one or two groups ahead, and unpacks them with packed f32 arithmetic, lane = (64-value chunk, row), into the
+//     128-byte-swizzled operand tiles of four K steps.  No barrier among the warps.
+//   * the MMA warp walks through its loop as a whole and elects a lane for the tcgen05 instructions only: loop counters and descriptors then
+//     live in uniform registers.  (With one lane in the loop every MMA needed a dozen vector instructions, each of which waits its turn
+//     among the producers: 190 cycles an MMA whatever its width.)
+//   * the accumulators are double-buffered in TMEM (2 x 256 columns): four epilogue warps store tile i while tile i + 1 is computed.
+//   * BN is chosen on the host so that the tiles fill the pairs evenly (mmq_pair_plan): 512 columns are 2 x 256 or 3 x 176, whichever leaves
+//     the last wave fuller.  In the grouped form (routed experts) the width of every tile follows its rows.
+// Every wait has a limit (PAIR_WAIT_LIMIT); a role that gives up tells its CTA and goes on without waiting, nothing is stored from then on,
+// *timeout is set, and the CTA stays until copies and MMAs in flight have ended.
+#pragma once
+
+namespace b200 {
+
+constexpr long long PAIR_WAIT_LIMIT = 4000000000LL;  // clock cycles: about two seconds
+constexpr int PAIR_PRODUCERS = 16;                   // warps that unpack, 8 rows of the CTA's 128 each
+constexpr int PAIR_MAX_STAGES = 8;
+constexpr int PAIR_SMEM = 232448 - 1024 - 1024;      // dynamic shared memory: what a CTA can have, less static data and alignment
+
+// 256-value groups of 128 rows as they lie in memory: 16-byte pieces a row (a 2-byte aligned row starts up to 14 bytes into its first one)
+__host__ __device__ constexpr bool raw_aligned(int t) { return t == B200_TYPE_Q4_K || t == B200_TYPE_Q5_K; }
+__host__ __device__ constexpr int raw_pieces(int t) { return (group256_bytes(t) + (raw_aligned(t) ? 0 : 14) + 15) / 16; }
+__host__ __device__ constexpr int raw_row(int t) { return (raw_pieces(t) | 1) * 16; }  // odd: rows start in different 16-byte bank groups
+__host__ __device__ constexpr int raw_slots(int t) { return t == B200_TYPE_BF16 ? 0 : raw_row(t) <= 192 ? 3 : 2; }
+__host__ __device__ constexpr int raw_bytes(int t) { return t == B200_TYPE_BF16 ? 0 : raw_slots(t) * MQ_BM * raw_row(t); }
+
+struct PairParams {
+    MmqParams q;
+    int64_t w_rows_per_product;  // dense weights by TMA: rows from one product (batch, expert) to the next
+    int bn;                      // columns of a tile (grouped: at most), a multiple of 16; grouped: of 32
+    int box;                     // activation rows of one TMA box
+    int stages;
+    int n_tiles_n, n_tiles_m;    // n_tiles_n of the grouped form: read from the tile table
+    int *timeout;
+};
+
+// ---------------------------------------------------------------- the pair's wrappers
+__device__ __forceinline__ unsigned cluster_rank() { unsigned r; asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r)); return r; }
+__device__ __forceinline__ void pair_sync() { asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+__device__ __forceinline__ bool elect_lane() {
+    unsigned e;
+    asm volatile("{\n.reg .pred p;\nelect.sync _|p, 0xffffffff;\nselp.u32 %0, 1, 0, p;\n}\n" : "=r"(e));
+    return e != 0;
+}
+__device__ __forceinline__ void tmem_alloc2(unsigned *smem_dst, unsigned ncols) {
+    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(smem_dst)), "r"(ncols) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void tmem_dealloc2(unsigned taddr, unsigned ncols) {
+    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
+}
+__device__ __forceinline__ void tc_mma2_bf16(unsigned tmem_d, unsigned long long adesc, unsigned long long bdesc, unsigned idesc, unsigned accumulate) {
+    asm volatile(
+        "{\n"
+        ".reg .pred p;\n"
+        "setp.ne.b32 p, %4, 0;\n"
+        "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n"
+        "}\n" ::"r"(tmem_d),
+        "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
+        : "memory");
+}
+// arrives on `bar` of both CTAs when the MMAs issued so far have retired
+__device__ __forceinline__ void tc_commit2(unsigned bar) {
+    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(bar), "h"((unsigned short)3) : "memory");
+}
+// arrive on `bar` of the pair's first CTA.  (The default semantics: what the barrier guards is in shared memory or TMEM and complete when the
+// arrival is issued; a release at cluster scope would wait for the thread's outstanding memory operations, about 1000 cycles a K step.)
+__device__ __forceinline__ void mbar_arrive_leader(unsigned bar) {
+    asm volatile(
+        "{\n"
+        ".reg .b32 ra;\n"
+        "mapa.shared::cluster.u32 ra, %0, 0;\n"
+        "mbarrier.arrive.shared::cluster.b64 _, [ra];\n"
+        "}\n" ::"r"(bar)
+        : "memory");
+}
+__device__ __forceinline__ bool mbar_try(unsigned bar, unsigned parity) {
+    unsigned done;
+    asm volatile(
+        "{\n"
+        ".reg .pred p;\n"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
+        "selp.u32 %0, 1, 0, p;\n"
+        "}\n"
+        : "=r"(done)
+        : "r"(bar), "r"(parity)
+        : "memory");
+    return done != 0;
+}
+// wait with the limit; at once when a role of the CTA has given up.  SLEEP: nanoseconds between two looks (a failing try_wait comes back within some
+// 50 cycles whatever time it is offered, and a dozen polling warps take the issue slots of the others).  The caller's control flow does not
+// depend on the outcome.
+template <int SLEEP>
+__device__ __forceinline__ void pair_wait_slow(unsigned bar, unsigned parity, volatile int *failed) {
+    const long long t0 = clock64();
+    while (!mbar_try(bar, parity)) {
+        if (SLEEP > 0) __nanosleep(SLEEP);
+        if (*failed) return;
+        if (clock64() - t0 > PAIR_WAIT_LIMIT) { *failed = 1; return; }
+    }
+}
+template <int SLEEP>
+__device__ __forceinline__ void pair_wait(unsigned bar, unsigned parity, volatile int *failed) {
+    if (!mbar_try(bar, parity)) pair_wait_slow<SLEEP>(bar, parity, failed);
+}
+
+// ---------------------------------------------------------------- 64 values of a row out of shared memory -> 32 packed bf16 pairs
+// Two values at a time (packed f32: one issue slot for both): four small unsigned integers, one per byte of x, become d * q + c as two bf16
+// pairs.  Integers below 128 take the upper mantissa bits of 128 (0x43qq0000 = 128 + q), so that PRMT alone makes the float and the 128
+// goes into the constant, c - 128 d: that constant is off by 2^-17 d at most, far below the bf16 rounding of the result.
+struct Scale2 { unsigned long long d, c; };
+__device__ __forceinline__ unsigned long long pack_f2(float a, float b) {
+    unsigned long long r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ unsigned fma2_bf16(unsigned long long x, const Scale2 &s) {
+    unsigned long long r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(x), "l"(s.d), "l"(s.c));
+    float lo, hi;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(r));
+    return pack_bf16(lo, hi);
+}
+__device__ __forceinline__ Scale2 scale_q7(float d, float c) {
+    const float c128 = fmaf(-128.0f, d, c);
+    return {pack_f2(d, d), pack_f2(c128, c128)};
+}
+__device__ __forceinline__ void unpack_q7x4(unsigned x, const Scale2 &s, unsigned *o) {
+    const float a = __uint_as_float(__byte_perm(x, 0x43000000u, 0x7044)), b = __uint_as_float(__byte_perm(x, 0x43000000u, 0x7144));
+    const float e = __uint_as_float(__byte_perm(x, 0x43000000u, 0x7244)), f = __uint_as_float(__byte_perm(x, 0x43000000u, 0x7344));
+    o[0] = fma2_bf16(pack_f2(a, b), s);
+    o[1] = fma2_bf16(pack_f2(e, f), s);
+}
+// bytes 0..255: float(byte) first, exact
+__device__ __forceinline__ void unpack_u8x4(unsigned x, const Scale2 &s, unsigned *o) {
+    o[0] = fma2_bf16(pack_f2(byte_f<0>(x), byte_f<1>(x)), s);
+    o[1] = fma2_bf16(pack_f2(byte_f<2>(x), byte_f<3>(x)), s);
+}
+// N consecutive words at a 2-byte aligned shared address: 8-byte loads from the aligned-down one, a word select and a 16-bit funnel shift
+template <int N>
+__device__ __forceinline__ void lds_run(const unsigned char *at, unsigned (&w)[N]) {
+    const unsigned a = smem_u32(at);
+    const uint2 *p = reinterpret_cast<const uint2 *>(at - (a & 7u));
+    const bool odd = (a & 4u) != 0;
+    const unsigned sh = (a & 2u) * 8u;
+    constexpr int NP = (N + 3) / 2;
+    unsigned u[2 * NP];
+#pragma unroll
+    for (int i = 0; i < NP; i++) { const uint2 v = p[i]; u[2 * i] = v.x; u[2 * i + 1] = v.y; }
+#pragma unroll
+    for (int i = 0; i < N; i++) w[i] = __funnelshift_r(odd ? u[i + 1] : u[i], odd ? u[i + 2] : u[i + 1], sh);
+}
+// word of the four bytes that start at an even byte offset, known at compile time
+__device__ __forceinline__ unsigned word_at(const unsigned *w, int byte_off) {
+    return (byte_off & 2) ? __funnelshift_r(w[byte_off >> 2], w[(byte_off >> 2) + 1], 16) : w[byte_off >> 2];
+}
+
+// run(g, c, o): g -> first byte of the 256-value group, c = 64-value chunk 0..3 inside it (differs between the lanes).  Formats as at Dequant64.
+template <int TYPE> struct Unpack;
+
+template <int TYPE>
+struct UnpackK45 {  // the scales and minima of sub-blocks 2c and 2c + 1 are two neighbouring bytes of the 12 (get_scale_min_k4)
+    static __device__ __forceinline__ void run(const unsigned char *g, int c, unsigned (&o)[32]) {
+        const uint4 hdr = *reinterpret_cast<const uint4 *>(g);
+        const float d = f16lo(hdr.x), dmin = f16hi(hdr.x);
+        const unsigned sh = 16u * (c & 1), y = hdr.y >> sh, z = hdr.z >> sh, w = hdr.w >> sh;
+        const unsigned sc = c < 2 ? y & 0x3F3Fu : (w & 0x0F0Fu) | ((y >> 2) & 0x3030u), mn = c < 2 ? z & 0x3F3Fu : ((w >> 4) & 0x0F0Fu) | ((z >> 2) & 0x3030u);
+        const Scale2 s0 = scale_q7(d * byte_f<0>(sc), -(dmin * byte_f<0>(mn))), s1 = scale_q7(d * byte_f<1>(sc), -(dmin * byte_f<1>(mn)));
+        const uint4 *qp = reinterpret_cast<const uint4 *>(g + (TYPE == B200_TYPE_Q4_K ? 16 : 48) + 32 * c);
+        const uint4 qa = qp[0], qb = qp[1];
+        const unsigned q[8] = {qa.x, qa.y, qa.z, qa.w, qb.x, qb.y, qb.z, qb.w};
+        unsigned h[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+        if constexpr (TYPE == B200_TYPE_Q5_K) {
+            const uint4 ha = *reinterpret_cast<const uint4 *>(g + 16), hb = *reinterpret_cast<const uint4 *>(g + 32);
+            h[0] = ha.x >> (2 * c); h[1] = ha.y >> (2 * c); h[2] = ha.z >> (2 * c); h[3] = ha.w >> (2 * c);
+            h[4] = hb.x >> (2 * c); h[5] = hb.y >> (2 * c); h[6] = hb.z >> (2 * c); h[7] = hb.w >> (2 * c);
+        }
+#pragma unroll
+        for (int i = 0; i < 8; i++) {
+            unsigned lo = q[i] & 0x0F0F0F0Fu, hi = (q[i] >> 4) & 0x0F0F0F0Fu;
+            if constexpr (TYPE == B200_TYPE_Q5_K) { lo += (h[i] & 0x01010101u) * 16u; hi += (h[i] & 0x02020202u) * 8u; }
+            unpack_q7x4(lo, s0, o + 2 * i);
+            unpack_q7x4(hi, s1, o + 16 + 2 * i);
+        }
+    }
+};
+template <> struct Unpack<B200_TYPE_Q4_K> : UnpackK45<B200_TYPE_Q4_K> {};
+template <> struct Unpack<B200_TYPE_Q5_K> : UnpackK45<B200_TYPE_Q5_K> {};
+
+template <> struct Unpack<B200_TYPE_Q6_K> {
+    static __device__ __forceinline__ void run(const unsigned char *g, int c, unsigned (&o)[32]) {
+        const int half = c >> 1, hi = c & 1;
+        unsigned ql[16], qh[8], sc[1];
+        lds_run<16>(g + 64 * half, ql);
+        lds_run<8>(g + 128 + 32 * half, qh);
+        lds_run<1>(g + 192 + 4 * c, sc);
+        const float d = h2f(*reinterpret_cast<const unsigned short *>(g + 208));
+#pragma unroll
+        for (int i = 0; i < 8; i++) qh[i] >>= 4 * hi;
+#pragma unroll
+        for (int gr = 0; gr < 4; gr++) {  // 16 values of one scale each
+            const float ds = d * (float)(int)(signed char)((sc[0] >> (8 * gr)) & 0xff);
+            const Scale2 s = scale_q7(ds, -32.0f * ds);
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+                const int lw = 4 * (gr & 1) + i;
+                const unsigned x = ((ql[8 * (gr >> 1) + lw] >> (4 * hi)) & 0x0F0F0F0Fu) + ((gr >> 1) ? (qh[lw] & 0x0C0C0C0Cu) * 4u : (qh[lw] & 0x03030303u) * 16u);
+                unpack_q7x4(x, s, o + 8 * gr + 2 * i);
+            }
+        }
+    }
+};
+
+template <> struct Unpack<B200_TYPE_Q4_0> {
+    static __device__ __forceinline__ void run(const unsigned char *g, int c, unsigned (&o)[32]) {
+        unsigned w[9];
+        lds_run<9>(g + 36 * c, w);
+#pragma unroll
+        for (int b = 0; b < 2; b++) {
+            const float d = f16_at(w, 18 * b);
+            const Scale2 s = scale_q7(d, -8.0f * d);
+#pragma unroll
+            for (int j = 0; j < 4; j++) {
+                const unsigned q = word_at(w, 18 * b + 2 + 4 * j);
+                unpack_q7x4(q & 0x0F0F0F0Fu, s, o + 16 * b + 2 * j);
+                unpack_q7x4((q >> 4) & 0x0F0F0F0Fu, s, o + 16 * b + 8 + 2 * j);
+            }
+        }
+    }
+};
+template <> struct Unpack<B200_TYPE_Q8_0> {
+    static __device__ __forceinline__ void run(const unsigned char *g, int c, unsigned (&o)[32]) {
+        unsigned w[17];
+        lds_run<17>(g + 68 * c, w);
+#pragma unroll
+        for (int b = 0; b < 2; b++) {
+            const float d = f16_at(w, 34 * b);
+            const Scale2 s = {pack_f2(d, d), pack_f2(-128.0f * d, -128.0f * d)};
+#pragma unroll
+            for (int j = 0; j < 8; j++) unpack_u8x4(word_at(w, 34 * b + 2 + 4 * j) ^ 0x80808080u, s, o + 16 * b + 2 * j);  // int8 + 128
+        }
+    }
+};
+template <int TYPE>
+struct UnpackLegacy {  // q4_1, q5_0, q5_1
+    static __device__ __forceinline__ void run(const unsigned char *g, int c, unsigned (&o)[32]) {
+        using L = LegacyLayout<TYPE>;
+        unsigned w[L::BB / 2];
+        lds_run<L::BB / 2>(g + 2 * L::BB * c, w);
+#pragma unroll
+        for (int b = 0; b < 2; b++) {
+            const int base = L::BB * b;
+            const float d = f16_at(w, base);
+            const Scale2 s = scale_q7(d, L::HAS_M ? f16_at(w, base + 2) : d * -16.0f);
+            const unsigned qh = L::HAS_H ? word_at(w, base + L::QH) : 0u;
+#pragma unroll
+            for (int j = 0; j < 4; j++) {
+                const unsigned q = word_at(w, base + L::QS + 4 * j);
+                unsigned lo = q & 0x0F0F0F0Fu, hi = (q >> 4) & 0x0F0F0F0Fu;
+                if constexpr (L::HAS_H) {  // the fifth bits of four values: nibble j (and 4 + j) of qh, a bit to each byte
+                    const unsigned hl = (qh >> (4 * j)) & 15u, hh = (qh >> (16 + 4 * j)) & 15u;
+                    lo |= ((hl * 0x00204081u) & 0x01010101u) << 4;
+                    hi |= ((hh * 0x00204081u) & 0x01010101u) << 4;
+                }
+                unpack_q7x4(lo, s, o + 16 * b + 2 * j);
+                unpack_q7x4(hi, s, o + 16 * b + 8 + 2 * j);
+            }
+        }
+    }
+};
+template <> struct Unpack<B200_TYPE_Q4_1> : UnpackLegacy<B200_TYPE_Q4_1> {};
+template <> struct Unpack<B200_TYPE_Q5_0> : UnpackLegacy<B200_TYPE_Q5_0> {};
+template <> struct Unpack<B200_TYPE_Q5_1> : UnpackLegacy<B200_TYPE_Q5_1> {};
+
+// 16 nibble bytes of an iq4 sub-block as four words: levels + 128, eight at a time
+__device__ __forceinline__ void unpack_iq4x32(const unsigned (&q)[4], float dl, unsigned *o) {
+    const Scale2 s = {pack_f2(dl, dl), pack_f2(-128.0f * dl, -128.0f * dl)};
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        unsigned lo, hi;
+        iq4_levels(q[i], lo, hi);
+        unpack_u8x4(lo ^ 0x80808080u, s, o + 2 * i);
+        unpack_u8x4(hi ^ 0x80808080u, s, o + 8 + 2 * i);
+    }
+}
+template <> struct Unpack<B200_TYPE_IQ4_NL> {
+    static __device__ __forceinline__ void run(const unsigned char *g, int c, unsigned (&o)[32]) {
+        unsigned w[9];
+        lds_run<9>(g + 36 * c, w);
+#pragma unroll
+        for (int b = 0; b < 2; b++) {
+            const unsigned q[4] = {word_at(w, 18 * b + 2), word_at(w, 18 * b + 6), word_at(w, 18 * b + 10), word_at(w, 18 * b + 14)};
+            unpack_iq4x32(q, f16_at(w, 18 * b), o + 16 * b);
+        }
+    }
+};
+template <> struct Unpack<B200_TYPE_IQ4_XS> {
+    static __device__ __forceinline__ void run(const unsigned char *g, int c, unsigned (&o)[32]) {
+        unsigned hdr[2], w[8];
+        lds_run<2>(g, hdr);
+        lds_run<8>(g + 8 + 32 * c, w);
+        const float d = f16lo(hdr[0]);
+#pragma unroll
+        for (int b = 0; b < 2; b++) {
+            const unsigned q[4] = {w[4 * b], w[4 * b + 1], w[4 * b + 2], w[4 * b + 3]};
+            unpack_iq4x32(q, d * iq4xs_scale(hdr[1], hdr[0] >> 16, 2 * c + b), o + 16 * b);
+        }
+    }
+};
+// q2_K / q3_K: chunk c is bit fields 2 (c & 1) and 2 (c & 1) + 1 of half c >> 1; its four scales are bytes 4c .. 4c + 3 of the 16
+template <> struct Unpack<B200_TYPE_Q2_K> {
+    static __device__ __forceinline__ void run(const unsigned char *g, int c, unsigned (&o)[32]) {
+        unsigned q[8], sc[1], dm[1];
+        lds_run<8>(g + 16 + 32 * (c >> 1), q);
+        lds_run<1>(g + 4 * c, sc);
+        lds_run<1>(g + 80, dm);
+        const float d = f16lo(dm[0]), dmin = f16hi(dm[0]);
+#pragma unroll
+        for (int gr = 0; gr < 4; gr++) {
+            const unsigned b = (sc[0] >> (8 * gr)) & 0xff;
+            const Scale2 s = scale_q7(d * (float)(b & 15), -(dmin * (float)(b >> 4)));
+#pragma unroll
+            for (int i = 0; i < 4; i++) unpack_q7x4((q[4 * (gr & 1) + i] >> (4 * (c & 1) + 2 * (gr >> 1))) & 0x03030303u, s, o + 8 * gr + 2 * i);
+        }
+    }
+};
+template <> struct Unpack<B200_TYPE_Q3_K> {
+    static __device__ __forceinline__ void run(const unsigned char *g, int c, unsigned (&o)[32]) {
+        unsigned q[8], h[8], sw[3];
+        lds_run<8>(g + 32 + 32 * (c >> 1), q);
+        lds_run<8>(g, h);
+        lds_run<3>(g + 96, sw);
+        const float d = h2f(*reinterpret_cast<const unsigned short *>(g + 108));
+        // word c of the 16 scales (q3k_scales)
+        const unsigned sc = ((((c & 1) ? sw[1] : sw[0]) >> (c & 2 ? 4 : 0)) & 0x0f0f0f0fu) | (((sw[2] >> (2 * c)) & 0x03030303u) << 4);
+#pragma unroll
+        for (int gr = 0; gr < 4; gr++) {
+            const float dl = d * (float)((int)((sc >> (8 * gr)) & 0xff) - 32);
+            const Scale2 s = scale_q7(dl, -4.0f * dl);
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+                const int l = 4 * (gr & 1) + i;
+                unpack_q7x4(((q[l] >> (4 * (c & 1) + 2 * (gr >> 1))) & 0x03030303u) + ((h[l] >> (2 * c + (gr >> 1))) & 0x01010101u) * 4u, s, o + 8 * gr + 2 * i);
+            }
+        }
+    }
+};
+
+// ---------------------------------------------------------------- the tile that comes next
+struct PairTile {
+    int64_t m0;          // first weight row of the pair's tile
+    int64_t n0, n_end;   // columns
+    int64_t product;     // batch entry or expert
+    int n;               // columns the MMA computes
+    int kb0, nkb;        // K steps of 64
+};
+template <bool GROUPED>
+__device__ __forceinline__ PairTile pair_tile(const PairParams &p, int t, int nt, int ksteps_unit) {
+    PairTile r;
+    const int ni = t % nt;
+    int rest = t / nt;
+    r.m0 = (int64_t)(rest % p.n_tiles_m) * 256;
+    rest /= p.n_tiles_m;
+    r.kb0 = 0;
+    r.nkb = (int)(p.q.K / MQ_BK);
+    if constexpr (GROUPED) {
+        const int *te = p.q.tile_tab + 1 + 3 * ni;
+        r.product = __ldg(te);
+        r.n0 = __ldg(te + 1);
+        const int64_t end = __ldg(te + 2);
+        r.n_end = end < r.n0 + p.bn ? end : r.n0 + p.bn;
+        r.n = ((int)(r.n_end - r.n0) + 31) / 32 * 32;
+    } else {
+        r.n0 = (int64_t)ni * p.bn;
+        r.n_end = r.n0 + p.bn < p.q.N ? r.n0 + p.bn : p.q.N;
+        r.n = p.bn;
+        if (p.q.n_batch > 1) {
+            r.product = rest;
+        } else {
+            r.product = 0;
+            const int units = r.nkb / ksteps_unit, u0 = rest * units / p.q.ksplit, u1 = (rest + 1) * units / p.q.ksplit;
+            r.kb0 = u0 * ksteps_unit;
+            r.nkb = (u1 - u0) * ksteps_unit;
+        }
+    }
+    return r;
+}
+
+template <int TYPE>
+__host__ __device__ constexpr int pair_threads() { return 32 * ((TYPE == B200_TYPE_BF16 ? 0 : PAIR_PRODUCERS) + 6); }
+
+template <int TYPE, bool GROUPED>
+__global__ void __launch_bounds__(pair_threads<TYPE>(), 1) mmq_pair_kernel(const __grid_constant__ TmapBytes tmA, const __grid_constant__ TmapBytes tmB, const __grid_constant__ PairParams p) {
+    constexpr bool DENSE = TYPE == B200_TYPE_BF16;
+    constexpr int NP = DENSE ? 0 : PAIR_PRODUCERS, A_BYTES = MQ_BM * MQ_BK * 2, UNIT = DENSE ? 1 : 4;
+    constexpr int G256 = DENSE ? 0 : group256_bytes(TYPE);
+    extern __shared__ unsigned char smem_raw[];
+    unsigned char *smem = reinterpret_cast<unsigned char *>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+    __shared__ __align__(8) unsigned long long full_bar[PAIR_MAX_STAGES], peer_bar[PAIR_MAX_STAGES], empty_bar[PAIR_MAX_STAGES], acc_full[2], acc_empty[2];
+    __shared__ unsigned tmem_base_s;
+    __shared__ volatile int failed;
+    const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31, tid = threadIdx.x;
+    const int rank = (int)cluster_rank(), pair = (int)(blockIdx.x >> 1), n_pairs = (int)(gridDim.x >> 1);
+    const int S = p.stages, stage_bytes = A_BYTES + p.bn * MQ_BK;  // (bn / 2 activation rows of 128 bytes)
+    const int nt = GROUPED ? __ldg(p.q.tile_tab) : p.n_tiles_n;
+    const int n_tiles = nt * p.n_tiles_m * (GROUPED ? 1 : p.q.n_batch > 1 ? p.q.n_batch : p.q.ksplit);
+    const unsigned full0 = smem_u32(full_bar), peer0 = smem_u32(peer_bar), empty0 = smem_u32(empty_bar), acc_full0 = smem_u32(acc_full), acc_empty0 = smem_u32(acc_empty);
+
+    if (tid == 0) {
+        for (int s = 0; s < S; s++) {
+            mbar_init(&full_bar[s], DENSE ? 1 : PAIR_PRODUCERS + 1);
+            mbar_init(&peer_bar[s], 1);
+            mbar_init(&empty_bar[s], 1);
+        }
+        for (int b = 0; b < 2; b++) { mbar_init(&acc_full[b], 1); mbar_init(&acc_empty[b], 8); }
+        failed = 0;
+        mbar_fence_init();
+    }
+    if (warp == NP) tmem_alloc2(&tmem_base_s, 512);
+    tc_fence_before();
+    __syncthreads();
+    pair_sync();
+    tc_fence_after();
+    const unsigned tmem_base = tmem_base_s;
+
+    if (warp < NP) {
+        // ===== producers: rows 8 * warp .. 8 * warp + 7 of this CTA's 128
+        if constexpr (!DENSE) {
+            constexpr int PIECES = raw_pieces(TYPE), ROW = raw_row(TYPE), SLOTS = raw_slots(TYPE), PER = (8 * PIECES + 31) / 32;
+            unsigned char *raw = smem + (size_t)S * stage_bytes + (size_t)warp * SLOTS * 8 * ROW;
+            // first byte of row r (0..7) of this warp in the tile's first group; rows past the matrix read its last one (their results are not stored)
+            auto row_base = [&](const PairTile &ti, int r) {
+                const int64_t row = ti.m0 + rank * MQ_BM + 8 * warp + r;
+                return p.q.W + (size_t)ti.product * (GROUPED ? p.q.expert_bytes : p.q.w_batch_bytes) + (size_t)(ti.kb0 / 4) * G256 + (size_t)(row < p.q.M ? row : p.q.M - 1) * p.q.w_row_bytes;
+            };
+            // the copy runs SLOTS - 1 groups ahead of the unpacking, over tile ends too
+            int ct = pair, left = 0, slot_in = 0;
+            const unsigned char *src[PER];
+            unsigned to[PER];  // where piece j of this lane goes in slot 0
+#pragma unroll
+            for (int j = 0; j < PER; j++) to[j] = smem_u32(raw) + (unsigned)((lane + 32 * j) / PIECES * ROW + (lane + 32 * j) % PIECES * 16);
+            auto copy_group = [&]() {
+                if (left == 0 && ct < n_tiles) {
+                    const PairTile ti = pair_tile<GROUPED>(p, ct, nt, UNIT);
+                    left = ti.nkb / 4;
+                    ct += n_pairs;
+#pragma unroll
+                    for (int j = 0; j < PER; j++) {
+                        const int i = lane + 32 * j;
+                        src[j] = row_base(ti, i / PIECES & 7) + (raw_aligned(TYPE) ? i % PIECES * 16 : 0);
+                    }
+                }
+                if (left > 0) {
+                    left--;
+                    const unsigned slot_off = (unsigned)(slot_in * 8 * ROW);
+#pragma unroll
+                    for (int j = 0; j < PER; j++) {
+                        const bool mine = 32 * (j + 1) <= 8 * PIECES || lane + 32 * j < 8 * PIECES;
+                        if constexpr (raw_aligned(TYPE)) {
+                            if (mine) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(to[j] + slot_off), "l"(src[j]) : "memory");
+                        } else {
+                            const unsigned off = (unsigned)(uintptr_t)src[j] & 15u, at = (unsigned)((lane + 32 * j) % PIECES * 16);
+                            if (mine && at < off + G256) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(to[j] + slot_off), "l"(src[j] + (int)(at - off)) : "memory");
+                        }
+                        src[j] += G256;
+                    }
+                }
+                cp_async_commit();
+                slot_in = slot_in + 1 == SLOTS ? 0 : slot_in + 1;
+            };
+            for (int i = 0; i < SLOTS - 1; i++) copy_group();
+            const int c = lane >> 3, r = lane & 7;
+            const unsigned a_row = smem_u32(smem) + (unsigned)(warp * 1024 + r * 128 + (r << 4));  // piece q of the row lies at a_row ^ (q << 4)
+            int s0 = 0, slot = 0;       // stage of the group's first K step
+            unsigned ph0 = 1;           // parity of its empty barrier: the first pass finds it free
+            for (int t = pair; t < n_tiles; t += n_pairs) {
+                const PairTile ti = pair_tile<GROUPED>(p, t, nt, UNIT);
+                unsigned at = raw_aligned(TYPE) ? 0u : (unsigned)(uintptr_t)row_base(ti, r) & 15u;  // where in its first piece the row's group starts
+#pragma unroll 1
+                for (int g = ti.nkb / 4; g > 0; g--) {
+                    cp_async_wait<SLOTS - 2>();
+                    __syncwarp();  // the group has landed for all lanes, and all have left the one before
+                    copy_group();
+                    unsigned o[32];
+                    Unpack<TYPE>::run(raw + (slot * 8 + r) * ROW + at, c, o);
+                    if constexpr (!raw_aligned(TYPE)) at = (at + G256) & 15u;
+                    slot = slot + 1 == SLOTS ? 0 : slot + 1;
+                    // stages are freed in order: the last of the four stands for all
+                    const bool wrap = s0 + 3 >= S;
+                    pair_wait<20>(empty0 + 8u * (unsigned)(wrap ? s0 + 3 - S : s0 + 3), wrap ? ph0 ^ 1u : ph0, &failed);
+                    const int mine = s0 + c >= S ? s0 + c - S : s0 + c;
+                    const unsigned d = a_row + (unsigned)(mine * stage_bytes);
+#pragma unroll
+                    for (int q = 0; q < 8; q++)
+                        asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(d ^ (q << 4)), "r"(o[4 * q]), "r"(o[4 * q + 1]), "r"(o[4 * q + 2]), "r"(o[4 * q + 3]) : "memory");
+                    fence_proxy_async_smem();
+                    __syncwarp();
+                    if (r == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(full0 + 8u * (unsigned)mine) : "memory");
+                    s0 += 4;
+                    if (s0 >= S) { s0 -= S; ph0 ^= 1u; }
+                }
+            }
+            cp_async_wait<0>();
+        }
+    } else if (warp == NP) {
+        // ===== the pair's MMAs (first CTA); the second CTA passes on that its half of a stage is ready
+        const unsigned long long desc0 = umma_desc_sw128(smem_u32(smem));
+        const bool elected = elect_lane();
+        int s = 0, buf = 0;
+        unsigned ph = 0, aph = 1;
+        for (int t = pair; t < n_tiles; t += n_pairs) {
+            const PairTile ti = pair_tile<GROUPED>(p, t, nt, UNIT);
+            if (rank != 0) {
+                for (int kb = 0; kb < ti.nkb; kb++) {
+                    pair_wait<0>(full0 + 8u * s, ph, &failed);
+                    if (elected) mbar_arrive_leader(peer0 + 8u * s);
+                    if (++s == S) { s = 0; ph ^= 1u; }
+                }
+                continue;
+            }
+            const unsigned idesc = umma_idesc_bf16(256, 16) + ((unsigned)((ti.n - 16) >> 3) << 17), acc = tmem_base + (unsigned)buf * 256u;
+            pair_wait<0>(acc_empty0 + 8u * buf, aph, &failed);
+            tc_fence_after();
+            unsigned accumulate = 0;
+#pragma unroll 1
+            for (int kb = 0; kb < ti.nkb; kb++) {
+                pair_wait<0>(full0 + 8u * s, ph, &failed);
+                pair_wait<0>(peer0 + 8u * s, ph, &failed);
+                tc_fence_after();
+                const unsigned long long ad = desc0 + (unsigned)(s * (stage_bytes >> 4)), bd = ad + (A_BYTES >> 4);
+                if (elected) {
+                    // 16 bf16 = 32 bytes further along K inside the swizzle atom: +2 in the (address >> 4) field
+                    tc_mma2_bf16(acc, ad, bd, idesc, accumulate);
+#pragma unroll
+                    for (int k = 1; k < MQ_BK / 16; k++) tc_mma2_bf16(acc, ad + 2u * k, bd + 2u * k, idesc, 1u);
+                    tc_commit2(empty0 + 8u * s);
+                }
+                __syncwarp();
+                accumulate = 1;
+                if (++s == S) { s = 0; ph ^= 1u; }
+            }
+            if (elected) tc_commit2(acc_full0 + 8u * buf);
+            __syncwarp();
+            buf ^= 1;
+            if (buf == 0) aph ^= 1u;
+        }
+    } else if (warp == NP + 1) {
+        // ===== copies: this CTA's half of the activation rows (dense weights: its 128 weight rows too)
+        if (lane == 0) {
+            int s = 0;
+            unsigned ph = 1;
+            for (int t = pair; t < n_tiles; t += n_pairs) {
+                const PairTile ti = pair_tile<GROUPED>(p, t, nt, UNIT);
+                const int half = ti.n / 2, row = (int)(ti.n0 + rank * half + (GROUPED ? 0 : ti.product * p.q.n_pad));
+                for (int kb = 0; kb < ti.nkb; kb++) {
+                    pair_wait<20>(empty0 + 8u * s, ph, &failed);
+                    if (failed) break;  // no copy without a free stage
+                    unsigned char *st = smem + (size_t)s * stage_bytes;
+                    mbar_expect_tx(&full_bar[s], (unsigned)(half * MQ_BK * 2 + (DENSE ? A_BYTES : 0)));
+                    const int k = (ti.kb0 + kb) * MQ_BK;
+                    if constexpr (DENSE) tma_load_2d(st, &tmA, k, (int)(ti.product * p.w_rows_per_product + ti.m0 + rank * MQ_BM), &full_bar[s]);
+                    for (int r = 0; r < half; r += p.box) tma_load_2d(st + A_BYTES + r * MQ_BK * 2, &tmB, k, row + r, &full_bar[s]);
+                    if (++s == S) { s = 0; ph ^= 1u; }
+                }
+            }
+        }
+        __syncwarp();
+    } else {
+        // ===== epilogue: TMEM lanes 32 * (warp % 4) .. of this CTA's 128 rows
+        int buf = 0;
+        unsigned ph = 0;
+        const int quarter = warp & 3;
+        for (int t = pair; t < n_tiles; t += n_pairs) {
+            const PairTile ti = pair_tile<GROUPED>(p, t, nt, UNIT);
+            pair_wait<200>(acc_full0 + 8u * buf, ph, &failed);
+            tc_fence_after();
+            const int64_t m = ti.m0 + rank * MQ_BM + quarter * 32 + lane;
+            const bool row_ok = m < p.q.M && !failed;
+            float *drow = p.q.dst + m + (!GROUPED && p.q.n_batch > 1 ? ti.product * p.q.dst_batch : 0);
+            const int cols = (int)(ti.n_end - ti.n0);
+#pragma unroll 1
+            for (int c0 = 0; c0 < cols; c0 += 32) {
+                float v[32];
+                __syncwarp();
+                tmem_ld32(tmem_base + (unsigned)buf * 256u + ((unsigned)(quarter * 32) << 16) + (unsigned)c0, v);
+                if (row_ok) {
+#pragma unroll
+                    for (int j = 0; j < 32; j++) {
+                        if (c0 + j >= cols) continue;
+                        const int64_t n = ti.n0 + c0 + j;
+                        if constexpr (GROUPED) drow[(int64_t)__ldg(p.q.row_dst + n)] = v[j];    // scatter: sorted row -> (token, slot)
+                        else if (p.q.ksplit > 1) atomicAdd(drow + n * p.q.dst_stride, v[j]);    // (result unused: RED.ADD.F32)
+                        else drow[n * p.q.dst_stride] = v[j];
+                    }
+                }
+            }
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive_leader(acc_empty0 + 8u * buf);
+            buf ^= 1;
+            if (buf == 0) ph ^= 1u;
+        }
+    }
+    __syncwarp();
+    __syncthreads();
+    if (failed) {  // copies and MMAs that were requested end within this time
+        if (tid == 0 && p.timeout) atomicExch(p.timeout, 1);
+        for (const long long t0 = clock64(); clock64() - t0 < 4000000LL;) {}
+    }
+    tc_fence_before();
+    pair_sync();
+    if (warp == NP) {
+        tc_fence_after();
+        tmem_dealloc2(tmem_base, 512);
+    }
+}
+
+// ---------------------------------------------------------------- host side
+// Tile width and K split by the length of the longest pair's work, in tensor cycles: a K step of 64 takes 2 * BN of them (8192 MACs a cycle
+// and pair), or as long as the producers need to unpack it (measured, per format), a tile about 1500 more; two halves of K add into a
+// zeroed dst, which costs about as much as 4000.  Widths are N / 1, N / 2, ... rounded up to 16.
+struct PairPlan { int bn, ksplit, n_tiles_n; };
+static inline PairPlan mmq_pair_plan(int64_t M, int64_t N, int64_t K, int n_batch, int pairs, int unpack) {
+    PairPlan best = {256, 1, 1};
+    double best_cost = -1;
+    const int64_t mt = (M + 255) / 256;
+    for (int64_t parts = (N + 255) / 256; parts <= (N + 31) / 32; parts++) {
+        const int64_t even = ((N + parts - 1) / parts + 15) / 16 * 16, bn = even < 32 ? 32 : even;
+        const int64_t nt = (N + bn - 1) / bn;
+        for (int ks = 1; ks <= 2; ks++) {
+            if (ks == 2 && (n_batch > 1 || K < 2048)) break;
+            const int64_t tiles = mt * nt * n_batch * ks, waves = (tiles + pairs - 1) / pairs;
+            const double step = 2.0 * bn > unpack ? 2.0 * bn : unpack;
+            const double cost = waves * ((double)(K / MQ_BK) / ks * step + 1500.0) + (ks == 2 ? 4000.0 : 0.0);
+            if (best_cost < 0 || cost < 0.98 * best_cost) { best_cost = cost; best = {(int)bn, ks, (int)nt}; }
+        }
+    }
+    return best;
+}
+
+// pairs of CTAs that the device can hold at once (the same for every instantiation: one CTA an SM by its shared memory)
+static int mmq_pairs() {
+    static int pairs = 0;
+    if (!pairs) {
+        int dev = 0, sms = 0;
+        if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) { cudaGetLastError(); sms = 148; }
+        pairs = sms / 2;
+    }
+    return pairs;
+}
+
+template <int TYPE> constexpr int pair_unpack_cycles() { return TYPE == B200_TYPE_BF16 ? 0 : TYPE == B200_TYPE_Q4_K || TYPE == B200_TYPE_Q4_0 || TYPE == B200_TYPE_Q5_K ? 300 : 420; }
+
+template <int TYPE, bool GROUPED>
+static int mmq_pair_launch(const MmqParams &q, int64_t n_pad, int64_t w_rows_per_product, int64_t max_tiles_n, int64_t grouped_bn, cudaStream_t st) {
+    const auto kern = mmq_pair_kernel<TYPE, GROUPED>;
+    static bool attr_set_dev[16] = {};  // cudaFuncSetAttribute is per device
+    int cur_dev = 0;
+    B200_CUDA_TRY(cudaGetDevice(&cur_dev));
+    bool &attr_set = attr_set_dev[cur_dev & 15];
+    if (!attr_set) {
+        B200_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, PAIR_SMEM));
+        attr_set = true;
+    }
+    PairParams p;
+    p.q = q;
+    p.w_rows_per_product = w_rows_per_product;
+    p.timeout = g_gemm_timeout;
+    p.n_tiles_m = (int)((q.M + 255) / 256);
+    if (GROUPED) {
+        p.bn = (int)grouped_bn;
+        p.box = 16;
+        p.n_tiles_n = 0;
+        p.q.ksplit = 1;
+    } else {
+        const PairPlan pl = mmq_pair_plan(q.M, q.N, q.K, q.n_batch, mmq_pairs(), pair_unpack_cycles<TYPE>());
+        p.bn = pl.bn;
+        p.box = pl.bn / 2;
+        p.n_tiles_n = pl.n_tiles_n;
+        p.q.ksplit = pl.ksplit;
+    }
+    const int stage = MQ_BM * MQ_BK * 2 + p.bn * MQ_BK;
+    p.stages = (PAIR_SMEM - 1024 - raw_bytes(TYPE)) / stage;
+    if (p.stages > PAIR_MAX_STAGES) p.stages = PAIR_MAX_STAGES;
+    TmapBytes tmA = {}, tmB;
+    if (TYPE == B200_TYPE_BF16) {
+        const int64_t products = GROUPED ? q.n_expert : q.n_batch;
+        const int rc = encode_rows(tmA, q.W, q.K, (products - 1) * w_rows_per_product + q.M, q.w_row_bytes, MQ_BM);
+        if (rc != B200_OK) return rc;
+    }
+    const int rc = encode_rows(tmB, q.Xb, q.K, n_pad * (q.n_batch > 1 ? q.n_batch : 1), (size_t)q.K * 2, p.box);
+    if (rc != B200_OK) return rc;
+    if (p.q.ksplit > 1) {
+        if (q.dst_stride == q.M) B200_CUDA_TRY(cudaMemsetAsync(q.dst, 0, (size_t)q.M * q.N * sizeof(float), st));
+        else B200_CUDA_TRY(cudaMemset2DAsync(q.dst, (size_t)q.dst_stride * sizeof(float), 0, (size_t)q.M * sizeof(float), (size_t)q.N, st));
+    }
+    const int64_t tiles = (int64_t)p.n_tiles_m * (GROUPED ? max_tiles_n : p.n_tiles_n) * (GROUPED ? 1 : q.n_batch > 1 ? q.n_batch : p.q.ksplit);
+    if (tiles > 0x3fffffff) { set_error("b200_mul_mat_q: too many tiles"); return B200_ERR_UNSUPPORTED; }
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(2 * (tiles < mmq_pairs() ? tiles : mmq_pairs())));
+    cfg.blockDim = dim3(pair_threads<TYPE>());
+    cfg.dynamicSmemBytes = PAIR_SMEM;
+    cfg.stream = st;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = 2;
+    at[0].val.clusterDim.y = 1;
+    at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    B200_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, tmA, tmB, p));
+    return B200_OK;
+}
+
+}  // namespace b200
