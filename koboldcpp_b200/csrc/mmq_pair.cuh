@@ -8,8 +8,8 @@
 // share a 256 x BN tile: each unpacks its own 128 weight rows into its shared memory and fetches HALF of the activation rows, and the
 // pair's one MMA reads both halves.
 //   * 16 producer warps a CTA, 8 weight rows each: a warp copies the raw blocks of its rows (256 values of each, contiguous 16-byte cp.async) into
-//     a ring of its own, one or two groups ahead, and unpacks them with packed f32 arithmetic, lane = (64-value chunk, row), into the
-//     128-byte-swizzled operand tiles of four K steps.  No barrier among the warps.
+//     a ring of its own, one or two groups ahead, and unpacks them with packed f32 arithmetic, lane = (K step, half, row), two K
+//     steps at a time into the 128-byte-swizzled operand tiles.  No barrier among the warps.
 //   * the MMA warp walks through its loop as a whole and elects a lane for the tcgen05 instructions only: loop counters and descriptors then
 //     live in uniform registers.  (With one lane in the loop every MMA needed a dozen vector instructions, each of which waits its turn
 //     among the producers: 190 cycles an MMA whatever its width.)
@@ -114,7 +114,7 @@ __device__ __forceinline__ void pair_wait(unsigned bar, unsigned parity, volatil
     if (!mbar_try(bar, parity)) pair_wait_slow<SLEEP>(bar, parity, failed);
 }
 
-// ---------------------------------------------------------------- 64 values of a row out of shared memory -> 32 packed bf16 pairs
+// ---------------------------------------------------------------- 32 values of a row out of shared memory -> 16 packed bf16 pairs
 // Two values at a time (packed f32: one issue slot for both): four small unsigned integers, one per byte of x, become d * q + c as two bf16
 // pairs.  Integers below 128 take the upper mantissa bits of 128 (0x43qq0000 = 128 + q), so that PRMT alone makes the float and the 128
 // goes into the constant, c - 128 d: that constant is off by 2^-17 d at most, far below the bf16 rounding of the result.
@@ -160,130 +160,119 @@ __device__ __forceinline__ void lds_run(const unsigned char *at, unsigned (&w)[N
 #pragma unroll
     for (int i = 0; i < N; i++) w[i] = __funnelshift_r(odd ? u[i + 1] : u[i], odd ? u[i + 2] : u[i + 1], sh);
 }
-// word of the four bytes that start at an even byte offset, known at compile time
-__device__ __forceinline__ unsigned word_at(const unsigned *w, int byte_off) {
-    return (byte_off & 2) ? __funnelshift_r(w[byte_off >> 2], w[(byte_off >> 2) + 1], 16) : w[byte_off >> 2];
-}
 
-// run(g, c, o): g -> first byte of the 256-value group, c = 64-value chunk 0..3 inside it (differs between the lanes).  Formats as at Dequant64.
-template <int TYPE> struct Unpack;
+// run(g, c, h, o): g -> first byte of the 256-value group, c = 64-value chunk 0..3 of it, h = which half of the chunk's bytes (c and h differ between the
+// lanes).  o[0..7] are the 16 values from unpack_first(TYPE, h) on, o[8..15] those from unpack_second on.  Formats as at Dequant64: in a K-quant's
+// chunk 16 bytes hold values 16h.. (low bits) and 32 + 16h.. (high bits), in a 32-value block low and high nibbles are neighbouring values.
+__host__ __device__ constexpr bool unpack_block32(int t) { return t != B200_TYPE_Q4_K && t != B200_TYPE_Q5_K && t != B200_TYPE_Q6_K && t != B200_TYPE_Q2_K && t != B200_TYPE_Q3_K; }
+__host__ __device__ constexpr int unpack_first(int t, int h) { return unpack_block32(t) ? 32 * h : 16 * h; }
+__host__ __device__ constexpr int unpack_second(int t, int h) { return unpack_block32(t) ? 32 * h + 16 : 32 + 16 * h; }
+template <int TYPE> struct Unpack32;
+
+// four words of nibbles: low ones with scale a, high ones with scale b
+__device__ __forceinline__ void unpack_nibbles(const unsigned (&q)[4], const Scale2 &a, const Scale2 &b, unsigned (&o)[16]) {
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        unpack_q7x4(q[i] & 0x0F0F0F0Fu, a, o + 2 * i);
+        unpack_q7x4((q[i] >> 4) & 0x0F0F0F0Fu, b, o + 8 + 2 * i);
+    }
+}
+__device__ __forceinline__ unsigned spread4(unsigned b) { return ((b & 15u) * 0x00204081u) & 0x01010101u; }  // four bits, one to each byte
 
 template <int TYPE>
-struct UnpackK45 {  // the scales and minima of sub-blocks 2c and 2c + 1 are two neighbouring bytes of the 12 (get_scale_min_k4)
-    static __device__ __forceinline__ void run(const unsigned char *g, int c, unsigned (&o)[32]) {
+struct UnpackK45 {
+    static __device__ __forceinline__ void run(const unsigned char *g, int c, int h, unsigned (&o)[16]) {
         const uint4 hdr = *reinterpret_cast<const uint4 *>(g);
-        const float d = f16lo(hdr.x), dmin = f16hi(hdr.x);
+        const uint4 qv = *reinterpret_cast<const uint4 *>(g + (TYPE == B200_TYPE_Q4_K ? 16 : 48) + 32 * c + 16 * h);
+        // 6-bit scales and minima of sub-blocks 2c and 2c + 1: two neighbouring bytes of the 12 (get_scale_min_k4)
         const unsigned sh = 16u * (c & 1), y = hdr.y >> sh, z = hdr.z >> sh, w = hdr.w >> sh;
         const unsigned sc = c < 2 ? y & 0x3F3Fu : (w & 0x0F0Fu) | ((y >> 2) & 0x3030u), mn = c < 2 ? z & 0x3F3Fu : ((w >> 4) & 0x0F0Fu) | ((z >> 2) & 0x3030u);
-        const Scale2 s0 = scale_q7(d * byte_f<0>(sc), -(dmin * byte_f<0>(mn))), s1 = scale_q7(d * byte_f<1>(sc), -(dmin * byte_f<1>(mn)));
-        const uint4 *qp = reinterpret_cast<const uint4 *>(g + (TYPE == B200_TYPE_Q4_K ? 16 : 48) + 32 * c);
-        const uint4 qa = qp[0], qb = qp[1];
-        const unsigned q[8] = {qa.x, qa.y, qa.z, qa.w, qb.x, qb.y, qb.z, qb.w};
-        unsigned h[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-        if constexpr (TYPE == B200_TYPE_Q5_K) {
-            const uint4 ha = *reinterpret_cast<const uint4 *>(g + 16), hb = *reinterpret_cast<const uint4 *>(g + 32);
-            h[0] = ha.x >> (2 * c); h[1] = ha.y >> (2 * c); h[2] = ha.z >> (2 * c); h[3] = ha.w >> (2 * c);
-            h[4] = hb.x >> (2 * c); h[5] = hb.y >> (2 * c); h[6] = hb.z >> (2 * c); h[7] = hb.w >> (2 * c);
-        }
-#pragma unroll
-        for (int i = 0; i < 8; i++) {
-            unsigned lo = q[i] & 0x0F0F0F0Fu, hi = (q[i] >> 4) & 0x0F0F0F0Fu;
-            if constexpr (TYPE == B200_TYPE_Q5_K) { lo += (h[i] & 0x01010101u) * 16u; hi += (h[i] & 0x02020202u) * 8u; }
-            unpack_q7x4(lo, s0, o + 2 * i);
-            unpack_q7x4(hi, s1, o + 16 + 2 * i);
-        }
-    }
-};
-template <> struct Unpack<B200_TYPE_Q4_K> : UnpackK45<B200_TYPE_Q4_K> {};
-template <> struct Unpack<B200_TYPE_Q5_K> : UnpackK45<B200_TYPE_Q5_K> {};
-
-template <> struct Unpack<B200_TYPE_Q6_K> {
-    static __device__ __forceinline__ void run(const unsigned char *g, int c, unsigned (&o)[32]) {
-        const int half = c >> 1, hi = c & 1;
-        unsigned ql[16], qh[8], sc[1];
-        lds_run<16>(g + 64 * half, ql);
-        lds_run<8>(g + 128 + 32 * half, qh);
-        lds_run<1>(g + 192 + 4 * c, sc);
-        const float d = h2f(*reinterpret_cast<const unsigned short *>(g + 208));
-#pragma unroll
-        for (int i = 0; i < 8; i++) qh[i] >>= 4 * hi;
-#pragma unroll
-        for (int gr = 0; gr < 4; gr++) {  // 16 values of one scale each
-            const float ds = d * (float)(int)(signed char)((sc[0] >> (8 * gr)) & 0xff);
-            const Scale2 s = scale_q7(ds, -32.0f * ds);
+        const float d = f16lo(hdr.x), dmin = f16hi(hdr.x);
+        const Scale2 a = scale_q7(d * byte_f<0>(sc), -(dmin * byte_f<0>(mn))), b = scale_q7(d * byte_f<1>(sc), -(dmin * byte_f<1>(mn)));
+        const unsigned q[4] = {qv.x, qv.y, qv.z, qv.w};
+        if constexpr (TYPE == B200_TYPE_Q4_K) {
+            unpack_nibbles(q, a, b, o);
+        } else {
+            const uint4 hv = *reinterpret_cast<const uint4 *>(g + 16 + 16 * h);
+            const unsigned f[4] = {hv.x >> (2 * c), hv.y >> (2 * c), hv.z >> (2 * c), hv.w >> (2 * c)};
 #pragma unroll
             for (int i = 0; i < 4; i++) {
-                const int lw = 4 * (gr & 1) + i;
-                const unsigned x = ((ql[8 * (gr >> 1) + lw] >> (4 * hi)) & 0x0F0F0F0Fu) + ((gr >> 1) ? (qh[lw] & 0x0C0C0C0Cu) * 4u : (qh[lw] & 0x03030303u) * 16u);
-                unpack_q7x4(x, s, o + 8 * gr + 2 * i);
+                unpack_q7x4((q[i] & 0x0F0F0F0Fu) + (f[i] & 0x01010101u) * 16u, a, o + 2 * i);
+                unpack_q7x4(((q[i] >> 4) & 0x0F0F0F0Fu) + (f[i] & 0x02020202u) * 8u, b, o + 8 + 2 * i);
             }
         }
     }
 };
+template <> struct Unpack32<B200_TYPE_Q4_K> : UnpackK45<B200_TYPE_Q4_K> {};
+template <> struct Unpack32<B200_TYPE_Q5_K> : UnpackK45<B200_TYPE_Q5_K> {};
 
-template <> struct Unpack<B200_TYPE_Q4_0> {
-    static __device__ __forceinline__ void run(const unsigned char *g, int c, unsigned (&o)[32]) {
-        unsigned w[9];
-        lds_run<9>(g + 36 * c, w);
+template <> struct Unpack32<B200_TYPE_Q6_K> {  // bytes 16h.. of both 32-byte rows of the half, nibbles c & 1
+    static __device__ __forceinline__ void run(const unsigned char *g, int c, int h, unsigned (&o)[16]) {
+        unsigned qa[4], qb[4], qh[4];
+        lds_run<4>(g + 64 * (c >> 1) + 16 * h, qa);
+        lds_run<4>(g + 64 * (c >> 1) + 32 + 16 * h, qb);
+        lds_run<4>(g + 128 + 32 * (c >> 1) + 16 * h, qh);
+        const float d = h2f(*reinterpret_cast<const unsigned short *>(g + 208));
+        const signed char *sc = reinterpret_cast<const signed char *>(g + 192 + 4 * c + h);
+        const float da = d * (float)sc[0], db = d * (float)sc[2];
+        const Scale2 a = scale_q7(da, -32.0f * da), b = scale_q7(db, -32.0f * db);
+        const int n = 4 * (c & 1);
 #pragma unroll
-        for (int b = 0; b < 2; b++) {
-            const float d = f16_at(w, 18 * b);
-            const Scale2 s = scale_q7(d, -8.0f * d);
-#pragma unroll
-            for (int j = 0; j < 4; j++) {
-                const unsigned q = word_at(w, 18 * b + 2 + 4 * j);
-                unpack_q7x4(q & 0x0F0F0F0Fu, s, o + 16 * b + 2 * j);
-                unpack_q7x4((q >> 4) & 0x0F0F0F0Fu, s, o + 16 * b + 8 + 2 * j);
-            }
+        for (int i = 0; i < 4; i++) {
+            const unsigned f = qh[i] >> n;
+            unpack_q7x4(((qa[i] >> n) & 0x0F0F0F0Fu) + (f & 0x03030303u) * 16u, a, o + 2 * i);
+            unpack_q7x4(((qb[i] >> n) & 0x0F0F0F0Fu) + (f & 0x0C0C0C0Cu) * 4u, b, o + 8 + 2 * i);
         }
     }
 };
-template <> struct Unpack<B200_TYPE_Q8_0> {
-    static __device__ __forceinline__ void run(const unsigned char *g, int c, unsigned (&o)[32]) {
-        unsigned w[17];
-        lds_run<17>(g + 68 * c, w);
+template <> struct Unpack32<B200_TYPE_Q4_0> {
+    static __device__ __forceinline__ void run(const unsigned char *g, int c, int h, unsigned (&o)[16]) {
+        const unsigned char *blk = g + 36 * c + 18 * h;
+        const float d = h2f(*reinterpret_cast<const unsigned short *>(blk));
+        const Scale2 s = scale_q7(d, -8.0f * d);
+        unsigned q[4];
+        lds_run<4>(blk + 2, q);
+        unpack_nibbles(q, s, s, o);
+    }
+};
+template <> struct Unpack32<B200_TYPE_Q8_0> {
+    static __device__ __forceinline__ void run(const unsigned char *g, int c, int h, unsigned (&o)[16]) {
+        const unsigned char *blk = g + 68 * c + 34 * h;
+        const float d = h2f(*reinterpret_cast<const unsigned short *>(blk));
+        const Scale2 s = {pack_f2(d, d), pack_f2(-128.0f * d, -128.0f * d)};
+        unsigned q[8];
+        lds_run<8>(blk + 2, q);
 #pragma unroll
-        for (int b = 0; b < 2; b++) {
-            const float d = f16_at(w, 34 * b);
-            const Scale2 s = {pack_f2(d, d), pack_f2(-128.0f * d, -128.0f * d)};
-#pragma unroll
-            for (int j = 0; j < 8; j++) unpack_u8x4(word_at(w, 34 * b + 2 + 4 * j) ^ 0x80808080u, s, o + 16 * b + 2 * j);  // int8 + 128
-        }
+        for (int i = 0; i < 8; i++) unpack_u8x4(q[i] ^ 0x80808080u, s, o + 2 * i);  // int8 + 128
     }
 };
 template <int TYPE>
-struct UnpackLegacy {  // q4_1, q5_0, q5_1
-    static __device__ __forceinline__ void run(const unsigned char *g, int c, unsigned (&o)[32]) {
+struct UnpackLegacy {  // q4_1, q5_0, q5_1: as q4_0, with a minimum and / or the fifth bits in qh
+    static __device__ __forceinline__ void run(const unsigned char *g, int c, int h, unsigned (&o)[16]) {
         using L = LegacyLayout<TYPE>;
-        unsigned w[L::BB / 2];
-        lds_run<L::BB / 2>(g + 2 * L::BB * c, w);
+        const unsigned char *blk = g + 2 * L::BB * c + L::BB * h;
+        const float d = h2f(*reinterpret_cast<const unsigned short *>(blk));
+        const Scale2 s = scale_q7(d, L::HAS_M ? h2f(*reinterpret_cast<const unsigned short *>(blk + 2)) : d * -16.0f);
+        unsigned q[4];
+        lds_run<4>(blk + L::QS, q);
+        if constexpr (L::HAS_H) {
+            const unsigned fl = *reinterpret_cast<const unsigned short *>(blk + L::QH), fh = *reinterpret_cast<const unsigned short *>(blk + L::QH + 2);
 #pragma unroll
-        for (int b = 0; b < 2; b++) {
-            const int base = L::BB * b;
-            const float d = f16_at(w, base);
-            const Scale2 s = scale_q7(d, L::HAS_M ? f16_at(w, base + 2) : d * -16.0f);
-            const unsigned qh = L::HAS_H ? word_at(w, base + L::QH) : 0u;
-#pragma unroll
-            for (int j = 0; j < 4; j++) {
-                const unsigned q = word_at(w, base + L::QS + 4 * j);
-                unsigned lo = q & 0x0F0F0F0Fu, hi = (q >> 4) & 0x0F0F0F0Fu;
-                if constexpr (L::HAS_H) {  // the fifth bits of four values: nibble j (and 4 + j) of qh, a bit to each byte
-                    const unsigned hl = (qh >> (4 * j)) & 15u, hh = (qh >> (16 + 4 * j)) & 15u;
-                    lo |= ((hl * 0x00204081u) & 0x01010101u) << 4;
-                    hi |= ((hh * 0x00204081u) & 0x01010101u) << 4;
-                }
-                unpack_q7x4(lo, s, o + 16 * b + 2 * j);
-                unpack_q7x4(hi, s, o + 16 * b + 8 + 2 * j);
+            for (int i = 0; i < 4; i++) {
+                unpack_q7x4((q[i] & 0x0F0F0F0Fu) + spread4(fl >> (4 * i)) * 16u, s, o + 2 * i);
+                unpack_q7x4(((q[i] >> 4) & 0x0F0F0F0Fu) + spread4(fh >> (4 * i)) * 16u, s, o + 8 + 2 * i);
             }
+        } else {
+            unpack_nibbles(q, s, s, o);
         }
     }
 };
-template <> struct Unpack<B200_TYPE_Q4_1> : UnpackLegacy<B200_TYPE_Q4_1> {};
-template <> struct Unpack<B200_TYPE_Q5_0> : UnpackLegacy<B200_TYPE_Q5_0> {};
-template <> struct Unpack<B200_TYPE_Q5_1> : UnpackLegacy<B200_TYPE_Q5_1> {};
+template <> struct Unpack32<B200_TYPE_Q4_1> : UnpackLegacy<B200_TYPE_Q4_1> {};
+template <> struct Unpack32<B200_TYPE_Q5_0> : UnpackLegacy<B200_TYPE_Q5_0> {};
+template <> struct Unpack32<B200_TYPE_Q5_1> : UnpackLegacy<B200_TYPE_Q5_1> {};
 
-// 16 nibble bytes of an iq4 sub-block as four words: levels + 128, eight at a time
-__device__ __forceinline__ void unpack_iq4x32(const unsigned (&q)[4], float dl, unsigned *o) {
+// an iq4 sub-block of 32: levels + 128
+__device__ __forceinline__ void unpack_iq4x32(const unsigned (&q)[4], float dl, unsigned (&o)[16]) {
     const Scale2 s = {pack_f2(dl, dl), pack_f2(-128.0f * dl, -128.0f * dl)};
 #pragma unroll
     for (int i = 0; i < 4; i++) {
@@ -293,65 +282,54 @@ __device__ __forceinline__ void unpack_iq4x32(const unsigned (&q)[4], float dl, 
         unpack_u8x4(hi ^ 0x80808080u, s, o + 8 + 2 * i);
     }
 }
-template <> struct Unpack<B200_TYPE_IQ4_NL> {
-    static __device__ __forceinline__ void run(const unsigned char *g, int c, unsigned (&o)[32]) {
-        unsigned w[9];
-        lds_run<9>(g + 36 * c, w);
-#pragma unroll
-        for (int b = 0; b < 2; b++) {
-            const unsigned q[4] = {word_at(w, 18 * b + 2), word_at(w, 18 * b + 6), word_at(w, 18 * b + 10), word_at(w, 18 * b + 14)};
-            unpack_iq4x32(q, f16_at(w, 18 * b), o + 16 * b);
-        }
+template <> struct Unpack32<B200_TYPE_IQ4_NL> {
+    static __device__ __forceinline__ void run(const unsigned char *g, int c, int h, unsigned (&o)[16]) {
+        const unsigned char *blk = g + 36 * c + 18 * h;
+        unsigned q[4];
+        lds_run<4>(blk + 2, q);
+        unpack_iq4x32(q, h2f(*reinterpret_cast<const unsigned short *>(blk)), o);
     }
 };
-template <> struct Unpack<B200_TYPE_IQ4_XS> {
-    static __device__ __forceinline__ void run(const unsigned char *g, int c, unsigned (&o)[32]) {
-        unsigned hdr[2], w[8];
+template <> struct Unpack32<B200_TYPE_IQ4_XS> {
+    static __device__ __forceinline__ void run(const unsigned char *g, int c, int h, unsigned (&o)[16]) {
+        unsigned hdr[2], q[4];
         lds_run<2>(g, hdr);
-        lds_run<8>(g + 8 + 32 * c, w);
-        const float d = f16lo(hdr[0]);
-#pragma unroll
-        for (int b = 0; b < 2; b++) {
-            const unsigned q[4] = {w[4 * b], w[4 * b + 1], w[4 * b + 2], w[4 * b + 3]};
-            unpack_iq4x32(q, d * iq4xs_scale(hdr[1], hdr[0] >> 16, 2 * c + b), o + 16 * b);
-        }
+        lds_run<4>(g + 8 + 32 * c + 16 * h, q);
+        unpack_iq4x32(q, f16lo(hdr[0]) * iq4xs_scale(hdr[1], hdr[0] >> 16, 2 * c + h), o);
     }
 };
 // q2_K / q3_K: chunk c is bit fields 2 (c & 1) and 2 (c & 1) + 1 of half c >> 1; its four scales are bytes 4c .. 4c + 3 of the 16
-template <> struct Unpack<B200_TYPE_Q2_K> {
-    static __device__ __forceinline__ void run(const unsigned char *g, int c, unsigned (&o)[32]) {
-        unsigned q[8], sc[1], dm[1];
-        lds_run<8>(g + 16 + 32 * (c >> 1), q);
-        lds_run<1>(g + 4 * c, sc);
-        lds_run<1>(g + 80, dm);
-        const float d = f16lo(dm[0]), dmin = f16hi(dm[0]);
+template <> struct Unpack32<B200_TYPE_Q2_K> {
+    static __device__ __forceinline__ void run(const unsigned char *g, int c, int h, unsigned (&o)[16]) {
+        unsigned q[4];
+        lds_run<4>(g + 16 + 32 * (c >> 1) + 16 * h, q);
+        const unsigned ba = g[4 * c + h], bb = g[4 * c + 2 + h];
+        const float d = h2f(*reinterpret_cast<const unsigned short *>(g + 80)), dmin = h2f(*reinterpret_cast<const unsigned short *>(g + 82));
+        const Scale2 a = scale_q7(d * (float)(ba & 15), -(dmin * (float)(ba >> 4))), b = scale_q7(d * (float)(bb & 15), -(dmin * (float)(bb >> 4)));
 #pragma unroll
-        for (int gr = 0; gr < 4; gr++) {
-            const unsigned b = (sc[0] >> (8 * gr)) & 0xff;
-            const Scale2 s = scale_q7(d * (float)(b & 15), -(dmin * (float)(b >> 4)));
-#pragma unroll
-            for (int i = 0; i < 4; i++) unpack_q7x4((q[4 * (gr & 1) + i] >> (4 * (c & 1) + 2 * (gr >> 1))) & 0x03030303u, s, o + 8 * gr + 2 * i);
+        for (int i = 0; i < 4; i++) {
+            const unsigned f = q[i] >> (4 * (c & 1));
+            unpack_q7x4(f & 0x03030303u, a, o + 2 * i);
+            unpack_q7x4((f >> 2) & 0x03030303u, b, o + 8 + 2 * i);
         }
     }
 };
-template <> struct Unpack<B200_TYPE_Q3_K> {
-    static __device__ __forceinline__ void run(const unsigned char *g, int c, unsigned (&o)[32]) {
-        unsigned q[8], h[8], sw[3];
-        lds_run<8>(g + 32 + 32 * (c >> 1), q);
-        lds_run<8>(g, h);
+template <> struct Unpack32<B200_TYPE_Q3_K> {
+    static __device__ __forceinline__ void run(const unsigned char *g, int c, int h, unsigned (&o)[16]) {
+        unsigned q[4], m[4], sw[3];
+        lds_run<4>(g + 32 + 32 * (c >> 1) + 16 * h, q);
+        lds_run<4>(g + 16 * h, m);
         lds_run<3>(g + 96, sw);
-        const float d = h2f(*reinterpret_cast<const unsigned short *>(g + 108));
         // word c of the 16 scales (q3k_scales)
         const unsigned sc = ((((c & 1) ? sw[1] : sw[0]) >> (c & 2 ? 4 : 0)) & 0x0f0f0f0fu) | (((sw[2] >> (2 * c)) & 0x03030303u) << 4);
+        const float d = h2f(*reinterpret_cast<const unsigned short *>(g + 108));
+        const float da = d * (float)((int)((sc >> (8 * h)) & 0xff) - 32), db = d * (float)((int)((sc >> (16 + 8 * h)) & 0xff) - 32);
+        const Scale2 a = scale_q7(da, -4.0f * da), b = scale_q7(db, -4.0f * db);
 #pragma unroll
-        for (int gr = 0; gr < 4; gr++) {
-            const float dl = d * (float)((int)((sc >> (8 * gr)) & 0xff) - 32);
-            const Scale2 s = scale_q7(dl, -4.0f * dl);
-#pragma unroll
-            for (int i = 0; i < 4; i++) {
-                const int l = 4 * (gr & 1) + i;
-                unpack_q7x4(((q[l] >> (4 * (c & 1) + 2 * (gr >> 1))) & 0x03030303u) + ((h[l] >> (2 * c + (gr >> 1))) & 0x01010101u) * 4u, s, o + 8 * gr + 2 * i);
-            }
+        for (int i = 0; i < 4; i++) {
+            const unsigned f = q[i] >> (4 * (c & 1)), k = m[i] >> (2 * c);
+            unpack_q7x4((f & 0x03030303u) + (k & 0x01010101u) * 4u, a, o + 2 * i);
+            unpack_q7x4(((f >> 2) & 0x03030303u) + (k & 0x02020202u) * 2u, b, o + 8 + 2 * i);
         }
     }
 };
@@ -479,10 +457,13 @@ __global__ void __launch_bounds__(pair_threads<TYPE>(), 1) mmq_pair_kernel(const
                 slot_in = slot_in + 1 == SLOTS ? 0 : slot_in + 1;
             };
             for (int i = 0; i < SLOTS - 1; i++) copy_group();
-            const int c = lane >> 3, r = lane & 7;
-            const unsigned a_row = smem_u32(smem) + (unsigned)(warp * 1024 + r * 128 + (r << 4));  // piece q of the row lies at a_row ^ (q << 4)
-            int s0 = 0, slot = 0;       // stage of the group's first K step
-            unsigned ph0 = 1;           // parity of its empty barrier: the first pass finds it free
+            const int cc = lane >> 4, h = (lane >> 3) & 1, r = lane & 7;  // chunk of a pair of K steps, half of its bytes, row
+            // the lane's four 16-byte pieces of row r, swizzled
+            const unsigned a_row = smem_u32(smem) + (unsigned)(warp * 1024 + r * 128);
+            const int f0 = unpack_first(TYPE, h) / 8, f1 = unpack_second(TYPE, h) / 8;
+            const unsigned p0 = a_row + (unsigned)((f0 ^ r) << 4), p1 = a_row + (unsigned)(((f0 + 1) ^ r) << 4), p2 = a_row + (unsigned)((f1 ^ r) << 4), p3 = a_row + (unsigned)(((f1 + 1) ^ r) << 4);
+            int s = 0, slot = 0;        // stage of the first K step of the pair
+            unsigned ph = 1;            // parity of its empty barrier: the first pass finds it free
             for (int t = pair; t < n_tiles; t += n_pairs) {
                 const PairTile ti = pair_tile<GROUPED>(p, t, nt, UNIT);
                 unsigned at = raw_aligned(TYPE) ? 0u : (unsigned)(uintptr_t)row_base(ti, r) & 15u;  // where in its first piece the row's group starts
@@ -491,23 +472,31 @@ __global__ void __launch_bounds__(pair_threads<TYPE>(), 1) mmq_pair_kernel(const
                     cp_async_wait<SLOTS - 2>();
                     __syncwarp();  // the group has landed for all lanes, and all have left the one before
                     copy_group();
-                    unsigned o[32];
-                    Unpack<TYPE>::run(raw + (slot * 8 + r) * ROW + at, c, o);
+                    const unsigned char *row = raw + (slot * 8 + r) * ROW + at;
                     if constexpr (!raw_aligned(TYPE)) at = (at + G256) & 15u;
                     slot = slot + 1 == SLOTS ? 0 : slot + 1;
-                    // stages are freed in order: the last of the four stands for all
-                    const bool wrap = s0 + 3 >= S;
-                    pair_wait<20>(empty0 + 8u * (unsigned)(wrap ? s0 + 3 - S : s0 + 3), wrap ? ph0 ^ 1u : ph0, &failed);
-                    const int mine = s0 + c >= S ? s0 + c - S : s0 + c;
-                    const unsigned d = a_row + (unsigned)(mine * stage_bytes);
 #pragma unroll
-                    for (int q = 0; q < 8; q++)
-                        asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(d ^ (q << 4)), "r"(o[4 * q]), "r"(o[4 * q + 1]), "r"(o[4 * q + 2]), "r"(o[4 * q + 3]) : "memory");
-                    fence_proxy_async_smem();
-                    __syncwarp();
-                    if (r == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(full0 + 8u * (unsigned)mine) : "memory");
-                    s0 += 4;
-                    if (s0 >= S) { s0 -= S; ph0 ^= 1u; }
+                    for (int c2 = 0; c2 < 4; c2 += 2) {
+                        unsigned o[16];
+                        Unpack32<TYPE>::run(row, c2 + cc, h, o);
+                        // stages are freed in order: the second of the two stands for both
+                        const bool wrap = s + 1 >= S;
+                        const int s1 = wrap ? s + 1 - S : s + 1;
+                        const unsigned ph1 = wrap ? ph ^ 1u : ph;
+                        pair_wait<20>(empty0 + 8u * s1, ph1, &failed);
+                        const int mine = cc ? s1 : s;
+                        const unsigned d = (unsigned)(mine * stage_bytes);
+                        asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(p0 + d), "r"(o[0]), "r"(o[1]), "r"(o[2]), "r"(o[3]) : "memory");
+                        asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(p1 + d), "r"(o[4]), "r"(o[5]), "r"(o[6]), "r"(o[7]) : "memory");
+                        asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(p2 + d), "r"(o[8]), "r"(o[9]), "r"(o[10]), "r"(o[11]) : "memory");
+                        asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(p3 + d), "r"(o[12]), "r"(o[13]), "r"(o[14]), "r"(o[15]) : "memory");
+                        fence_proxy_async_smem();
+                        __syncwarp();
+                        if ((lane & 15) == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(full0 + 8u * mine) : "memory");
+                        s = s1 + 1;
+                        ph = ph1;
+                        if (s == S) { s = 0; ph ^= 1u; }
+                    }
                 }
             }
             cp_async_wait<0>();
