@@ -7,15 +7,12 @@
 // fallback that koboldcpp uses by default (ggml-cuda.cu:1186-1284: whole-tensor dequant to f16 in HBM, then cublasGemmEx).
 //
 // B200 design (the one dense contraction of the path: tensor-pipe bound once N is a few hundred):
-//   * weights are dequantised ON THE FLY into bf16 operand tiles in shared memory (never to HBM) by 4 producer warps --
-//     thread t owns weight row t of the 128-row tile and writes its 64-value K-step straight into the 128-byte-swizzled
-//     K-major layout the tensor core reads; activations are converted f32 -> bf16 once per call by a pre-pass and staged
-//     with 16-byte cp.async into the same swizzled layout;
-//   * one elected thread issues tcgen05.mma (kind::f16, bf16 x bf16 -> f32, M=128, N<=256, K=16 x4 per stage); the f32
-//     accumulator tile lives in TMEM (N columns x 128 lanes), so the producers' registers are free for unpacking;
-//   * 4-stage shared-memory ring with mbarrier full/empty pairs; tcgen05.commit releases a stage when the MMAs that read
-//     it retire -- no CTA-wide barrier in the K loop;
-//   * epilogue: the same 4 warps read their TMEM lane quarter (tcgen05.ld 32x32b) and store f32 rows coalesced along m.
+//   * weights are dequantised ON THE FLY into bf16 operand tiles in shared memory (never to HBM), in the 128-byte-swizzled K-major layout
+//     the tensor core reads; activations are converted f32 -> bf16 once per call by a pre-pass;
+//   * tcgen05.mma (kind::f16, bf16 x bf16 -> f32), the f32 accumulators in TMEM; a shared-memory ring with mbarrier full/empty pairs,
+//     tcgen05.commit releases a stage when the MMAs that read it retire -- no CTA-wide barrier in the K loop.
+// mmq_pair.cuh holds the kernel of almost every call (K a multiple of 256, dense rows); here are the formats' definitions, mmq_tc_kernel for
+// the legacy formats with other K, a dense kernel for odd strides, MUL_MAT_ID's grouping, and the entry points.
 // Why bf16 and not kind::i8: per-32 (per-16 for Q6_K) group scales would force a TMEM read-out after every K=32 MMA,
 // which is epilogue-bound; bf16 operands keep the whole K loop inside the tensor pipe.  Activations carry 8 mantissa bits
 // (q8_1 carries 7 + sign per 32-block), weights are rounded once from their exact f32 dequantised value.
@@ -510,32 +507,17 @@ __global__ void __launch_bounds__(MQ_THREADS, 1) mmq_tc_kernel(const __grid_cons
     }
 }
 
-// ---------------------------------------------------------------- register-resident variant (software-pipelined producers)
-// A thread keeps the raw bytes of one 256-value group of its row in registers (w[], block start at word 0) and unpacks chunk
-// C (compile time) from them.  Small integers become floats without I2F: PRMT drops the byte into the mantissa of 2^23
-// (0x4B0000bb = 8388608 + b), one exact FADD removes the bias.
-__host__ __device__ constexpr int group256_words(int t) { return (group256_bytes(t) + 3) / 4; }
+// small integers become floats without I2F: PRMT drops the byte into the mantissa of 2^23 (0x4B0000bb = 8388608 + b), one exact FADD removes the bias
 template <int K> __device__ __forceinline__ float byte_f(unsigned x) {  // float(byte K of x), exact
     return __uint_as_float(__byte_perm(x, 0x4B000000u, 0x7650 + K)) - 8388608.0f;
 }
-__device__ __forceinline__ float f16_at(const unsigned *w, int byte_off) {  // fp16 at an even byte offset
-    return (byte_off & 2) ? f16hi(w[byte_off >> 2]) : f16lo(w[byte_off >> 2]);
-}
 
-// ================================================================ v2: asynchronous operand supply
-// Same tensor-core pipeline, but neither operand waits on a global load inside the producers:
-//   * B (bf16 activations) arrives by TMA (cp.async.bulk.tensor.2d, 128-byte swizzle applied by the copy engine) issued by
-//     a dedicated warp as soon as a stage is free;
-//   * the raw quantised blocks of the NEXT 256-value group of each of the 128 rows are staged in shared memory by 1-D bulk
-//     copies (one per row, issued by the row's own thread, aligned-down windows like the decode GEMV) two groups ahead, so the
-//     producers unpack from shared memory.  A thread only ever reads its own row's slot: re-arming a slot needs no CTA barrier.
+// ================================================================ dense bf16 rows whose products lie at odd strides
+// What one tensor map cannot cover (an expert or batch stride that is no multiple of the row stride): the weight rows pass through the
+// producers' registers, the activations arrive by TMA (cp.async.bulk.tensor.2d, 128-byte swizzle applied by the copy engine), issued by a
+// dedicated warp as soon as a stage is free.  Everything else runs on the pair kernel (mmq_pair.cuh).
 constexpr int MQ2_STAGES = 4;
 constexpr int MQ2_THREADS = MQ_PRODUCERS + 64;  // + MMA warp + TMA warp
-// per-row slot stride: >= group bytes + 14 bytes of head misalignment (2-byte aligned formats), rounded to 16, and an ODD
-// number of 16-byte units so that the 8 threads of a quarter-warp hit distinct bank groups with 16-byte accesses
-__host__ __device__ constexpr int raw_stride(int t) {
-    return t == B200_TYPE_Q4_K ? 144 : t == B200_TYPE_Q5_K ? 176 : t == B200_TYPE_Q6_K ? 240 : t == B200_TYPE_Q8_0 ? 304 : 176;
-}
 
 __device__ __forceinline__ void tma_load_2d(void *dst, const void *tmap, int c0, int c1, unsigned long long *bar) {
     asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(smem_u32(dst)),
@@ -680,120 +662,6 @@ __global__ void __launch_bounds__(MQ2_THREADS, 1) mmq_tc2_kernel(const __grid_co
     }
 }
 
-// ================================================================ dense bf16 weights: both operands by TMA
-// Dense rows need no unpacking, so nothing stands between HBM and the tensor core: one warp's elected lane requests the weight tile
-// [128 rows x 64] and the activation tile [BN rows x 64] of every stage (128-byte swizzle by the copy engine) as soon as the stage is
-// free, one lane issues the MMAs, four warps read the accumulators out of TMEM.  The stages are as many as shared memory takes, all
-// of them in flight.  Every wait has a limit: a role that gives up says so in shared memory, the others run into their own limits, the
-// copies in flight are waited for, TMEM is freed, nothing is stored and *timeout is set.
-constexpr long long BG_WAIT_LIMIT = 4000000000LL;  // clock cycles: about two seconds
-template <int BN> constexpr int bg_stages() { return BN >= 256 ? 4 : BN >= 128 ? 6 : 8; }
-template <int BN, bool GROUPED>
-__global__ void __launch_bounds__(MQ2_THREADS, 1) bf16_gemm_kernel(const __grid_constant__ TmapBytes tmA, const __grid_constant__ TmapBytes tmB, const __grid_constant__ MmqParams p,
-                                                                   int64_t w_rows_per_product, int *timeout) {
-    constexpr int STAGES = bg_stages<BN>(), A_BYTES = MQ_BM * MQ_BK * 2, B_BYTES = BN * MQ_BK * 2, STAGE_BYTES = A_BYTES + B_BYTES;
-    int64_t n0 = (int64_t)blockIdx.y * BN, n_end = p.N, a_row = (int64_t)blockIdx.x * MQ_BM;
-    const int64_t m0 = a_row;
-    if constexpr (GROUPED) {  // uniform over the CTA: tiles past the table's end have nothing to do
-        if ((int)blockIdx.y >= __ldg(p.tile_tab)) return;
-        const int *te = p.tile_tab + 1 + 3 * blockIdx.y;
-        a_row += (int64_t)__ldg(te) * w_rows_per_product;
-        n0 = __ldg(te + 1);
-        n_end = __ldg(te + 2);
-    }
-    extern __shared__ unsigned char smem_raw[];
-    unsigned char *smem = reinterpret_cast<unsigned char *>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-    __shared__ __align__(8) unsigned long long full_bar[STAGES], empty_bar[STAGES], tmem_full_bar;
-    __shared__ unsigned tmem_base_s;
-    __shared__ volatile int failed;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, tid = threadIdx.x;
-    const int nkb_all = (int)(p.K / MQ_BK);
-    const int ksplit = GROUPED ? 1 : p.ksplit;  // split-K: this CTA's steps [kb0, kb0 + nkb)
-    const bool batched = !GROUPED && p.n_batch > 1;
-    const int zk = batched ? 0 : (int)blockIdx.z, zb = batched ? (int)blockIdx.z : 0;
-    a_row += zb * w_rows_per_product;
-    const int kb0 = (int)(((int64_t)zk * nkb_all) / ksplit), nkb = (int)(((int64_t)(zk + 1) * nkb_all) / ksplit) - kb0;
-
-    if (tid == 0) {
-        for (int s = 0; s < STAGES; s++) { mbar_init(&full_bar[s], 1); mbar_init(&empty_bar[s], 1); }
-        mbar_init(&tmem_full_bar, 1);
-        failed = 0;
-        mbar_fence_init();
-    }
-    if (warp == 4) tmem_alloc(&tmem_base_s, BN);
-    tc_fence_before();
-    __syncthreads();
-    tc_fence_after();
-    const unsigned tmem_base = tmem_base_s;
-
-    if (warp == 5) {
-        if (lane == 0) {
-            int kb = 0;
-            for (; kb < nkb; kb++) {
-                const int s = kb % STAGES;
-                if (!mbar_wait_limited(&empty_bar[s], ((unsigned)(kb / STAGES) & 1u) ^ 1u, BG_WAIT_LIMIT)) { failed = 1; break; }
-                unsigned char *st = smem + (size_t)s * STAGE_BYTES;
-                mbar_expect_tx(&full_bar[s], (unsigned)STAGE_BYTES);
-                tma_load_2d(st, &tmA, (kb0 + kb) * MQ_BK, (int)a_row, &full_bar[s]);
-                tma_load_2d(st + A_BYTES, &tmB, (kb0 + kb) * MQ_BK, (int)n0 + (batched ? zb * (int)p.n_pad : 0), &full_bar[s]);
-            }
-            if (kb < nkb)  // gave up: the copies that were requested still have to land before this CTA may end
-                for (int j = kb > STAGES ? kb - STAGES : 0; j < kb; j++) mbar_wait_limited(&full_bar[j % STAGES], (unsigned)(j / STAGES) & 1u, BG_WAIT_LIMIT);
-        }
-    } else if (warp == 4) {
-        constexpr unsigned idesc = umma_idesc_bf16(MQ_BM, BN);
-        int kb = 0;
-        for (; kb < nkb; kb++) {
-            const int s = kb % STAGES;
-            const bool ok = mbar_wait_limited(&full_bar[s], (unsigned)(kb / STAGES) & 1u, BG_WAIT_LIMIT);
-            if (!__all_sync(0xffffffffu, ok)) { failed = 1; break; }
-            tc_fence_after();
-            if (lane == 0) {
-                const unsigned a_addr = smem_u32(smem + (size_t)s * STAGE_BYTES), b_addr = a_addr + A_BYTES;
-#pragma unroll
-                for (int k = 0; k < MQ_BK / 16; k++)
-                    tc_mma_bf16(tmem_base, umma_desc_sw128(a_addr) + 2u * k, umma_desc_sw128(b_addr) + 2u * k, idesc, (kb | k) != 0 ? 1u : 0u);
-                tc_commit(&empty_bar[s]);
-                if (kb == nkb - 1) tc_commit(&tmem_full_bar);
-            }
-            __syncwarp();
-        }
-        if (kb < nkb && lane == 0) tc_commit(&tmem_full_bar);  // gave up: releases the epilogue once the MMAs issued so far have retired
-        __syncwarp();
-        tc_fence_before();
-    } else {
-        bool ok = mbar_wait_limited(&tmem_full_bar, 0u, 3 * BG_WAIT_LIMIT);
-        ok = __all_sync(0xffffffffu, ok);
-        if (!ok) failed = 1;
-        tc_fence_after();
-        const int64_t m = m0 + tid;
-        const bool row_ok = m < p.M && ok && !failed;
-        float *drow = p.dst + m + (batched ? (int64_t)zb * p.dst_batch : 0);
-#pragma unroll 1
-        for (int c0 = 0; c0 < BN; c0 += 32) {
-            float v[32];
-            tmem_ld32(tmem_base + ((unsigned)(warp * 32) << 16) + (unsigned)c0, v);
-            if (row_ok) {
-#pragma unroll
-                for (int j = 0; j < 32; j++) {
-                    const int64_t n = n0 + c0 + j;
-                    if (n >= n_end) continue;
-                    if constexpr (GROUPED) drow[(int64_t)__ldg(p.row_dst + n)] = v[j];  // scatter: sorted row -> (token, slot)
-                    else if (ksplit > 1) atomicAdd(drow + n * p.dst_stride, v[j]);      // (result unused: RED.ADD.F32)
-                    else drow[n * p.dst_stride] = v[j];
-                }
-            }
-        }
-        tc_fence_before();
-    }
-    __syncthreads();
-    if (tid == 0 && failed && timeout) atomicExch(timeout, 1);
-    if (warp == 4) {
-        tc_fence_after();
-        tmem_dealloc(tmem_base, BN);
-    }
-}
-
 // ---------------------------------------------------------------- host side
 // set by a GEMM whose pipeline gave up; pinned host memory, so that reading it after a synchronisation costs nothing
 static int *g_gemm_timeout = nullptr;
@@ -852,47 +720,8 @@ static int encode_rows(TmapBytes &tm, const void *base, int64_t K, int64_t rows,
 #include "mmq_pair.cuh"
 namespace b200 {
 
-template <int BN, bool GROUPED>
-static int bf16_gemm_launch(const MmqParams &p, int64_t n_pad, int64_t w_rows_per_product, cudaStream_t st, unsigned grid_y) {
-    constexpr size_t smem = (size_t)bg_stages<BN>() * (MQ_BM * MQ_BK * 2 + BN * MQ_BK * 2) + 1024;
-    static bool attr_set_dev[16] = {};  // cudaFuncSetAttribute is per device
-    int cur_dev = 0;
-    B200_CUDA_TRY(cudaGetDevice(&cur_dev));
-    bool &attr_set = attr_set_dev[cur_dev & 15];
-    if (!attr_set) {
-        B200_CUDA_TRY(cudaFuncSetAttribute(bf16_gemm_kernel<BN, GROUPED>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        attr_set = true;
-    }
-    const int64_t products = GROUPED ? p.n_expert : p.n_batch;
-    TmapBytes tmA, tmB;
-    int rc = encode_rows(tmA, p.W, p.K, (products - 1) * w_rows_per_product + p.M, p.w_row_bytes, MQ_BM);
-    if (rc != B200_OK) return rc;
-    rc = encode_rows(tmB, p.Xb, p.K, n_pad * (p.n_batch > 1 ? p.n_batch : 1), (size_t)p.K * 2, BN);
-    if (rc != B200_OK) return rc;
-    dim3 grid((unsigned)((p.M + MQ_BM - 1) / MQ_BM), GROUPED ? grid_y : (unsigned)((p.N + BN - 1) / BN));
-    MmqParams q = p;
-    q.ksplit = 1;
-    if (p.n_batch > 1) {
-        grid.z = (unsigned)p.n_batch;
-    } else if (!GROUPED && (int64_t)grid.x * grid.y * 2 <= 148 && p.K >= 2048) {
-        // fewer tiles than half the SMs: two CTAs share a tile's K range and add into a zeroed dst (two partials only: the sum is
-        // independent of the arrival order)
-        q.ksplit = 2;
-        grid.z = 2;
-        if (p.dst_stride == p.M) B200_CUDA_TRY(cudaMemsetAsync(p.dst, 0, (size_t)p.M * p.N * sizeof(float), st));
-        else B200_CUDA_TRY(cudaMemset2DAsync(p.dst, (size_t)p.dst_stride * sizeof(float), 0, (size_t)p.M * sizeof(float), (size_t)p.N, st));
-    }
-    bf16_gemm_kernel<BN, GROUPED><<<grid, MQ2_THREADS, smem, st>>>(tmA, tmB, q, w_rows_per_product, g_gemm_timeout);
-    B200_CUDA_TRY(cudaGetLastError());
-    return B200_OK;
-}
-
 template <int TYPE, int BN, bool GROUPED = false>
 static int mmq2_launch(const MmqParams &p, int64_t n_pad, cudaStream_t st, unsigned grid_y = 0) {
-    if constexpr (TYPE == B200_TYPE_BF16) {  // products whose weight rows lie at one stride over all of them: one tensor map covers the stack
-        const size_t step = GROUPED ? p.expert_bytes : p.n_batch > 1 ? p.w_batch_bytes : 0;
-        if (step % p.w_row_bytes == 0) return bf16_gemm_launch<BN, GROUPED>(p, n_pad, (int64_t)(step / p.w_row_bytes), st, grid_y);
-    }
     constexpr size_t smem = (size_t)MQ2_STAGES * (MQ_BM * MQ_BK * 2 + BN * MQ_BK * 2) + 1024;
     static bool attr_set_dev[16] = {};  // cudaFuncSetAttribute is per device
     int cur_dev = 0;
@@ -935,12 +764,11 @@ static int mmq2_launch(const MmqParams &p, int64_t n_pad, cudaStream_t st, unsig
 
 template <int TYPE>
 static int mmq_dispatch_bn(const MmqParams &p, cudaStream_t st) {
-    if constexpr (TYPE == B200_TYPE_BF16) {  // dense rows: the asynchronous kernel only, any K that is a multiple of the K step
+    if constexpr (TYPE == B200_TYPE_BF16) {  // dense rows: any K that is a multiple of the K step
         const int64_t n_pad = mmq_n_pad(p.N);
-        // few rows of weights: narrower tiles until they fill the device at least by half (with the two halves of K)
-        int64_t bn = mmq_bn(p.N);
-        while (bn > 32 && (p.M + MQ_BM - 1) / MQ_BM * ((p.N + bn - 1) / bn) * p.n_batch * 4 <= 148) bn /= 2;
-        switch (bn) {
+        // products whose weight rows lie at one stride over all of them: one tensor map covers the stack
+        if (p.n_batch == 1 || p.w_batch_bytes % p.w_row_bytes == 0) return mmq_pair_launch<TYPE, false>(p, n_pad, p.n_batch > 1 ? (int64_t)(p.w_batch_bytes / p.w_row_bytes) : 0, 0, 0, st);
+        switch (mmq_bn(p.N)) {
             case 32: return mmq2_launch<TYPE, 32>(p, n_pad, st);
             case 64: return mmq2_launch<TYPE, 64>(p, n_pad, st);
             case 128: return mmq2_launch<TYPE, 128>(p, n_pad, st);
@@ -1026,23 +854,26 @@ __global__ void mid_gather_bf16_kernel(const float *__restrict__ b, const int *_
 
 static int64_t mid_bn(int64_t n_rows, int n_expert) { return mmq_bn((n_rows + n_expert - 1) / n_expert); }
 static int64_t mid_max_tiles(int64_t bn, int64_t n_rows, int n_expert) { return (n_rows + bn - 1) / bn + n_expert; }
-// quantised experts: the tile's width follows its rows, so the table's tiles are as wide as the accumulators allow unless experts are small
-static int64_t mid_tile(int type, int64_t n_rows, int n_expert) {
+// experts whose rows lie at one stride over the stack (quantised ones need no stack): the pair kernel
+static bool mid_pair(int type, size_t w_row_bytes, size_t expert_bytes) { return type != B200_TYPE_BF16 || expert_bytes % w_row_bytes == 0; }
+// there the width of a tile follows its rows, so the table's tiles are as wide as the accumulators allow unless experts are small
+static int64_t mid_tile(bool pair, int64_t n_rows, int n_expert) {
     const int64_t bn = mid_bn(n_rows, n_expert);
-    return type == B200_TYPE_BF16 ? bn : bn < 128 ? 2 * bn : 256;
+    return !pair ? bn : bn < 128 ? 2 * bn : 256;
 }
 static size_t mid_xb_bytes(int64_t n_rows, int64_t K) { return ((size_t)n_rows * (size_t)K * 2 + 255) / 256 * 256; }
 
 template <int TYPE>
 static int mid_dispatch_bn(const MmqParams &p, int64_t bn, int64_t n_rows, unsigned grid_y, cudaStream_t st) {
-    if constexpr (TYPE != B200_TYPE_BF16) return mmq_pair_launch<TYPE, true>(p, n_rows, 0, grid_y, bn, st);
-    else
+    if (mid_pair(TYPE, p.w_row_bytes, p.expert_bytes)) return mmq_pair_launch<TYPE, true>(p, n_rows, (int64_t)(p.expert_bytes / p.w_row_bytes), grid_y, bn, st);
+    if constexpr (TYPE == B200_TYPE_BF16)
     switch (bn) {
         case 32: return mmq2_launch<TYPE, 32, true>(p, n_rows, st, grid_y);
         case 64: return mmq2_launch<TYPE, 64, true>(p, n_rows, st, grid_y);
         case 128: return mmq2_launch<TYPE, 128, true>(p, n_rows, st, grid_y);
         default: return mmq2_launch<TYPE, 256, true>(p, n_rows, st, grid_y);
     }
+    return B200_ERR_UNSUPPORTED;
 }
 
 }  // namespace b200
@@ -1181,7 +1012,7 @@ extern "C" int b200_mul_mat_id_q(int type, const void *as, size_t w_row_bytes, s
         return B200_ERR_INVALID;
     }
     const cudaStream_t st = (cudaStream_t)stream;
-    const int64_t bn = mid_tile(type, n_rows, n_expert), max_tiles = mid_max_tiles(bn, n_rows, n_expert);
+    const int64_t bn = mid_tile(mid_pair(type, w_row_bytes, expert_bytes), n_rows, n_expert), max_tiles = mid_max_tiles(bn, n_rows, n_expert);
     __nv_bfloat16 *xb = (__nv_bfloat16 *)workspace;
     MidTables t;
     t.tile_tab = (int *)((unsigned char *)workspace + mid_xb_bytes(n_rows, K));

@@ -38,7 +38,7 @@ struct PairParams {
     MmqParams q;
     int64_t w_rows_per_product;  // dense weights by TMA: rows from one product (batch, expert) to the next
     int bn;                      // columns of a tile (grouped: at most), a multiple of 16; grouped: of 32
-    int box;                     // activation rows of one TMA box
+    int box;                     // activation rows of one TMA box: all of the CTA's, grouped: 16
     int stages;
     int n_tiles_n, n_tiles_m;    // n_tiles_n of the grouped form: read from the tile table
     int *timeout;
@@ -46,7 +46,8 @@ struct PairParams {
 
 // ---------------------------------------------------------------- the pair's wrappers
 __device__ __forceinline__ unsigned cluster_rank() { unsigned r; asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r)); return r; }
-__device__ __forceinline__ void pair_sync() { asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+__device__ __forceinline__ void pair_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void pair_await() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
 __device__ __forceinline__ bool elect_lane() {
     unsigned e;
     asm volatile("{\n.reg .pred p;\nelect.sync _|p, 0xffffffff;\nselp.u32 %0, 1, 0, p;\n}\n" : "=r"(e));
@@ -73,17 +74,15 @@ __device__ __forceinline__ void tc_mma2_bf16(unsigned tmem_d, unsigned long long
 __device__ __forceinline__ void tc_commit2(unsigned bar) {
     asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(bar), "h"((unsigned short)3) : "memory");
 }
-// arrive on `bar` of the pair's first CTA.  (The default semantics: what the barrier guards is in shared memory or TMEM and complete when the
-// arrival is issued; a release at cluster scope would wait for the thread's outstanding memory operations, about 1000 cycles a K step.)
-__device__ __forceinline__ void mbar_arrive_leader(unsigned bar) {
-    asm volatile(
-        "{\n"
-        ".reg .b32 ra;\n"
-        "mapa.shared::cluster.u32 ra, %0, 0;\n"
-        "mbarrier.arrive.shared::cluster.b64 _, [ra];\n"
-        "}\n" ::"r"(bar)
-        : "memory");
+// the pair's first CTA's copy of a shared variable, and an arrival there.  (The default semantics: what the barrier guards is in shared memory or TMEM
+// and complete when the arrival is issued; a release at cluster scope would wait for the thread's outstanding memory operations, about 1000
+// cycles a K step.)
+__device__ __forceinline__ unsigned leader_addr(unsigned local) {
+    unsigned r;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(r) : "r"(local));
+    return r;
 }
+__device__ __forceinline__ void mbar_arrive_remote(unsigned bar) { asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory"); }
 __device__ __forceinline__ bool mbar_try(unsigned bar, unsigned parity) {
     unsigned done;
     asm volatile(
@@ -97,21 +96,18 @@ __device__ __forceinline__ bool mbar_try(unsigned bar, unsigned parity) {
         : "memory");
     return done != 0;
 }
-// wait with the limit; at once when a role of the CTA has given up.  SLEEP: nanoseconds between two looks (a failing try_wait comes back within some
-// 50 cycles whatever time it is offered, and a dozen polling warps take the issue slots of the others).  The caller's control flow does not
-// depend on the outcome.
+// wait with the limit; false, at once, when a role of the CTA has given up.  SLEEP: nanoseconds between two looks (a failing try_wait comes back within
+// some 50 cycles whatever time it is offered, and a dozen polling warps take the issue slots of the others).
 template <int SLEEP>
-__device__ __forceinline__ void pair_wait_slow(unsigned bar, unsigned parity, volatile int *failed) {
+__device__ __forceinline__ bool pair_wait(unsigned bar, unsigned parity, volatile int *failed) {
+    if (mbar_try(bar, parity)) return true;
     const long long t0 = clock64();
     while (!mbar_try(bar, parity)) {
         if (SLEEP > 0) __nanosleep(SLEEP);
-        if (*failed) return;
-        if (clock64() - t0 > PAIR_WAIT_LIMIT) { *failed = 1; return; }
+        if (*failed) return false;
+        if (clock64() - t0 > PAIR_WAIT_LIMIT) { *failed = 1; return false; }
     }
-}
-template <int SLEEP>
-__device__ __forceinline__ void pair_wait(unsigned bar, unsigned parity, volatile int *failed) {
-    if (!mbar_try(bar, parity)) pair_wait_slow<SLEEP>(bar, parity, failed);
+    return true;
 }
 
 // ---------------------------------------------------------------- 32 values of a row out of shared memory -> 16 packed bf16 pairs
@@ -334,6 +330,7 @@ template <> struct Unpack32<B200_TYPE_Q3_K> {
     }
 };
 
+// words per 256-value group are read at up to 14 bytes behind the slot's row start: raw_row leaves room for the last 8-byte load
 // ---------------------------------------------------------------- the tile that comes next
 struct PairTile {
     int64_t m0;          // first weight row of the pair's tile
@@ -407,7 +404,9 @@ __global__ void __launch_bounds__(pair_threads<TYPE>(), 1) mmq_pair_kernel(const
     if (warp == NP) tmem_alloc2(&tmem_base_s, 512);
     tc_fence_before();
     __syncthreads();
-    pair_sync();
+    // producers and copies touch their own CTA only: they start at once, and wait for the other CTA to be there when they are done
+    pair_arrive();
+    if (warp == NP || warp >= NP + 2) pair_await();
     tc_fence_after();
     const unsigned tmem_base = tmem_base_s;
 
@@ -505,6 +504,7 @@ __global__ void __launch_bounds__(pair_threads<TYPE>(), 1) mmq_pair_kernel(const
         // ===== the pair's MMAs (first CTA); the second CTA passes on that its half of a stage is ready
         const unsigned long long desc0 = umma_desc_sw128(smem_u32(smem));
         const bool elected = elect_lane();
+        const unsigned peer_remote = leader_addr(peer0);
         int s = 0, buf = 0;
         unsigned ph = 0, aph = 1;
         for (int t = pair; t < n_tiles; t += n_pairs) {
@@ -512,7 +512,8 @@ __global__ void __launch_bounds__(pair_threads<TYPE>(), 1) mmq_pair_kernel(const
             if (rank != 0) {
                 for (int kb = 0; kb < ti.nkb; kb++) {
                     pair_wait<0>(full0 + 8u * s, ph, &failed);
-                    if (elected) mbar_arrive_leader(peer0 + 8u * s);
+                    if (elected) mbar_arrive_remote(peer_remote + 8u * s);
+                    __syncwarp();
                     if (++s == S) { s = 0; ph ^= 1u; }
                 }
                 continue;
@@ -545,30 +546,40 @@ __global__ void __launch_bounds__(pair_threads<TYPE>(), 1) mmq_pair_kernel(const
         }
     } else if (warp == NP + 1) {
         // ===== copies: this CTA's half of the activation rows (dense weights: its 128 weight rows too)
-        if (lane == 0) {
-            int s = 0;
-            unsigned ph = 1;
-            for (int t = pair; t < n_tiles; t += n_pairs) {
-                const PairTile ti = pair_tile<GROUPED>(p, t, nt, UNIT);
-                const int half = ti.n / 2, row = (int)(ti.n0 + rank * half + (GROUPED ? 0 : ti.product * p.q.n_pad));
-                for (int kb = 0; kb < ti.nkb; kb++) {
-                    pair_wait<20>(empty0 + 8u * s, ph, &failed);
-                    if (failed) break;  // no copy without a free stage
-                    unsigned char *st = smem + (size_t)s * stage_bytes;
-                    mbar_expect_tx(&full_bar[s], (unsigned)(half * MQ_BK * 2 + (DENSE ? A_BYTES : 0)));
-                    const int k = (ti.kb0 + kb) * MQ_BK;
-                    if constexpr (DENSE) tma_load_2d(st, &tmA, k, (int)(ti.product * p.w_rows_per_product + ti.m0 + rank * MQ_BM), &full_bar[s]);
-                    for (int r = 0; r < half; r += p.box) tma_load_2d(st + A_BYTES + r * MQ_BK * 2, &tmB, k, row + r, &full_bar[s]);
-                    if (++s == S) { s = 0; ph ^= 1u; }
+        // (the whole warp loops, as above)
+        const bool elected = elect_lane();
+        bool dead = false;
+        int s = 0;
+        unsigned ph = 1;
+        for (int t = pair; t < n_tiles; t += n_pairs) {
+            const PairTile ti = pair_tile<GROUPED>(p, t, nt, UNIT);
+            const int half = ti.n / 2, row = (int)(ti.n0 + rank * half + (GROUPED ? 0 : ti.product * p.q.n_pad));
+            const int a_row = DENSE ? (int)(ti.product * p.w_rows_per_product + ti.m0 + rank * MQ_BM) : 0;
+            const unsigned tx = (unsigned)(half * MQ_BK * 2 + (DENSE ? A_BYTES : 0));
+            int k = ti.kb0 * MQ_BK;
+#pragma unroll 1
+            for (int kb = 0; kb < ti.nkb; kb++, k += MQ_BK) {
+                if (!pair_wait<20>(empty0 + 8u * s, ph, &failed)) dead = true;
+                if (elected && !dead) {  // no copy without a free stage
+                    unsigned char *st = smem + (size_t)(s * stage_bytes);
+                    mbar_expect_tx(&full_bar[s], tx);
+                    if constexpr (DENSE) tma_load_2d(st, &tmA, k, a_row, &full_bar[s]);
+                    if constexpr (GROUPED) {
+                        for (int r = 0; r < half; r += 16) tma_load_2d(st + A_BYTES + r * MQ_BK * 2, &tmB, k, row + r, &full_bar[s]);
+                    } else {
+                        tma_load_2d(st + A_BYTES, &tmB, k, row, &full_bar[s]);
+                    }
                 }
+                __syncwarp();
+                if (++s == S) { s = 0; ph ^= 1u; }
             }
         }
-        __syncwarp();
     } else {
         // ===== epilogue: TMEM lanes 32 * (warp % 4) .. of this CTA's 128 rows
         int buf = 0;
         unsigned ph = 0;
         const int quarter = warp & 3;
+        const unsigned acc_remote = leader_addr(acc_empty0);
         for (int t = pair; t < n_tiles; t += n_pairs) {
             const PairTile ti = pair_tile<GROUPED>(p, t, nt, UNIT);
             pair_wait<200>(acc_full0 + 8u * buf, ph, &failed);
@@ -595,19 +606,21 @@ __global__ void __launch_bounds__(pair_threads<TYPE>(), 1) mmq_pair_kernel(const
             }
             tc_fence_before();
             __syncwarp();
-            if (lane == 0) mbar_arrive_leader(acc_empty0 + 8u * buf);
+            if (lane == 0) mbar_arrive_remote(acc_remote + 8u * buf);
             buf ^= 1;
             if (buf == 0) ph ^= 1u;
         }
     }
     __syncwarp();
+    if (warp < NP || warp == NP + 1) pair_await();
     __syncthreads();
     if (failed) {  // copies and MMAs that were requested end within this time
         if (tid == 0 && p.timeout) atomicExch(p.timeout, 1);
         for (const long long t0 = clock64(); clock64() - t0 < 4000000LL;) {}
     }
     tc_fence_before();
-    pair_sync();
+    pair_arrive();
+    pair_await();
     if (warp == NP) {
         tc_fence_after();
         tmem_dealloc2(tmem_base, 512);
@@ -615,22 +628,23 @@ __global__ void __launch_bounds__(pair_threads<TYPE>(), 1) mmq_pair_kernel(const
 }
 
 // ---------------------------------------------------------------- host side
-// Tile width and K split by the length of the longest pair's work, in tensor cycles: a K step of 64 takes 2 * BN of them (8192 MACs a cycle
-// and pair), or as long as the producers need to unpack it (measured, per format), a tile about 1500 more; two halves of K add into a
-// zeroed dst, which costs about as much as 4000.  Widths are N / 1, N / 2, ... rounded up to 16.
+// Tile width and K split by the time of the longest pair's work, in microseconds.  A K step of 64 costs `unpack` plus 0.6 ns a column while the
+// producers are the slower ones (measured, 18944 rows: q4_K 0.29 at 64 columns, 0.43 at 256; q6_K 0.47 and 0.54), dense weights take 1.25 ns a
+// column but 0.2 at least; a tile more costs about 1.  Two halves of K add into a zeroed dst: that much more traffic, at 1.5 TB/s, and a
+// launch more.  Widths are N / 1, N / 2, ... rounded up to 16.
 struct PairPlan { int bn, ksplit, n_tiles_n; };
-static inline PairPlan mmq_pair_plan(int64_t M, int64_t N, int64_t K, int n_batch, int pairs, int unpack) {
+static inline PairPlan mmq_pair_plan(int64_t M, int64_t N, int64_t K, int n_batch, int pairs, double unpack) {
     PairPlan best = {256, 1, 1};
     double best_cost = -1;
     const int64_t mt = (M + 255) / 256;
     for (int64_t parts = (N + 255) / 256; parts <= (N + 31) / 32; parts++) {
         const int64_t even = ((N + parts - 1) / parts + 15) / 16 * 16, bn = even < 32 ? 32 : even;
         const int64_t nt = (N + bn - 1) / bn;
+        const double dense = 1.25e-3 * bn < 0.2 ? 0.2 : 1.25e-3 * bn, step = unpack > 0 ? unpack + 0.6e-3 * bn : dense;
         for (int ks = 1; ks <= 2; ks++) {
             if (ks == 2 && (n_batch > 1 || K < 2048)) break;
             const int64_t tiles = mt * nt * n_batch * ks, waves = (tiles + pairs - 1) / pairs;
-            const double step = 2.0 * bn > unpack ? 2.0 * bn : unpack;
-            const double cost = waves * ((double)(K / MQ_BK) / ks * step + 1500.0) + (ks == 2 ? 4000.0 : 0.0);
+            const double cost = waves * ((double)(K / MQ_BK) / ks * step + 1.0) + (ks == 2 ? 2.0 + (double)M * N * 4 / 1.5e6 : 0.0);
             if (best_cost < 0 || cost < 0.98 * best_cost) { best_cost = cost; best = {(int)bn, ks, (int)nt}; }
         }
     }
@@ -648,7 +662,7 @@ static int mmq_pairs() {
     return pairs;
 }
 
-template <int TYPE> constexpr int pair_unpack_cycles() { return TYPE == B200_TYPE_BF16 ? 0 : TYPE == B200_TYPE_Q4_K || TYPE == B200_TYPE_Q4_0 || TYPE == B200_TYPE_Q5_K ? 300 : 420; }
+template <int TYPE> constexpr double pair_unpack_us() { return TYPE == B200_TYPE_BF16 ? 0 : TYPE == B200_TYPE_Q4_K || TYPE == B200_TYPE_Q4_0 ? 0.27 : TYPE == B200_TYPE_Q5_K || TYPE == B200_TYPE_Q8_0 ? 0.33 : 0.43; }
 
 template <int TYPE, bool GROUPED>
 static int mmq_pair_launch(const MmqParams &q, int64_t n_pad, int64_t w_rows_per_product, int64_t max_tiles_n, int64_t grouped_bn, cudaStream_t st) {
@@ -672,7 +686,7 @@ static int mmq_pair_launch(const MmqParams &q, int64_t n_pad, int64_t w_rows_per
         p.n_tiles_n = 0;
         p.q.ksplit = 1;
     } else {
-        const PairPlan pl = mmq_pair_plan(q.M, q.N, q.K, q.n_batch, mmq_pairs(), pair_unpack_cycles<TYPE>());
+        const PairPlan pl = mmq_pair_plan(q.M, q.N, q.K, q.n_batch, mmq_pairs(), pair_unpack_us<TYPE>());
         p.bn = pl.bn;
         p.box = pl.bn / 2;
         p.n_tiles_n = pl.n_tiles_n;

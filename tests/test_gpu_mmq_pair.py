@@ -1,0 +1,86 @@
+"""The paired-SM prompt GEMM where it can go wrong: weight rows and columns around the tile edges, rows that start at any even byte, two halves
+of K, results inside wider rows, batches of products and experts of uneven size.  Against float64 over the dequantised weights; the bound is
+that of tests/test_gpu_mmq.py (both operands rounded to bf16: 2^-9 / sqrt(3) each, relative to the product)."""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+import koboldcpp_b200.host as H
+import orc as O
+from koboldcpp_b200.lib import BF16, Q2_K, Q3_K, Q4_0, Q4_K, Q5_0, Q5_1, Q5_K, Q6_K, Q8_0, IQ4_XS, check, lib, row_size
+from koboldcpp_b200.llama import random_blocks
+
+pytestmark = pytest.mark.gpu
+
+
+def rel(a, b):
+    return float(np.linalg.norm(a - b) / np.linalg.norm(b))
+
+
+def product(t, w, x, K, M, offset=0, row_bytes=None, dst_stride=None):
+    """b200_mul_mat_q with the weight rows `row_bytes` apart, the first one `offset` bytes into its allocation."""
+    N, rs = x.shape[0], row_size(t, K)
+    row_bytes, dst_stride = row_bytes or rs, dst_stride or M
+    raw = np.zeros(offset + M * row_bytes + 64, np.uint8)
+    for m in range(M):
+        raw[offset + m * row_bytes:offset + m * row_bytes + rs] = w[m]
+    dw, dx, dd = H.DeviceBuffer.from_numpy(raw), H.DeviceBuffer.from_numpy(x), H.DeviceBuffer.from_numpy(np.full((N, dst_stride), np.nan, np.float32))
+    need = lib().b200_mul_mat_q_workspace_bytes(t, K, M, N)
+    ws = H.DeviceBuffer(need + 16)
+    check(lib().b200_mul_mat_q(t, dw.ptr + offset, row_bytes, dx.ptr, K, dd.ptr, dst_stride, K, M, N, ws.ptr, need, None))
+    return dd.to_numpy(np.float32, (N, dst_stride))
+
+
+def expected(t, w, x, K):
+    return x.astype(np.float64) @ np.stack([O.dequantize(t, r, K) for r in w]).astype(np.float64).T
+
+
+@pytest.mark.parametrize("t", [Q4_K, Q5_K, Q6_K, Q4_0, Q8_0])
+@pytest.mark.parametrize("K,M,N", [(256, 1, 9), (256, 255, 31), (512, 257, 33), (2304, 129, 177), (2048, 513, 16), (768, 700, 257)])
+def test_edges_of_tiles(t, K, M, N):
+    rng = np.random.default_rng(K + M + N + t)
+    w, x = random_blocks(rng, t, M, K), rng.standard_normal((N, K)).astype(np.float32)
+    got = product(t, w, x, K, M, dst_stride=M + 5)
+    assert np.isnan(got[:, M:]).all()
+    assert rel(got[:, :M], expected(t, w, x, K)) < 4e-3
+
+
+@pytest.mark.parametrize("t", [Q6_K, Q8_0, Q4_0, Q2_K, Q3_K, Q5_0, Q5_1, IQ4_XS])
+@pytest.mark.parametrize("offset,pad", [(0, 0), (2, 0), (6, 2), (14, 10), (4, 6), (8, 12)])
+def test_rows_at_any_even_byte(t, offset, pad):
+    K, M, N = 1024, 40, 20
+    rng = np.random.default_rng(t + offset)
+    w, x = random_blocks(rng, t, M, K), rng.standard_normal((N, K)).astype(np.float32)
+    assert rel(product(t, w, x, K, M, offset, row_size(t, K) + pad), expected(t, w, x, K)) < 4e-3
+
+
+@pytest.mark.parametrize("K,M,N,batch", [(64, 130, 20, 3), (320, 256, 100, 5), (128, 300, 300, 2)])
+def test_batches_of_dense_products(K, M, N, batch):
+    rng = np.random.default_rng(K + M)
+    w = rng.standard_normal((batch, M, K)).astype(np.float32)
+    bits = (w.view(np.uint32) >> 16).astype(np.uint16)
+    w = (bits.astype(np.uint32) << 16).view(np.float32)
+    x = rng.standard_normal((batch, N, K)).astype(np.float32)
+    for gap in (0, 8):  # values between two products: with 8 the stride is no multiple of a row
+        stack = np.zeros((batch, M * K + gap), np.uint16)
+        stack[:, :M * K] = bits.reshape(batch, -1)
+        dw, dx, dd = H.DeviceBuffer.from_numpy(stack), H.DeviceBuffer.from_numpy(x), H.DeviceBuffer(4 * batch * N * M)
+        need = batch * lib().b200_mul_mat_q_workspace_bytes(BF16, K, M, N)
+        ws = H.DeviceBuffer(need + 16)
+        check(lib().b200_mul_mat_bf16_batched(dw.ptr, 2 * K, 2 * (M * K + gap), dx.ptr, K, N * K, dd.ptr, M, N * M, K, M, N, batch, ws.ptr, need, None))
+        assert rel(dd.to_numpy(np.float32, (batch, N, M)), np.einsum("bnk,bmk->bnm", x.astype(np.float64), w.astype(np.float64))) < 4e-3
+
+
+@pytest.mark.parametrize("t", [Q4_K, Q6_K])
+@pytest.mark.parametrize("T,n_expert,hot", [(9, 4, 0.5), (300, 4, 0.9), (520, 8, 0.6)])
+def test_experts_of_uneven_size(t, T, n_expert, hot):
+    """One expert takes most pairs (several full tiles and a remainder), another none."""
+    K, M, used = 512, 300, 2
+    rng = np.random.default_rng(T + t)
+    w, b = random_blocks(rng, t, n_expert * M, K), rng.standard_normal((T, 1, K)).astype(np.float32)
+    ids = np.where(rng.random((T, used)) < hot, 1, rng.integers(0, n_expert - 1, (T, used))).astype(np.int32)
+    got = H.mul_mat_id_q(t, w, ids, b, K, M, n_expert)
+    W = [np.stack([O.dequantize(t, r, K) for r in w[e * M:(e + 1) * M]]).astype(np.float64) for e in range(n_expert)]
+    exp = np.stack([[W[ids[i, s]] @ b[i, 0].astype(np.float64) for s in range(used)] for i in range(T)])
+    assert rel(got, exp) < 4e-3
