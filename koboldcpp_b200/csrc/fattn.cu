@@ -641,8 +641,7 @@ static int fa_launch_mma(const FaParams &p, const FaPlan &pl, cudaStream_t st, b
 
 template <int D>
 static int fa_launch_prefill(const FaParams &p, const FaPlan &pl, cudaStream_t st, bool pdl) {
-    using G = MmaGeo<B200_TYPE_F16, D>;
-    const size_t smem = (size_t)FP_NBUF * 2 * G::TILE_BYTES;
+    const size_t smem = (size_t)FP_NBUF * fp_stage_bytes<D>();
     static bool attr_set_dev[16] = {};  // cudaFuncSetAttribute is per device
     int cur_dev = 0;
     B200_CUDA_TRY(cudaGetDevice(&cur_dev));

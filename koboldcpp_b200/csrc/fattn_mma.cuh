@@ -626,33 +626,100 @@ __global__ void __launch_bounds__(FM_NW * 32, 2) fattn_mma_kernel(const __grid_c
 
 // ------------------------------------------------------------------------------------------------ prompt batches (a12)
 // Flash-prefill form of the same arithmetic: a CTA serves 64 query columns of one kv-head (each of its 4 warps owns 16 of them for
-// the whole KV range -- no cross-warp merge, no splits) and the 4 warps SHARE every (K, V) tile: one CTA-wide cp.async ring, one
-// __syncthreads per tile.  The decode kernel above gives every warp its own tiles instead (right for 1..16 columns); run on a
-// 512-token batch it launched 1024 CTAs whose 4 warps saw ~4 tiles each and spent their time in prologue and merge (7B pp512:
-// 165 us per layer, 27 % of the step: profiles/r02_launches_pp512_7b.txt).  Causal structure: tile i is skipped by a warp when the
-// mask is -inf for all its 16 columns, and not even loaded when that holds for all 64 (the skip words cover the LAST 64 tiles of
-// the range: that is where the upper triangle lives).
-constexpr int FP_NBUF = 4;   // stages of the CTA ring
+// the whole KV range -- no cross-warp merge, no splits) and the 4 warps SHARE every (K, V) tile through a CTA-wide cp.async ring.
+// What bounds it: instruction issue.  A tile is 64 keys (32 for wider heads), so that barrier, maximum, rescaling and the bookkeeping of a tile
+// are paid once per 64 keys, and two CTAs an SM hide one another's softmax: 7B, 512 tokens behind 1536: 222 us with 16-key tiles that
+// loaded the mask for every score; 121 here.  The mask is looked at 16 bytes a lane, one tile ahead: a tile whose mask is 0 throughout
+// needs no additions, one that is -inf throughout is skipped by the warp; only the diagonal goes value by value.  Tiles behind the last one
+// that any column of the CTA sees are not loaded at all.
+constexpr int FP_NBUF = 3;   // stages of the CTA ring
 constexpr int FP_COLS = 64;  // query columns per CTA
+template <int D> constexpr int fp_keys() { return D > 128 ? 32 : 64; }  // keys of a tile: the scores' registers beside 2 D accumulators
+template <int D> constexpr int fp_stage_bytes() { return 2 * fp_keys<D>() * MmaGeo<B200_TYPE_F16, D>::ROW_STRIDE; }
 
 template <int D>
 __global__ void __launch_bounds__(FM_NW * 32, 2) fattn_mma_prefill_kernel(const __grid_constant__ FaParams p) {
     using G = MmaGeo<B200_TYPE_F16, D>;
-    constexpr int KS = D / 16;
+    constexpr int KS = D / 16, KT = fp_keys<D>(), NB = KT / 8, TILE = KT * G::ROW_STRIDE;
+    constexpr float LOG2E = 1.4426950408889634f;
     extern __shared__ __align__(128) unsigned char smem[];
-    __shared__ unsigned long long skip_w[FM_NW];
+    __shared__ int last_tile[FM_NW];
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int g = lane >> 2, t4 = lane & 3;
     const int hk = blockIdx.y, ct = blockIdx.x;
     const int col0 = ct * FP_COLS + warp * FM_MAXC;        // this warp's 16 columns
     const int ncol = max(0, min(FM_MAXC, p.n_cols - col0));
-    const int n_tiles = (p.n_kv + FM_TP - 1) / FM_TP;
+    const int n_tiles_all = (p.n_kv + KT - 1) / KT;
     const unsigned char *kbase = p.k + (size_t)hk * p.k_nb2;
     const unsigned char *vbase = p.v + (size_t)hk * p.v_nb2;
 
     pdl_wait();
     pdl_trigger();
+
+    // ---- the mask of this warp's columns in a tile, 16 bytes a lane: all 0 / all -inf / mixed.  Lane l looks at columns l / CH, l / CH + 32 / CH, ...
+    constexpr int CH = KT / 8, RP = 32 / CH;               // 16-byte pieces of a mask row in a tile; rows per pass
+    const bool m16 = (((uintptr_t)p.mask | p.mask_nb1) & 15) == 0;
+    enum { ZERO = 0, MIXED = 1, HIDDEN = 2 };
+    auto mask_load = [&](int t, uint4 (&u)[16 / RP]) {
+        const int key = t * KT + (lane % CH) * 8;
+#pragma unroll
+        for (int i = 0; i < 16 / RP; i++) {
+            const int c = min(lane / CH + i * RP, ncol - 1);
+            u[i] = make_uint4(0u, 0u, 0u, 0u);
+            if (key + 8 <= p.n_kv) u[i] = __ldg(reinterpret_cast<const uint4 *>(p.mask + (size_t)((col0 + c) / p.gqa) * p.mask_nb1 + 2 * (size_t)key));
+        }
+    };
+    auto mask_kind = [&](int t, const uint4 (&u)[16 / RP]) {
+        unsigned any = 0, all = 0xffffffffu, inf = 0;
+#pragma unroll
+        for (int i = 0; i < 16 / RP; i++) {
+            const unsigned o = u[i].x | u[i].y | u[i].z | u[i].w, n = u[i].x & u[i].y & u[i].z & u[i].w;
+            any |= o;
+            inf |= o ^ 0xfc00fc00u;
+            all &= n;
+        }
+        const bool whole = (t + 1) * KT <= p.n_kv;         // a ragged last tile goes value by value
+        if (!__any_sync(0xffffffffu, any != 0u || !whole)) return (int)ZERO;
+        return __any_sync(0xffffffffu, inf != 0u || all != 0xfc00fc00u || !whole) ? (int)MIXED : (int)HIDDEN;
+    };
+    // ---- the last tile that a column of this warp sees, from the back (the causal triangle); then of the CTA
+    int n_tiles = n_tiles_all;
+    if (ncol == 0) n_tiles = 0;
+    else if (p.mask != nullptr && m16) {
+        while (n_tiles > 0) {
+            uint4 u[16 / RP];
+            mask_load(n_tiles - 1, u);
+            if (mask_kind(n_tiles - 1, u) != HIDDEN) break;
+            n_tiles--;
+        }
+    }
+    if (lane == 0) last_tile[warp] = n_tiles;
+    __syncthreads();
+    const int cta_tiles = max(max(last_tile[0], last_tile[1]), max(last_tile[2], last_tile[3]));
+
+    // ---- CTA ring: stage = (K tile, V tile)
+    constexpr int CPR = G::ROW_BYTES / 16;
+    auto load_stage = [&](int tt, int st) {
+        if (tt < cta_tiles) {
+            unsigned char *base = smem + (size_t)st * 2 * TILE;
+#pragma unroll 4
+            for (int i = threadIdx.x; i < KT * CPR; i += FM_NW * 32) {
+                const int r = i / CPR, c = i - r * CPR, row = tt * KT + r;
+                unsigned char *d = base + r * G::ROW_STRIDE + c * 16;
+                if (row < p.n_kv) {
+                    cp_async16(d, kbase + (size_t)row * p.k_nb1 + c * 16);
+                    cp_async16(d + TILE, vbase + (size_t)row * p.v_nb1 + c * 16);
+                } else {
+                    *reinterpret_cast<uint4 *>(d) = make_uint4(0, 0, 0, 0);
+                    *reinterpret_cast<uint4 *>(d + TILE) = make_uint4(0, 0, 0, 0);
+                }
+            }
+        }
+        cp_async_commit();
+    };
+#pragma unroll
+    for (int st = 0; st < FP_NBUF - 1; st++) load_stage(st, st);
 
     // ---- Q fragments, mask rows, slopes of this warp's columns
     unsigned qa[KS][4];
@@ -679,79 +746,112 @@ __global__ void __launch_bounds__(FM_NW * 32, 2) fattn_mma_prefill_kernel(const 
             qa[s][2 + hh] = pack_h2(hi.x, hi.y);
         }
     }
-    // ---- skip words: bit i <-> tile t_skip0 + i is masked for all columns of this warp (lane i checks tile i)
-    const int t_skip0 = n_tiles > 64 ? n_tiles - 64 : 0;
-    unsigned long long skip = 0;
-    if (p.mask != nullptr) {
-        const bool al16 = (((uintptr_t)p.mask | p.mask_nb1) & 15) == 0;
-#pragma unroll 1
-        for (int pass = 0; pass < 2; pass++) {
-            const int tt = t_skip0 + pass * 32 + lane;
-            bool masked = false;
-            if (tt < n_tiles) {
-                masked = true;
-                const int key = tt * FM_TP;
-                for (int c = 0; c < ncol; c++) {
-                    const unsigned char *mr = p.mask + (size_t)((col0 + c) / p.gqa) * p.mask_nb1 + 2 * (size_t)key;
-                    if (al16 && key + FM_TP <= p.n_kv) {
-                        const uint4 u0 = __ldg(reinterpret_cast<const uint4 *>(mr)), u1 = __ldg(reinterpret_cast<const uint4 *>(mr) + 1);
-                        masked = masked && (u0.x & u0.y & u0.z & u0.w & u1.x & u1.y & u1.z & u1.w) == 0xfc00fc00u &&
-                                 (u0.x | u0.y | u0.z | u0.w | u1.x | u1.y | u1.z | u1.w) == 0xfc00fc00u;
-                    } else {
-                        for (int e = 0; e < FM_TP; e++)
-                            if (key + e < p.n_kv) masked = masked && *reinterpret_cast<const unsigned short *>(mr + 2 * e) == 0xfc00;
-                    }
-                }
-            }
-            skip |= (unsigned long long)__ballot_sync(0xffffffffu, masked) << (32 * pass);
-        }
-    }
-    if (ncol == 0) skip = ~0ull;  // a warp without columns never needs a tile
-    if (lane == 0) skip_w[warp] = skip;
-    __syncthreads();
-    const unsigned long long skip_cta = skip_w[0] & skip_w[1] & skip_w[2] & skip_w[3];
-    auto is_skipped = [&](unsigned long long w, int tt) { return tt >= t_skip0 && ((w >> (tt - t_skip0)) & 1ull) != 0; };
-    // a warp without columns must still not read tiles before t_skip0: give it nothing to do
-    const bool idle = ncol == 0;
-
-    // ---- CTA ring: stage = (K tile, V tile); 128 threads copy a tile pair (2 x 16 rows x D/8 chunks of 16 bytes)
-    constexpr int CPR = G::ROW_BYTES / 16;
-    constexpr int CHUNKS = 2 * FM_TP * CPR;
-    auto load_stage = [&](int tt, int st) {
-        if (tt < n_tiles && !is_skipped(skip_cta, tt)) {
-            unsigned char *base = smem + (size_t)st * 2 * G::TILE_BYTES;
-#pragma unroll
-            for (int i = threadIdx.x; i < CHUNKS; i += FM_NW * 32) {
-                const int kv = i / (FM_TP * CPR), j = i - kv * (FM_TP * CPR), r = j / CPR, c = j - r * CPR;
-                const int row = tt * FM_TP + r;
-                unsigned char *d = base + kv * G::TILE_BYTES + r * G::ROW_STRIDE + c * 16;
-                if (row < p.n_kv) cp_async16(d, (kv ? vbase + (size_t)row * p.v_nb1 : kbase + (size_t)row * p.k_nb1) + c * 16);
-                else *reinterpret_cast<uint4 *>(d) = make_uint4(0, 0, 0, 0);
-            }
-        }
-        cp_async_commit();
-    };
-#pragma unroll
-    for (int st = 0; st < FP_NBUF - 1; st++) load_stage(st, st);
-
     const bool mask_al4 = (((uintptr_t)p.mask | p.mask_nb1) & 3) == 0;
-    float scale = p.scale;
-    if (p.softcap != 0.0f) scale /= p.softcap;
-    float m[2] = {-INFINITY, -INFINITY}, l[2] = {0.f, 0.f};
+    const float scale = p.softcap != 0.0f ? p.scale / p.softcap : p.scale;
+    float m[2] = {-INFINITY, -INFINITY}, l[2] = {0.f, 0.f};  // maximum (times log2 e) and this lane's share of the sum
     float o[2 * KS][4];
 #pragma unroll
     for (int i = 0; i < 2 * KS; i++) o[i][0] = o[i][1] = o[i][2] = o[i][3] = 0.f;
     const int mi = lane >> 3, mr = lane & 7;
     const unsigned k_off = (unsigned)(((mi >> 1) * 8 + mr) * G::ROW_STRIDE + (mi & 1) * 16);
     const unsigned v_off = (unsigned)(((mi & 1) * 8 + mr) * G::ROW_STRIDE + (mi >> 1) * 16);
+    uint4 mu[16 / RP];
+    const bool looked = p.mask != nullptr && m16;
+    if (looked && n_tiles > 0) mask_load(0, mu);
 
-    for (int t = 0; t < n_tiles; t++) {
+    int stage = 0;
+    for (int t = 0; t < cta_tiles; t++) {
         cp_async_wait<FP_NBUF - 2>();   // tile t has landed (this thread's copies) ...
         __syncthreads();                // ... everybody's; and everybody is done with tile t - 1, whose stage is refilled now
-        load_stage(t + FP_NBUF - 1, (t + FP_NBUF - 1) % FP_NBUF);
-        if (idle || is_skipped(skip, t)) continue;
-        const unsigned kt = smem_u32(smem + (size_t)(t % FP_NBUF) * 2 * G::TILE_BYTES), vt = kt + G::TILE_BYTES;
-        mma_tile_step<D>(kt, vt, t, qa, m, l, o, mrow, slope, scale, p.softcap, p.n_kv, mask_al4, k_off, v_off, t4);
+        load_stage(t + FP_NBUF - 1, stage + FP_NBUF - 1 >= FP_NBUF ? stage - 1 : stage + FP_NBUF - 1);
+        const unsigned kt = smem_u32(smem + (size_t)stage * 2 * TILE), vt = kt + TILE;
+        stage = stage + 1 == FP_NBUF ? 0 : stage + 1;
+        if (t >= n_tiles) continue;
+        int kind = p.mask != nullptr || (t + 1) * KT > p.n_kv ? (int)MIXED : (int)ZERO;
+        if (looked) {
+            kind = mask_kind(t, mu);
+            if (t + 1 < n_tiles) mask_load(t + 1, mu);
+            if (kind == HIDDEN) continue;
+        }
+        float s[NB][4];
+#pragma unroll
+        for (int j = 0; j < NB; j++) s[j][0] = s[j][1] = s[j][2] = s[j][3] = 0.f;
+#pragma unroll
+        for (int ks = 0; ks < KS; ks++) {
+#pragma unroll
+            for (int j = 0; j < NB / 2; j++) {
+                unsigned b0, b1, b2, b3;
+                ldsm_x4(kt + k_off + (unsigned)(j * 16 * G::ROW_STRIDE) + ks * 32, b0, b1, b2, b3);
+                mma_f16(s[2 * j], qa[ks], b0, b1);
+                mma_f16(s[2 * j + 1], qa[ks], b2, b3);
+            }
+        }
+        // scores times log2 e.  s[j][2 hh + e]: column g + 8 hh, key KT t + 8 j + 2 t4 + e
+        float alpha[2];
+#pragma unroll
+        for (int hh = 0; hh < 2; hh++) {
+            float mx = -INFINITY;
+#pragma unroll
+            for (int j = 0; j < NB; j++) {
+                float s0 = s[j][2 * hh], s1 = s[j][2 * hh + 1];
+                if (p.softcap != 0.0f) {
+                    s0 = p.softcap * LOG2E * tanhf(s0 * scale); s1 = p.softcap * LOG2E * tanhf(s1 * scale);
+                } else {
+                    s0 *= scale * LOG2E; s1 *= scale * LOG2E;
+                }
+                if (kind == MIXED) {
+                    const int key = t * KT + 8 * j + 2 * t4;
+                    if (mrow[hh] != nullptr && key < p.n_kv) {
+                        float2 mf;
+                        if (mask_al4 && key + 1 < p.n_kv) {
+                            mf = __half22float2(*reinterpret_cast<const __half2 *>(mrow[hh] + 2 * (size_t)key));
+                        } else {
+                            mf.x = __half2float(*reinterpret_cast<const __half *>(mrow[hh] + 2 * (size_t)key));
+                            mf.y = key + 1 < p.n_kv ? __half2float(*reinterpret_cast<const __half *>(mrow[hh] + 2 * (size_t)key + 2)) : 0.f;
+                        }
+                        s0 += slope[hh] * LOG2E * mf.x;
+                        s1 += slope[hh] * LOG2E * mf.y;
+                    }
+                    s0 = key < p.n_kv ? s0 : -INFINITY;
+                    s1 = key + 1 < p.n_kv ? s1 : -INFINITY;
+                }
+                s[j][2 * hh] = s0;
+                s[j][2 * hh + 1] = s1;
+                mx = fmaxf(mx, fmaxf(s0, s1));
+            }
+            mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
+            mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
+            const float mn = fmaxf(m[hh], mx), mb = mn == -INFINITY ? 0.f : mn;  // (nothing seen yet: exp2(-inf) = 0 throughout)
+            alpha[hh] = mn == -INFINITY ? 1.0f : exp2f(m[hh] - mb);
+            m[hh] = mn;
+            float sum = 0.f;
+#pragma unroll
+            for (int j = 0; j < NB; j++) {
+                s[j][2 * hh] = exp2f(s[j][2 * hh] - mb);
+                s[j][2 * hh + 1] = exp2f(s[j][2 * hh + 1] - mb);
+                sum += s[j][2 * hh] + s[j][2 * hh + 1];
+            }
+            l[hh] = l[hh] * alpha[hh] + sum;
+        }
+        if (__any_sync(0xffffffffu, alpha[0] != 1.0f || alpha[1] != 1.0f)) {
+#pragma unroll
+            for (int i = 0; i < 2 * KS; i++) {
+                o[i][0] *= alpha[0]; o[i][1] *= alpha[0];
+                o[i][2] *= alpha[1]; o[i][3] *= alpha[1];
+            }
+        }
+#pragma unroll
+        for (int kk = 0; kk < KT / 16; kk++) {
+            const unsigned pa[4] = {pack_h2(s[2 * kk][0], s[2 * kk][1]), pack_h2(s[2 * kk][2], s[2 * kk][3]), pack_h2(s[2 * kk + 1][0], s[2 * kk + 1][1]),
+                                    pack_h2(s[2 * kk + 1][2], s[2 * kk + 1][3])};
+#pragma unroll
+            for (int j = 0; j < KS; j++) {
+                unsigned b0, b1, b2, b3;
+                ldsm_x4_t(vt + v_off + (unsigned)(kk * 16 * G::ROW_STRIDE) + j * 32, b0, b1, b2, b3);
+                mma_f16(o[2 * j], pa, b0, b1);
+                mma_f16(o[2 * j + 1], pa, b2, b3);
+            }
+        }
     }
     cp_async_wait<0>();
 #pragma unroll
