@@ -629,11 +629,13 @@ __global__ void __launch_bounds__(FM_NW * 32, 2) fattn_mma_kernel(const __grid_c
 // the whole KV range -- no cross-warp merge, no splits) and the 4 warps SHARE every (K, V) tile through a CTA-wide cp.async ring.
 // What bounds it: instruction issue.  A tile is 64 keys (32 for wider heads), so that barrier, maximum, rescaling and the bookkeeping of a tile
 // are paid once per 64 keys, and two CTAs an SM hide one another's softmax: 7B, 512 tokens behind 1536: 222 us with 16-key tiles that
-// loaded the mask for every score; 121 here.  The mask is looked at 16 bytes a lane, one tile ahead: a tile whose mask is 0 throughout
+// loaded the mask for every score; 84 here (121 before the common tile lost its branches and a scaling per score).  The mask is looked at 16 bytes a lane, one tile ahead: a tile whose mask is 0 throughout
 // needs no additions, one that is -inf throughout is skipped by the warp; only the diagonal goes value by value.  Tiles behind the last one
 // that any column of the CTA sees are not loaded at all.
 constexpr int FP_NBUF = 3;   // stages of the CTA ring
 constexpr int FP_COLS = 64;  // query columns per CTA
+// 2^x to two ulp; results below 2^-126 become 0 (beside a sum of at least 1 they vanish)
+__device__ __forceinline__ float ex2(float x) { float y; asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x)); return y; }
 template <int D> constexpr int fp_keys() { return D > 128 ? 32 : 64; }  // keys of a tile: the scores' registers beside 2 D accumulators
 template <int D> constexpr int fp_stage_bytes() { return 2 * fp_keys<D>() * MmaGeo<B200_TYPE_F16, D>::ROW_STRIDE; }
 
@@ -786,22 +788,18 @@ __global__ void __launch_bounds__(FM_NW * 32, 2) fattn_mma_prefill_kernel(const 
                 mma_f16(s[2 * j + 1], qa[ks], b2, b3);
             }
         }
-        // scores times log2 e.  s[j][2 hh + e]: column g + 8 hh, key KT t + 8 j + 2 t4 + e
-        float alpha[2];
+        // s[j][2 hh + e]: column g + 8 hh, key KT t + 8 j + 2 t4 + e.  The common tile (no soft cap, mask 0) keeps the raw products, `c` takes them to
+        // scaled scores times log2 e inside the exponent's FMA; the others are brought there value by value, c = 1.
+        float c = scale * LOG2E;
+        if (kind == MIXED || p.softcap != 0.0f || !(scale > 0.f)) {
 #pragma unroll
-        for (int hh = 0; hh < 2; hh++) {
-            float mx = -INFINITY;
+            for (int hh = 0; hh < 2; hh++) {
 #pragma unroll
-            for (int j = 0; j < NB; j++) {
-                float s0 = s[j][2 * hh], s1 = s[j][2 * hh + 1];
-                if (p.softcap != 0.0f) {
-                    s0 = p.softcap * LOG2E * tanhf(s0 * scale); s1 = p.softcap * LOG2E * tanhf(s1 * scale);
-                } else {
-                    s0 *= scale * LOG2E; s1 *= scale * LOG2E;
-                }
-                if (kind == MIXED) {
+                for (int j = 0; j < NB; j++) {
+                    float s0 = s[j][2 * hh] * scale, s1 = s[j][2 * hh + 1] * scale;
+                    if (p.softcap != 0.0f) { s0 = p.softcap * tanhf(s0); s1 = p.softcap * tanhf(s1); }
                     const int key = t * KT + 8 * j + 2 * t4;
-                    if (mrow[hh] != nullptr && key < p.n_kv) {
+                    if (kind == MIXED && mrow[hh] != nullptr && key < p.n_kv) {
                         float2 mf;
                         if (mask_al4 && key + 1 < p.n_kv) {
                             mf = __half22float2(*reinterpret_cast<const __half2 *>(mrow[hh] + 2 * (size_t)key));
@@ -809,29 +807,35 @@ __global__ void __launch_bounds__(FM_NW * 32, 2) fattn_mma_prefill_kernel(const 
                             mf.x = __half2float(*reinterpret_cast<const __half *>(mrow[hh] + 2 * (size_t)key));
                             mf.y = key + 1 < p.n_kv ? __half2float(*reinterpret_cast<const __half *>(mrow[hh] + 2 * (size_t)key + 2)) : 0.f;
                         }
-                        s0 += slope[hh] * LOG2E * mf.x;
-                        s1 += slope[hh] * LOG2E * mf.y;
+                        s0 += slope[hh] * mf.x;
+                        s1 += slope[hh] * mf.y;
                     }
-                    s0 = key < p.n_kv ? s0 : -INFINITY;
-                    s1 = key + 1 < p.n_kv ? s1 : -INFINITY;
+                    s[j][2 * hh] = key < p.n_kv ? s0 * LOG2E : -INFINITY;
+                    s[j][2 * hh + 1] = key + 1 < p.n_kv ? s1 * LOG2E : -INFINITY;
                 }
-                s[j][2 * hh] = s0;
-                s[j][2 * hh + 1] = s1;
-                mx = fmaxf(mx, fmaxf(s0, s1));
             }
+            c = 1.0f;
+        }
+        float alpha[2];
+#pragma unroll
+        for (int hh = 0; hh < 2; hh++) {
+            float mx = fmaxf(s[0][2 * hh], s[0][2 * hh + 1]);
+#pragma unroll
+            for (int j = 1; j < NB; j++) mx = fmaxf(mx, fmaxf(s[j][2 * hh], s[j][2 * hh + 1]));
             mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
             mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
-            const float mn = fmaxf(m[hh], mx), mb = mn == -INFINITY ? 0.f : mn;  // (nothing seen yet: exp2(-inf) = 0 throughout)
-            alpha[hh] = mn == -INFINITY ? 1.0f : exp2f(m[hh] - mb);
+            const float mn = fmaxf(m[hh], mx * c), mb = mn == -INFINITY ? 0.f : mn;  // (nothing seen yet: 2^-inf = 0 throughout)
+            alpha[hh] = mn == -INFINITY ? 1.0f : ex2(m[hh] - mb);
             m[hh] = mn;
-            float sum = 0.f;
+            float sum0 = 0.f, sum1 = 0.f;
 #pragma unroll
             for (int j = 0; j < NB; j++) {
-                s[j][2 * hh] = exp2f(s[j][2 * hh] - mb);
-                s[j][2 * hh + 1] = exp2f(s[j][2 * hh + 1] - mb);
-                sum += s[j][2 * hh] + s[j][2 * hh + 1];
+                s[j][2 * hh] = ex2(fmaf(s[j][2 * hh], c, -mb));
+                s[j][2 * hh + 1] = ex2(fmaf(s[j][2 * hh + 1], c, -mb));
+                sum0 += s[j][2 * hh];
+                sum1 += s[j][2 * hh + 1];
             }
-            l[hh] = l[hh] * alpha[hh] + sum;
+            l[hh] = l[hh] * alpha[hh] + (sum0 + sum1);
         }
         if (__any_sync(0xffffffffu, alpha[0] != 1.0f || alpha[1] != 1.0f)) {
 #pragma unroll
