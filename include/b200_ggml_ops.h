@@ -336,7 +336,8 @@ typedef struct {
 } b200_sink_attn_args;
 B200_API int b200_op_sink_attn(const b200_sink_attn_args *a, b200_stream_t stream);
 /* The same with a workspace of b200_sink_attn_workspace_bytes(a) bytes (16-byte aligned; 0: none needed): with few tokens and
- * many cells (decode) the cells of a (token, head) pair are split over several CTAs whose partial results meet there. */
+ * many cells (decode) the cells of a (token, head) pair are split over several CTAs whose partial results meet there; prompt batches
+ * with bf16 products keep the rounded cache rows there. */
 B200_API size_t b200_sink_attn_workspace_bytes(const b200_sink_attn_args *a);
 B200_API int b200_op_sink_attn_ws(const b200_sink_attn_args *a, void *workspace, size_t workspace_bytes, b200_stream_t stream);
 

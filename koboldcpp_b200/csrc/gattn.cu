@@ -553,6 +553,10 @@ static int launch_sink_attn_mma(const b200_sink_attn_args *a, cudaStream_t st) {
     return launch_sink_attn_mma1<8>(a, st);
 }
 
+}  // namespace b200
+#include "sink_tile.cuh"
+namespace b200 {
+
 // ------------------------------------------------------------------------------------------------ linear attention with decay
 // The columns of the state never interact: a warp owns LA_CW columns of one (sequence, head) and keeps them in registers over
 // the whole token loop, a lane the rows d = lane, lane + 32, ...  The inputs of LA_CHUNK tokens are staged in shared memory
@@ -715,7 +719,7 @@ extern "C" int b200_op_qkv_store(const b200_qkv_store_args *args, b200_stream_t 
 
 extern "C" size_t b200_sink_attn_workspace_bytes(const b200_sink_attn_args *a) {
     if (!a || a->n_tokens <= 0 || a->n_head <= 0 || a->vdim <= 0) return 0;
-    if (a->bf16_products && a->n_tokens >= 16 && a->dim <= 128 && a->vdim <= 128) return 0;
+    if (sink_attn_mma_ok(a)) return a->n_head_kv > 0 && st_wanted(a) ? st_workspace(a) : 0;
     const int s = sink_attn_splits(a);
     return s > 1 ? (size_t)a->n_tokens * a->n_head * s * (a->vdim + 2) * sizeof(float) : 0;
 }
@@ -734,7 +738,10 @@ extern "C" int b200_op_sink_attn_ws(const b200_sink_attn_args *args, void *works
     OPX_REQUIRE(a->softcap >= 0.f, B200_ERR_INVALID, "b200_op_sink_attn: soft cap below zero");
     if (a->n_tokens == 0) return B200_OK;
     const cudaStream_t st = (cudaStream_t)stream;
-    if (sink_attn_mma_ok(a)) return launch_sink_attn_mma(a, st);
+    if (sink_attn_mma_ok(a)) {
+        const bool room = workspace && ((uintptr_t)workspace & 15) == 0 && st_wanted(a) && workspace_bytes >= st_workspace(a);
+        return room ? st_launch(a, workspace, st) : launch_sink_attn_mma(a, st);
+    }
     int n_split = sink_attn_splits(a);
     if (n_split > 1 && (!workspace || workspace_bytes < b200_sink_attn_workspace_bytes(a) || ((uintptr_t)workspace & 15))) n_split = 1;  // no room to merge through
     float *part = (float *)workspace;
