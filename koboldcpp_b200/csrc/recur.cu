@@ -73,159 +73,182 @@ __global__ void __launch_bounds__(128) short_conv_kernel(const b200_short_conv_a
 // ------------------------------------------------------------------------------------------------ gated delta rule
 // The columns of the state never interact: column j of S [dim, vdim] sees  S_j <- g S_j + k u_j  with  u_j = beta (v_j - g k.S_j),
 // and the read-out is  o_j = q.S_j(new) = g q.S_j(old) + (q.k) u_j,  so one pass over the old column gives both sums a token
-// needs.  A warp owns DR_CW * DR_CPL columns of one (sequence, head); 8 lanes share DR_CPL columns, lane r of them keeping the rows
-// 4 (r + 8 i) .. + 3 of each in registers over the whole token loop, so a sum over a column is three exchanges among 8 lanes and
-// the q and k values a lane reads from shared memory serve DR_CPL columns (the loads, not the arithmetic, are what two CTAs on one
-// SM compete for).
-// The inputs of DR_CHUNK tokens (16, or 8) are staged in shared memory: q and k as unit vectors (q scaled), q.k, the decay and beta once per
-// token; the next chunk's values travel to registers while the current chunk is worked on.
+// needs.  8 lanes share DR_CPL columns, lane r of them keeping the rows 4 (r + 8 i) .. + 3 of each in registers over the whole token loop, so a sum
+// over a column is three exchanges among 8 lanes, and two rows are worked on at a time (packed f32: one issue slot for both).
+// What bounds it: the chain S -> sums -> u -> S of a token, and the shared-memory pipe (a 16-byte load of a warp takes four of its cycles however
+// few addresses differ).  So every q and k piece that is loaded serves two columns, the four warps that carry the state do nothing else, and
+// four more warps prepare the next chunk of tokens meanwhile: q and k as unit vectors (q scaled), q.k, the decay and beta once per token.  512
+// tokens, 32 heads of 128 x 128: 183 us with one column a lane, eight warps that staged and scanned in turn, and unpacked arithmetic; 134 us here.
 // CHAN: the decay is one factor per key channel (row of S) instead of one per head.  The old column is multiplied by it first, then
 // ks, qs are sums over the decayed column and  o_j = qs + (q.k) u_j;  the factors of a chunk are staged like q and k.
-constexpr int DR_CW = 4, DR_CPL = 1, DR_WARPS = 8, DR_COLS = DR_CW * DR_CPL * DR_WARPS;
+constexpr int DR_CW = 4, DR_CPL = 2, DR_WARPS = 4, DR_COLS = DR_CW * DR_CPL * DR_WARPS;
+template <int DQ, bool CHAN> constexpr int dr_chunk() { return DQ * (CHAN ? 3 : 2) <= 8 ? 16 : DQ * (CHAN ? 3 : 2) <= 16 ? 8 : 4; }  // two chunks in 48 KB
+__device__ __forceinline__ unsigned long long dr_pack(float lo, float hi) { unsigned long long r; asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi)); return r; }
+__device__ __forceinline__ float2 dr_unpack(unsigned long long x) { float2 r; asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(x)); return r; }
+__device__ __forceinline__ unsigned long long dr_fma(unsigned long long x, unsigned long long y, unsigned long long z) {
+    unsigned long long r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(x), "l"(y), "l"(z));
+    return r;
+}
+__device__ __forceinline__ unsigned long long dr_mul(unsigned long long x, unsigned long long y) {
+    unsigned long long r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(x), "l"(y));
+    return r;
+}
 template <int DQ, bool CHAN>  // float4 groups per lane: dim <= 32 DQ
-__global__ void __launch_bounds__(DR_WARPS * 32) delta_rule_scan_kernel(const b200_delta_rule_args a) {
-    constexpr int DP = 32 * DQ, DR_CHUNK = CHAN && DQ > 4 ? 8 : 16, DR_TPW = DR_CHUNK / DR_WARPS;  // (three staged rows of 256 values: half the tokens fit)
-    __shared__ __align__(16) float sq[DR_CHUNK][DP], sk[DR_CHUNK][DP];
-    __shared__ __align__(16) float sgc[CHAN ? DR_CHUNK : 1][CHAN ? DP : 4];
-    __shared__ float sbias[CHAN ? DP : 1];  // (not added where a.a is read: the test of the pointer would make those loads wait for one another)
-    __shared__ float sv[DR_CHUNK][DR_COLS], sqk[DR_CHUNK], sg[DR_CHUNK], sbeta[DR_CHUNK];
+__global__ void __launch_bounds__(DR_WARPS * 64) delta_rule_scan_kernel(const b200_delta_rule_args a) {
+    constexpr int DP = 32 * DQ, DR_CHUNK = dr_chunk<DQ, CHAN>();
+    __shared__ __align__(16) float sq[2][DR_CHUNK][DP], sk[2][DR_CHUNK][DP];
+    __shared__ __align__(16) float sgc[CHAN ? 2 : 1][CHAN ? DR_CHUNK : 1][CHAN ? DP : 4];
+    __shared__ float sv[2][DR_CHUNK][DR_COLS];
+    __shared__ __align__(16) float4 stok[2][DR_CHUNK];  // g, g (1 with CHAN), beta, q.k
     const int h = blockIdx.y, s = blockIdx.z, kvh = h / (a.heads / a.kv_heads);
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, tid = threadIdx.x;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int D = a.dim, V = a.vdim;
     const int first = a.seq_info[s], count = a.seq_info[a.n_seq + s], slot = a.seq_info[2 * a.n_seq + s], fresh = a.seq_info[3 * a.n_seq + s];
     if (count <= 0) return;
-    const int cb = blockIdx.x * DR_COLS, cw = lane >> 3, r = lane & 7, lc0 = warp * DR_CW * DR_CPL + cw;  // the lane's columns: cb + lc0 + DR_CW c
-    float *Sp = a.state + (int64_t)slot * a.slot_stride + ((int64_t)h * V + cb + lc0) * D;                // column c at Sp + DR_CW c D
-    float S[DR_CPL][DQ][4];
-#pragma unroll
-    for (int c = 0; c < DR_CPL; c++)
-#pragma unroll
-        for (int i = 0; i < DQ; i++)
-#pragma unroll
-            for (int e = 0; e < 4; e++) {
-                const int d = 4 * (r + 8 * i) + e;
-                S[c][i][e] = (!fresh && d < D && cb + lc0 + DR_CW * c < V) ? Sp[(int64_t)DR_CW * c * D + d] : 0.f;
-            }
-    const float decay_rate = expf(a.a_log[h]), dtb = !CHAN && a.dt_bias ? a.dt_bias[h] : 0.f;
-    // staging: the raw values of a chunk travel to registers (every thread a slice of the chunk), are parked in shared memory, and
-    // warp w then turns the tokens w, w + DR_WARPS, ... into unit vectors in place
-    constexpr int NQ = DR_CHUNK * DP / (DR_WARPS * 32), NVV = (DR_CHUNK * DR_COLS) / (DR_WARPS * 32);
-    float pq[NQ], pk[NQ], pg[CHAN ? NQ : 1], pv[NVV], pa = 0.f, pb = 0.f;
-    auto fetch = [&](int t0) {
-        const int nt = min(DR_CHUNK, count - t0);
-#pragma unroll
-        for (int j = 0; j < NQ; j++) {
-            const int idx = tid + j * DR_WARPS * 32, tt = idx / DP, d = idx - tt * DP;
-            const bool ok = tt < nt && d < D;
-            const int64_t tok = first + t0 + tt;
-            pq[j] = ok ? a.q[tok * a.q_stride + (int64_t)kvh * D + d] : 0.f;
-            pk[j] = ok ? a.k[tok * a.k_stride + (int64_t)kvh * D + d] : 0.f;
-            if (CHAN) pg[CHAN ? j : 0] = ok ? a.a[tok * a.a_stride + (int64_t)h * D + d] : 0.f;
-        }
-#pragma unroll
-        for (int j = 0; j < NVV; j++) {
-            const int idx = tid + j * DR_WARPS * 32, tt = idx / DR_COLS, c = idx - tt * DR_COLS;
-            pv[j] = (tt < nt && cb + c < V) ? a.v[(int64_t)(first + t0 + tt) * a.v_stride + (int64_t)h * V + cb + c] : 0.f;
-        }
-        if (tid < DR_CHUNK) {
-            if (!CHAN) pa = tid < nt ? a.a[(int64_t)(first + t0 + tid) * a.a_stride + h] : 0.f;
-            pb = tid < nt ? a.b[(int64_t)(first + t0 + tid) * a.b_stride + h] : 0.f;
-        }
-    };
-    fetch(0);
-    if (CHAN) for (int d = tid; d < DP; d += DR_WARPS * 32) sbias[d] = a.dt_bias && d < D ? a.dt_bias[(int64_t)h * D + d] : 0.f;
-    for (int t0 = 0; t0 < count; t0 += DR_CHUNK) {
-        const int nt = min(DR_CHUNK, count - t0);
-        __syncthreads();  // the previous chunk has been read
-#pragma unroll
-        for (int j = 0; j < NQ; j++) { (&sq[0][0])[tid + j * DR_WARPS * 32] = pq[j]; (&sk[0][0])[tid + j * DR_WARPS * 32] = pk[j]; }
-#pragma unroll
-        for (int j = 0; j < NVV; j++) (&sv[0][0])[tid + j * DR_WARPS * 32] = pv[j];
+    const int cb = blockIdx.x * DR_COLS, n_chunks = (count + DR_CHUNK - 1) / DR_CHUNK;
+    if (warp >= DR_WARPS) {
+        // ===== staging: a warp takes the tokens w, w + DR_WARPS, ... of a chunk, all their loads in flight at once
+        constexpr int TPW = (DR_CHUNK + DR_WARPS - 1) / DR_WARPS;
+        const int w = warp - DR_WARPS;
+        const float decay_rate = expf(a.a_log[h]), dtb = !CHAN && a.dt_bias ? a.dt_bias[h] : 0.f;
+        float bias[CHAN ? DQ : 1];
         if (CHAN) {
 #pragma unroll
-            for (int j = 0; j < NQ; j++) (&sgc[0][0])[tid + j * DR_WARPS * 32] = expf(-decay_rate * softplus_f(pg[CHAN ? j : 0] + sbias[CHAN ? (tid + j * DR_WARPS * 32) % DP : 0]));
+            for (int j = 0; j < DQ; j++) bias[CHAN ? j : 0] = a.dt_bias && lane + 32 * j < D ? a.dt_bias[(int64_t)h * D + lane + 32 * j] : 0.f;
         }
-        if (tid < DR_CHUNK) {
-            if (!CHAN) sg[tid] = expf(-decay_rate * softplus_f(pa + dtb));
-            sbeta[tid] = sigmoidf_(pb);
-        }
-        __syncthreads();
+        for (int c = 0; c < n_chunks; c++) {
+            const int buf = c & 1;
+            float q[TPW][DQ], k[TPW][DQ], z[CHAN ? TPW : 1][CHAN ? DQ : 1], v[TPW], ga[TPW], be[TPW];
 #pragma unroll
-        for (int u = 0; u < DR_TPW; u++) {
-            const int tt = warp + u * DR_WARPS;
-            float qv[DQ], kv[DQ], qq = 0.f, kk = 0.f, qk = 0.f;
+            for (int u = 0; u < TPW; u++) {
+                const int t = c * DR_CHUNK + w + u * DR_WARPS;
+                const bool ok = w + u * DR_WARPS < DR_CHUNK && t < count;
+                const int64_t tok = first + t;
 #pragma unroll
-            for (int j = 0; j < DQ; j++) {
-                qv[j] = sq[tt][lane + 32 * j]; kv[j] = sk[tt][lane + 32 * j];
-                qq += qv[j] * qv[j]; kk += kv[j] * kv[j];
+                for (int j = 0; j < DQ; j++) {
+                    const int d = lane + 32 * j;
+                    q[u][j] = ok && d < D ? a.q[tok * a.q_stride + (int64_t)kvh * D + d] : 0.f;
+                    k[u][j] = ok && d < D ? a.k[tok * a.k_stride + (int64_t)kvh * D + d] : 0.f;
+                    if (CHAN) z[CHAN ? u : 0][CHAN ? j : 0] = ok && d < D ? a.a[tok * a.a_stride + (int64_t)h * D + d] : 0.f;
+                }
+                v[u] = ok && cb + lane < V ? a.v[tok * a.v_stride + (int64_t)h * V + cb + lane] : 0.f;
+                ga[u] = !CHAN && ok ? a.a[tok * a.a_stride + h] : 0.f;
+                be[u] = ok ? a.b[tok * a.b_stride + h] : 0.f;
             }
-            qq = warp_sum(qq); kk = warp_sum(kk);
-            const float fq = (a.unit_qk ? 1.0f / sqrtf(qq + a.unit_eps) : 1.0f) * a.q_scale, fk = a.unit_qk ? 1.0f / sqrtf(kk + a.unit_eps) : 1.0f;
 #pragma unroll
-            for (int j = 0; j < DQ; j++) {
-                qv[j] *= fq; kv[j] *= fk;
-                qk += qv[j] * kv[j];
-                sq[tt][lane + 32 * j] = qv[j]; sk[tt][lane + 32 * j] = kv[j];
+            for (int u = 0; u < TPW; u++) {
+                const int tt = w + u * DR_WARPS;
+                float qq = 0.f, kk = 0.f, qk = 0.f;
+#pragma unroll
+                for (int j = 0; j < DQ; j++) { qq += q[u][j] * q[u][j]; kk += k[u][j] * k[u][j]; }
+                qq = warp_sum(qq); kk = warp_sum(kk);
+                const float fq = (a.unit_qk ? 1.0f / sqrtf(qq + a.unit_eps) : 1.0f) * a.q_scale, fk = a.unit_qk ? 1.0f / sqrtf(kk + a.unit_eps) : 1.0f;
+#pragma unroll
+                for (int j = 0; j < DQ; j++) { q[u][j] *= fq; k[u][j] *= fk; qk += q[u][j] * k[u][j]; }
+                qk = warp_sum(qk);
+                if (tt < DR_CHUNK) {
+#pragma unroll
+                    for (int j = 0; j < DQ; j++) {
+                        sq[buf][tt][lane + 32 * j] = q[u][j];
+                        sk[buf][tt][lane + 32 * j] = k[u][j];
+                        if (CHAN) sgc[CHAN ? buf : 0][CHAN ? tt : 0][CHAN ? lane + 32 * j : 0] = expf(-decay_rate * softplus_f(z[CHAN ? u : 0][CHAN ? j : 0] + bias[CHAN ? j : 0]));
+                    }
+                    sv[buf][tt][lane] = v[u];
+                    if (lane == 0) {
+                        const float g = CHAN ? 1.0f : expf(-decay_rate * softplus_f(ga[u] + dtb));
+                        stok[buf][tt] = make_float4(g, g, sigmoidf_(be[u]), qk);
+                    }
+                }
             }
-            qk = warp_sum(qk);
-            if (lane == 0) sqk[tt] = qk;
+            __syncthreads();  // chunk c is ready; chunk c - 1, whose room the next one takes, has been read
         }
+        return;
+    }
+    // ===== the state: columns cb + lc + DR_CW c of the lane
+    const int r = lane & 7, lc = warp * DR_CW * DR_CPL + (lane >> 3);
+    float *Sp = a.state + (int64_t)slot * a.slot_stride + ((int64_t)h * V + cb + lc) * D;  // column c at Sp + DR_CW c D
+    unsigned long long S[DR_CPL][DQ][2];
+#pragma unroll
+    for (int c = 0; c < DR_CPL; c++) {
+#pragma unroll
+        for (int i = 0; i < DQ; i++) {
+            float x[4];
+#pragma unroll
+            for (int e = 0; e < 4; e++) { const int d = 4 * (r + 8 * i) + e; x[e] = (!fresh && d < D && cb + lc + DR_CW * c < V) ? Sp[(int64_t)DR_CW * c * D + d] : 0.f; }
+            S[c][i][0] = dr_pack(x[0], x[1]);
+            S[c][i][1] = dr_pack(x[2], x[3]);
+        }
+    }
+    float *out = a.dst + (int64_t)first * a.dst_stride + (int64_t)h * V + cb + lc;
+    for (int ch = 0; ch < n_chunks; ch++) {
+        const int nt = min(DR_CHUNK, count - ch * DR_CHUNK), buf = ch & 1;
         __syncthreads();
-        if (t0 + DR_CHUNK < count) fetch(t0 + DR_CHUNK);
         // unrolled so that the shared-memory loads of the following tokens are issued ahead of the chain S -> sums -> u -> S
-#pragma unroll 4
+#pragma unroll 2
         for (int tt = 0; tt < nt; tt++) {
+            const float4 tok = stok[buf][tt];
+            ulonglong2 kv[DQ], qv[DQ];
             float ks[DR_CPL], qs[DR_CPL];
-            float4 kv[DQ];
-#pragma unroll
-            for (int c = 0; c < DR_CPL; c++) ks[c] = qs[c] = 0.f;
 #pragma unroll
             for (int i = 0; i < DQ; i++) {
-                kv[i] = *reinterpret_cast<const float4 *>(&sk[tt][4 * (r + 8 * i)]);
-                const float4 qv = *reinterpret_cast<const float4 *>(&sq[tt][4 * (r + 8 * i)]);
+                kv[i] = *reinterpret_cast<const ulonglong2 *>(&sk[buf][tt][4 * (r + 8 * i)]);
+                qv[i] = *reinterpret_cast<const ulonglong2 *>(&sq[buf][tt][4 * (r + 8 * i)]);
                 if (CHAN) {
-                    const float4 gv = *reinterpret_cast<const float4 *>(&sgc[CHAN ? tt : 0][CHAN ? 4 * (r + 8 * i) : 0]);
+                    const ulonglong2 gv = *reinterpret_cast<const ulonglong2 *>(&sgc[CHAN ? buf : 0][CHAN ? tt : 0][CHAN ? 4 * (r + 8 * i) : 0]);
 #pragma unroll
-                    for (int c = 0; c < DR_CPL; c++) { S[c][i][0] *= gv.x; S[c][i][1] *= gv.y; S[c][i][2] *= gv.z; S[c][i][3] *= gv.w; }
-                }
-#pragma unroll
-                for (int c = 0; c < DR_CPL; c++) {
-                    ks[c] += (kv[i].x * S[c][i][0] + kv[i].z * S[c][i][2]) + (kv[i].y * S[c][i][1] + kv[i].w * S[c][i][3]);
-                    qs[c] += (qv.x * S[c][i][0] + qv.z * S[c][i][2]) + (qv.y * S[c][i][1] + qv.w * S[c][i][3]);
+                    for (int c = 0; c < DR_CPL; c++) { S[c][i][0] = dr_mul(S[c][i][0], gv.x); S[c][i][1] = dr_mul(S[c][i][1], gv.y); }
                 }
             }
-#pragma unroll
-            for (int off = 4; off >= 1; off >>= 1)
-#pragma unroll
-                for (int c = 0; c < DR_CPL; c++) { ks[c] += __shfl_xor_sync(0xffffffffu, ks[c], off); qs[c] += __shfl_xor_sync(0xffffffffu, qs[c], off); }
-            const float g = CHAN ? 1.0f : sg[tt];
 #pragma unroll
             for (int c = 0; c < DR_CPL; c++) {
-                const float u = sbeta[tt] * (sv[tt][lc0 + DR_CW * c] - g * ks[c]);
+                unsigned long long k0 = dr_mul(kv[0].x, S[c][0][0]), k1 = dr_mul(kv[0].y, S[c][0][1]), q0 = dr_mul(qv[0].x, S[c][0][0]), q1 = dr_mul(qv[0].y, S[c][0][1]);
+#pragma unroll
+                for (int i = 1; i < DQ; i++) {
+                    k0 = dr_fma(kv[i].x, S[c][i][0], k0); k1 = dr_fma(kv[i].y, S[c][i][1], k1);
+                    q0 = dr_fma(qv[i].x, S[c][i][0], q0); q1 = dr_fma(qv[i].y, S[c][i][1], q1);
+                }
+                const float2 ka = dr_unpack(k0), kb = dr_unpack(k1), qa = dr_unpack(q0), qb = dr_unpack(q1);
+                ks[c] = (ka.x + kb.x) + (ka.y + kb.y);
+                qs[c] = (qa.x + qb.x) + (qa.y + qb.y);
+            }
+#pragma unroll
+            for (int off = 4; off >= 1; off >>= 1) {
+#pragma unroll
+                for (int c = 0; c < DR_CPL; c++) { ks[c] += __shfl_xor_sync(0xffffffffu, ks[c], off); qs[c] += __shfl_xor_sync(0xffffffffu, qs[c], off); }
+            }
+            const unsigned long long g2 = dr_pack(tok.x, tok.y);
+#pragma unroll
+            for (int c = 0; c < DR_CPL; c++) {
+                const float u = tok.z * (sv[buf][tt][lc + DR_CW * c] - tok.x * ks[c]);
+                const unsigned long long u2 = dr_pack(u, u);
 #pragma unroll
                 for (int i = 0; i < DQ; i++) {
-                    S[c][i][0] = g * S[c][i][0] + kv[i].x * u; S[c][i][1] = g * S[c][i][1] + kv[i].y * u;
-                    S[c][i][2] = g * S[c][i][2] + kv[i].z * u; S[c][i][3] = g * S[c][i][3] + kv[i].w * u;
+                    S[c][i][0] = dr_fma(kv[i].x, u2, CHAN ? S[c][i][0] : dr_mul(S[c][i][0], g2));
+                    S[c][i][1] = dr_fma(kv[i].y, u2, CHAN ? S[c][i][1] : dr_mul(S[c][i][1], g2));
                 }
-                if (r == 0 && cb + lc0 + DR_CW * c < V) a.dst[(int64_t)(first + t0 + tt) * a.dst_stride + (int64_t)h * V + cb + lc0 + DR_CW * c] = g * qs[c] + sqk[tt] * u;
+                if (r == 0 && cb + lc + DR_CW * c < V) out[DR_CW * c] = tok.x * qs[c] + tok.w * u;
             }
+            out += a.dst_stride;
         }
     }
 #pragma unroll
-    for (int c = 0; c < DR_CPL; c++)
+    for (int c = 0; c < DR_CPL; c++) {
 #pragma unroll
-        for (int i = 0; i < DQ; i++)
+        for (int i = 0; i < DQ; i++) {
+            const float2 x = dr_unpack(S[c][i][0]), y = dr_unpack(S[c][i][1]);
+            const float z[4] = {x.x, x.y, y.x, y.y};
 #pragma unroll
-            for (int e = 0; e < 4; e++) {
-                const int d = 4 * (r + 8 * i) + e;
-                if (d < D && cb + lc0 + DR_CW * c < V) Sp[(int64_t)DR_CW * c * D + d] = S[c][i][e];
-            }
+            for (int e = 0; e < 4; e++) { const int d = 4 * (r + 8 * i) + e; if (d < D && cb + lc + DR_CW * c < V) Sp[(int64_t)DR_CW * c * D + d] = z[e]; }
+        }
+    }
 }
 
 template <int DQ, bool CHAN>
 static int launch_delta_rule2(const b200_delta_rule_args *a, cudaStream_t st) {
     const dim3 grid((unsigned)((a->vdim + DR_COLS - 1) / DR_COLS), (unsigned)a->heads, (unsigned)a->n_seq);
-    delta_rule_scan_kernel<DQ, CHAN><<<grid, DR_WARPS * 32, 0, st>>>(*a);
+    delta_rule_scan_kernel<DQ, CHAN><<<grid, DR_WARPS * 64, 0, st>>>(*a);
     B200_CUDA_TRY(cudaGetLastError());
     return B200_OK;
 }
