@@ -272,30 +272,39 @@ static int device_props() {
     return B200_OK;
 }
 
-template <int TYPE, int NCOLS, bool MULTI>
-static int launch_mmvq(MmvqParams &p, cudaStream_t st, bool pdl) {
-    using G = Geo<TYPE>;
-    int rc = device_props();
+struct MmvqPlan { int64_t units, grid; size_t act_bytes, tab_bytes; };  // units: rows, or (gate, up) pairs
+// split over the SMs, and whether row table and activations fit: what several columns may ask for, whichever kernel serves them
+template <int TYPE>
+static int mmvq_plan(MmvqParams &p, int ncols, bool multi, MmvqPlan &pl) {
+    const int rc = device_props();
     if (rc) return rc;
-    const size_t bar_bytes = MMVQ_BAR_BYTES;
-    const size_t act_bytes = ((size_t)NCOLS * act_col_bytes(p.n_it) + 127) / 128 * 128;
-    const int64_t units = p.silu_pair ? p.total_rows / 2 : p.total_rows;  // rows, or (gate, up) pairs
-    const int64_t grid = units < g_sm_count ? units : g_sm_count;
-    const int64_t rows_per_cta = p.silu_pair ? 2 * MMVQ_NW * (((units + grid - 1) / grid + MMVQ_NW - 1) / MMVQ_NW) : (p.total_rows + grid - 1) / grid;
-    if (MULTI && rows_per_cta > MMVQ_MAX_TAB) {
+    pl.act_bytes = ((size_t)ncols * act_col_bytes(p.n_it) + 127) / 128 * 128;
+    pl.units = p.silu_pair ? p.total_rows / 2 : p.total_rows;
+    pl.grid = pl.units < g_sm_count ? pl.units : g_sm_count;
+    const int64_t rows_per_cta = p.silu_pair ? 2 * MMVQ_NW * (((pl.units + pl.grid - 1) / pl.grid + MMVQ_NW - 1) / MMVQ_NW) : (p.total_rows + pl.grid - 1) / pl.grid;
+    if (multi && rows_per_cta > MMVQ_MAX_TAB) {
         set_error("b200_mul_mat_vec_q_multi: %lld rows exceed the per-CTA row table", (long long)p.total_rows);
         return B200_ERR_UNSUPPORTED;
     }
-    p.tab_rows = MULTI ? (int)((rows_per_cta + 63) / 64 * 64) : 0;
-    const size_t tab_bytes = MULTI ? (size_t)17 * p.tab_rows + 64 : 0;
+    p.tab_rows = multi ? (int)((rows_per_cta + 63) / 64 * 64) : 0;
+    pl.tab_bytes = multi ? (size_t)17 * p.tab_rows + 64 : 0;
     // (measured: 8 warps + half-SM rings so that consecutive launches overlap under PDL lost 15 %: a 93 KB ring cannot cover
     // the HBM latency-bandwidth product of one SM on the large matrices)
-    const size_t min_need = bar_bytes + act_bytes + 2 * (size_t)MMVQ_NW * G::STAGE_BYTES + tab_bytes + 256;
-    const size_t cap = g_smem_optin;
-    if (min_need > cap) {
-        set_error("b200_mul_mat_vec_q: K=%lld x N=%d activations do not fit in shared memory", (long long)p.K, NCOLS);
+    if (MMVQ_BAR_BYTES + pl.act_bytes + 2 * (size_t)MMVQ_NW * Geo<TYPE>::STAGE_BYTES + pl.tab_bytes + 256 > g_smem_optin) {
+        set_error("b200_mul_mat_vec_q: K=%lld x N=%d activations do not fit in shared memory", (long long)p.K, ncols);
         return B200_ERR_UNSUPPORTED;
     }
+    return B200_OK;
+}
+
+template <int TYPE, int NCOLS, bool MULTI>
+static int launch_mmvq(MmvqParams &p, cudaStream_t st, bool pdl) {
+    using G = Geo<TYPE>;
+    MmvqPlan pl;
+    const int rc = mmvq_plan<TYPE>(p, NCOLS, MULTI, pl);
+    if (rc) return rc;
+    const size_t bar_bytes = MMVQ_BAR_BYTES, act_bytes = pl.act_bytes, tab_bytes = pl.tab_bytes, cap = g_smem_optin;
+    const int64_t units = pl.units, grid = pl.grid;
     const size_t budget = cap - 256 - tab_bytes;
     size_t ns = (budget - bar_bytes - act_bytes) / ((size_t)MMVQ_NW * G::STAGE_BYTES);
     // no point in more stages than a warp has steps: rows per warp ~ total_rows / (SMs * NW)
@@ -397,6 +406,10 @@ static int launch_mmvq3(MmvqParams &p, cudaStream_t st, bool pdl) {
     return B200_OK;
 }
 
+}  // namespace b200
+#include "mmvq_mma.cuh"
+namespace b200 {
+
 template <int TYPE>
 static int dispatch_cols(MmvqParams &p, int N, cudaStream_t st, bool pdl) {
     const bool multi = p.n_jobs > 1 || p.ids != nullptr;
@@ -406,6 +419,20 @@ static int dispatch_cols(MmvqParams &p, int N, cudaStream_t st, bool pdl) {
         for (int j = 1; j < p.n_jobs; j++) same_x = same_x && p.jobs[j].X == p.jobs[0].X;
         if (same_x) {
             const int rc = multi ? launch_mmvq3<TYPE, true>(p, st, pdl) : launch_mmvq3<TYPE, false>(p, st, pdl);
+            if (rc != -1000) return rc;
+        }
+    }
+    // Several columns of one activation matrix: the integer tensor cores, whose cost hardly grows with the columns.  The line lies where the dp4a form
+    // begins to lose over all measured shapes (K 512 .. 14336, M 64 .. 32000), dp4a -> tensor: q4_K 4096 x 14336 at 4 columns 24.2 -> 17.7 us, at 8
+    // 40.5 -> 19.9; q5_K 24.5 -> 20.1 and 41.4 -> 22.4; q6_K, whose rows lie at any even byte, 27.0 -> 27.6 at 4, 35.1 -> 28.4 at 6.  Few rows leave
+    // each warp one block: q5_K 2048 x 256 at 4 columns 5.6 -> 5.9, 4096 x 1024 7.8 -> 7.5.
+    if constexpr (TYPE == B200_TYPE_Q4_K || TYPE == B200_TYPE_Q5_K || TYPE == B200_TYPE_Q6_K) {
+        bool same_x = p.ids == nullptr;
+        for (int j = 1; j < p.n_jobs; j++) same_x = same_x && p.jobs[j].X == p.jobs[0].X;
+        if (N >= (TYPE == B200_TYPE_Q6_K ? 6 : 4) && p.total_rows >= 512 && same_x && (!multi || N <= 4)) {
+            MmvqPlan pl;
+            int rc = mmvq_plan<TYPE>(p, N, multi, pl);
+            if (!rc) rc = launch_mmvq_mma<TYPE>(p, N, st, pdl);
             if (rc != -1000) return rc;
         }
     }

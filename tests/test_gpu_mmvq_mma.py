@@ -1,0 +1,86 @@
+"""The GEMV of several columns on the integer tensor cores: row tiles of 16 and their remainders, K parts for 1 to 16 warps, odd and even column counts,
+rows at any even byte, jobs of different sizes, norm prologue, residual and raw results.  Against the oracle's q8_1 arithmetic: sums of K / 32 exact
+products in f32, 2^-24 sqrt(K / 32) of their size, bound 3e-5 as for the other GEMV kernels."""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+import koboldcpp_b200.host as H
+import orc as O
+from koboldcpp_b200.lib import Q4_K, Q5_K, Q6_K, GemvFuse, GemvJob, check, lib, row_size
+from koboldcpp_b200.llama import random_blocks
+
+pytestmark = pytest.mark.gpu
+
+
+def close(got, want):
+    return float(np.abs(got - want).max() / np.abs(want).max()) < 3e-5
+
+
+@pytest.mark.parametrize("t", [Q4_K, Q5_K, Q6_K])
+@pytest.mark.parametrize("K,M,N", [(256, 511, 8), (256, 512, 8), (256, 513, 7), (512, 527, 5), (1024, 700, 8), (2816, 545, 7), (4096, 2500, 4), (5120, 530, 6), (11008, 512, 5), (13824, 560, 4)])
+def test_columns(t, K, M, N):
+    rng = np.random.default_rng(K + M + N + t)
+    w, x = random_blocks(rng, t, M, K), rng.standard_normal((N, K)).astype(np.float32)
+    assert close(H.mul_mat_vec_q(t, w, x, K, M), O.mul_mat_q8_1(t, w, x, K, M))
+
+
+@pytest.mark.parametrize("offset,pad", [(2, 0), (6, 2), (14, 10), (8, 4)])
+def test_rows_at_any_even_byte(offset, pad):
+    t, K, M, N = Q6_K, 1024, 515, 6
+    rng = np.random.default_rng(offset)
+    w, x = random_blocks(rng, t, M, K), rng.standard_normal((N, K)).astype(np.float32)
+    rs = row_size(t, K)
+    raw = np.zeros(offset + M * (rs + pad) + 64, np.uint8)
+    for m in range(M):
+        raw[offset + m * (rs + pad):offset + m * (rs + pad) + rs] = w[m]
+    dw, dx, dd = H.DeviceBuffer.from_numpy(raw), H.DeviceBuffer.from_numpy(x), H.DeviceBuffer(4 * N * M)
+    check(lib().b200_mul_mat_vec_q(t, dw.ptr + offset, rs + pad, dx.ptr, K, dd.ptr, M, K, M, N, None))
+    assert close(dd.to_numpy(np.float32, (N, M)), O.mul_mat_q8_1(t, w, x, K, M))
+
+
+@pytest.mark.parametrize("t", [Q4_K, Q5_K])
+def test_jobs_with_norm_and_residual(t):
+    K, N, Ms, eps = 1280, 4, [100, 16, 433], 1e-5
+    rng = np.random.default_rng(N + t)
+    ws = [random_blocks(rng, t, M, K) for M in Ms]
+    x, nw = rng.standard_normal((N, K)).astype(np.float32), rng.standard_normal(K).astype(np.float32)
+    total = sum(Ms)
+    res = rng.standard_normal((N, total)).astype(np.float32)
+    scale = (1.0 / np.sqrt((x.astype(np.float64) ** 2).mean(1, keepdims=True) + eps)).astype(np.float32)
+    xn = x * scale * nw
+    dx, dn, dr = H.DeviceBuffer.from_numpy(x), H.DeviceBuffer.from_numpy(nw), H.DeviceBuffer.from_numpy(res)
+    dws = [H.DeviceBuffer.from_numpy(w, pad=16) for w in ws]
+    dd, draw, dnorm, dmul = (H.DeviceBuffer(4 * N * n) for n in (total, total, K, K))
+    jobs, fuse, at = (GemvJob * len(Ms))(), GemvFuse(), 0
+    fuse.norm_weight, fuse.norm_eps, fuse.norm_out, fuse.norm_mul_out = dn.ptr, eps, dnorm.ptr, dmul.ptr
+    for i, (w, M) in enumerate(zip(dws, Ms)):
+        jobs[i].W, jobs[i].X, jobs[i].dst, jobs[i].M, jobs[i].id_index = w.ptr, dx.ptr, dd.ptr + 4 * at, M, -1
+        if i != 1:
+            fuse.residual[i], fuse.raw_dst[i] = dr.ptr + 4 * at, draw.ptr + 4 * at
+        at += M
+    check(lib().b200_mul_mat_vec_q_fused(t, jobs, len(Ms), row_size(t, K), K, total, K, N, C.byref(fuse), None))
+    got, raw = dd.to_numpy(np.float32, (N, total)), draw.to_numpy(np.float32, (N, total))
+    np.testing.assert_allclose(dnorm.to_numpy(np.float32, (N, K)), x * scale, rtol=3e-6, atol=3e-6)
+    np.testing.assert_allclose(dmul.to_numpy(np.float32, (N, K)), xn, rtol=3e-6, atol=3e-6)
+    at = 0
+    for i, (w, M) in enumerate(zip(ws, Ms)):
+        want = O.mul_mat_q8_1(t, w, xn, K, M)
+        sl = slice(at, at + M)
+        # (a value on the edge between two quants may fall to the other side with the norm's last bit: one step of 2^-7 of a block)
+        tol = 2e-3 * np.abs(want).max()
+        assert np.abs(got[:, sl] - (want + (res[:, sl] if i != 1 else 0))).max() < tol
+        if i != 1:
+            assert np.abs(raw[:, sl] - want).max() < tol
+        at += M
+
+
+def test_five_columns_of_several_jobs_stay_refused():
+    K, M = 256, 272
+    w = H.DeviceBuffer(row_size(Q4_K, K) * M + 16, zero=True)
+    x, d = H.DeviceBuffer(4 * 5 * K, zero=True), H.DeviceBuffer(4 * 5 * 2 * M)
+    jobs = (GemvJob * 2)()
+    for i in range(2):
+        jobs[i].W, jobs[i].X, jobs[i].dst, jobs[i].M, jobs[i].id_index = w.ptr, x.ptr, d.ptr + 4 * M * i, M, -1
+    assert lib().b200_mul_mat_vec_q_multi(Q4_K, jobs, 2, row_size(Q4_K, K), K, 2 * M, K, 5, None, 0, 0, None) == 1
