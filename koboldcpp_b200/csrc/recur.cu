@@ -225,8 +225,9 @@ __global__ void __launch_bounds__(DR_WARPS * 64) delta_rule_scan_kernel(const b2
                 const unsigned long long u2 = dr_pack(u, u);
 #pragma unroll
                 for (int i = 0; i < DQ; i++) {
-                    S[c][i][0] = dr_fma(kv[i].x, u2, CHAN ? S[c][i][0] : dr_mul(S[c][i][0], g2));
-                    S[c][i][1] = dr_fma(kv[i].y, u2, CHAN ? S[c][i][1] : dr_mul(S[c][i][1], g2));
+                    // (the small term k u is the one that is rounded first)
+                    S[c][i][0] = CHAN ? dr_fma(kv[i].x, u2, S[c][i][0]) : dr_fma(S[c][i][0], g2, dr_mul(kv[i].x, u2));
+                    S[c][i][1] = CHAN ? dr_fma(kv[i].y, u2, S[c][i][1]) : dr_fma(S[c][i][1], g2, dr_mul(kv[i].y, u2));
                 }
                 if (r == 0 && cb + lc + DR_CW * c < V) out[DR_CW * c] = tok.x * qs[c] + tok.w * u;
             }
