@@ -448,8 +448,9 @@ static bool fa_use_mma(const b200_fattn_args *a) {
     if (a->D != 64 && a->D != 128) return true;  // head sizes 80 / 96 / 112 / 256 exist on the tensor-core kernels only
     if (a->type_k == B200_TYPE_Q4_0) return true;  // a q4_0 cache too (tiles dequantised to f16 in shared memory)
     if (off) return false;
-    // q8_0 cache: the tile is dequantised to f16 in shared memory first (~2 instructions per value); that pays as soon as several
-    // query columns share it (GQA group, prompt batch): 32/8 heads @ 32k 67 -> 54 us, but one column per kv-head 28 -> 31 us
+    // q8_0 cache: the tile is unpacked to f16 fragments (~2 instructions per value); that pays as soon as several query columns share it (GQA
+    // group, prompt batch): 32/8 heads @ 32k 67 us in the scalar kernel, 37 here.  One column per kv-head stays with the scalar kernel, which
+    // keeps the unpacked values in f32
     if (a->type_k == B200_TYPE_Q8_0) return a->N * (a->n_head / a->n_head_kv) >= 2;
     // a tiny cache with one or two kv-heads (a rank's share under 8-way tensor parallelism: 8 q-heads on 1 kv-head, 2 MB) is
     // pure latency: the scalar kernel spreads the q-heads over 8x more CTAs and finishes in 10.6 us against 12.6 us here
@@ -589,8 +590,8 @@ static int fa_launch(const FaParams &p, const FaPlan &pl, cudaStream_t st, bool 
     return B200_OK;
 }
 
-template <int TYPE, int D>
-static int fa_launch_mma(const FaParams &p, const FaPlan &pl, cudaStream_t st, bool pdl) {
+template <int TYPE, int D, bool WIDE>
+static int fa_launch_mma_cols(const FaParams &p, const FaPlan &pl, cudaStream_t st, bool pdl) {
     using G = MmaGeo<TYPE, D>;
     size_t smem = (size_t)FM_NW * G::WARP_BYTES;
     const size_t merge = ((size_t)(FM_NW + 1) * FM_MAXC * (D + FA_RS_PAD) + 2 * FM_MAXC * FM_MAX_CLUSTER + 2 * FM_MAXC * FA_MAX_SPLITS) * sizeof(float);
@@ -600,8 +601,8 @@ static int fa_launch_mma(const FaParams &p, const FaPlan &pl, cudaStream_t st, b
     B200_CUDA_TRY(cudaGetDevice(&cur_dev));
     bool &attr_set = attr_set_dev[cur_dev & 15];
     if (!attr_set) {
-        B200_CUDA_TRY(cudaFuncSetAttribute(fattn_mma_kernel<TYPE, D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        B200_CUDA_TRY(cudaFuncSetAttribute(fattn_mma_kernel<TYPE, D>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+        B200_CUDA_TRY(cudaFuncSetAttribute(fattn_mma_kernel<TYPE, D, WIDE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        B200_CUDA_TRY(cudaFuncSetAttribute(fattn_mma_kernel<TYPE, D, WIDE>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
         attr_set = true;
     }
     cudaLaunchConfig_t cfg = {};
@@ -625,7 +626,7 @@ static int fa_launch_mma(const FaParams &p, const FaPlan &pl, cudaStream_t st, b
     }
     cfg.attrs = at;
     cfg.numAttrs = na;
-    cudaError_t e = cudaLaunchKernelEx(&cfg, fattn_mma_kernel<TYPE, D>, p);
+    cudaError_t e = cudaLaunchKernelEx(&cfg, fattn_mma_kernel<TYPE, D, WIDE>, p);
     if (e != cudaSuccess && pl.cluster) {
         // the device could not place the cluster (size, shared memory, a partitioned GPU): same splits, merged through global memory
         cudaGetLastError();
@@ -633,10 +634,17 @@ static int fa_launch_mma(const FaParams &p, const FaPlan &pl, cudaStream_t st, b
         q.cluster_merge = 0;
         q.dyn_tiles = 0;
         cfg.numAttrs = pdl ? 1 : 0;
-        e = cudaLaunchKernelEx(&cfg, fattn_mma_kernel<TYPE, D>, q);
+        e = cudaLaunchKernelEx(&cfg, fattn_mma_kernel<TYPE, D, WIDE>, q);
     }
     if (e != cudaSuccess) return cuda_fail(e, "cudaLaunchKernelEx(fattn_mma_kernel)");
     return B200_OK;
+}
+template <int TYPE, int D>
+static int fa_launch_mma(const FaParams &p, const FaPlan &pl, cudaStream_t st, bool pdl) {
+    // up to 8 columns: half the softmax (f16, 32 heads @ 32k 101 -> 93 us); not with q4_0 and 128 dims, whose unpacking is what bounds a tile (32/8 @ 8k
+    // 19.1 us wide, 20.1 narrow)
+    if constexpr (TYPE == B200_TYPE_Q4_0 && D == 128) return fa_launch_mma_cols<TYPE, D, true>(p, pl, st, pdl);
+    else return pl.C > 8 ? fa_launch_mma_cols<TYPE, D, true>(p, pl, st, pdl) : fa_launch_mma_cols<TYPE, D, false>(p, pl, st, pdl);
 }
 
 template <int D>

@@ -7,7 +7,7 @@
 //   S (16 q x 16 keys) = Q (16 x D, f16 A fragments resident in registers) . K^T   -- K rows come out of shared memory with
 //                                                                                     ldmatrix (B fragments, keys = n)
 //   O (16 q x D)      += P (the S accumulators, repacked as A fragments) . V        -- V through ldmatrix.trans
-// ~190 instructions per tile whatever the number of columns <= 16, so a GQA group or a q8_0... (f16 here) long-context decode is
+// ~190 instructions per f16 tile whatever the number of columns <= 16, so a GQA group or a long-context decode is
 // no longer issue-bound; the KV stream (per-warp cp.async rings, split-K over CTAs, ticket merge) is the one of fattn.cu.
 // Semantics: ggml_compute_forward_flash_attn_ext_f16 (ggml/src/ggml.c:15667-15877): Q rounded to f16, scores scaled in f32,
 // optional softcap / mask / ALiBi slope, online softmax, f32 accumulation of P.V with P rounded to f16 (the reference rounds
@@ -30,13 +30,15 @@ struct MmaGeo {
     static constexpr int ROW_BYTES  = D * 2;           // f16 tile (what ldmatrix reads)
     static constexpr int ROW_STRIDE = ROW_BYTES + 16;  // ldmatrix: 8 rows x 16 bytes must hit 8 different bank groups
     static constexpr int TILE_BYTES = FM_TP * ROW_STRIDE;
-    // q8_0 / q4_0 cache: the ring holds raw rows (D/32 blocks of 34 / 18 bytes, 8- or 4-byte aligned); a warp dequantises the tile it is
-    // about to use into ONE f16 tile pair of its own
+    // q8_0 / q4_0 cache: the ring holds raw rows (D/32 blocks of 34 / 18 bytes, 8- or 4-byte aligned).  q8_0 goes from there to the fragments
+    // (row stride 16 or 48 modulo 128 bytes: 8 rows x 4 words lie in 32 different banks); of q4_0 a warp dequantises the tile it is about to
+    // use into ONE f16 tile pair of its own
+    static constexpr bool Q4        = TYPE == B200_TYPE_Q4_0;
     static constexpr int RAW_ROW    = D / 32 * BLK;
-    static constexpr int RAW_STRIDE = (RAW_ROW + 15) / 16 * 16 + 8;
+    static constexpr int RAW_STRIDE = (RAW_ROW + 15) / 16 * 16 + (Q4 ? 8 : 0);
     static constexpr int RAW_TILE   = (FM_TP * RAW_STRIDE + 16 + 127) / 128 * 128;
     static constexpr int RING_TILE  = Q8 ? RAW_TILE : TILE_BYTES;                                  // one K or V tile in the ring
-    static constexpr int WARP_BYTES = FM_NBUF * 2 * RING_TILE + (Q8 ? 2 * TILE_BYTES : 0);         // ring (+ f16 scratch pair)
+    static constexpr int WARP_BYTES = FM_NBUF * 2 * RING_TILE + (Q4 ? 2 * TILE_BYTES : 0);         // ring (+ f16 scratch pair)
 };
 
 __device__ __forceinline__ void ldsm_x4(unsigned addr, unsigned &r0, unsigned &r1, unsigned &r2, unsigned &r3) {
@@ -115,6 +117,24 @@ __device__ __forceinline__ void mma_load_tile_q8(unsigned char *dst, const unsig
     using G = MmaGeo<TYPE, D>;
     constexpr int CH = G::RAW_ROW % 8 == 0 ? 8 : 4;  // q8_0: D = 128: 136 = 17 x 8, D = 64: 68 = 17 x 4; q4_0: 72 = 9 x 8, 36 = 9 x 4
     constexpr int CPR = G::RAW_ROW / CH;
+    if constexpr (CPR == 17) {  // q8_0: 16 lanes a row, the last pieces of all rows in one go; no division and no check in a whole tile
+        if (row0 + FM_TP <= n_kv) {
+            const unsigned char *src = base + (size_t)(row0 + (lane >> 4)) * nb1 + (lane & 15) * CH;
+            unsigned char *d = dst + (lane >> 4) * G::RAW_STRIDE + (lane & 15) * CH;
+#pragma unroll
+            for (int i = 0; i < FM_TP / 2; i++) {
+                if constexpr (CH == 8) cp_async8(d + 2 * i * G::RAW_STRIDE, src);
+                else cp_async4(d + 2 * i * G::RAW_STRIDE, src);
+                src += 2 * nb1;
+            }
+            if (lane < FM_TP) {
+                src = base + (size_t)(row0 + lane) * nb1 + 16 * CH;
+                if constexpr (CH == 8) cp_async8(dst + lane * G::RAW_STRIDE + 16 * CH, src);
+                else cp_async4(dst + lane * G::RAW_STRIDE + 16 * CH, src);
+            }
+            return;
+        }
+    }
     for (int i = lane; i < FM_TP * CPR; i += 32) {
         const int r = i / CPR, c = i - r * CPR;
         unsigned char *d = dst + r * G::RAW_STRIDE + c * CH;
@@ -142,9 +162,9 @@ __device__ __forceinline__ void u4x4_to_h2x2(unsigned w, __half2 &lo, __half2 &h
     lo = __hsub2(*reinterpret_cast<const __half2 *>(&a), off);
     hi = __hsub2(*reinterpret_cast<const __half2 *>(&b), off);
 }
-// dequantise one raw q8_0 / q4_0 tile (16 rows x D/32 blocks) into an f16 tile: value = fp16(d * q) (one f16 rounding, 2^-11 relative)
+// dequantise one raw q4_0 tile (16 rows x D/32 blocks) into an f16 tile: value = fp16(d * q) (one f16 rounding, 2^-11 relative)
 template <int TYPE, int D>
-__device__ __forceinline__ void mma_dequant_tile_q8(unsigned char *dst, const unsigned char *raw, int lane) {
+__device__ __forceinline__ void mma_dequant_tile_q4(unsigned char *dst, const unsigned char *raw, int lane) {
     using G = MmaGeo<TYPE, D>;
     constexpr int NB = D / 32;
 #pragma unroll
@@ -155,59 +175,114 @@ __device__ __forceinline__ void mma_dequant_tile_q8(unsigned char *dst, const un
         const __half dh = *reinterpret_cast<const __half *>(src);
         const __half2 d2 = __half2half2(dh);
         uint4 out[4];
-        if constexpr (TYPE == B200_TYPE_Q4_0) {
-            // 16 bytes: low nibbles are values 0..15, high nibbles 16..31 (dequantize_row_q4_0, ggml-quants.c:1523-1541)
-            unsigned w[4];
-            lds_words<4>(src + 2, w);
+        // 16 bytes: low nibbles are values 0..15, high nibbles 16..31 (dequantize_row_q4_0, ggml-quants.c:1523-1541)
+        unsigned w[4];
+        lds_words<4>(src + 2, w);
 #pragma unroll
-            for (int k = 0; k < 4; k++) {
-                __half2 lo, hi;
-                u4x4_to_h2x2(w[k] & 0x0f0f0f0fu, lo, hi);
-                reinterpret_cast<__half2 *>(out)[2 * k] = __hmul2(lo, d2);
-                reinterpret_cast<__half2 *>(out)[2 * k + 1] = __hmul2(hi, d2);
-                u4x4_to_h2x2((w[k] >> 4) & 0x0f0f0f0fu, lo, hi);
-                reinterpret_cast<__half2 *>(out)[8 + 2 * k] = __hmul2(lo, d2);
-                reinterpret_cast<__half2 *>(out)[8 + 2 * k + 1] = __hmul2(hi, d2);
-            }
-        } else {
-            unsigned w[8];
-            lds_words<8>(src + 2, w);
-#pragma unroll
-            for (int k = 0; k < 8; k++) {
-                __half2 lo, hi;
-                i8x4_to_h2x2(w[k], lo, hi);
-                lo = __hmul2(lo, d2);
-                hi = __hmul2(hi, d2);
-                reinterpret_cast<__half2 *>(out)[2 * k] = lo;
-                reinterpret_cast<__half2 *>(out)[2 * k + 1] = hi;
-            }
+        for (int k = 0; k < 4; k++) {
+            __half2 lo, hi;
+            u4x4_to_h2x2(w[k] & 0x0f0f0f0fu, lo, hi);
+            reinterpret_cast<__half2 *>(out)[2 * k] = __hmul2(lo, d2);
+            reinterpret_cast<__half2 *>(out)[2 * k + 1] = __hmul2(hi, d2);
+            u4x4_to_h2x2((w[k] >> 4) & 0x0f0f0f0fu, lo, hi);
+            reinterpret_cast<__half2 *>(out)[8 + 2 * k] = __hmul2(lo, d2);
+            reinterpret_cast<__half2 *>(out)[8 + 2 * k + 1] = __hmul2(hi, d2);
         }
         uint4 *o = reinterpret_cast<uint4 *>(dst + r * G::ROW_STRIDE + b * 64);
         o[0] = out[0]; o[1] = out[1]; o[2] = out[2]; o[3] = out[3];
     }
 }
+// word `i` of the quants of block b of a raw q8_0 row (4-byte aligned): they start 34 b + 2 bytes on, in the middle of a word for even b
+__device__ __forceinline__ unsigned q8_word(const unsigned char *row, int b, int i) {
+    if (b & 1) return *reinterpret_cast<const unsigned *>(row + 34 * b + 2 + 4 * i);
+    const unsigned *w = reinterpret_cast<const unsigned *>(row + 34 * b + 4 * i);
+    return __byte_perm(w[0], w[1], 0x5432);
+}
+__device__ __forceinline__ unsigned h2_bits(__half2 h) { return *reinterpret_cast<const unsigned *>(&h); }
 
-// One (16 keys x K, V) tile against the warp's 16 query columns: S = Q.K^T on the tensor cores, online softmax on the accumulator
-// fragments, O += P.V.  kt / vt: shared addresses of the f16 tiles; t: tile number (keys 16 t ..).
+// Scores of a raw q8_0 tile, K from the ring straight into fragments: value = fp16(d * q).  A contraction may take its dims in any order, so the
+// four that a lane holds of each step of 16 are neighbours (one word), and so are Q's.  What bounds such a tile: issue and the chain copy -> unpack ->
+// product -> softmax, two warps a scheduler.  Unpacking through an f16 tile in shared memory took 1292 instructions a tile and a round trip:
+// 32/8 heads @ 32k 57.3 us; 792 and 36.9 here.  (Measured and not taken: three CTAs an SM with up to 55 splits 39.2 us; mask values asked for ahead
+// of the scores 37.3.)
 template <int D>
-__device__ __forceinline__ void mma_tile_step(unsigned kt, unsigned vt, int t, const unsigned (&qa)[D / 16][4], float (&m)[2], float (&l)[2],
-                                              float (&o)[D / 8][4], const unsigned char *const (&mrow)[2], const float (&slope)[2], float scale,
-                                              float softcap, int n_kv, bool mask_al4, unsigned k_off, unsigned v_off, int t4) {
-    constexpr int KS = D / 16;
-    constexpr float LOG2E = 1.4426950408889634f;
-    float s[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
+__device__ __forceinline__ void mma_scores_q8(const unsigned char *raw, const unsigned (&qa)[D / 16][4], float (&s)[2][4], int g, int t4) {
+    using G = MmaGeo<B200_TYPE_Q8_0, D>;
 #pragma unroll
-    for (int ks = 0; ks < KS; ks++) {
+    for (int nb = 0; nb < 2; nb++) {
+        const unsigned char *row = raw + (g + 8 * nb) * G::RAW_STRIDE;
+#pragma unroll
+        for (int b = 0; b < D / 32; b++) {
+            const __half2 d2 = __half2half2(*reinterpret_cast<const __half *>(row + 34 * b));
+#pragma unroll
+            for (int kk = 0; kk < 2; kk++) {
+                __half2 lo, hi;
+                i8x4_to_h2x2(q8_word(row, b, 4 * kk + t4), lo, hi);
+                mma_f16(s[nb], qa[2 * b + kk], h2_bits(__hmul2(lo, d2)), h2_bits(__hmul2(hi, d2)));
+            }
+        }
+    }
+}
+// O += P . V of a raw q8_0 tile: of every block a lane takes word g of its four keys and pairs the keys' bytes; n-tile 4 b + j, column n: dim 32 b + 4 n + j
+template <int D>
+__device__ __forceinline__ void mma_values_q8(const unsigned char *raw, const unsigned (&pa)[4], float (&o)[D / 8][4], int g, int t4) {
+    using G = MmaGeo<B200_TYPE_Q8_0, D>;
+    const unsigned char *row = raw + 2 * t4 * G::RAW_STRIDE;
+#pragma unroll
+    for (int b = 0; b < D / 32; b++) {
+        unsigned f[2][4];  // keys 2 t4, 2 t4 + 1 and those 8 on; dims 4 g + 0 .. 3 of the block
+#pragma unroll
+        for (int e = 0; e < 2; e++) {
+            const unsigned char *r0 = row + 8 * e * G::RAW_STRIDE, *r1 = r0 + G::RAW_STRIDE;
+            const __half2 d2 = __halves2half2(*reinterpret_cast<const __half *>(r0 + 34 * b), *reinterpret_cast<const __half *>(r1 + 34 * b));
+            const unsigned w0 = q8_word(r0, b, g), w1 = q8_word(r1, b, g);
+            __half2 v[4];
+            i8x4_to_h2x2(__byte_perm(w0, w1, 0x5140), v[0], v[1]);
+            i8x4_to_h2x2(__byte_perm(w0, w1, 0x7362), v[2], v[3]);
+#pragma unroll
+            for (int j = 0; j < 4; j++) f[e][j] = h2_bits(__hmul2(v[j], d2));
+        }
+#pragma unroll
+        for (int j = 0; j < 4; j++) mma_f16(o[4 * b + j], pa, f[0][j], f[1][j]);
+    }
+}
+
+// scores of an f16 tile (shared address kt): S = Q.K^T
+template <int D>
+__device__ __forceinline__ void mma_scores(unsigned kt, const unsigned (&qa)[D / 16][4], float (&s)[2][4], unsigned k_off) {
+#pragma unroll
+    for (int ks = 0; ks < D / 16; ks++) {
         unsigned b0, b1, b2, b3;
         ldsm_x4(kt + k_off + ks * 32, b0, b1, b2, b3);
         mma_f16(s[0], qa[ks], b0, b1);  // keys 0-7
         mma_f16(s[1], qa[ks], b2, b3);  // keys 8-15
     }
+}
+// O += P.V of an f16 tile
+template <int D>
+__device__ __forceinline__ void mma_values(unsigned vt, const unsigned (&pa)[4], float (&o)[D / 8][4], unsigned v_off) {
+#pragma unroll
+    for (int j = 0; j < D / 16; j++) {
+        unsigned b0, b1, b2, b3;
+        ldsm_x4_t(vt + v_off + j * 32, b0, b1, b2, b3);
+        mma_f16(o[2 * j], pa, b0, b1);      // dims 16 j .. 16 j + 7
+        mma_f16(o[2 * j + 1], pa, b2, b3);  // dims 16 j + 8 .. 16 j + 15
+    }
+}
+// Online softmax of one tile (keys 16 t ..) on the accumulator fragments of the warp's 16 query columns; pa: P as A fragments; the rows of O are
+// rescaled.  Without WIDE the columns 8 .. 15 do not exist: their P is 0.
+template <int D, bool WIDE>
+__device__ __forceinline__ void mma_softmax(float (&s)[2][4], int t, unsigned (&pa)[4], float (&m)[2], float (&l)[2], float (&o)[D / 8][4],
+                                            const unsigned char *const (&mrow)[2], const float (&slope)[2], float scale, float softcap, int n_kv,
+                                            bool mask_al4, int t4) {
+    constexpr int KS = D / 16;
+    constexpr float LOG2E = 1.4426950408889634f;
     // s[nb][2 hh + e]: column g + 8 hh, key 16 t + 8 nb + 2 t4 + e
     const int key0 = t * FM_TP + 2 * t4;
     float tmax[2];
 #pragma unroll
     for (int hh = 0; hh < 2; hh++) {
+        if (hh == 1 && !WIDE) continue;
 #pragma unroll
         for (int nb = 0; nb < 2; nb++) {
             const int key = key0 + 8 * nb;
@@ -232,10 +307,14 @@ __device__ __forceinline__ void mma_tile_step(unsigned kt, unsigned vt, int t, c
         mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
         tmax[hh] = mx;
     }
-    unsigned pa[4];
     float alpha[2];
 #pragma unroll
     for (int hh = 0; hh < 2; hh++) {
+        if (hh == 1 && !WIDE) {
+            pa[1] = pa[3] = 0u;
+            alpha[1] = 1.0f;
+            continue;
+        }
         const float mn = fmaxf(m[hh], tmax[hh]);
         const float mb = mn == -INFINITY ? 0.f : mn * LOG2E;
         alpha[hh] = mn == -INFINITY ? 1.0f : exp2f(m[hh] * LOG2E - mb);
@@ -255,16 +334,9 @@ __device__ __forceinline__ void mma_tile_step(unsigned kt, unsigned vt, int t, c
             o[i][2] *= alpha[1]; o[i][3] *= alpha[1];
         }
     }
-#pragma unroll
-    for (int j = 0; j < KS; j++) {
-        unsigned b0, b1, b2, b3;
-        ldsm_x4_t(vt + v_off + j * 32, b0, b1, b2, b3);
-        mma_f16(o[2 * j], pa, b0, b1);      // dims 16 j .. 16 j + 7
-        mma_f16(o[2 * j + 1], pa, b2, b3);  // dims 16 j + 8 .. 16 j + 15
-    }
 }
 
-template <int TYPE, int D>
+template <int TYPE, int D, bool WIDE>  // WIDE: more than 8 query columns a CTA
 __global__ void __launch_bounds__(FM_NW * 32, 2) fattn_mma_kernel(const __grid_constant__ FaParams p) {
     using G = MmaGeo<TYPE, D>;
     constexpr bool Q8 = G::Q8;
@@ -313,8 +385,9 @@ __global__ void __launch_bounds__(FM_NW * 32, 2) fattn_mma_kernel(const __grid_c
         for (int s = 0; s < KS; s++) {
             qraw[hh][s][0] = qraw[hh][s][1] = make_float2(0.f, 0.f);
             if (ok) {
-                qraw[hh][s][0] = __ldcg(reinterpret_cast<const float2 *>(qrow + 16 * s + 2 * t4));
-                qraw[hh][s][1] = __ldcg(reinterpret_cast<const float2 *>(qrow + 16 * s + 8 + 2 * t4));
+                // (q8_0: four neighbours, see mma_scores_q8)
+                qraw[hh][s][0] = __ldcg(reinterpret_cast<const float2 *>(qrow + 16 * s + (Q8 && !G::Q4 ? 4 : 2) * t4));
+                qraw[hh][s][1] = __ldcg(reinterpret_cast<const float2 *>(qrow + 16 * s + (Q8 && !G::Q4 ? 2 + 4 * t4 : 8 + 2 * t4)));
             }
         }
     }
@@ -440,20 +513,25 @@ __global__ void __launch_bounds__(FM_NW * 32, 2) fattn_mma_kernel(const __grid_c
             cbuf = cbuf + 1 == FM_NBUF ? 0 : cbuf + 1;
             continue;
         }
-        unsigned kt, vt;
-        if constexpr (Q8) {
-            const unsigned char *rk = my_tiles + (size_t)cbuf * 2 * G::RING_TILE;
-            mma_dequant_tile_q8<TYPE, D>(my_f16, rk, lane);
-            mma_dequant_tile_q8<TYPE, D>(my_f16 + G::TILE_BYTES, rk + G::RING_TILE, lane);
-            __syncwarp();
-            kt = smem_u32(my_f16);
-            vt = kt + G::TILE_BYTES;
+        float s[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
+        unsigned pa[4];
+        const unsigned char *raw = my_tiles + (size_t)cbuf * 2 * G::RING_TILE;
+        if constexpr (Q8 && !G::Q4) {
+            mma_scores_q8<D>(raw, qa, s, g, t4);
+            mma_softmax<D, WIDE>(s, t, pa, m, l, o, mrow, slope, scale, p.softcap, p.n_kv, mask_al4, t4);
+            mma_values_q8<D>(raw + G::RING_TILE, pa, o, g, t4);
         } else {
-            kt = smem_u32(my_tiles + (size_t)cbuf * 2 * G::RING_TILE);
-            vt = kt + G::TILE_BYTES;
+            unsigned kt = smem_u32(raw);
+            if constexpr (G::Q4) {
+                mma_dequant_tile_q4<TYPE, D>(my_f16, raw, lane);
+                mma_dequant_tile_q4<TYPE, D>(my_f16 + G::TILE_BYTES, raw + G::RING_TILE, lane);
+                __syncwarp();
+                kt = smem_u32(my_f16);
+            }
+            mma_scores<D>(kt, qa, s, k_off);
+            mma_softmax<D, WIDE>(s, t, pa, m, l, o, mrow, slope, scale, p.softcap, p.n_kv, mask_al4, t4);
+            mma_values<D>(kt + G::TILE_BYTES, pa, o, v_off);
         }
-
-        mma_tile_step<D>(kt, vt, t, qa, m, l, o, mrow, slope, scale, p.softcap, p.n_kv, mask_al4, k_off, v_off, t4);
         __syncwarp();  // all lanes are done with this buffer before it is refilled two iterations from now
         cbuf = cbuf + 1 == FM_NBUF ? 0 : cbuf + 1;
     }
@@ -475,7 +553,13 @@ __global__ void __launch_bounds__(FM_NW * 32, 2) fattn_mma_kernel(const __grid_c
         if (c < ncol) {
             float *orow = red + ((size_t)warp * C + c) * RS;
 #pragma unroll
-            for (int i = 0; i < 2 * KS; i++) *reinterpret_cast<float2 *>(orow + 8 * i + 2 * t4) = make_float2(o[i][2 * hh], o[i][2 * hh + 1]);
+            for (int i = 0; i < 2 * KS; i++) {
+                if constexpr (Q8 && !G::Q4) { if (i % 4 == 0) {  // (the dims as mma_values_q8 lays them)
+#pragma unroll
+                    for (int e = 0; e < 2; e++)
+                        *reinterpret_cast<float4 *>(orow + 8 * i + 8 * t4 + 4 * e) = make_float4(o[i][2 * hh + e], o[i + 1][2 * hh + e], o[i + 2][2 * hh + e], o[i + 3][2 * hh + e]);
+                } } else *reinterpret_cast<float2 *>(orow + 8 * i + 2 * t4) = make_float2(o[i][2 * hh], o[i][2 * hh + 1]);
+            }
             if (t4 == 0) { orow[D] = m[hh]; orow[D + 1] = l[hh]; }
         }
     }

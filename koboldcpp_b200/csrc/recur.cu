@@ -78,7 +78,7 @@ __global__ void __launch_bounds__(128) short_conv_kernel(const b200_short_conv_a
 // What bounds it: the chain S -> sums -> u -> S of a token, and the shared-memory pipe (a 16-byte load of a warp takes four of its cycles however
 // few addresses differ).  So every q and k piece that is loaded serves two columns, the four warps that carry the state do nothing else, and
 // four more warps prepare the next chunk of tokens meanwhile: q and k as unit vectors (q scaled), q.k, the decay and beta once per token.  512
-// tokens, 32 heads of 128 x 128: 183 us with one column a lane, eight warps that staged and scanned in turn, and unpacked arithmetic; 134 us here.
+// tokens, 32 heads of 128 x 128: 183 us with one column a lane, eight warps that staged and scanned in turn, and unpacked arithmetic; 139 us here.
 // CHAN: the decay is one factor per key channel (row of S) instead of one per head.  The old column is multiplied by it first, then
 // ks, qs are sums over the decayed column and  o_j = qs + (q.k) u_j;  the factors of a chunk are staged like q and k.
 constexpr int DR_CW = 4, DR_CPL = 2, DR_WARPS = 4, DR_COLS = DR_CW * DR_CPL * DR_WARPS;
