@@ -3,7 +3,7 @@
 //   dst[n][m] = sum_k W[m][k] * X[n][k],  W quantised (Q4_0, Q8_0, Q4_K, Q5_K, Q6_K), X f32, any N.
 //
 // Replaces ggml_cuda_op_mul_mat_q / mul_mat_q<type,...> (mma.sync m16n8k32 int8 tiles with ALU-side unpack and two CTA
-// barriers per 128-K half step, /root/reference/ggml/src/ggml-cuda/mmq.cuh:2495-2905) and the cuBLAS dequantise-then-GEMM
+// barriers per 128-K half step, ggml/src/ggml-cuda/mmq.cuh:2495-2905) and the cuBLAS dequantise-then-GEMM
 // fallback that koboldcpp uses by default (ggml-cuda.cu:1186-1284: whole-tensor dequant to f16 in HBM, then cublasGemmEx).
 //
 // B200 design (the one dense contraction of the path: tensor-pipe bound once N is a few hundred):
@@ -789,7 +789,7 @@ static int mmq_dispatch_bn(const MmqParams &p, cudaStream_t st) {
 
 
 // ================================================================ (a9) MUL_MAT_ID for batches: group by expert on the device
-// Replaces the batch branch of ggml_cuda_mul_mat_id (/root/reference/ggml/src/ggml-cuda.cu:2066-2139: ids copied to the host +
+// Replaces the batch branch of ggml_cuda_mul_mat_id (ggml/src/ggml-cuda.cu:2066-2139: ids copied to the host +
 // stream sync, then per expert k_copy_src1_to_contiguous -> mul_mat -> k_copy_dst_from_contiguous, :1954-2001).  Here nothing
 // leaves the device: one small kernel counts the (token, slot) pairs per expert, prefix-sums them, writes the sorted row lists and
 // the tile table; a gather pass converts the selected activation rows to bf16 in sorted order; ONE grouped tensor-core launch
