@@ -95,6 +95,8 @@ __device__ __forceinline__ unsigned long long dr_mul(unsigned long long x, unsig
     asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(x), "l"(y));
     return r;
 }
+// the meeting of both roles: all warps of the CTA, from whichever branch they come (__syncthreads() wants one place for all threads)
+__device__ __forceinline__ void dr_meet() { asm volatile("bar.sync 1, %0;" ::"n"(DR_WARPS * 64) : "memory"); }
 template <int DQ, bool CHAN>  // float4 groups per lane: dim <= 32 DQ
 __global__ void __launch_bounds__(DR_WARPS * 64) delta_rule_scan_kernel(const b200_delta_rule_args a) {
     constexpr int DP = 32 * DQ, DR_CHUNK = dr_chunk<DQ, CHAN>();
@@ -162,7 +164,7 @@ __global__ void __launch_bounds__(DR_WARPS * 64) delta_rule_scan_kernel(const b2
                     }
                 }
             }
-            __syncthreads();  // chunk c is ready; chunk c - 1, whose room the next one takes, has been read
+            dr_meet();  // chunk c is ready; chunk c - 1, whose room the next one takes, has been read
         }
         return;
     }
@@ -184,7 +186,7 @@ __global__ void __launch_bounds__(DR_WARPS * 64) delta_rule_scan_kernel(const b2
     float *out = a.dst + (int64_t)first * a.dst_stride + (int64_t)h * V + cb + lc;
     for (int ch = 0; ch < n_chunks; ch++) {
         const int nt = min(DR_CHUNK, count - ch * DR_CHUNK), buf = ch & 1;
-        __syncthreads();
+        dr_meet();
         // unrolled so that the shared-memory loads of the following tokens are issued ahead of the chain S -> sums -> u -> S
 #pragma unroll 2
         for (int tt = 0; tt < nt; tt++) {
