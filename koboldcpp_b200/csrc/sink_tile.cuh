@@ -5,13 +5,15 @@
 // one of the query heads that share the keys, 16 columns a warp.  sink_attn_mma_kernel, which needs no workspace, converts every tile for every query head
 // and block of 64 tokens, with its loads in front of its products: 214 us for 512 tokens behind 512, 32 heads over 8 of 128; both launches here
 // take 70.  Bound by instruction issue (scores, exponentials), as fattn_mma_prefill_kernel, whose tile step this is.
-// Whether a tile is seen wholly, partly or not at all follows from the positions of the warp's tokens (their smallest and largest) when they
-// belong to one sequence; only partly seen tiles, and those with a soft cap or a distance bias, go value by value.
+// Whether half a tile is seen wholly, partly or not at all follows from the positions of the warp's tokens (their smallest and largest) when they
+// belong to one sequence; only partly seen halves, and those with a soft cap or a distance bias, go value by value.
+// A softmax step is 32 cells, half a tile: the running maximum and with it the bf16 roundings of the weights are those of sink_attn_mma_kernel,
+// and cells of a half that none of the warp's tokens sees stay out of its products, whatever they hold.
 #pragma once
 
 namespace b200 {
 
-constexpr int ST_CELLS = 64, ST_COLS = 64, ST_WARPS = 4, ST_NBUF = 3;
+constexpr int ST_CELLS = 64, ST_STEP = 32, ST_COLS = 64, ST_WARPS = 4, ST_NBUF = 3;
 
 __device__ __forceinline__ float st_ex2(float x) { float y; asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x)); return y; }
 
@@ -47,7 +49,7 @@ __global__ void __launch_bounds__(256) sink_rows_bf16_kernel(const b200_sink_att
 
 template <int KS, int VS>
 __global__ void __launch_bounds__(ST_WARPS * 32, 2) sink_attn_tile_kernel(const b200_sink_attn_args a, const unsigned char *__restrict__ kd, const unsigned char *__restrict__ vd, int64_t cells) {
-    constexpr int KROW = KS * 32, VROW = VS * 32, KSTRIDE = KROW + 16, VSTRIDE = VROW + 16, KTILE = ST_CELLS * KSTRIDE, STAGE = KTILE + ST_CELLS * VSTRIDE, NB = ST_CELLS / 8;
+    constexpr int KROW = KS * 32, VROW = VS * 32, KSTRIDE = KROW + 16, VSTRIDE = VROW + 16, KTILE = ST_CELLS * KSTRIDE, STAGE = KTILE + ST_CELLS * VSTRIDE, NB = ST_STEP / 8;
     constexpr float LOG2E = 1.4426950408889634f;
     extern __shared__ __align__(128) unsigned char st_smem[];
     __shared__ int cseq[ST_NBUF][ST_CELLS], cpos[ST_NBUF][ST_CELLS];
@@ -70,31 +72,36 @@ __global__ void __launch_bounds__(ST_WARPS * 32, 2) sink_attn_tile_kernel(const 
     const int lo_start = sa_chunk_start(lo_pos, a.chunk), hi_start = sa_chunk_start(hi_pos, a.chunk);
     const int rs0 = __shfl_sync(0xffffffffu, my_seq, g), rp0 = __shfl_sync(0xffffffffu, my_pos, g), rl0 = sa_chunk_start(rp0, a.chunk);
     const int rs1 = __shfl_sync(0xffffffffu, my_seq, g + 8), rp1 = __shfl_sync(0xffffffffu, my_pos, g + 8), rl1 = sa_chunk_start(rp1, a.chunk);
-    enum { WHOLE = 0, PART = 1, HIDDEN = 2 };
-    auto tile_kind = [&](int t) {  // lane looks at cells lane and lane + 32
-        bool all = true, none = true;
+    enum { WHOLE = 0, PART = 1, HIDDEN = 2, BOTH_HIDDEN = HIDDEN | HIDDEN << 2 };
+    auto tile_kinds = [&](int t) {  // of the tile's halves, two bits each; lane looks at cells lane and lane + 32
+        int kinds = 0;
 #pragma unroll
         for (int i = 0; i < 2; i++) {
             const int64_t c = (int64_t)t * ST_CELLS + lane + 32 * i;
             int cs = -1, cp = 0;
             if (c < a.n_kv) { cs = a.cell_seq[c]; cp = a.cell_pos[c]; }
+            bool all, none;
             if (!uniform) {  // any token of this cell's sequence?
                 all = false;
-                none = none && cs < 0;
-                continue;
+                none = cs < 0;
+            } else {
+                all = cs == seq0 && cs >= 0 && cp <= lo_pos && cp >= hi_start && (a.window <= 0 || hi_pos - cp < a.window || cp < a.keep_first);
+                none = cs != seq0 || cs < 0 || cp > hi_pos || cp < lo_start || (a.window > 0 && lo_pos - cp >= a.window && cp >= a.keep_first);
             }
-            all = all && cs == seq0 && cs >= 0 && cp <= lo_pos && cp >= hi_start && (a.window <= 0 || hi_pos - cp < a.window || cp < a.keep_first);
-            none = none && (cs != seq0 || cs < 0 || cp > hi_pos || cp < lo_start || (a.window > 0 && lo_pos - cp >= a.window && cp >= a.keep_first));
+            const bool hidden = __all_sync(0xffffffffu, none), whole = __all_sync(0xffffffffu, all);
+            kinds |= (hidden ? HIDDEN : whole ? WHOLE : PART) << (2 * i);
         }
-        if (__all_sync(0xffffffffu, none)) return (int)HIDDEN;
-        return __all_sync(0xffffffffu, all) ? (int)WHOLE : (int)PART;
+        return ncol > 0 ? kinds : (int)BOTH_HIDDEN;
     };
 
-    // the CTA's next tile that one of its warps sees: the same for all threads
+    // the CTA's next tile that one of its warps sees: the same for all threads; what this warp sees of it
     int next = 0;
-    auto advance = [&]() {
-        while (next < n_tiles && !__syncthreads_or(ncol > 0 && tile_kind(next) != HIDDEN)) next++;
-        return next < n_tiles ? next++ : -1;
+    auto advance = [&](int &kinds) {
+        for (; next < n_tiles; next++) {
+            kinds = tile_kinds(next);
+            if (__syncthreads_or(kinds != BOTH_HIDDEN)) return next++;
+        }
+        return -1;
     };
     auto load_stage = [&](int t, int st) {
         if (t >= 0) {
@@ -112,9 +119,9 @@ __global__ void __launch_bounds__(ST_WARPS * 32, 2) sink_attn_tile_kernel(const 
         }
         cp_async_commit();
     };
-    int ahead[ST_NBUF];  // tiles in the ring, oldest first
+    int ahead[ST_NBUF], seen[ST_NBUF];  // tiles in the ring, oldest first, and their kinds
 #pragma unroll
-    for (int i = 0; i < ST_NBUF - 1; i++) { ahead[i] = advance(); load_stage(ahead[i], i); }
+    for (int i = 0; i < ST_NBUF - 1; i++) { ahead[i] = advance(seen[i]); load_stage(ahead[i], i); }
 
     // queries as bf16 A fragments, straight from the f32 rows
     unsigned qa[KS][4];
@@ -147,100 +154,105 @@ __global__ void __launch_bounds__(ST_WARPS * 32, 2) sink_attn_tile_kernel(const 
 
     int stage = 0;
     for (;;) {
-        const int t = ahead[0];
-        if (t < 0) break;
+        if (ahead[0] < 0) break;
+        const int kinds = seen[0];
+        int kinds_n = BOTH_HIDDEN;
         cp_async_wait<ST_NBUF - 2>();
-        const int tn = advance();  // (its barriers: the tile has landed for everybody, and everybody is done with the one before)
+        const int tn = advance(kinds_n);  // (its barriers: the tile has landed for everybody, and everybody is done with the one before)
         __syncthreads();
 #pragma unroll
-        for (int i = 0; i < ST_NBUF - 2; i++) ahead[i] = ahead[i + 1];
+        for (int i = 0; i < ST_NBUF - 2; i++) { ahead[i] = ahead[i + 1]; seen[i] = seen[i + 1]; }
         ahead[ST_NBUF - 2] = tn;
+        seen[ST_NBUF - 2] = kinds_n;
         load_stage(tn, stage == 0 ? ST_NBUF - 1 : stage - 1);
         const int st = stage;
         stage = stage + 1 == ST_NBUF ? 0 : stage + 1;
-        const int kind = ncol > 0 ? tile_kind(t) : (int)HIDDEN;
-        if (kind == HIDDEN) continue;
-        const unsigned kt = smem_u32(st_smem + (size_t)st * STAGE), vt = kt + KTILE;
-        float s[NB][4];
+#pragma unroll 1
+        for (int half = 0; half < ST_CELLS / ST_STEP; half++) {
+            const int kind = kinds >> (2 * half) & 3, x0 = half * ST_STEP;
+            if (kind == HIDDEN) continue;
+            const unsigned kt = smem_u32(st_smem + (size_t)st * STAGE) + (unsigned)(x0 * KSTRIDE), vt = smem_u32(st_smem + (size_t)st * STAGE) + KTILE + (unsigned)(x0 * VSTRIDE);
+            float s[NB][4];
 #pragma unroll
-        for (int j = 0; j < NB; j++) s[j][0] = s[j][1] = s[j][2] = s[j][3] = 0.f;
+            for (int j = 0; j < NB; j++) s[j][0] = s[j][1] = s[j][2] = s[j][3] = 0.f;
 #pragma unroll
-        for (int ks = 0; ks < KS; ks++) {
+            for (int ks = 0; ks < KS; ks++) {
 #pragma unroll
-            for (int j = 0; j < NB / 2; j++) {
-                unsigned b0, b1, b2, b3;
-                gm_ldsm4(kt + k_off + (unsigned)(j * 16 * KSTRIDE) + ks * 32, b0, b1, b2, b3);
-                gm_mma_bf16(s[2 * j], qa[ks], b0, b1);
-                gm_mma_bf16(s[2 * j + 1], qa[ks], b2, b3);
-            }
-        }
-        // s[j][2 hh + e]: column g + 8 hh, cell 8 j + 2 t4 + e.  `c` takes raw products to scaled scores times log2 e inside the exponent's FMA
-        float c = a.scale * LOG2E;
-        if (kind == PART || !plain) {
-#pragma unroll
-            for (int j = 0; j < NB; j++) {
-#pragma unroll
-                for (int e = 0; e < 2; e++) {
-                    const int x = 8 * j + 2 * t4 + e, xs = cseq[st][x], xp = cpos[st][x];
-                    const bool v0 = xs >= 0 && sa_visible(xs, xp, rs0, rp0, a.window, a.keep_first, rl0), v1 = xs >= 0 && sa_visible(xs, xp, rs1, rp1, a.window, a.keep_first, rl1);
-                    float s0 = s[j][e] * a.scale, s1 = s[j][2 + e] * a.scale;
-                    if (a.softcap > 0.f) { s0 = sa_cap_fast(s0, a.softcap, two_over_cap); s1 = sa_cap_fast(s1, a.softcap, two_over_cap); }
-                    if (a.dist_bias) {
-                        if (v0) s0 += sa_dist_bias(a, rp0 - xp, hd[0], lin[0]);
-                        if (v1) s1 += sa_dist_bias(a, rp1 - xp, hd[1], lin[1]);
-                    }
-                    s[j][e] = v0 ? (sig ? s0 : s0 * LOG2E) : -INFINITY;
-                    s[j][2 + e] = v1 ? (sig ? s1 : s1 * LOG2E) : -INFINITY;
+                for (int j = 0; j < NB / 2; j++) {
+                    unsigned b0, b1, b2, b3;
+                    gm_ldsm4(kt + k_off + (unsigned)(j * 16 * KSTRIDE) + ks * 32, b0, b1, b2, b3);
+                    gm_mma_bf16(s[2 * j], qa[ks], b0, b1);
+                    gm_mma_bf16(s[2 * j + 1], qa[ks], b2, b3);
                 }
             }
-            c = 1.0f;
-        }
-        if (sig) {  // every visible key's weight is the sigmoid of its own score (0 for the others: the sigmoid of -inf)
-#pragma unroll
-            for (int j = 0; j < NB; j++) {
-#pragma unroll
-                for (int e = 0; e < 4; e++) s[j][e] = sa_sigmoid_fast(s[j][e]);
-            }
-        } else {
-            float alpha[2];
-#pragma unroll
-            for (int hh = 0; hh < 2; hh++) {
-                float mx = fmaxf(s[0][2 * hh], s[0][2 * hh + 1]);
-#pragma unroll
-                for (int j = 1; j < NB; j++) mx = fmaxf(mx, fmaxf(s[j][2 * hh], s[j][2 * hh + 1]));
-                mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
-                mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
-                const float mn = fmaxf(m[hh], mx * c), mb = mn == -INFINITY ? 0.f : mn;  // (nothing seen yet: 2^-inf = 0 throughout)
-                alpha[hh] = mn == -INFINITY ? 1.0f : st_ex2(m[hh] - mb);
-                m[hh] = mn;
-                float sum0 = 0.f, sum1 = 0.f;
+            // s[j][2 hh + e]: column g + 8 hh, cell x0 + 8 j + 2 t4 + e.  `c` takes raw products to scaled scores times log2 e inside the exponent's FMA
+            float c = a.scale * LOG2E;
+            if (kind == PART || !plain) {
 #pragma unroll
                 for (int j = 0; j < NB; j++) {
-                    s[j][2 * hh] = st_ex2(fmaf(s[j][2 * hh], c, -mb));
-                    s[j][2 * hh + 1] = st_ex2(fmaf(s[j][2 * hh + 1], c, -mb));
-                    sum0 += s[j][2 * hh];
-                    sum1 += s[j][2 * hh + 1];
+#pragma unroll
+                    for (int e = 0; e < 2; e++) {
+                        const int x = x0 + 8 * j + 2 * t4 + e, xs = cseq[st][x], xp = cpos[st][x];
+                        const bool v0 = xs >= 0 && sa_visible(xs, xp, rs0, rp0, a.window, a.keep_first, rl0), v1 = xs >= 0 && sa_visible(xs, xp, rs1, rp1, a.window, a.keep_first, rl1);
+                        float s0 = s[j][e] * a.scale, s1 = s[j][2 + e] * a.scale;
+                        if (a.softcap > 0.f) { s0 = sa_cap_fast(s0, a.softcap, two_over_cap); s1 = sa_cap_fast(s1, a.softcap, two_over_cap); }
+                        if (a.dist_bias) {
+                            if (v0) s0 += sa_dist_bias(a, rp0 - xp, hd[0], lin[0]);
+                            if (v1) s1 += sa_dist_bias(a, rp1 - xp, hd[1], lin[1]);
+                        }
+                        s[j][e] = v0 ? (sig ? s0 : s0 * LOG2E) : -INFINITY;
+                        s[j][2 + e] = v1 ? (sig ? s1 : s1 * LOG2E) : -INFINITY;
+                    }
                 }
-                l[hh] = l[hh] * alpha[hh] + (sum0 + sum1);
+                c = 1.0f;
             }
-            if (__any_sync(0xffffffffu, alpha[0] != 1.0f || alpha[1] != 1.0f)) {
+            if (sig) {  // every visible key's weight is the sigmoid of its own score (0 for the others: the sigmoid of -inf)
 #pragma unroll
-                for (int i = 0; i < 2 * VS; i++) {
-                    o[i][0] *= alpha[0]; o[i][1] *= alpha[0];
-                    o[i][2] *= alpha[1]; o[i][3] *= alpha[1];
+                for (int j = 0; j < NB; j++) {
+#pragma unroll
+                    for (int e = 0; e < 4; e++) s[j][e] = sa_sigmoid_fast(s[j][e]);
+                }
+            } else {
+                float alpha[2];
+#pragma unroll
+                for (int hh = 0; hh < 2; hh++) {
+                    float mx = fmaxf(s[0][2 * hh], s[0][2 * hh + 1]);
+#pragma unroll
+                    for (int j = 1; j < NB; j++) mx = fmaxf(mx, fmaxf(s[j][2 * hh], s[j][2 * hh + 1]));
+                    mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
+                    mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
+                    const float mn = fmaxf(m[hh], mx * c), mb = mn == -INFINITY ? 0.f : mn;  // (nothing seen yet: 2^-inf = 0 throughout)
+                    alpha[hh] = mn == -INFINITY ? 1.0f : st_ex2(m[hh] - mb);
+                    m[hh] = mn;
+                    float sum0 = 0.f, sum1 = 0.f;
+#pragma unroll
+                    for (int j = 0; j < NB; j++) {
+                        s[j][2 * hh] = st_ex2(fmaf(s[j][2 * hh], c, -mb));
+                        s[j][2 * hh + 1] = st_ex2(fmaf(s[j][2 * hh + 1], c, -mb));
+                        sum0 += s[j][2 * hh];
+                        sum1 += s[j][2 * hh + 1];
+                    }
+                    l[hh] = l[hh] * alpha[hh] + (sum0 + sum1);
+                }
+                if (__any_sync(0xffffffffu, alpha[0] != 1.0f || alpha[1] != 1.0f)) {
+#pragma unroll
+                    for (int i = 0; i < 2 * VS; i++) {
+                        o[i][0] *= alpha[0]; o[i][1] *= alpha[0];
+                        o[i][2] *= alpha[1]; o[i][3] *= alpha[1];
+                    }
                 }
             }
-        }
 #pragma unroll
-        for (int kk = 0; kk < ST_CELLS / 16; kk++) {
-            const unsigned pa[4] = {gm_pack_bf2(s[2 * kk][0], s[2 * kk][1]), gm_pack_bf2(s[2 * kk][2], s[2 * kk][3]), gm_pack_bf2(s[2 * kk + 1][0], s[2 * kk + 1][1]),
-                                    gm_pack_bf2(s[2 * kk + 1][2], s[2 * kk + 1][3])};
+            for (int kk = 0; kk < ST_STEP / 16; kk++) {
+                const unsigned pa[4] = {gm_pack_bf2(s[2 * kk][0], s[2 * kk][1]), gm_pack_bf2(s[2 * kk][2], s[2 * kk][3]), gm_pack_bf2(s[2 * kk + 1][0], s[2 * kk + 1][1]),
+                                        gm_pack_bf2(s[2 * kk + 1][2], s[2 * kk + 1][3])};
 #pragma unroll
-            for (int j = 0; j < VS; j++) {
-                unsigned b0, b1, b2, b3;
-                gm_ldsm4_t(vt + v_off + (unsigned)(kk * 16 * VSTRIDE) + j * 32, b0, b1, b2, b3);
-                gm_mma_bf16(o[2 * j], pa, b0, b1);
-                gm_mma_bf16(o[2 * j + 1], pa, b2, b3);
+                for (int j = 0; j < VS; j++) {
+                    unsigned b0, b1, b2, b3;
+                    gm_ldsm4_t(vt + v_off + (unsigned)(kk * 16 * VSTRIDE) + j * 32, b0, b1, b2, b3);
+                    gm_mma_bf16(o[2 * j], pa, b0, b1);
+                    gm_mma_bf16(o[2 * j + 1], pa, b2, b3);
+                }
             }
         }
     }
