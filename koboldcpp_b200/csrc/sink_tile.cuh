@@ -6,7 +6,7 @@
 // and block of 64 tokens, with its loads in front of its products: 214 us for 512 tokens behind 512, 32 heads over 8 of 128; both launches here
 // take 70.  Bound by instruction issue (scores, exponentials), as fattn_mma_prefill_kernel, whose tile step this is.
 // Whether half a tile is seen wholly, partly or not at all follows from the positions of the warp's tokens (their smallest and largest) when they
-// belong to one sequence; only partly seen halves, and those with a soft cap or a distance bias, go value by value.
+// belong to one sequence, else token by token; only partly seen halves, and those with a soft cap or a distance bias, go value by value.
 // A softmax step is 32 cells, half a tile: the running maximum and with it the bf16 roundings of the weights are those of sink_attn_mma_kernel,
 // and cells of a half that none of the warp's tokens sees stay out of its products, whatever they hold.
 #pragma once
@@ -63,6 +63,7 @@ __global__ void __launch_bounds__(ST_WARPS * 32, 2) sink_attn_tile_kernel(const 
     // the columns' tokens: lane i < 16 holds column i; the warp's one sequence (or not) and its range of positions
     int my_seq = -2, my_pos = 0;
     if (lane < ncol) { const int t = (col0 + lane) / gqa; my_seq = a.tok_seq[t]; my_pos = a.tok_pos[t]; }
+    const int my_start = sa_chunk_start(my_pos, a.chunk);
     const int seq0 = __shfl_sync(0xffffffffu, my_seq, 0);
     const bool uniform = __all_sync(0xffffffffu, lane >= ncol || my_seq == seq0);
     int lo_pos = lane < ncol ? my_pos : 0x7fffffff, hi_pos = lane < ncol ? my_pos : -0x7fffffff;
@@ -81,9 +82,14 @@ __global__ void __launch_bounds__(ST_WARPS * 32, 2) sink_attn_tile_kernel(const 
             int cs = -1, cp = 0;
             if (c < a.n_kv) { cs = a.cell_seq[c]; cp = a.cell_pos[c]; }
             bool all, none;
-            if (!uniform) {  // any token of this cell's sequence?
-                all = false;
-                none = cs < 0;
+            if (!uniform) {  // token by token: its columns follow one another
+                all = none = true;
+                for (int i = 0; i < ncol; i += gqa - (col0 + i) % gqa) {
+                    const int ts = __shfl_sync(0xffffffffu, my_seq, i), tp = __shfl_sync(0xffffffffu, my_pos, i), tl = __shfl_sync(0xffffffffu, my_start, i);
+                    const bool v = cs >= 0 && sa_visible(cs, cp, ts, tp, a.window, a.keep_first, tl);
+                    all = all && v;
+                    none = none && !v;
+                }
             } else {
                 all = cs == seq0 && cs >= 0 && cp <= lo_pos && cp >= hi_start && (a.window <= 0 || hi_pos - cp < a.window || cp < a.keep_first);
                 none = cs != seq0 || cs < 0 || cp > hi_pos || cp < lo_start || (a.window > 0 && lo_pos - cp >= a.window && cp >= a.keep_first);

@@ -162,3 +162,24 @@ def test_hidden_group_of_32_cells_beside_a_visible_one():
     k[other], v[other] = 0.0, 0.0
     exact = oracle({}, q, k, v, cell_seq, cell_pos, tok_seq, tok_pos, Hh, G, D, D, {})
     assert np.linalg.norm(got - exact) < 2.3e-3 * np.linalg.norm(exact)
+
+
+def test_tokens_of_many_sequences_in_turn():
+    """Columns of one warp that belong to several sequences: what it sees of a half tile follows from its own tokens, not from whether cells are in use."""
+    T, Hh, G, D, n_seq, each = 192, 16, 16, 64, 6, 128
+    rng = np.random.default_rng(21)
+    cells = n_seq * each
+    q, k, v = (rng.standard_normal((n, w * D)).astype(np.float32) for n, w in ((T, Hh), (cells, G), (cells, G)))
+    cell_seq, cell_pos = (np.arange(cells) // each).astype(np.int32), (np.arange(cells) % each).astype(np.int32)
+    # tokens 0 .. 95: sequences 0 and 1 in turn; 96 .. 191: 2 to 5 in turn
+    tok_seq = np.where(np.arange(T) < 96, np.arange(T) % 2, 2 + np.arange(T) % 4).astype(np.int32)
+    tok_pos = np.where(np.arange(T) < 96, np.arange(T) // 2 + each - 48, (np.arange(T) - 96) // 4 + each - 24).astype(np.int32)
+    for f in ({}, {"window": 30}, {"chunk": 64}):
+        got = run_plain(q, k, v, cell_seq, cell_pos, tok_seq, tok_pos, Hh, G, D, window=f.get("window", 0), chunk=f.get("chunk", 0))
+        exact = oracle(f, q, k, v, cell_seq, cell_pos, tok_seq, tok_pos, Hh, G, D, D, {})
+        assert np.linalg.norm(got - exact) < 2.3e-3 * np.linalg.norm(exact)
+    # what sequences 2 to 5 hold does not reach the first tokens' results
+    other = cell_seq >= 2
+    k[other], v[other] = np.inf, np.nan
+    got = run_plain(q, k, v, cell_seq, cell_pos, tok_seq, tok_pos, Hh, G, D)
+    assert np.isfinite(got[:96]).all()
