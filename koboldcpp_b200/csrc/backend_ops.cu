@@ -760,7 +760,16 @@ size_t node_scratch_bytes(const ggml_tensor *n) {
     if (n->op == GGML_OP_MAP_CUSTOM1 && (uint32_t)n->op_params[0] == B200_EXT_TAG && n->op_params[1] == B200_EXT_SINK_ATTN) {
         b200_sink_attn_args a;
         fill_sink_attn_args(n, a);
-        return b200_sink_attn_workspace_bytes(&a);
+        size_t need = b200_sink_attn_workspace_bytes(&a);
+        // prompt batches keep the rounded rows of all visible cells there: room for the whole cache at once, since a scratch that grew with every 256
+        // cells would move each time, and every captured graph with it
+        const ggml_tensor *cache = n->src[1]->view_src;
+        if (cache && a.n_tokens >= 16 && cache->ne[1] > a.n_kv && cache->ne[0] == n->src[1]->ne[0]) {
+            a.n_kv = (int32_t)cache->ne[1];
+            const size_t whole = b200_sink_attn_workspace_bytes(&a);
+            if (whole > need) need = whole;
+        }
+        return need;
     }
     if (n->op == GGML_OP_MAP_CUSTOM1 && (uint32_t)n->op_params[0] == B200_EXT_TAG && n->op_params[1] == B200_EXT_MUL_MAT_ID && ext_mul_mat_id_gemm_ok(n))
         return b200_mul_mat_id_q_workspace_bytes(n->src[0]->type, n->src[0]->ne[0], n->src[0]->ne[1], n->src[2]->ne[0], n->src[2]->ne[1], (int32_t)n->src[0]->ne[2]);

@@ -488,3 +488,32 @@ def test_model_folder_command_line_and_trace_runner(tmp_path, capsys):
     for n, w in want.items():
         got = np.fromfile(out / f"{n}.f32", dtype="<f4").reshape(-1, cfg["vocab"])
         assert got.shape == w.shape and logits_err(got, w) < 1e-4, n
+
+
+def test_longer_prompts_keep_captured_graphs():
+    """bf16 serving mode: the attention of a prompt keeps its rounded cache rows in the backend's scratch.  Prompts that reach further and further into
+    the cache neither move it nor drop the captured graphs of other steps: a single-token request between them is replayed each time."""
+    from koboldcpp_b200.llama import _l
+    cfg = R.make_config([R.attn_layer(heads=8, kv_heads=8, dim=64, vdim=64, rot_dims=64, chunk=700, mlp=R.dense(64))], width=64, vocab=64)
+    W = R.random_weights(cfg, seed=2)
+    m = Z.build(cfg, R.as_tensors(W), dtype="bfloat16", n_ctx=6144, n_seq_max=2, max_batch=512)
+    eng, L = Engine(m), _l()
+
+    def probe():
+        n = [C.c_int64() for _ in range(6)]
+        L.ggml_backend_b200_get_stats(*(C.byref(x) for x in n[:3]))
+        eng.step([("p", [3], [0])])
+        L.ggml_backend_b200_get_stats(*(C.byref(x) for x in n[3:]))
+        eng.finish("p")
+        return n[5].value - n[2].value  # graphs captured by the step
+
+    try:
+        captured = []
+        for length in range(1024, 5633, 512):
+            for at in range(0, length, 512):
+                eng.step([("a", [(7 * i) % 64 for i in range(at, at + 512)], [])])
+            eng.finish("a")
+            captured.append(probe())
+        assert captured[1:] == [0] * (len(captured) - 1), captured
+    finally:
+        m.close()
