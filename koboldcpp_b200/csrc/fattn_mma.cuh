@@ -713,15 +713,38 @@ __global__ void __launch_bounds__(FM_NW * 32, 2) fattn_mma_kernel(const __grid_c
 // the whole KV range -- no cross-warp merge, no splits) and the 4 warps SHARE every (K, V) tile through a CTA-wide cp.async ring.
 // What bounds it: instruction issue.  A tile is 64 keys (32 for wider heads), so that barrier, maximum, rescaling and the bookkeeping of a tile
 // are paid once per 64 keys, and two CTAs an SM hide one another's softmax: 7B, 512 tokens behind 1536: 222 us with 16-key tiles that
-// loaded the mask for every score; 84 here (121 before the common tile lost its branches and a scaling per score).  The mask is looked at 16 bytes a lane, one tile ahead: a tile whose mask is 0 throughout
-// needs no additions, one that is -inf throughout is skipped by the warp; only the diagonal goes value by value.  Tiles behind the last one
-// that any column of the CTA sees are not loaded at all.
+// loaded the mask for every score; 84 here (121 before the common tile lost its branches and a scaling per score).  The mask is looked at 16
+// bytes a lane, one tile ahead: a tile whose mask is 0 throughout needs no additions, one that is -inf throughout is skipped by the warp;
+// only the diagonal goes value by value, and there groups of 16 keys that none of the warp's columns sees are left out, whatever they hold.
+// Tiles behind the last one that any column of the CTA sees are not loaded at all.  Masks with rows at other places, and a ragged last
+// tile, are looked at value by value (mask_kind_any).
 constexpr int FP_NBUF = 3;   // stages of the CTA ring
 constexpr int FP_COLS = 64;  // query columns per CTA
 // 2^x to two ulp; results below 2^-126 become 0 (beside a sum of at least 1 they vanish)
 __device__ __forceinline__ float ex2(float x) { float y; asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x)); return y; }
 template <int D> constexpr int fp_keys() { return D > 128 ? 32 : 64; }  // keys of a tile: the scores' registers beside 2 D accumulators
 template <int D> constexpr int fp_stage_bytes() { return 2 * fp_keys<D>() * MmaGeo<B200_TYPE_F16, D>::ROW_STRIDE; }
+
+// what a warp's columns see of a tile, whatever the place of the mask's rows (keys behind n_kv count as -inf): kind (0: mask 0 throughout, 1: mixed, 2: nothing) | groups << 2,
+// bit i of groups: keys 16 i .. 16 i + 15.  Lane l looks at keys l, l + 32 of all columns.  Not inlined: its addresses would be kept over the caller's loop.
+template <int KT>
+__device__ __noinline__ unsigned mask_kind_any(const unsigned char *mask, size_t nb1, int col0, int ncol, int gqa, int n_kv, int t, int lane) {
+    unsigned groups = 0, any = 0;
+    for (int half = 0; half < KT / 32; half++) {
+        const int key = t * KT + 32 * half + lane;
+        unsigned seen = 0;
+#pragma unroll 4
+        for (int c = 0; c < ncol; c++) {
+            const unsigned h = key < n_kv ? __ldg(reinterpret_cast<const unsigned short *>(mask + (size_t)((col0 + c) / gqa) * nb1 + 2 * (size_t)key)) : 0xfc00u;
+            any |= h;
+            seen |= h ^ 0xfc00u;
+        }
+        const unsigned lanes = __ballot_sync(0xffffffffu, seen != 0u);
+        groups |= ((lanes & 0xffffu) != 0u ? 1u : 0u) << (2 * half) | ((lanes >> 16) != 0u ? 2u : 0u) << (2 * half);
+    }
+    if (!__any_sync(0xffffffffu, any != 0u)) return 0u | groups << 2;
+    return (groups == 0u ? 2u : 1u) | groups << 2;
+}
 
 template <int D>
 __global__ void __launch_bounds__(FM_NW * 32, 2) fattn_mma_prefill_kernel(const __grid_constant__ FaParams p) {
@@ -730,6 +753,7 @@ __global__ void __launch_bounds__(FM_NW * 32, 2) fattn_mma_prefill_kernel(const 
     constexpr float LOG2E = 1.4426950408889634f;
     extern __shared__ __align__(128) unsigned char smem[];
     __shared__ int last_tile[FM_NW];
+    __shared__ uint4 zeros[2 * D / 16];  // a row of values
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int g = lane >> 2, t4 = lane & 3;
@@ -756,7 +780,8 @@ __global__ void __launch_bounds__(FM_NW * 32, 2) fattn_mma_prefill_kernel(const 
             if (key + 8 <= p.n_kv) u[i] = __ldg(reinterpret_cast<const uint4 *>(p.mask + (size_t)((col0 + c) / p.gqa) * p.mask_nb1 + 2 * (size_t)key));
         }
     };
-    auto mask_kind = [&](int t, const uint4 (&u)[16 / RP]) {
+    // groups: bit i of a tile that is mixed: some column sees one of its keys 16 i .. 16 i + 15
+    auto mask_kind = [&](const uint4 (&u)[16 / RP], unsigned &groups) {
         unsigned any = 0, all = 0xffffffffu, inf = 0;
 #pragma unroll
         for (int i = 0; i < 16 / RP; i++) {
@@ -765,22 +790,38 @@ __global__ void __launch_bounds__(FM_NW * 32, 2) fattn_mma_prefill_kernel(const 
             inf |= o ^ 0xfc00fc00u;
             all &= n;
         }
-        const bool whole = (t + 1) * KT <= p.n_kv;         // a ragged last tile goes value by value
-        if (!__any_sync(0xffffffffu, any != 0u || !whole)) return (int)ZERO;
-        return __any_sync(0xffffffffu, inf != 0u || all != 0xfc00fc00u || !whole) ? (int)MIXED : (int)HIDDEN;
+        if (!__any_sync(0xffffffffu, any != 0u)) return (int)ZERO;
+        const unsigned seen = __ballot_sync(0xffffffffu, inf != 0u || all != 0xfc00fc00u);
+        if (seen == 0u) return (int)HIDDEN;
+        groups = 0;
+#pragma unroll
+        for (int i = 0; i < KT / 16; i++) groups |= (seen & (CH == 8 ? 0x03030303u : 0x33333333u) << (2 * i)) != 0u ? 1u << i : 0u;
+        return (int)MIXED;
+    };
+    auto fast = [&](int t) { return m16 && (t + 1) * KT <= p.n_kv; };
+    auto mask_kind_slow = [&](int t, unsigned &groups) {
+        const unsigned r = mask_kind_any<KT>(p.mask, p.mask_nb1, col0, ncol, p.gqa, p.n_kv, t, lane);
+        groups = r >> 2;
+        return (int)(r & 3u);
     };
     // ---- the last tile that a column of this warp sees, from the back (the causal triangle); then of the CTA
     int n_tiles = n_tiles_all;
     if (ncol == 0) n_tiles = 0;
-    else if (p.mask != nullptr && m16) {
+    else if (p.mask != nullptr) {
         while (n_tiles > 0) {
-            uint4 u[16 / RP];
-            mask_load(n_tiles - 1, u);
-            if (mask_kind(n_tiles - 1, u) != HIDDEN) break;
+            unsigned groups;
+            if (fast(n_tiles - 1)) {
+                uint4 u[16 / RP];
+                mask_load(n_tiles - 1, u);
+                if (mask_kind(u, groups) != HIDDEN) break;
+            } else if (mask_kind_slow(n_tiles - 1, groups) != HIDDEN) {
+                break;
+            }
             n_tiles--;
         }
     }
     if (lane == 0) last_tile[warp] = n_tiles;
+    if (threadIdx.x < 2 * D / 16) zeros[threadIdx.x] = make_uint4(0u, 0u, 0u, 0u);
     __syncthreads();
     const int cta_tiles = max(max(last_tile[0], last_tile[1]), max(last_tile[2], last_tile[3]));
 
@@ -832,6 +873,7 @@ __global__ void __launch_bounds__(FM_NW * 32, 2) fattn_mma_prefill_kernel(const 
             qa[s][2 + hh] = pack_h2(hi.x, hi.y);
         }
     }
+    const unsigned zeros_at = smem_u32(zeros);
     const bool mask_al4 = (((uintptr_t)p.mask | p.mask_nb1) & 3) == 0;
     const float scale = p.softcap != 0.0f ? p.scale / p.softcap : p.scale;
     float m[2] = {-INFINITY, -INFINITY}, l[2] = {0.f, 0.f};  // maximum (times log2 e) and this lane's share of the sum
@@ -842,8 +884,7 @@ __global__ void __launch_bounds__(FM_NW * 32, 2) fattn_mma_prefill_kernel(const 
     const unsigned k_off = (unsigned)(((mi >> 1) * 8 + mr) * G::ROW_STRIDE + (mi & 1) * 16);
     const unsigned v_off = (unsigned)(((mi & 1) * 8 + mr) * G::ROW_STRIDE + (mi >> 1) * 16);
     uint4 mu[16 / RP];
-    const bool looked = p.mask != nullptr && m16;
-    if (looked && n_tiles > 0) mask_load(0, mu);
+    if (p.mask != nullptr && m16 && n_tiles > 0) mask_load(0, mu);
 
     int stage = 0;
     for (int t = 0; t < cta_tiles; t++) {
@@ -853,10 +894,12 @@ __global__ void __launch_bounds__(FM_NW * 32, 2) fattn_mma_prefill_kernel(const 
         const unsigned kt = smem_u32(smem + (size_t)stage * 2 * TILE), vt = kt + TILE;
         stage = stage + 1 == FP_NBUF ? 0 : stage + 1;
         if (t >= n_tiles) continue;
-        int kind = p.mask != nullptr || (t + 1) * KT > p.n_kv ? (int)MIXED : (int)ZERO;
-        if (looked) {
-            kind = mask_kind(t, mu);
-            if (t + 1 < n_tiles) mask_load(t + 1, mu);
+        int kind = (t + 1) * KT > p.n_kv ? (int)MIXED : (int)ZERO;
+        constexpr unsigned ALL_GROUPS = (1u << (KT / 16)) - 1;
+        unsigned groups = ALL_GROUPS;
+        if (p.mask != nullptr) {
+            kind = fast(t) ? mask_kind(mu, groups) : mask_kind_slow(t, groups);
+            if (m16 && t + 1 < n_tiles) mask_load(t + 1, mu);
             if (kind == HIDDEN) continue;
         }
         float s[NB][4];
@@ -891,8 +934,8 @@ __global__ void __launch_bounds__(FM_NW * 32, 2) fattn_mma_prefill_kernel(const 
                             mf.x = __half2float(*reinterpret_cast<const __half *>(mrow[hh] + 2 * (size_t)key));
                             mf.y = key + 1 < p.n_kv ? __half2float(*reinterpret_cast<const __half *>(mrow[hh] + 2 * (size_t)key + 2)) : 0.f;
                         }
-                        s0 += slope[hh] * mf.x;
-                        s1 += slope[hh] * mf.y;
+                        s0 = mf.x == -INFINITY ? -INFINITY : s0 + slope[hh] * mf.x;  // (whatever a hidden key's row holds)
+                        s1 = mf.y == -INFINITY ? -INFINITY : s1 + slope[hh] * mf.y;
                     }
                     s[j][2 * hh] = key < p.n_kv ? s0 * LOG2E : -INFINITY;
                     s[j][2 * hh + 1] = key + 1 < p.n_kv ? s1 * LOG2E : -INFINITY;
@@ -930,12 +973,15 @@ __global__ void __launch_bounds__(FM_NW * 32, 2) fattn_mma_prefill_kernel(const 
         }
 #pragma unroll
         for (int kk = 0; kk < KT / 16; kk++) {
+            // (16 keys that no column sees: their P is 0, their values are read as zeros, whatever they hold.  A choice of address: branches or a second copy of the
+            // step take this loop from the exponentials' side and cost 15 %, masking the fragments 6 %)
+            const unsigned va = groups >> kk & 1u ? vt + v_off + (unsigned)(kk * 16 * G::ROW_STRIDE) : zeros_at;
             const unsigned pa[4] = {pack_h2(s[2 * kk][0], s[2 * kk][1]), pack_h2(s[2 * kk][2], s[2 * kk][3]), pack_h2(s[2 * kk + 1][0], s[2 * kk + 1][1]),
                                     pack_h2(s[2 * kk + 1][2], s[2 * kk + 1][3])};
 #pragma unroll
             for (int j = 0; j < KS; j++) {
                 unsigned b0, b1, b2, b3;
-                ldsm_x4_t(vt + v_off + (unsigned)(kk * 16 * G::ROW_STRIDE) + j * 32, b0, b1, b2, b3);
+                ldsm_x4_t(va + j * 32, b0, b1, b2, b3);
                 mma_f16(o[2 * j], pa, b0, b1);
                 mma_f16(o[2 * j + 1], pa, b2, b3);
             }
