@@ -208,6 +208,12 @@ B200_API int b200_gemm_status(void);
 B200_API int b200_mul_mat_q(int type, const void *W, size_t w_row_bytes, const float *X, int64_t x_stride,
                             float *dst, int64_t dst_stride, int64_t K, int64_t M, int64_t N,
                             void *workspace, size_t workspace_bytes, b200_stream_t stream);
+/* The same with the limit of each of the kernel's own waits in clock cycles (b200_mul_mat_q: about two seconds' worth), where the product runs on the
+ * paired-SM kernel (K a multiple of 256; bf16).  When one runs out the product ends early: values of dst that were stored are right, the
+ * others are as they were (zero, or short of one half of K, where K was split). */
+B200_API int b200_mul_mat_q_wait(int type, const void *W, size_t w_row_bytes, const float *X, int64_t x_stride,
+                                 float *dst, int64_t dst_stride, int64_t K, int64_t M, int64_t N,
+                                 void *workspace, size_t workspace_bytes, int64_t wait_cycles, b200_stream_t stream);
 
 /* Dense bf16 weights: b200_mul_mat_q also takes B200_TYPE_BF16 (rows 16-byte aligned, K a multiple of 64).  A batch of n_batch
  * independent products of one shape (the per-head matrices of an attention layer) runs as ONE launch: product b reads

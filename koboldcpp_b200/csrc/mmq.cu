@@ -381,6 +381,7 @@ __global__ void mmq_x_to_bf16_kernel(const float *__restrict__ x, int64_t x_stri
     *reinterpret_cast<uint2 *>(out + n * K + i4 * 4) = pk;
 }
 
+constexpr long long PAIR_WAIT_LIMIT = 4000000000LL;  // clock cycles: about two seconds
 struct MmqParams {
     const unsigned char *W;
     size_t w_row_bytes;
@@ -401,6 +402,7 @@ struct MmqParams {
     size_t w_batch_bytes;
     int64_t dst_batch, n_pad;
     int n_expert;  // grouped: experts in the stack
+    long long wait_limit = PAIR_WAIT_LIMIT;  // mmq_pair_kernel: clock cycles
 };
 
 template <int TYPE, int BN>
@@ -890,6 +892,12 @@ extern "C" size_t b200_mul_mat_q_workspace_bytes(int type, int64_t K, int64_t M,
 
 extern "C" int b200_mul_mat_q(int type, const void *W, size_t w_row_bytes, const float *X, int64_t x_stride, float *dst, int64_t dst_stride,
                               int64_t K, int64_t M, int64_t N, void *workspace, size_t workspace_bytes, b200_stream_t stream) {
+    return b200_mul_mat_q_wait(type, W, w_row_bytes, X, x_stride, dst, dst_stride, K, M, N, workspace, workspace_bytes, PAIR_WAIT_LIMIT, stream);
+}
+
+extern "C" int b200_mul_mat_q_wait(int type, const void *W, size_t w_row_bytes, const float *X, int64_t x_stride, float *dst, int64_t dst_stride, int64_t K, int64_t M,
+                                   int64_t N, void *workspace, size_t workspace_bytes, int64_t wait_cycles, b200_stream_t stream) {
+    if (wait_cycles < 0) { set_error("b200_mul_mat_q_wait: limit below zero"); return B200_ERR_INVALID; }
     if (!W || !dst) { set_error("b200_mul_mat_q: NULL argument"); return B200_ERR_INVALID; }
     const int bv = type_block_values(type);
     if (!(type == B200_TYPE_Q4_0 || type == B200_TYPE_Q8_0 || type == B200_TYPE_Q4_K || type == B200_TYPE_Q5_K || type == B200_TYPE_Q6_K ||
@@ -926,6 +934,7 @@ extern "C" int b200_mul_mat_q(int type, const void *W, size_t w_row_bytes, const
     p.W = (const unsigned char *)W; p.w_row_bytes = w_row_bytes; p.Xb = xb; p.dst = dst; p.dst_stride = dst_stride; p.K = K; p.M = M; p.N = N;
     p.tile_tab = nullptr; p.row_dst = nullptr; p.expert_bytes = 0;
     p.n_batch = 1; p.w_batch_bytes = 0; p.dst_batch = 0; p.n_pad = n_pad; p.n_expert = 1;
+    p.wait_limit = wait_cycles;
     switch (type) {
         case B200_TYPE_Q4_0: return mmq_dispatch_bn<B200_TYPE_Q4_0>(p, st);
         case B200_TYPE_Q8_0: return mmq_dispatch_bn<B200_TYPE_Q8_0>(p, st);

@@ -16,13 +16,15 @@
 //   * the accumulators are double-buffered in TMEM (2 x 256 columns): four epilogue warps store tile i while tile i + 1 is computed.
 //   * BN is chosen on the host so that the tiles fill the pairs evenly (mmq_pair_plan): 512 columns are 2 x 256 or 3 x 176, whichever leaves
 //     the last wave fuller.  In the grouped form (routed experts) the width of every tile follows its rows.
-// Every wait has a limit (PAIR_WAIT_LIMIT); a role that gives up tells its CTA and goes on without waiting, nothing is stored from then on,
-// *timeout is set, and the CTA stays until copies and MMAs in flight have ended.
+// Every wait has a limit (MmqParams::wait_limit).  A role whose wait runs out sets `failed` of its CTA and leaves its loop: no store, copy or MMA, and no
+// arrival (an arrival that no wait stands before could find a phase whose arrivals are all there, waiting for bytes only).  Whoever
+// waits for it, in either CTA, gives up in turn.  An accumulator is announced when the operands of all its K steps had arrived, so what is
+// stored is right (of two halves of K: what is added); the rest of the result stays as it was, *timeout is set, and the CTA stays until
+// copies and MMAs in flight have ended.
 #pragma once
 
 namespace b200 {
 
-constexpr long long PAIR_WAIT_LIMIT = 4000000000LL;  // clock cycles: about two seconds
 constexpr int PAIR_PRODUCERS = 16;                   // warps that unpack, 8 rows of the CTA's 128 each
 constexpr int PAIR_MAX_STAGES = 8;
 constexpr int PAIR_SMEM = 232448 - 1024 - 1024;      // dynamic shared memory: what a CTA can have, less static data and alignment
@@ -99,13 +101,13 @@ __device__ __forceinline__ bool mbar_try(unsigned bar, unsigned parity) {
 // wait with the limit; false, at once, when a role of the CTA has given up.  SLEEP: nanoseconds between two looks (a failing try_wait comes back within
 // some 50 cycles whatever time it is offered, and a dozen polling warps take the issue slots of the others).
 template <int SLEEP>
-__device__ __forceinline__ bool pair_wait(unsigned bar, unsigned parity, volatile int *failed) {
+__device__ __forceinline__ bool pair_wait(unsigned bar, unsigned parity, volatile int *failed, long long limit) {
     if (mbar_try(bar, parity)) return true;
     const long long t0 = clock64();
     while (!mbar_try(bar, parity)) {
         if (SLEEP > 0) __nanosleep(SLEEP);
         if (*failed) return false;
-        if (clock64() - t0 > PAIR_WAIT_LIMIT) { *failed = 1; return false; }
+        if (clock64() - t0 > limit) { *failed = 1; return false; }
     }
     return true;
 }
@@ -386,6 +388,7 @@ __global__ void __launch_bounds__(pair_threads<TYPE>(), 1) mmq_pair_kernel(const
     __shared__ volatile int failed;
     const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31, tid = threadIdx.x;
     const int rank = (int)cluster_rank(), pair = (int)(blockIdx.x >> 1), n_pairs = (int)(gridDim.x >> 1);
+    const long long limit = p.q.wait_limit;
     const int S = p.stages, stage_bytes = A_BYTES + p.bn * MQ_BK;  // (bn / 2 activation rows of 128 bytes)
     const int nt = GROUPED ? __ldg(p.q.tile_tab) : p.n_tiles_n;
     const int n_tiles = nt * p.n_tiles_m * (GROUPED ? 1 : p.q.n_batch > 1 ? p.q.n_batch : p.q.ksplit);
@@ -463,11 +466,12 @@ __global__ void __launch_bounds__(pair_threads<TYPE>(), 1) mmq_pair_kernel(const
             const unsigned p0 = a_row + (unsigned)((f0 ^ r) << 4), p1 = a_row + (unsigned)(((f0 + 1) ^ r) << 4), p2 = a_row + (unsigned)((f1 ^ r) << 4), p3 = a_row + (unsigned)(((f1 + 1) ^ r) << 4);
             int s = 0, slot = 0;        // stage of the first K step of the pair
             unsigned ph = 1;            // parity of its empty barrier: the first pass finds it free
-            for (int t = pair; t < n_tiles; t += n_pairs) {
+            bool ok = true;  // (the same in all lanes)
+            for (int t = pair; t < n_tiles && ok; t += n_pairs) {
                 const PairTile ti = pair_tile<GROUPED>(p, t, nt, UNIT);
                 unsigned at = raw_aligned(TYPE) ? 0u : (unsigned)(uintptr_t)row_base(ti, r) & 15u;  // where in its first piece the row's group starts
 #pragma unroll 1
-                for (int g = ti.nkb / 4; g > 0; g--) {
+                for (int g = ti.nkb / 4; g > 0 && ok; g--) {
                     cp_async_wait<SLOTS - 2>();
                     __syncwarp();  // the group has landed for all lanes, and all have left the one before
                     copy_group();
@@ -482,7 +486,8 @@ __global__ void __launch_bounds__(pair_threads<TYPE>(), 1) mmq_pair_kernel(const
                         const bool wrap = s + 1 >= S;
                         const int s1 = wrap ? s + 1 - S : s + 1;
                         const unsigned ph1 = wrap ? ph ^ 1u : ph;
-                        pair_wait<20>(empty0 + 8u * s1, ph1, &failed);
+                        ok = __all_sync(0xffffffffu, pair_wait<20>(empty0 + 8u * s1, ph1, &failed, limit));
+                        if (!ok) break;
                         const int mine = cc ? s1 : s;
                         const unsigned d = (unsigned)(mine * stage_bytes);
                         asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(p0 + d), "r"(o[0]), "r"(o[1]), "r"(o[2]), "r"(o[3]) : "memory");
@@ -507,11 +512,13 @@ __global__ void __launch_bounds__(pair_threads<TYPE>(), 1) mmq_pair_kernel(const
         const unsigned peer_remote = leader_addr(peer0);
         int s = 0, buf = 0;
         unsigned ph = 0, aph = 1;
-        for (int t = pair; t < n_tiles; t += n_pairs) {
+        bool ok = true;  // (the same in all lanes)
+        for (int t = pair; t < n_tiles && ok; t += n_pairs) {
             const PairTile ti = pair_tile<GROUPED>(p, t, nt, UNIT);
             if (rank != 0) {
                 for (int kb = 0; kb < ti.nkb; kb++) {
-                    pair_wait<0>(full0 + 8u * s, ph, &failed);
+                    ok = __all_sync(0xffffffffu, pair_wait<0>(full0 + 8u * s, ph, &failed, limit));
+                    if (!ok) break;
                     if (elected) mbar_arrive_remote(peer_remote + 8u * s);
                     __syncwarp();
                     if (++s == S) { s = 0; ph ^= 1u; }
@@ -519,13 +526,15 @@ __global__ void __launch_bounds__(pair_threads<TYPE>(), 1) mmq_pair_kernel(const
                 continue;
             }
             const unsigned idesc = umma_idesc_bf16(256, 16) + ((unsigned)((ti.n - 16) >> 3) << 17), acc = tmem_base + (unsigned)buf * 256u;
-            pair_wait<0>(acc_empty0 + 8u * buf, aph, &failed);
+            ok = __all_sync(0xffffffffu, pair_wait<0>(acc_empty0 + 8u * buf, aph, &failed, limit));
+            if (!ok) break;
             tc_fence_after();
             unsigned accumulate = 0;
 #pragma unroll 1
             for (int kb = 0; kb < ti.nkb; kb++) {
-                pair_wait<0>(full0 + 8u * s, ph, &failed);
-                pair_wait<0>(peer0 + 8u * s, ph, &failed);
+                const bool here = pair_wait<0>(full0 + 8u * s, ph, &failed, limit), there = pair_wait<0>(peer0 + 8u * s, ph, &failed, limit);
+                ok = __all_sync(0xffffffffu, here && there);
+                if (!ok) break;
                 tc_fence_after();
                 const unsigned long long ad = desc0 + (unsigned)(s * (stage_bytes >> 4)), bd = ad + (A_BYTES >> 4);
                 if (elected) {
@@ -539,6 +548,7 @@ __global__ void __launch_bounds__(pair_threads<TYPE>(), 1) mmq_pair_kernel(const
                 accumulate = 1;
                 if (++s == S) { s = 0; ph ^= 1u; }
             }
+            if (!ok) break;
             if (elected) tc_commit2(acc_full0 + 8u * buf);
             __syncwarp();
             buf ^= 1;
@@ -559,7 +569,7 @@ __global__ void __launch_bounds__(pair_threads<TYPE>(), 1) mmq_pair_kernel(const
             int k = ti.kb0 * MQ_BK;
 #pragma unroll 1
             for (int kb = 0; kb < ti.nkb; kb++, k += MQ_BK) {
-                if (!pair_wait<20>(empty0 + 8u * s, ph, &failed)) dead = true;
+                if (!dead && !pair_wait<20>(empty0 + 8u * s, ph, &failed, limit)) dead = true;
                 if (elected && !dead) {  // no copy without a free stage
                     unsigned char *st = smem + (size_t)(s * stage_bytes);
                     mbar_expect_tx(&full_bar[s], tx);
@@ -576,16 +586,17 @@ __global__ void __launch_bounds__(pair_threads<TYPE>(), 1) mmq_pair_kernel(const
         }
     } else {
         // ===== epilogue: TMEM lanes 32 * (warp % 4) .. of this CTA's 128 rows
+        bool ok = true;
         int buf = 0;
         unsigned ph = 0;
         const int quarter = warp & 3;
         const unsigned acc_remote = leader_addr(acc_empty0);
         for (int t = pair; t < n_tiles; t += n_pairs) {
             const PairTile ti = pair_tile<GROUPED>(p, t, nt, UNIT);
-            pair_wait<200>(acc_full0 + 8u * buf, ph, &failed);
+            ok = ok && pair_wait<200>(acc_full0 + 8u * buf, ph, &failed, limit);
             tc_fence_after();
             const int64_t m = ti.m0 + rank * MQ_BM + quarter * 32 + lane;
-            const bool row_ok = m < p.q.M && !failed;
+            const bool row_ok = m < p.q.M && ok;
             float *drow = p.q.dst + m + (!GROUPED && p.q.n_batch > 1 ? ti.product * p.q.dst_batch : 0);
             const int cols = (int)(ti.n_end - ti.n0);
 #pragma unroll 1
@@ -606,7 +617,7 @@ __global__ void __launch_bounds__(pair_threads<TYPE>(), 1) mmq_pair_kernel(const
             }
             tc_fence_before();
             __syncwarp();
-            if (lane == 0) mbar_arrive_remote(acc_remote + 8u * buf);
+            if (lane == 0 && ok) mbar_arrive_remote(acc_remote + 8u * buf);
             buf ^= 1;
             if (buf == 0) ph ^= 1u;
         }

@@ -2,6 +2,9 @@
 of K, results inside wider rows, batches of products and experts of uneven size.  Against float64 over the dequantised weights; the bound is
 that of tests/test_gpu_mmq.py (both operands rounded to bf16: 2^-9 / sqrt(3) each, relative to the product)."""
 import ctypes as C
+import subprocess
+import sys
+from pathlib import Path
 
 import numpy as np
 import pytest
@@ -84,3 +87,46 @@ def test_experts_of_uneven_size(t, T, n_expert, hot):
     W = [np.stack([O.dequantize(t, r, K) for r in w[e * M:(e + 1) * M]]).astype(np.float64) for e in range(n_expert)]
     exp = np.stack([[W[ids[i, s]] @ b[i, 0].astype(np.float64) for s in range(used)] for i in range(T)])
     assert rel(got, exp) < 4e-3
+
+
+GIVE_UP = """
+import sys, numpy as np
+sys.path[:0] = [{root!r}, {tests!r}]
+import koboldcpp_b200.host as H, orc as O
+from koboldcpp_b200.lib import Q4_K, check, lib, row_size
+from koboldcpp_b200.llama import random_blocks
+K, M, N = 1792, 19500, 200
+rng = np.random.default_rng(0)
+w, x = random_blocks(rng, Q4_K, M, K), rng.standard_normal((N, K)).astype(np.float32)
+want = x.astype(np.float64) @ np.stack([O.dequantize(Q4_K, r, K) for r in w]).astype(np.float64).T
+dw, dx = H.DeviceBuffer.from_numpy(w.reshape(-1)), H.DeviceBuffer.from_numpy(x)
+need = lib().b200_mul_mat_q_workspace_bytes(Q4_K, K, M, N)
+ws = H.DeviceBuffer(need + 16)
+def run(limit):
+    dd = H.DeviceBuffer.from_numpy(np.full((N, M), np.nan, np.float32))
+    check(lib().b200_mul_mat_q_wait(Q4_K, dw.ptr, row_size(Q4_K, K), dx.ptr, K, dd.ptr, M, K, M, N, ws.ptr, need, limit, None))
+    return dd.to_numpy(np.float32, (N, M))
+whole = run(4_000_000_000)
+assert np.isfinite(whole).all() and np.linalg.norm(whole - want) < 4e-3 * np.linalg.norm(want)
+assert lib().b200_gemm_status() == 0
+for limit in {limits}:
+    got = run(limit)
+    stored = ~np.isnan(got)
+    print(limit, stored.mean())
+    assert np.array_equal(got[stored], whole[stored]), limit
+assert not stored.all()
+{more}
+"""
+
+
+def give_up(more="", limits=(0,)):
+    """The statements above in a process of their own (that a product gave up is remembered for the life of a process), then `more`."""
+    tests = Path(__file__).resolve().parent
+    r = subprocess.run([sys.executable, "-c", GIVE_UP.format(root=str(tests.parent), tests=str(tests), more=more, limits=limits)], capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stdout[-2000:] + r.stderr[-2000:]
+
+
+def test_what_is_stored_is_right_when_waits_run_out():
+    """With a limit of some cycles the pipeline gives up at its start, in its middle or not at all, in either CTA of a pair: every value is the right one, to
+    the bit, or was never written."""
+    give_up(limits=(100_000, 20_000, 6_000, 2_000, 700, 200, 0))
