@@ -20,7 +20,9 @@
 
 #include <cuda_bf16.h>
 
+#include <atomic>
 #include <cstdlib>
+#include <mutex>
 
 namespace b200 {
 
@@ -665,13 +667,23 @@ __global__ void __launch_bounds__(MQ2_THREADS, 1) mmq_tc2_kernel(const __grid_co
 }
 
 // ---------------------------------------------------------------- host side
-// set by a GEMM whose pipeline gave up; pinned host memory, so that reading it after a synchronisation costs nothing
-static int *g_gemm_timeout = nullptr;
-void gemm_status_prepare() {
-    if (g_gemm_timeout) return;
+// set by a GEMM whose pipeline gave up; pinned host memory, so that reading it after a synchronisation costs nothing.  Allocated before the first
+// launch that may set it, whoever makes it and on whichever thread; legal while a stream is being captured.
+static std::atomic<int *> g_gemm_timeout{nullptr};
+static int gemm_status_prepare() {
+    static std::mutex lock;
+    if (g_gemm_timeout.load(std::memory_order_acquire)) return B200_OK;
+    std::lock_guard<std::mutex> guard(lock);
+    if (g_gemm_timeout.load(std::memory_order_relaxed)) return B200_OK;
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    B200_CUDA_TRY(cudaThreadExchangeStreamCaptureMode(&mode));
     int *p = nullptr;
-    if (cudaHostAlloc((void **)&p, sizeof(int), cudaHostAllocPortable | cudaHostAllocMapped) == cudaSuccess) { *p = 0; g_gemm_timeout = p; }
-    else cudaGetLastError();
+    const cudaError_t rc = cudaHostAlloc((void **)&p, sizeof(int), cudaHostAllocPortable | cudaHostAllocMapped);
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    B200_CUDA_TRY(rc);
+    *p = 0;
+    g_gemm_timeout.store(p, std::memory_order_release);
+    return B200_OK;
 }
 
 static int64_t mmq_bn(int64_t N) { return N <= 32 ? 32 : N <= 64 ? 64 : N <= 128 ? 128 : 256; }
@@ -882,7 +894,10 @@ static int mid_dispatch_bn(const MmqParams &p, int64_t bn, int64_t n_rows, unsig
 
 using namespace b200;
 
-extern "C" int b200_gemm_status(void) { return g_gemm_timeout ? *(volatile int *)g_gemm_timeout : 0; }
+extern "C" int b200_gemm_status(void) {
+    const volatile int *p = g_gemm_timeout.load(std::memory_order_acquire);
+    return p ? *p : 0;
+}
 
 extern "C" size_t b200_mul_mat_q_workspace_bytes(int type, int64_t K, int64_t M, int64_t N) {
     (void)type; (void)M;

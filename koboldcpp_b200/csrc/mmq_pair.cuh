@@ -626,7 +626,7 @@ __global__ void __launch_bounds__(pair_threads<TYPE>(), 1) mmq_pair_kernel(const
     if (warp < NP || warp == NP + 1) pair_await();
     __syncthreads();
     if (failed) {  // copies and MMAs that were requested end within this time
-        if (tid == 0 && p.timeout) atomicExch(p.timeout, 1);
+        if (tid == 0) atomicExch(p.timeout, 1);
         for (const long long t0 = clock64(); clock64() - t0 < 4000000LL;) {}
     }
     tc_fence_before();
@@ -689,7 +689,9 @@ static int mmq_pair_launch(const MmqParams &q, int64_t n_pad, int64_t w_rows_per
     PairParams p;
     p.q = q;
     p.w_rows_per_product = w_rows_per_product;
-    p.timeout = g_gemm_timeout;
+    const int status_rc = gemm_status_prepare();
+    if (status_rc != B200_OK) return status_rc;
+    p.timeout = g_gemm_timeout.load(std::memory_order_acquire);
     p.n_tiles_m = (int)((q.M + 255) / 256);
     if (GROUPED) {
         p.bn = (int)grouped_bn;

@@ -130,3 +130,7 @@ def test_what_is_stored_is_right_when_waits_run_out():
     """With a limit of some cycles the pipeline gives up at its start, in its middle or not at all, in either CTA of a pair: every value is the right one, to
     the bit, or was never written."""
     give_up(limits=(100_000, 20_000, 6_000, 2_000, 700, 200, 0))
+
+
+def test_status_is_set_for_a_caller_without_a_backend():
+    give_up("assert lib().b200_gemm_status() == 1")
