@@ -659,9 +659,11 @@ int enqueue_decode(b200_llama *m, const int32_t *tokens, int32_t n_tokens, int32
 
 }  // namespace
 
-// Tensor parallel: an all-reduce whose peer never arrived gives up after its timeout and flags the window (comm.cu); the sums of
-// that step are stale, so the step must not be reported as done.  One 4-byte read per synchronised step, tensor-parallel runs only.
-static int peer_check(b200_llama *m) {
+// What only a synchronisation shows; the step must not be reported as done.  A prompt's product that gave up waiting for its operands has left its
+// results incomplete (mmq_pair.cuh).  Tensor parallel: an all-reduce whose peer never arrived gives up after its timeout and flags the window
+// (comm.cu); the sums of that step are stale.  One 4-byte read each per synchronised step.
+static int step_check(b200_llama *m) {
+    LL_REQUIRE(b200_gemm_status() == 0, B200_ERR_CUDA, "b200_llama: a product gave up waiting for its operands: the step's results are invalid");
     if (m->hp.tp_world <= 1) return B200_OK;
     const int st = b200_comm_peer_status();
     LL_REQUIRE(st == 0, B200_ERR_CUDA, "b200_llama: a tensor-parallel peer did not arrive in time (peer status %d): the step's results are invalid", st);
@@ -674,7 +676,7 @@ extern "C" int b200_llama_decode_async(b200_llama *m, const int32_t *tokens, int
 extern "C" int b200_llama_synchronize(b200_llama *m) {
     LL_REQUIRE(m && m->be, B200_ERR_INVALID, "b200_llama_synchronize: NULL model");
     m->be->iface.synchronize(m->be);
-    return peer_check(m);
+    return step_check(m);
 }
 extern "C" int b200_llama_decode(b200_llama *m, const int32_t *tokens, int32_t n_tokens, int32_t n_past, float *logits, int32_t logits_all) {
     const int rc = enqueue_decode(m, tokens, n_tokens, n_past, logits, logits_all);
@@ -682,7 +684,7 @@ extern "C" int b200_llama_decode(b200_llama *m, const int32_t *tokens, int32_t n
     const auto ts0 = std::chrono::steady_clock::now();
     m->be->iface.synchronize(m->be);
     m->t_sync += std::chrono::duration<double>(std::chrono::steady_clock::now() - ts0).count();
-    return peer_check(m);
+    return step_check(m);
 }
 extern "C" int b200_llama_replay(b200_llama *m) {
     LL_REQUIRE(m && m->finalized && m->graph.n_nodes > 0, B200_ERR_INVALID, "b200_llama_replay: nothing decoded yet");

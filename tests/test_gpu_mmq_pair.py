@@ -134,3 +134,26 @@ def test_what_is_stored_is_right_when_waits_run_out():
 
 def test_status_is_set_for_a_caller_without_a_backend():
     give_up("assert lib().b200_gemm_status() == 1")
+
+
+STEP = """
+import koboldcpp_b200.llama as L
+from koboldcpp_b200.lib import F16
+def failing(call):
+    try:
+        call()
+    except Exception as e:
+        assert "gave up waiting" in str(e), e
+        return
+    raise AssertionError("a step behind a product that gave up was reported as done")
+m = L.LlamaModel(L.SHAPES["test-dense"], 512, F16)
+m.init_random(1)
+m.finalize(64)
+failing(lambda: m.decode(list(range(40)), 0))
+m.decode_async(list(range(40)), 0)
+failing(m.synchronize)
+"""
+
+
+def test_decoder_reports_a_step_behind_a_product_that_gave_up():
+    give_up(STEP)
