@@ -272,6 +272,11 @@ static int device_props() {
     return B200_OK;
 }
 
+// one job's columns beside two ring stages of every warp
+template <int TYPE>
+static bool mmvq_fits(const MmvqParams &p, int ncols) {
+    return device_props() || MMVQ_BAR_BYTES + ((size_t)ncols * act_col_bytes(p.n_it) + 127) / 128 * 128 + 2 * (size_t)MMVQ_NW * Geo<TYPE>::STAGE_BYTES + 256 <= g_smem_optin;
+}
 struct MmvqPlan { int64_t units, grid; size_t act_bytes, tab_bytes; };  // units: rows, or (gate, up) pairs
 // split over the SMs, and whether row table and activations fit: what several columns may ask for, whichever kernel serves them
 template <int TYPE>
@@ -430,11 +435,28 @@ static int dispatch_cols(MmvqParams &p, int N, cudaStream_t st, bool pdl) {
         bool same_x = p.ids == nullptr;
         for (int j = 1; j < p.n_jobs; j++) same_x = same_x && p.jobs[j].X == p.jobs[0].X;
         if (N >= (TYPE == B200_TYPE_Q6_K ? 6 : 4) && p.total_rows >= 512 && same_x && (!multi || N <= 4)) {
-            MmvqPlan pl;
-            int rc = mmvq_plan<TYPE>(p, N, multi, pl);
+            int rc = B200_OK;
+            if (multi) {  // (several jobs have a limit of rows, whichever kernel serves them)
+                MmvqPlan pl;
+                rc = mmvq_plan<TYPE>(p, N, multi, pl);
+            }
             if (!rc) rc = launch_mmvq_mma<TYPE>(p, N, st, pdl);
             if (rc != -1000) return rc;
         }
+    }
+    if (!multi && N > 1 && !mmvq_fits<TYPE>(p, N)) {  // long rows: the columns' activations fill shared memory (13824 values: 7 or 8): half of them at a time
+        const int first = N / 2;
+        MmvqParams q = p;
+        int rc = dispatch_cols<TYPE>(q, first, st, pdl);
+        if (rc) return rc;
+        q = p;
+        q.jobs[0].X += first * p.x_stride;
+        q.jobs[0].dst += first * p.dst_stride;
+        if (q.residual[0]) q.residual[0] += first * p.dst_stride;
+        if (q.raw_dst[0]) q.raw_dst[0] += first * p.dst_stride;
+        if (q.norm_out) q.norm_out += first * p.K;
+        if (q.norm_mul_out) q.norm_mul_out += first * p.K;
+        return dispatch_cols<TYPE>(q, N - first, st, pdl);
     }
     if (multi) {  // fused / expert launches are decode-only: 1..4 columns
         switch (N) {

@@ -8,7 +8,7 @@ import pytest
 
 import koboldcpp_b200.host as H
 import orc as O
-from koboldcpp_b200.lib import Q4_K, Q5_K, Q6_K, GemvFuse, GemvJob, check, lib, row_size
+from koboldcpp_b200.lib import Q4_0, Q4_K, Q5_K, Q6_K, Q8_0, GemvFuse, GemvJob, check, lib, row_size
 from koboldcpp_b200.llama import random_blocks
 
 pytestmark = pytest.mark.gpu
@@ -84,3 +84,34 @@ def test_five_columns_of_several_jobs_stay_refused():
     for i in range(2):
         jobs[i].W, jobs[i].X, jobs[i].dst, jobs[i].M, jobs[i].id_index = w.ptr, x.ptr, d.ptr + 4 * M * i, M, -1
     assert lib().b200_mul_mat_vec_q_multi(Q4_K, jobs, 2, row_size(Q4_K, K), K, 2 * M, K, 5, None, 0, 0, None) == 1
+
+
+@pytest.mark.parametrize("t", [Q4_K, Q5_K, Q6_K, Q4_0, Q8_0])
+@pytest.mark.parametrize("K,N", [(13824, 7), (13824, 8), (20480, 5), (20480, 8)])
+def test_columns_of_long_rows(t, K, N):
+    """Where shared memory does not hold all columns' activations for the dp4a form: the tensor form holds more, else half of the columns at a time."""
+    M = 530
+    rng = np.random.default_rng(K + N + t)
+    w, x = random_blocks(rng, t, M, K), rng.standard_normal((N, K)).astype(np.float32)
+    assert close(H.mul_mat_vec_q(t, w, x, K, M), O.mul_mat_q8_1(t, w, x, K, M))
+
+
+def test_columns_of_long_rows_with_norm_and_residual():
+    t, K, M, N, eps = Q4_0, 13824, 300, 8, 1e-5
+    rng = np.random.default_rng(3)
+    w, x, nw = random_blocks(rng, t, M, K), rng.standard_normal((N, K)).astype(np.float32), rng.standard_normal(K).astype(np.float32)
+    res = rng.standard_normal((N, M)).astype(np.float32)
+    scale = (1.0 / np.sqrt((x.astype(np.float64) ** 2).mean(1, keepdims=True) + eps)).astype(np.float32)
+    xn = x * scale * nw
+    dw, dx, dn, dr = H.DeviceBuffer.from_numpy(w, pad=16), H.DeviceBuffer.from_numpy(x), H.DeviceBuffer.from_numpy(nw), H.DeviceBuffer.from_numpy(res)
+    dd, draw, dnorm, dmul = (H.DeviceBuffer(4 * N * n) for n in (M, M, K, K))
+    jobs, fuse = (GemvJob * 1)(), GemvFuse()
+    fuse.norm_weight, fuse.norm_eps, fuse.norm_out, fuse.norm_mul_out = dn.ptr, eps, dnorm.ptr, dmul.ptr
+    fuse.residual[0], fuse.raw_dst[0] = dr.ptr, draw.ptr
+    jobs[0].W, jobs[0].X, jobs[0].dst, jobs[0].M, jobs[0].id_index = dw.ptr, dx.ptr, dd.ptr, M, -1
+    check(lib().b200_mul_mat_vec_q_fused(t, jobs, 1, row_size(t, K), K, M, K, N, C.byref(fuse), None))
+    want = O.mul_mat_q8_1(t, w, xn, K, M)
+    tol = 2e-3 * np.abs(want).max()  # (as in test_jobs_with_norm_and_residual)
+    assert np.abs(dd.to_numpy(np.float32, (N, M)) - (want + res)).max() < tol and np.abs(draw.to_numpy(np.float32, (N, M)) - want).max() < tol
+    np.testing.assert_allclose(dnorm.to_numpy(np.float32, (N, K)), x * scale, rtol=3e-6, atol=3e-6)
+    np.testing.assert_allclose(dmul.to_numpy(np.float32, (N, K)), xn, rtol=3e-6, atol=3e-6)
