@@ -430,11 +430,13 @@ static int dispatch_cols(MmvqParams &p, int N, cudaStream_t st, bool pdl) {
     // Several columns of one activation matrix: the integer tensor cores, whose cost hardly grows with the columns.  The line lies where the dp4a form
     // begins to lose over all measured shapes (K 512 .. 14336, M 64 .. 32000), dp4a -> tensor: q4_K 4096 x 14336 at 4 columns 24.2 -> 17.7 us, at 8
     // 40.5 -> 19.9; q5_K 24.5 -> 20.1 and 41.4 -> 22.4; q6_K, whose rows lie at any even byte, 27.0 -> 27.6 at 4, 35.1 -> 28.4 at 6.  Few rows leave
-    // each warp one block: q5_K 2048 x 256 at 4 columns 5.6 -> 5.9, 4096 x 1024 7.8 -> 7.5.
+    // each warp one block: below 512 rows dp4a is ahead at 4 columns (q4_K 2048 x 256 7.3 -> 8.3, q5_K 8.0 -> 8.3), level at 5 and 6 (q4_K 2048 x 64 8.5 -> 8.4,
+    // q6_K 9.6 -> 10.5) and behind at 7 and 8 (q4_K 10.5 -> 8.5, q5_K 10.5 -> 8.5).  How K is cut, and with it the last bits, follows from the
+    // launch's rows.
     if constexpr (TYPE == B200_TYPE_Q4_K || TYPE == B200_TYPE_Q5_K || TYPE == B200_TYPE_Q6_K) {
         bool same_x = p.ids == nullptr;
         for (int j = 1; j < p.n_jobs; j++) same_x = same_x && p.jobs[j].X == p.jobs[0].X;
-        if (N >= (TYPE == B200_TYPE_Q6_K ? 6 : 4) && p.total_rows >= 512 && same_x && (!multi || N <= 4)) {
+        if (N >= (TYPE == B200_TYPE_Q6_K ? 6 : 4) && (p.total_rows >= 512 || N >= 7) && same_x && (!multi || N <= 4)) {
             int rc = B200_OK;
             if (multi) {  // (several jobs have a limit of rows, whichever kernel serves them)
                 MmvqPlan pl;

@@ -115,3 +115,11 @@ def test_columns_of_long_rows_with_norm_and_residual():
     assert np.abs(dd.to_numpy(np.float32, (N, M)) - (want + res)).max() < tol and np.abs(draw.to_numpy(np.float32, (N, M)) - want).max() < tol
     np.testing.assert_allclose(dnorm.to_numpy(np.float32, (N, K)), x * scale, rtol=3e-6, atol=3e-6)
     np.testing.assert_allclose(dmul.to_numpy(np.float32, (N, K)), xn, rtol=3e-6, atol=3e-6)
+
+
+@pytest.mark.parametrize("t", [Q4_K, Q5_K, Q6_K])
+@pytest.mark.parametrize("K,M,N", [(256, 1, 7), (2048, 64, 8), (1024, 300, 7), (4096, 511, 8)])
+def test_many_columns_of_few_rows(t, K, M, N):
+    rng = np.random.default_rng(K + M + t)
+    w, x = random_blocks(rng, t, M, K), rng.standard_normal((N, K)).astype(np.float32)
+    assert close(H.mul_mat_vec_q(t, w, x, K, M), O.mul_mat_q8_1(t, w, x, K, M))
