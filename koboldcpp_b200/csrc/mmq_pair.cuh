@@ -640,22 +640,24 @@ __global__ void __launch_bounds__(pair_threads<TYPE>(), 1) mmq_pair_kernel(const
 
 // ---------------------------------------------------------------- host side
 // Tile width and K split by the time of the longest pair's work, in microseconds.  A K step of 64 costs `unpack` plus 0.6 ns a column while the
-// producers are the slower ones (measured, 18944 rows: q4_K 0.29 at 64 columns, 0.43 at 256; q6_K 0.47 and 0.54), dense weights take 1.25 ns a
-// column but 0.2 at least; a tile more costs about 1.  Two halves of K add into a zeroed dst: that much more traffic, at 1.5 TB/s, and a
-// launch more.  Widths are N / 1, N / 2, ... rounded up to 16.
+// producers are the slower ones (measured with one tile a pair, see pair_unpack_us), dense weights take 1.25 ns a column but 0.2 at least; a tile
+// more costs about 1.  The last tile's values are stored with nothing behind them to hide it: 30 ns a column (dense 64 x 64 weights: 8.4 us for 64
+// columns, 12.6 for 512 in tiles of 256; dense 1024 x 1024 over 128 columns 14.5 us as 4 tiles of 128, 11.7 for a kernel with narrower ones).  Two halves of K
+// add into a zeroed dst: that much more traffic, at 1.5 TB/s, and a launch more.  Widths are N / 1, N / 2, ... rounded up to 16.
 struct PairPlan { int bn, ksplit, n_tiles_n; };
 static inline PairPlan mmq_pair_plan(int64_t M, int64_t N, int64_t K, int n_batch, int pairs, double unpack) {
     PairPlan best = {256, 1, 1};
     double best_cost = -1;
-    const int64_t mt = (M + 255) / 256;
-    for (int64_t parts = (N + 255) / 256; parts <= (N + 31) / 32; parts++) {
-        const int64_t even = ((N + parts - 1) / parts + 15) / 16 * 16, bn = even < 32 ? 32 : even;
-        const int64_t nt = (N + bn - 1) / bn;
+    const unsigned mt = (unsigned)((M + 255) / 256), n = (unsigned)N, np = (unsigned)pairs;  // (32-bit: the divisions of up to 30 candidates are host time of each call)
+    const double steps = (double)(K / MQ_BK), halves = 2.0 + (double)M * N * 4 / 1.5e6;
+    const int ks_max = n_batch > 1 || K < 2048 ? 1 : 2;
+    for (unsigned parts = (n + 255) / 256, last = (n + 31) / 32; parts <= last; parts++) {
+        const unsigned even = ((n + parts - 1) / parts + 15) / 16 * 16, bn = even < 32 ? 32 : even, nt = (n + bn - 1) / bn;
         const double dense = 1.25e-3 * bn < 0.2 ? 0.2 : 1.25e-3 * bn, step = unpack > 0 ? unpack + 0.6e-3 * bn : dense;
-        for (int ks = 1; ks <= 2; ks++) {
-            if (ks == 2 && (n_batch > 1 || K < 2048)) break;
-            const int64_t tiles = mt * nt * n_batch * ks, waves = (tiles + pairs - 1) / pairs;
-            const double cost = waves * ((double)(K / MQ_BK) / ks * step + 1.0) + (ks == 2 ? 2.0 + (double)M * N * 4 / 1.5e6 : 0.0);
+        for (int ks = 1; ks <= ks_max; ks++) {
+            const uint64_t tiles = (uint64_t)mt * nt * n_batch * ks;
+            const double waves = tiles <= np ? 1.0 : (double)((tiles + np - 1) / np);
+            const double cost = waves * (steps / ks * step + 1.0) + 0.03 * bn + (ks == 2 ? halves : 0.0);
             if (best_cost < 0 || cost < 0.98 * best_cost) { best_cost = cost; best = {(int)bn, ks, (int)nt}; }
         }
     }
@@ -673,7 +675,20 @@ static int mmq_pairs() {
     return pairs;
 }
 
-template <int TYPE> constexpr double pair_unpack_us() { return TYPE == B200_TYPE_BF16 ? 0 : TYPE == B200_TYPE_Q4_K || TYPE == B200_TYPE_Q4_0 ? 0.27 : TYPE == B200_TYPE_Q5_K || TYPE == B200_TYPE_Q8_0 ? 0.33 : 0.43; }
+// microseconds a K step of 64 takes while unpacking is the slower side, less 0.6 ns a column: one tile of 256 rows on each of 74 pairs, 64 columns, from the
+// difference between 8192 and 4096 values a row
+template <int TYPE> constexpr double pair_unpack_us() {
+    switch (TYPE) {
+        case B200_TYPE_BF16: return 0;
+        case B200_TYPE_Q4_0: return 0.29;
+        case B200_TYPE_Q4_K: return 0.30;
+        case B200_TYPE_Q2_K: return 0.32;
+        case B200_TYPE_Q4_1: case B200_TYPE_Q5_K: return 0.34;
+        case B200_TYPE_Q5_0: case B200_TYPE_Q8_0: return 0.38;
+        case B200_TYPE_Q5_1: case B200_TYPE_IQ4_NL: return 0.41;
+        default: return 0.44;  // q6_K, q3_K, iq4_XS
+    }
+}
 
 template <int TYPE, bool GROUPED>
 static int mmq_pair_launch(const MmqParams &q, int64_t n_pad, int64_t w_rows_per_product, int64_t max_tiles_n, int64_t grouped_bn, cudaStream_t st) {
