@@ -142,6 +142,7 @@ __global__ void __launch_bounds__(DR_WARPS * 64) delta_rule_scan_kernel(const b2
 #pragma unroll
             for (int u = 0; u < TPW; u++) {
                 const int tt = w + u * DR_WARPS;
+                if (c * DR_CHUNK + tt >= count) continue;  // (a short sequence does not wait for tokens that do not exist)
                 float qq = 0.f, kk = 0.f, qk = 0.f;
 #pragma unroll
                 for (int j = 0; j < DQ; j++) { qq += q[u][j] * q[u][j]; kk += k[u][j] * k[u][j]; }
