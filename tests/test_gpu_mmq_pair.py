@@ -157,3 +157,72 @@ failing(m.synchronize)
 
 def test_decoder_reports_a_step_behind_a_product_that_gave_up():
     give_up(STEP)
+
+
+@pytest.mark.parametrize("t", [Q4_K, Q6_K, Q8_0, Q4_0, Q5_1, IQ4_XS, BF16])
+@pytest.mark.parametrize("K,N", [(256, 300), (768, 177)])
+def test_several_tiles_a_pair(t, K, N):
+    """More than twice as many tiles as pairs of SMs: the second accumulator and its parity, stages and weight copies that run on into the next tile."""
+    M = 20000
+    rng = np.random.default_rng(K + t)
+    x = rng.standard_normal((N, K)).astype(np.float32)
+    if t == BF16:
+        bits = (rng.standard_normal((M, K)).astype(np.float32).view(np.uint32) >> 16).astype(np.uint16)
+        w, W = bits.view(np.uint8), (bits.astype(np.uint32) << 16).view(np.float32).astype(np.float64)
+    else:
+        w = random_blocks(rng, t, M, K).reshape(M, -1)
+        W = np.stack([O.dequantize(t, r, K) for r in w]).astype(np.float64)
+    got, want = product(t, w, x, K, M), x.astype(np.float64) @ W.T
+    assert rel(got, want) < 4e-3
+    # every tile by itself: 256 rows of the result each
+    for m in range(0, M, 256):
+        assert rel(got[:, m:m + 256], want[:, m:m + 256]) < 6e-3, m
+
+
+def test_several_tiles_a_pair_of_a_batch():
+    K, M, N, batch = 128, 3000, 300, 8
+    rng = np.random.default_rng(8)
+    bits = (rng.standard_normal((batch, M, K)).astype(np.float32).view(np.uint32) >> 16).astype(np.uint16)
+    W = (bits.astype(np.uint32) << 16).view(np.float32).astype(np.float64)
+    x = rng.standard_normal((batch, N, K)).astype(np.float32)
+    dw, dx, dd = H.DeviceBuffer.from_numpy(bits), H.DeviceBuffer.from_numpy(x), H.DeviceBuffer(4 * batch * N * M)
+    need = batch * lib().b200_mul_mat_q_workspace_bytes(BF16, K, M, N)
+    ws = H.DeviceBuffer(need + 16)
+    check(lib().b200_mul_mat_bf16_batched(dw.ptr, 2 * K, 2 * M * K, dx.ptr, K, N * K, dd.ptr, M, N * M, K, M, N, batch, ws.ptr, need, None))
+    got = dd.to_numpy(np.float32, (batch, N, M))
+    for b in range(batch):
+        assert rel(got[b], x[b].astype(np.float64) @ W[b].T) < 4e-3, b
+
+
+@pytest.mark.parametrize("t", [Q4_K, Q6_K, Q8_0])
+def test_several_tiles_a_pair_of_experts(t):
+    """Tiles of different widths follow one another on a pair: experts with 1 to 256 pairs and one with none."""
+    K, M, used, n_expert, T = 256, 5000, 2, 8, 300
+    rng = np.random.default_rng(t)
+    w, b = random_blocks(rng, t, n_expert * M, K).reshape(n_expert * M, -1), rng.standard_normal((T, 1, K)).astype(np.float32)
+    odds = np.array([0.45, 0.2, 0.15, 0.1, 0.06, 0.035, 0.005, 0.0])
+    ids = rng.choice(n_expert, (T, used), p=odds / odds.sum()).astype(np.int32)
+    ids[0] = 6
+    got = H.mul_mat_id_q(t, w, ids, b, K, M, n_expert)
+    for e in range(n_expert):
+        tok, slot = np.nonzero(ids == e)
+        if len(tok):
+            W = np.stack([O.dequantize(t, r, K) for r in w[e * M:(e + 1) * M]]).astype(np.float64)
+            assert rel(got[tok, slot], b[tok, 0].astype(np.float64) @ W.T) < 4e-3, e
+
+
+@pytest.mark.parametrize("gap", [0, 8])
+def test_dense_experts_at_odd_strides(gap):
+    """Values between two experts: with 8 their stride is no multiple of a row, which one tensor map cannot cover."""
+    K, M, used, n_expert, T = 192, 300, 2, 5, 120
+    rng = np.random.default_rng(gap)
+    bits = (rng.standard_normal((n_expert, M, K)).astype(np.float32).view(np.uint32) >> 16).astype(np.uint16)
+    W = (bits.astype(np.uint32) << 16).view(np.float32).astype(np.float64)
+    stack = np.zeros((n_expert, M * K + gap), np.uint16)
+    stack[:, :M * K] = bits.reshape(n_expert, -1)
+    b, ids = rng.standard_normal((T, 1, K)).astype(np.float32), rng.integers(0, n_expert, (T, used)).astype(np.int32)
+    need = lib().b200_mul_mat_id_q_workspace_bytes(BF16, K, M, used, T, n_expert)
+    dw, db, di, dd, ws = H.DeviceBuffer.from_numpy(stack), H.DeviceBuffer.from_numpy(b), H.DeviceBuffer.from_numpy(ids), H.DeviceBuffer(4 * T * used * M), H.DeviceBuffer(need + 512)
+    check(lib().b200_mul_mat_id_q(BF16, dw.ptr, 2 * K, 2 * (M * K + gap), n_expert, di.ptr, used, db.ptr, K, K, dd.ptr, M, used * M, K, M, used, 1, T, (ws.ptr + 255) // 256 * 256, need, None))
+    want = np.einsum("tsmk,tk->tsm", W[ids], b[:, 0].astype(np.float64))
+    assert rel(dd.to_numpy(np.float32, (T, used, M)), want) < 4e-3
