@@ -31,7 +31,7 @@ struct MmaGeo {
     static constexpr int ROW_STRIDE = ROW_BYTES + 16;  // ldmatrix: 8 rows x 16 bytes must hit 8 different bank groups
     static constexpr int TILE_BYTES = FM_TP * ROW_STRIDE;
     // q8_0 / q4_0 cache: the ring holds raw rows (D/32 blocks of 34 / 18 bytes, 8- or 4-byte aligned).  q8_0 goes from there to the fragments
-    // (row stride 16 or 48 modulo 128 bytes: 8 rows x 4 words lie in 32 different banks); of q4_0 a warp dequantises the tile it is about to
+    // (row stride 144 bytes for 128 dims, 80 for 64: 8 rows x 4 words lie in 32 different banks); of q4_0 a warp dequantises the tile it is about to
     // use into ONE f16 tile pair of its own
     static constexpr bool Q4        = TYPE == B200_TYPE_Q4_0;
     static constexpr int RAW_ROW    = D / 32 * BLK;

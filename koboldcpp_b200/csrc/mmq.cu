@@ -11,8 +11,8 @@
 //     the tensor core reads; activations are converted f32 -> bf16 once per call by a pre-pass;
 //   * tcgen05.mma (kind::f16, bf16 x bf16 -> f32), the f32 accumulators in TMEM; a shared-memory ring with mbarrier full/empty pairs,
 //     tcgen05.commit releases a stage when the MMAs that read it retire -- no CTA-wide barrier in the K loop.
-// mmq_pair.cuh holds the kernel of almost every call (K a multiple of 256, dense rows); here are the formats' definitions, mmq_tc_kernel for
-// the legacy formats with other K, a dense kernel for odd strides, MUL_MAT_ID's grouping, and the entry points.
+// mmq_pair.cuh holds the kernel of almost every call (K a multiple of 256, dense rows); here are mmq_tc_kernel for rows of 32-value blocks with other
+// K, a dense kernel for stacks at odd strides, MUL_MAT_ID's grouping, and the entry points.
 // Why bf16 and not kind::i8: per-32 (per-16 for Q6_K) group scales would force a TMEM read-out after every K=32 MMA,
 // which is epilogue-bound; bf16 operands keep the whole K loop inside the tensor pipe.  Activations carry 8 mantissa bits
 // (q8_1 carries 7 + sign per 32-block), weights are rounded once from their exact f32 dequantised value.
@@ -92,22 +92,19 @@ __host__ __device__ constexpr unsigned umma_idesc_bf16(int M, int N) {
 }
 
 // ---------------------------------------------------------------- raw block loads from 2-byte aligned global addresses
-// G = true: global memory through the read-only path; false: shared memory (raw blocks staged by the bulk-copy engine)
-template <bool G> __device__ __forceinline__ unsigned ld32(const unsigned *q) { if constexpr (G) return __ldg(q); else return *q; }
-template <bool G> __device__ __forceinline__ uint4 ld128(const uint4 *q) { if constexpr (G) return __ldg(q); else return *q; }
-template <bool G, int NW>
+template <int NW>
 __device__ __forceinline__ void ld_words(const unsigned char *p, unsigned (&w)[NW]) {
     const uintptr_t a = (uintptr_t)p;
     const unsigned *q = reinterpret_cast<const unsigned *>(a & ~(uintptr_t)3);
     const unsigned sh = (unsigned)(a & 3) * 8;
     if (sh == 0) {
 #pragma unroll
-        for (int i = 0; i < NW; i++) w[i] = ld32<G>(q + i);
+        for (int i = 0; i < NW; i++) w[i] = __ldg(q + i);
     } else {
-        unsigned prev = ld32<G>(q);
+        unsigned prev = __ldg(q);
 #pragma unroll
         for (int i = 0; i < NW; i++) {
-            const unsigned nxt = ld32<G>(q + i + 1);
+            const unsigned nxt = __ldg(q + i + 1);
             w[i] = __funnelshift_r(prev, nxt, sh);
             prev = nxt;
         }
@@ -121,21 +118,20 @@ __device__ __forceinline__ unsigned pack_bf16(float a, float b) {
 }
 
 // ---------------------------------------------------------------- 64 consecutive weights of one row -> 32 packed bf16x2 words
-// `row` points at the row's first block, kb is the 64-value step.  Arithmetic follows dequantize_row_* (ggml-quants.c:1523,
-// 1617, 2556, 2764, 2978) in f32; the result is rounded once to bf16.
+// Formats with blocks of 32 values.  Arithmetic follows dequantize_row_* (ggml-quants.c:1523, 1617) in f32; the result is rounded once to bf16.
 #define BYTE_OF(w, i) (((w)[(i) >> 2] >> (8 * ((i) & 3))) & 0xffu)
 
 // bytes of the 256-value group a K-step of 64 belongs to (one K-quant super-block, or 8 q4_0 / q8_0 blocks)
 __host__ __device__ constexpr int group256_bytes(int t) { return type_block_bytes(t) * 256 / type_block_values(t); }
 
-template <int TYPE, bool G>
+template <int TYPE>
 struct Dequant64;  // run(g, c, o): g -> first byte of the 256-value group, c = 64-value chunk 0..3 inside it
 
-template <bool G>
-struct Dequant64<B200_TYPE_Q4_0, G> {
+template <>
+struct Dequant64<B200_TYPE_Q4_0> {
     static __device__ __forceinline__ void run(const unsigned char *g, int c, unsigned (&o)[32]) {
         unsigned w[9];
-        ld_words<G, 9>(g + c * 2 * Q4_0_BYTES, w);
+        ld_words<9>(g + c * 2 * Q4_0_BYTES, w);
 #pragma unroll
         for (int b = 0; b < 2; b++) {
             const float d = __half2float(__ushort_as_half((unsigned short)(BYTE_OF(w, 18 * b) | (BYTE_OF(w, 18 * b + 1) << 8))));
@@ -156,13 +152,13 @@ struct LegacyLayout {
     static constexpr bool HAS_M = TYPE != B200_TYPE_Q5_0, HAS_H = TYPE != B200_TYPE_Q4_1;
     static constexpr int BB = type_block_bytes(TYPE), QH = 2 + (HAS_M ? 2 : 0), QS = QH + (HAS_H ? 4 : 0);
 };
-template <int TYPE, bool G>
+template <int TYPE>
 struct Dequant64Legacy {
     static __device__ __forceinline__ void run(const unsigned char *g, int c, unsigned (&o)[32]) {
         using L = LegacyLayout<TYPE>;
         constexpr int NWL = (2 * L::BB + 3) / 4;
         unsigned w[NWL];
-        ld_words<G, NWL>(g + c * 2 * L::BB, w);
+        ld_words<NWL>(g + c * 2 * L::BB, w);
 #pragma unroll
         for (int b = 0; b < 2; b++) {
             const int base = L::BB * b;
@@ -183,11 +179,11 @@ struct Dequant64Legacy {
         }
     }
 };
-template <bool G> struct Dequant64<B200_TYPE_Q4_1, G> : Dequant64Legacy<B200_TYPE_Q4_1, G> {};
-template <bool G> struct Dequant64<B200_TYPE_Q5_0, G> : Dequant64Legacy<B200_TYPE_Q5_0, G> {};
-template <bool G> struct Dequant64<B200_TYPE_Q5_1, G> : Dequant64Legacy<B200_TYPE_Q5_1, G> {};
+template <> struct Dequant64<B200_TYPE_Q4_1> : Dequant64Legacy<B200_TYPE_Q4_1> {};
+template <> struct Dequant64<B200_TYPE_Q5_0> : Dequant64Legacy<B200_TYPE_Q5_0> {};
+template <> struct Dequant64<B200_TYPE_Q5_1> : Dequant64Legacy<B200_TYPE_Q5_1> {};
 
-// IQ4_NL / IQ4_XS (dequantize_row_iq4_nl / iq4_xs, ggml-quants.c:3743-3785): dl * level[nibble], the levels looked up eight at a
+// IQ4_NL (dequantize_row_iq4_nl, ggml-quants.c:3743): dl * level[nibble], the levels looked up eight at a
 // time with the byte permute unit (iq4_levels, b200_common.cuh).  q(k) must yield byte k of the sub-block's 16 nibble bytes;
 // o16[0..7] receive values 0..15 (low nibbles), o16[8..15] values 16..31 (high nibbles).
 template <int K> __device__ __forceinline__ float s8_f(unsigned x) { return (float)(int)(signed char)((x >> (8 * K)) & 0xffu); }
@@ -208,11 +204,11 @@ __device__ __forceinline__ void iq4_unpack32(QFn q, float dl, unsigned *o16) {
 __device__ __forceinline__ float iq4xs_scale(unsigned sl, unsigned sh, int ib) {
     return (float)((int)(((sl >> (4 * ib)) & 0xFu) | (((sh >> (2 * ib)) & 3u) << 4)) - 32);
 }
-template <bool G>
-struct Dequant64<B200_TYPE_IQ4_NL, G> {
+template <>
+struct Dequant64<B200_TYPE_IQ4_NL> {
     static __device__ __forceinline__ void run(const unsigned char *g, int c, unsigned (&o)[32]) {
         unsigned w[9];
-        ld_words<G, 9>(g + c * 2 * IQ4_NL_BYTES, w);
+        ld_words<9>(g + c * 2 * IQ4_NL_BYTES, w);
 #pragma unroll
         for (int b = 0; b < 2; b++) {
             const int base = IQ4_NL_BYTES * b;
@@ -221,24 +217,11 @@ struct Dequant64<B200_TYPE_IQ4_NL, G> {
         }
     }
 };
-template <bool G>
-struct Dequant64<B200_TYPE_IQ4_XS, G> {
-    static __device__ __forceinline__ void run(const unsigned char *blk, int c, unsigned (&o)[32]) {
-        unsigned hdr[2], qw[8];
-        ld_words<G, 2>(blk, hdr);
-        ld_words<G, 8>(blk + 8 + 32 * c, qw);
-        const float d = f16lo(hdr[0]);
-#pragma unroll
-        for (int b = 0; b < 2; b++)
-            iq4_unpack32([&](int k) { return BYTE_OF(qw, 16 * b + k); }, d * iq4xs_scale(hdr[1], hdr[0] >> 16, 2 * c + b), o + 16 * b);
-    }
-};
-
-template <bool G>
-struct Dequant64<B200_TYPE_Q8_0, G> {
+template <>
+struct Dequant64<B200_TYPE_Q8_0> {
     static __device__ __forceinline__ void run(const unsigned char *g, int c, unsigned (&o)[32]) {
         unsigned w[17];
-        ld_words<G, 17>(g + c * 2 * Q8_0_BYTES, w);
+        ld_words<17>(g + c * 2 * Q8_0_BYTES, w);
 #pragma unroll
         for (int b = 0; b < 2; b++) {
             const float d = __half2float(__ushort_as_half((unsigned short)(BYTE_OF(w, 34 * b) | (BYTE_OF(w, 34 * b + 1) << 8))));
@@ -246,122 +229,6 @@ struct Dequant64<B200_TYPE_Q8_0, G> {
             for (int j = 0; j < 32; j += 2) {
                 const int q0 = (int)(signed char)BYTE_OF(w, 34 * b + 2 + j), q1 = (int)(signed char)BYTE_OF(w, 34 * b + 3 + j);
                 o[16 * b + j / 2] = pack_bf16(d * (float)q0, d * (float)q1);
-            }
-        }
-    }
-};
-
-template <int TYPE, bool G>
-struct DequantK45 {  // Q4_K / Q5_K: half d, half dmin, u8 scales[12], (u8 qh[32],) u8 qs[128]
-    static __device__ __forceinline__ void run(const unsigned char *blk, int c, unsigned (&o)[32]) {
-        const uint4 hdr = ld128<G>(reinterpret_cast<const uint4 *>(blk));  // rows are 16-byte aligned (checked on the host)
-        const float d = f16lo(hdr.x), dmin = f16hi(hdr.x);
-        const unsigned sw[3] = {hdr.y, hdr.z, hdr.w};
-        const uint4 *qp = reinterpret_cast<const uint4 *>(blk + (TYPE == B200_TYPE_Q4_K ? 16 : 48) + 32 * c);
-        const uint4 qa = ld128<G>(qp), qb = ld128<G>(qp + 1);
-        const unsigned q[8] = {qa.x, qa.y, qa.z, qa.w, qb.x, qb.y, qb.z, qb.w};
-        unsigned h[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-        if constexpr (TYPE == B200_TYPE_Q5_K) {
-            const uint4 ha = ld128<G>(reinterpret_cast<const uint4 *>(blk + 16)), hb = ld128<G>(reinterpret_cast<const uint4 *>(blk + 32));
-            h[0] = ha.x; h[1] = ha.y; h[2] = ha.z; h[3] = ha.w; h[4] = hb.x; h[5] = hb.y; h[6] = hb.z; h[7] = hb.w;
-        }
-#pragma unroll
-        for (int hf = 0; hf < 2; hf++) {  // hf = 0: low nibbles (sub-block 2c), 1: high nibbles (sub-block 2c+1)
-            const int sb = 2 * c + hf;
-            int sc, mn;
-            k4_scale_min(sw, sb, sc, mn);
-            const float d1 = d * (float)sc, m1 = dmin * (float)mn;
-#pragma unroll
-            for (int l = 0; l < 32; l += 2) {
-                unsigned q0 = (BYTE_OF(q, l) >> (4 * hf)) & 15, q1 = (BYTE_OF(q, l + 1) >> (4 * hf)) & 15;
-                if constexpr (TYPE == B200_TYPE_Q5_K) {
-                    q0 += ((BYTE_OF(h, l) >> sb) & 1) << 4;
-                    q1 += ((BYTE_OF(h, l + 1) >> sb) & 1) << 4;
-                }
-                o[16 * hf + l / 2] = pack_bf16(d1 * (float)q0 - m1, d1 * (float)q1 - m1);
-            }
-        }
-    }
-};
-template <bool G> struct Dequant64<B200_TYPE_Q4_K, G> : DequantK45<B200_TYPE_Q4_K, G> {};
-template <bool G> struct Dequant64<B200_TYPE_Q5_K, G> : DequantK45<B200_TYPE_Q5_K, G> {};
-
-// Q2_K / Q3_K (dequantize_row_q2_K / q3_K, ggml-quants.c:1980-2010, 2328-2373).  Chunk c (64 values) of a super-block is half
-// n = c >> 1, bit fields jb = 2 (c & 1) and jb + 1 of the half's 32 quant bytes; value vv of the chunk: field jb + vv / 32, byte
-// vv % 32, scale 8 n + 2 (jb + vv / 32) + (vv % 32) / 16.  W(i) must yield byte i of the block.
-template <int TYPE, typename ByteFn>
-__device__ __forceinline__ void dequant64_k23(ByteFn W, int c, unsigned (&o)[32]) {
-    constexpr bool Q2 = TYPE == B200_TYPE_Q2_K;
-    const int n = c >> 1, jb = 2 * (c & 1);
-    unsigned aux[4] = {0, 0, 0, 0};
-    float d, dmin = 0.f;
-    if constexpr (Q2) {
-        d = __half2float(__ushort_as_half((unsigned short)(W(80) | (W(81) << 8))));
-        dmin = __half2float(__ushort_as_half((unsigned short)(W(82) | (W(83) << 8))));
-    } else {
-        d = __half2float(__ushort_as_half((unsigned short)(W(108) | (W(109) << 8))));
-        unsigned sw[3];
-#pragma unroll
-        for (int k = 0; k < 3; k++) sw[k] = W(96 + 4 * k) | (W(97 + 4 * k) << 8) | (W(98 + 4 * k) << 16) | (W(99 + 4 * k) << 24);
-        q3k_scales(sw[0], sw[1], sw[2], aux);
-    }
-#pragma unroll
-    for (int gq = 0; gq < 4; gq++) {  // 16-value groups of the chunk
-        const int jj = jb + (gq >> 1), is = 8 * n + 2 * jj + (gq & 1);
-        float dl, ml = 0.f;
-        if constexpr (Q2) {
-            const unsigned sc = W(is);
-            dl = d * (float)(sc & 0xF);
-            ml = dmin * (float)(sc >> 4);
-        } else {
-            dl = d * (float)((int)((aux[is >> 2] >> (8 * (is & 3))) & 0xff) - 32);
-        }
-#pragma unroll
-        for (int e = 0; e < 16; e += 2) {
-            const int l = 16 * (gq & 1) + e;
-            const unsigned b0 = W((Q2 ? 16 : 32) + 32 * n + l), b1 = W((Q2 ? 16 : 32) + 32 * n + l + 1);
-            float x0 = (float)((b0 >> (2 * jj)) & 3), x1 = (float)((b1 >> (2 * jj)) & 3);
-            if constexpr (!Q2) {
-                x0 -= ((W(l) >> (4 * n + jj)) & 1) ? 0.f : 4.f;
-                x1 -= ((W(l + 1) >> (4 * n + jj)) & 1) ? 0.f : 4.f;
-            }
-            o[8 * gq + e / 2] = pack_bf16(dl * x0 - ml, dl * x1 - ml);
-        }
-    }
-}
-template <int TYPE, bool G>
-struct Dequant64K23 {
-    static __device__ __forceinline__ void run(const unsigned char *blk, int c, unsigned (&o)[32]) {
-        constexpr int NWB = (type_block_bytes(TYPE) + 3) / 4;
-        unsigned w[NWB];
-        ld_words<G, NWB>(blk, w);
-        dequant64_k23<TYPE>([&](int i) { return BYTE_OF(w, i); }, c, o);
-    }
-};
-template <bool G> struct Dequant64<B200_TYPE_Q2_K, G> : Dequant64K23<B200_TYPE_Q2_K, G> {};
-template <bool G> struct Dequant64<B200_TYPE_Q3_K, G> : Dequant64K23<B200_TYPE_Q3_K, G> {};
-
-template <bool G>
-struct Dequant64<B200_TYPE_Q6_K, G> {  // u8 ql[128], u8 qh[64], i8 scales[16], half d   (2-byte aligned blocks)
-    static __device__ __forceinline__ void run(const unsigned char *blk, int c, unsigned (&o)[32]) {
-        const int half = c >> 1, hi = c & 1;
-        unsigned ql[16], qh[8], sc[1], dw[1];
-        ld_words<G, 16>(blk + 64 * half, ql);
-        ld_words<G, 8>(blk + 128 + 32 * half, qh);
-        ld_words<G, 1>(blk + 192 + 8 * half + 4 * hi, sc);
-        ld_words<G, 1>(blk + 208, dw);
-        const float d = f16lo(dw[0]);
-#pragma unroll
-        for (int g = 0; g < 4; g++) {  // 16-value groups: jj = 16g .. 16g+15, one int8 scale each
-            const float ds = d * (float)(int)(signed char)BYTE_OF(sc, g);
-            const int rlow = g >> 1, r = 2 * hi + rlow;
-#pragma unroll
-            for (int e = 0; e < 16; e += 2) {
-                const int l = 16 * (g & 1) + e;
-                const unsigned b0 = BYTE_OF(ql, 32 * rlow + l), b1 = BYTE_OF(ql, 32 * rlow + l + 1);
-                const unsigned n0 = hi ? (b0 >> 4) : (b0 & 15), n1 = hi ? (b1 >> 4) : (b1 & 15);
-                const unsigned h0 = (BYTE_OF(qh, l) >> (2 * r)) & 3, h1 = (BYTE_OF(qh, l + 1) >> (2 * r)) & 3;
-                o[8 * g + e / 2] = pack_bf16(ds * (float)((int)(n0 | (h0 << 4)) - 32), ds * (float)((int)(n1 | (h1 << 4)) - 32));
             }
         }
     }
@@ -390,16 +257,16 @@ struct MmqParams {
     const __nv_bfloat16 *Xb;  // [n_pad][K]
     float *dst;
     int64_t dst_stride, K, M, N;
-    // grouped mode (MUL_MAT_ID batches, b200_mul_mat_id_q): blockIdx.y indexes a device-built tile table {n_tiles, (expert, first
+    // grouped mode (MUL_MAT_ID batches, b200_mul_mat_id_q): a device-built tile table {n_tiles, (expert, first
     // sorted row, end row) ...}; W advances by expert_bytes per expert; sorted row i is stored at dst[row_dst[i] + m]
     const int *tile_tab;
     const int *row_dst;
     size_t expert_bytes;
-    // split-K (mmq_tc2_kernel, not grouped): blockIdx.z owns a contiguous share of the 256-value groups and ADDS its tile into a
-    // zeroed dst (red.global.add.f32).  Only 1 or 2: the sum of two partials does not depend on their arrival order.
+    // split-K (mmq_pair_kernel, one product): a tile owns a contiguous share of K and ADDS its sums into a zeroed dst (red.global.add.f32).  Only 1
+    // or 2: the sum of two partials does not depend on their arrival order.
     int ksplit;
-    // batch of independent products of one shape (not grouped, no split-K): blockIdx.z picks the product; W advances by
-    // w_batch_bytes, dst by dst_batch floats, the bf16 activations by n_pad rows
+    // batch of independent products of one shape (not grouped, no split-K): W advances by w_batch_bytes, dst by dst_batch floats, the
+    // bf16 activations by n_pad rows
     int n_batch;
     size_t w_batch_bytes;
     int64_t dst_batch, n_pad;
@@ -453,7 +320,7 @@ __global__ void __launch_bounds__(MQ_THREADS, 1) mmq_tc_kernel(const __grid_cons
             }
             cp_async_commit();
             unsigned o[32];
-            if (row_ok) Dequant64<TYPE, true>::run(wrow + (size_t)(kb >> 2) * group256_bytes(TYPE), kb & 3, o);
+            if (row_ok) Dequant64<TYPE>::run(wrow + (size_t)(kb >> 2) * group256_bytes(TYPE), kb & 3, o);
             else {
 #pragma unroll
                 for (int i = 0; i < 32; i++) o[i] = 0u;
@@ -531,10 +398,9 @@ __device__ __forceinline__ void tma_load_2d(void *dst, const void *tmap, int c0,
 
 struct alignas(64) TmapBytes { unsigned char b[128]; };  // CUtensorMap without pulling <cuda.h> into device code
 
-template <int TYPE, int BN, bool GROUPED = false>
+template <int BN, bool GROUPED>  // GROUPED: experts; else a batch of products
 __global__ void __launch_bounds__(MQ2_THREADS, 1) mmq_tc2_kernel(const __grid_constant__ TmapBytes tmB, const __grid_constant__ MmqParams p) {
     constexpr int A_BYTES = MQ_BM * MQ_BK * 2, B_BYTES = BN * MQ_BK * 2, STAGE_BYTES = A_BYTES + B_BYTES;
-    constexpr int G256 = group256_bytes(TYPE);
     int64_t n0 = (int64_t)blockIdx.y * BN, n_end = p.N;
     const unsigned char *Wbase = p.W;
     if constexpr (GROUPED) {  // uniform over the CTA: tiles past the table's end have nothing to do
@@ -551,16 +417,8 @@ __global__ void __launch_bounds__(MQ2_THREADS, 1) mmq_tc2_kernel(const __grid_co
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, tid = threadIdx.x;
     const int64_t m0 = (int64_t)blockIdx.x * MQ_BM;
-    // K steps (64 values) per group: quantised formats are unpacked 256 values at a time, dense bf16 rows step by step
-    constexpr int KPG = TYPE == B200_TYPE_BF16 ? 1 : 4;
-    const int nsb_all = (int)(p.K / (MQ_BK * KPG));
-    // split-K: this CTA's groups [sb0, sb0 + nsb)
-    const int ksplit = GROUPED ? 1 : p.ksplit;
-    const bool batched = !GROUPED && p.n_batch > 1;
-    const int zk = batched ? 0 : (int)blockIdx.z, zb = batched ? (int)blockIdx.z : 0;
-    if (batched) Wbase += (size_t)zb * p.w_batch_bytes;
-    const int sb0 = (int)(((int64_t)zk * nsb_all) / ksplit);
-    const int nsb = (int)(((int64_t)(zk + 1) * nsb_all) / ksplit) - sb0, nkb = nsb * KPG;
+    const int nkb = (int)(p.K / MQ_BK), zb = GROUPED ? 0 : (int)blockIdx.z;
+    if (!GROUPED) Wbase += (size_t)zb * p.w_batch_bytes;
 
     if (tid == 0) {
         for (int s = 0; s < MQ2_STAGES; s++) { mbar_init(&full_bar[s], MQ_PRODUCERS + 1); mbar_init(&empty_bar[s], 1); }
@@ -590,7 +448,7 @@ __global__ void __launch_bounds__(MQ2_THREADS, 1) mmq_tc2_kernel(const __grid_co
         };
         {
             // dense bf16 rows: a K step is 128 bytes of the thread's row, stored as it is; the next step's bytes are in flight meanwhile
-            const uint4 *q4 = reinterpret_cast<const uint4 *>(wrow) + (size_t)sb0 * 8;
+            const uint4 *q4 = reinterpret_cast<const uint4 *>(wrow);
             uint4 cur[8], nxt[8];
 #pragma unroll
             for (int i = 0; i < 8; i++) cur[i] = row_ok ? __ldg(q4 + i) : make_uint4(0u, 0u, 0u, 0u);
@@ -610,7 +468,7 @@ __global__ void __launch_bounds__(MQ2_THREADS, 1) mmq_tc2_kernel(const __grid_co
         }
         mbar_wait(&tmem_full_bar, 0u);
         tc_fence_after();
-        float *drow = p.dst + m + (batched ? (int64_t)zb * p.dst_batch : 0);
+        float *drow = p.dst + m + (int64_t)zb * p.dst_batch;
 #pragma unroll 1
         for (int c0 = 0; c0 < BN; c0 += 32) {
             float v[32];
@@ -619,14 +477,9 @@ __global__ void __launch_bounds__(MQ2_THREADS, 1) mmq_tc2_kernel(const __grid_co
 #pragma unroll
                 for (int j = 0; j < 32; j++) {
                     const int64_t n = n0 + c0 + j;
-                    if constexpr (GROUPED) {
-                        if (n < n_end) drow[(int64_t)__ldg(p.row_dst + n)] = v[j];  // scatter: sorted row -> (token, slot)
-                    } else {
-                        if (n < n_end) {
-                            if (ksplit > 1) atomicAdd(drow + n * p.dst_stride, v[j]);  // (result unused: RED.ADD.F32)
-                            else drow[n * p.dst_stride] = v[j];
-                        }
-                    }
+                    if (n >= n_end) continue;
+                    if constexpr (GROUPED) drow[(int64_t)__ldg(p.row_dst + n)] = v[j];  // scatter: sorted row -> (token, slot)
+                    else drow[n * p.dst_stride] = v[j];
                 }
             }
         }
@@ -655,7 +508,7 @@ __global__ void __launch_bounds__(MQ2_THREADS, 1) mmq_tc2_kernel(const __grid_co
                 const int s = kb % MQ2_STAGES;
                 mbar_wait(&empty_bar[s], ((unsigned)(kb / MQ2_STAGES) & 1u) ^ 1u);
                 mbar_expect_tx(&full_bar[s], (unsigned)B_BYTES);
-                tma_load_2d(smem + (size_t)s * STAGE_BYTES + A_BYTES, &tmB, (sb0 * KPG + kb) * MQ_BK, (int)n0 + (batched ? zb * (int)p.n_pad : 0), &full_bar[s]);
+                tma_load_2d(smem + (size_t)s * STAGE_BYTES + A_BYTES, &tmB, kb * MQ_BK, (int)n0 + zb * (int)p.n_pad, &full_bar[s]);
             }
         }
     }
@@ -734,7 +587,7 @@ static int encode_rows(TmapBytes &tm, const void *base, int64_t K, int64_t rows,
 #include "mmq_pair.cuh"
 namespace b200 {
 
-template <int TYPE, int BN, bool GROUPED = false>
+template <int BN, bool GROUPED>
 static int mmq2_launch(const MmqParams &p, int64_t n_pad, cudaStream_t st, unsigned grid_y = 0) {
     constexpr size_t smem = (size_t)MQ2_STAGES * (MQ_BM * MQ_BK * 2 + BN * MQ_BK * 2) + 1024;
     static bool attr_set_dev[16] = {};  // cudaFuncSetAttribute is per device
@@ -742,36 +595,14 @@ static int mmq2_launch(const MmqParams &p, int64_t n_pad, cudaStream_t st, unsig
     B200_CUDA_TRY(cudaGetDevice(&cur_dev));
     bool &attr_set = attr_set_dev[cur_dev & 15];
     if (!attr_set) {
-        B200_CUDA_TRY(cudaFuncSetAttribute(mmq_tc2_kernel<TYPE, BN, GROUPED>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        B200_CUDA_TRY(cudaFuncSetAttribute(mmq_tc2_kernel<BN, GROUPED>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         attr_set = true;
     }
-    EncodeTiledFn enc = encode_tiled_fn();
-    if (!enc) { set_error("b200_mul_mat_q: cuTensorMapEncodeTiled not available"); return B200_ERR_CUDA; }
     TmapBytes tm;
-    const unsigned long long gdim[2] = {(unsigned long long)p.K, (unsigned long long)n_pad * (unsigned long long)(p.n_batch > 1 ? p.n_batch : 1)};
-    const unsigned long long gstr[1] = {(unsigned long long)p.K * 2};
-    const unsigned box[2] = {(unsigned)MQ_BK, (unsigned)BN};
-    const unsigned estr[2] = {1, 1};
-    // CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 = 9, INTERLEAVE_NONE = 0, SWIZZLE_128B = 3, L2_PROMOTION_L2_256B = 3, FLOAT_OOB_FILL_NONE = 0
-    const int rc = enc(&tm, 9, 2, (void *)p.Xb, gdim, gstr, box, estr, 0, 3, 3, 0);
-    if (rc != 0) { set_error("b200_mul_mat_q: cuTensorMapEncodeTiled failed (%d)", rc); return B200_ERR_CUDA; }
-    dim3 grid((unsigned)((p.M + MQ_BM - 1) / MQ_BM), GROUPED ? grid_y : (unsigned)((p.N + BN - 1) / BN));
-    MmqParams q = p;
-    q.ksplit = 1;
-    if constexpr (!GROUPED) {
-        // fewer tiles than half the SMs (M = 4096 x N = 512: 64 CTAs, every one bound by its own 128 dequantising threads): two
-        // CTAs share a tile's K range and add into a zeroed dst.  Two partials only: the sum is independent of the arrival order.
-        static const bool no_split = getenv("B200_MMQ_NO_SPLITK") != nullptr;
-        if (p.n_batch > 1) {
-            grid.z = (unsigned)p.n_batch;
-        } else if (!no_split && (int64_t)grid.x * grid.y * 2 <= 148 && p.K >= 2048) {
-            q.ksplit = 2;
-            grid.z = 2;
-            if (p.dst_stride == p.M) B200_CUDA_TRY(cudaMemsetAsync(p.dst, 0, (size_t)p.M * p.N * sizeof(float), st));
-            else B200_CUDA_TRY(cudaMemset2DAsync(p.dst, (size_t)p.dst_stride * sizeof(float), 0, (size_t)p.M * sizeof(float), (size_t)p.N, st));
-        }
-    }
-    mmq_tc2_kernel<TYPE, BN, GROUPED><<<grid, MQ2_THREADS, smem, st>>>(tm, q);
+    const int rc = encode_rows(tm, p.Xb, p.K, n_pad * p.n_batch, (size_t)p.K * 2, BN);
+    if (rc != B200_OK) return rc;
+    const dim3 grid((unsigned)((p.M + MQ_BM - 1) / MQ_BM), GROUPED ? grid_y : (unsigned)((p.N + BN - 1) / BN), (unsigned)p.n_batch);
+    mmq_tc2_kernel<BN, GROUPED><<<grid, MQ2_THREADS, smem, st>>>(tm, p);
     B200_CUDA_TRY(cudaGetLastError());
     return B200_OK;
 }
@@ -783,14 +614,15 @@ static int mmq_dispatch_bn(const MmqParams &p, cudaStream_t st) {
         // products whose weight rows lie at one stride over all of them: one tensor map covers the stack
         if (p.n_batch == 1 || p.w_batch_bytes % p.w_row_bytes == 0) return mmq_pair_launch<TYPE, false>(p, n_pad, p.n_batch > 1 ? (int64_t)(p.w_batch_bytes / p.w_row_bytes) : 0, 0, 0, st);
         switch (mmq_bn(p.N)) {
-            case 32: return mmq2_launch<TYPE, 32>(p, n_pad, st);
-            case 64: return mmq2_launch<TYPE, 64>(p, n_pad, st);
-            case 128: return mmq2_launch<TYPE, 128>(p, n_pad, st);
-            default: return mmq2_launch<TYPE, 256>(p, n_pad, st);
+            case 32: return mmq2_launch<32, false>(p, n_pad, st);
+            case 64: return mmq2_launch<64, false>(p, n_pad, st);
+            case 128: return mmq2_launch<128, false>(p, n_pad, st);
+            default: return mmq2_launch<256, false>(p, n_pad, st);
         }
-    } else
-    if (p.K % 256 == 0) return mmq_pair_launch<TYPE, false>(p, mmq_n_pad(p.N), 0, 0, 0, st);
-    if constexpr (TYPE != B200_TYPE_BF16) {
+    } else {
+        if (p.K % 256 == 0) return mmq_pair_launch<TYPE, false>(p, mmq_n_pad(p.N), 0, 0, 0, st);
+    }
+    if constexpr (type_block_values(TYPE) == 32) {  // (a K-quant's rows are whole groups of 256 values)
         switch (mmq_bn(p.N)) {
             case 32: return mmq_launch<TYPE, 32>(p, st);
             case 64: return mmq_launch<TYPE, 64>(p, st);
@@ -882,10 +714,10 @@ static int mid_dispatch_bn(const MmqParams &p, int64_t bn, int64_t n_rows, unsig
     if (mid_pair(TYPE, p.w_row_bytes, p.expert_bytes)) return mmq_pair_launch<TYPE, true>(p, n_rows, (int64_t)(p.expert_bytes / p.w_row_bytes), grid_y, bn, st);
     if constexpr (TYPE == B200_TYPE_BF16)
     switch (bn) {
-        case 32: return mmq2_launch<TYPE, 32, true>(p, n_rows, st, grid_y);
-        case 64: return mmq2_launch<TYPE, 64, true>(p, n_rows, st, grid_y);
-        case 128: return mmq2_launch<TYPE, 128, true>(p, n_rows, st, grid_y);
-        default: return mmq2_launch<TYPE, 256, true>(p, n_rows, st, grid_y);
+        case 32: return mmq2_launch<32, true>(p, n_rows, st, grid_y);
+        case 64: return mmq2_launch<64, true>(p, n_rows, st, grid_y);
+        case 128: return mmq2_launch<128, true>(p, n_rows, st, grid_y);
+        default: return mmq2_launch<256, true>(p, n_rows, st, grid_y);
     }
     return B200_ERR_UNSUPPORTED;
 }

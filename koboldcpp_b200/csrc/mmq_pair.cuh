@@ -115,7 +115,8 @@ __device__ __forceinline__ bool pair_wait(unsigned bar, unsigned parity, volatil
 // ---------------------------------------------------------------- 32 values of a row out of shared memory -> 16 packed bf16 pairs
 // Two values at a time (packed f32: one issue slot for both): four small unsigned integers, one per byte of x, become d * q + c as two bf16
 // pairs.  Integers below 128 take the upper mantissa bits of 128 (0x43qq0000 = 128 + q), so that PRMT alone makes the float and the 128
-// goes into the constant, c - 128 d: that constant is off by 2^-17 d at most, far below the bf16 rounding of the result.
+// goes into the constant, c - 128 d.  Without a minimum that constant is exact; with one (q4_K, q5_K, q2_K, q4_1, q5_1) it is rounded to f32, off by
+// 2^-17 d at most: small beside d, whatever is left of d q + c near 0.
 struct Scale2 { unsigned long long d, c; };
 __device__ __forceinline__ unsigned long long pack_f2(float a, float b) {
     unsigned long long r;

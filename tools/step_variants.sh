@@ -7,4 +7,3 @@ run B200_MMVQ_PREFILL=0
 run B200_MMVQ_PREFILL=2
 run B200_MMVQ_NO_MMVQ3=1
 run B200_FA_NO_CLUSTER=1
-run B200_MMQ_NO_SPLITK=1
