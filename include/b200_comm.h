@@ -1,6 +1,6 @@
 /* b200_comm.h -- the exchange step of the row-split (tensor-parallel) hot path: one process per GPU, NCCL over NVLink.
  *
- * Replaces the star-shaped peer copies of the reference's multi-GPU matmul loop (/root/reference/ggml/src/ggml-cuda.cu:1519-1657:
+ * Replaces the star-shaped peer copies of the reference's multi-GPU matmul loop (ggml/src/ggml-cuda.cu:1519-1657:
  * broadcast the quantised activations from the main GPU, gather output rows back, 2 peer memcpys + 2 event waits per device per
  * matmul from one host thread) with collectives that live INSIDE the captured decode graph:
  *   - weights that produce a layer's hidden state (attn_output, ffn_down) are split along K: every rank holds K/W columns and

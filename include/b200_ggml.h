@@ -1,7 +1,7 @@
 /* b200_ggml.h -- kernel-level C ABI of the B200-native GGML hot path (libkcpp_b200.so).
  *
  * Plain C: raw device pointers, sizes, strides and a CUDA stream handle.  No torch / C++ types.
- * Every entry point names the reference interface it replaces (paths under /root/reference/).
+ * Every entry point names the reference interface it replaces (paths within the reference's tree).
  * The ggml_backend-level drop-in boundary (reg / device / buffer type / buffer / backend vtables)
  * is declared in b200_ggml_backend.h and is built on top of these calls.
  *

@@ -1,12 +1,12 @@
 /* b200_ggml_abi.h -- the slice of the ggml ABI the B200 backend is called through.
  *
- * The drop-in boundary is the reference's ggml_backend interface (SURVEY.md 8b): the host program hands the
+ * The drop-in boundary is the reference's ggml_backend interface: the host program hands the
  * backend `struct ggml_tensor` / `struct ggml_cgraph` objects it built itself and calls through five vtables.
  * This header restates the binary layout of exactly those objects so that libkcpp_b200.so builds with no
  * reference checkout present.  It is an ABI description, not a copy of the reference headers: only the structs
  * that cross the boundary, and only the enum VALUES the backend dispatches on.
  *
- * Every definition cites the reference declaration it mirrors (paths under /root/reference/ggml/), and
+ * Every definition cites the reference declaration it mirrors (paths under ggml/), and
  * tests/cpp/abi_probe.cpp is compiled once against this file and once against the real headers and
  * tests/test_abi.py diffs every size, offset and enum value.  A maintainer integrating into a ggml tree compiles the backend with -DB200_USE_GGML_HEADERS instead,
  * which makes b200_ggml_backend.cpp include the tree's own ggml.h / ggml-backend-impl.h and skip this file.

@@ -1,12 +1,12 @@
 /* b200_ggml_backend.h -- the drop-in boundary: a ggml backend ("B200") behind the reference's own ggml_backend
- * interface (reg / device / buffer type / buffer / backend vtables, /root/reference/ggml/src/ggml-backend-impl.h).
+ * interface (reg / device / buffer type / buffer / backend vtables, ggml/src/ggml-backend-impl.h).
  *
- * Two ways to attach (SURVEY.md Appendix B):
+ * Two ways to attach:
  *   Route 2 (run time):  ggml_backend_register(ggml_backend_b200_reg());   before any llama_* call
  *   Route 1 (link time): link libkcpp_b200.so in place of ggml-cuda.o with -DGGML_USE_CUDA; the library also exports
  *                        the 12 public symbols of ggml/include/ggml-cuda.h:22-44 under their reference names.
  *
- * Each function cites the reference entry point it replaces (paths under /root/reference/ggml/).
+ * Each function cites the reference entry point it replaces (paths under ggml/).
  */
 #ifndef B200_GGML_BACKEND_H
 #define B200_GGML_BACKEND_H

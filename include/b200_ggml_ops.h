@@ -1,8 +1,8 @@
-/* b200_ggml_ops.h -- C ABI of the hot-path-adjacent ops (SURVEY.md 8f, row N1): everything else a llama / mixtral
+/* b200_ggml_ops.h -- C ABI of the hot-path-adjacent ops: everything else a llama / mixtral
  * graph contains, so that a whole decode graph stays on the device (no CPU fallback, CUDA-graph capturable).
  * Tensors are described the way ggml does: element counts ne[4] and BYTE strides nb[4] (ggml.h:584-619).
  * Each entry cites the reference CUDA kernel it replaces and the CPU function that defines its semantics
- * (paths under /root/reference/ggml/src/).
+ * (paths under ggml/src/).
  */
 #ifndef B200_GGML_OPS_H
 #define B200_GGML_OPS_H

@@ -1,8 +1,8 @@
 /* b200_llama.h -- C ABI of the host-side decoder that sits ABOVE the ggml_backend boundary (libkcpp_b200.so).
  *
- * This is the caller side of the hot path ("the callers either side of the path"): it does what
+ * This is the caller side of the hot path: it does what
  * llama.cpp does for a llama / mixtral model -- builds the per-batch ggml graph node for node like build_llama
- * (/root/reference/src/llama.cpp:10453-10617, llm_build_kv :9648-9680, llm_build_kv_store :9161-9203, llm_build_kqv
+ * (src/llama.cpp:10453-10617, llm_build_kv :9648-9680, llm_build_kv_store :9161-9203, llm_build_kqv
  * :9517-9646, llm_build_ffn :9289-9414, llm_build_moe_ffn :9416-9515), places weights / KV cache / activations in
  * buffers obtained through the backend's buffer-type vtable, feeds the graph inputs with set_tensor, and calls the
  * backend's graph_compute -- the same five vtables llama.cpp would call (b200_ggml_backend.h).  It exists so that

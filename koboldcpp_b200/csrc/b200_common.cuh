@@ -1,7 +1,7 @@
 // b200_common.cuh -- shared device helpers for the sm_100a kernels.
 //
 // Block layouts follow the reference's on-disk == in-memory GGUF formats
-// (/root/reference/ggml/src/ggml-common.h:144-335); we address bytes with explicit offsets
+// (ggml/src/ggml-common.h:144-335); we address bytes with explicit offsets
 // instead of packed structs because several formats are only 2-byte aligned (q4_0 18 B,
 // q8_0 34 B, q6_K 210 B) and the kernels read them out of shared memory with aligned-word
 // loads + funnel shifts.

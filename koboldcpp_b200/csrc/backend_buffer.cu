@@ -1,6 +1,6 @@
 // backend_buffer.cu -- buffer types and buffers of the B200 ggml backend (device, pinned host, row-split).
 //
-// Mirrors the contracts of /root/reference/ggml/src/ggml-cuda.cu:424-621 (device buffer + type), :623-953 (split buffer
+// Mirrors the contracts of ggml/src/ggml-cuda.cu:424-621 (device buffer + type), :623-953 (split buffer
 // + type), :955-1025 (host buffer type) behind the vtables of ggml-backend-impl.h:15-65.  Not a port: weights keep
 // their on-disk block layout (the GEMV streams raw blocks through the TMA engine), so set/get_tensor are plain copies
 // at any offset and no row padding is needed -- the buffer only over-allocates a fixed tail so kernels may read up to

@@ -1,5 +1,5 @@
 // backend_device.cu -- reg / device / backend (stream) objects of the B200 ggml backend.
-// Contracts: /root/reference/ggml/src/ggml-backend-impl.h:86-216; the reference implementation being replaced is
+// Contracts: ggml/src/ggml-backend-impl.h:86-216; the reference implementation being replaced is
 // ggml-cuda.cu:2355-2453 (backend), :2886-3256 (device), :3260-3340 (reg).
 #include <chrono>
 #include "backend_internal.h"

@@ -1,7 +1,7 @@
 // comm.cu -- the exchange step of the tensor-parallel hot path (include/b200_comm.h): a process-wide NCCL communicator,
 // loaded at run time so that single-GPU users of the library never need NCCL.
 //
-// Replaces the peer-copy star of ggml_cuda_op_mul_mat's split branch (/root/reference/ggml/src/ggml-cuda.cu:1519-1657,
+// Replaces the peer-copy star of ggml_cuda_op_mul_mat's split branch (ggml/src/ggml-cuda.cu:1519-1657,
 // ggml_cuda_Memcpy2DPeerAsync :1338-1356) with all-reduce / all-gather calls that are captured into the decode CUDA graph.
 #include <dlfcn.h>
 

@@ -1,7 +1,7 @@
 // fattn.cu -- (a10-a12) FLASH_ATTN_EXT over an f16 or q8_0 KV cache: split-K flash-decode with online softmax.
 //
 // Replaces flash_attn_vec_ext_f16/f32 + flash_attn_combine_results and (for now also) the wmma prefill kernel of
-// the reference (/root/reference/ggml/src/ggml-cuda/fattn-vec-f16.cuh:8-299, fattn-common.cuh:519-708,
+// the reference (ggml/src/ggml-cuda/fattn-vec-f16.cuh:8-299, fattn-common.cuh:519-708,
 // fattn-wmma-f16.cuh:13-506).  Semantics follow ggml_compute_forward_flash_attn_ext_f16 (ggml/src/ggml.c:15667-15877).
 //
 // B200 design (HBM-bound at decode: every K/V byte must be read exactly once and >= 40 KB kept in flight per SM):

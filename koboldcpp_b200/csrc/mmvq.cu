@@ -2,7 +2,7 @@
 // plus the expert-indexed (MUL_MAT_ID) and multi-matrix (fused Q/K/V, gate/up) forms.
 //
 // Replaces the reference's quantize_q8_1 + mul_mat_vec_q<type,ncols_y> pair
-// (/root/reference/ggml/src/ggml-cuda/quantize.cu:4-38, mmvq.cu:50-202, vecdotq.cuh:23-787) and, for MUL_MAT_ID,
+// (ggml/src/ggml-cuda/quantize.cu:4-38, mmvq.cu:50-202, vecdotq.cuh:23-787) and, for MUL_MAT_ID,
 // the host round trip in ggml_cuda_mul_mat_id (ggml-cuda.cu:2003-2139).
 //
 // B200 design (HBM-bound: the job is to keep >= ~40 KB of weight bytes in flight per SM and never touch a byte twice):

@@ -1,6 +1,6 @@
-// ops.cu -- the hot-path-adjacent ops of a llama / mixtral graph, so a whole decode graph runs on
+// ops.cu -- the hot-path-adjacent ops of a llama / mixtral graph so a whole decode graph runs on
 // the device with no CPU fallback.  All of them are HBM/L2-bound elementwise or row-reduction kernels; the design rule
-// is vector access + one pass.  Semantics cite /root/reference/ggml/src/ggml.c; see include/b200_ggml_ops.h.
+// is vector access + one pass.  Semantics cite the reference's ggml/src/ggml.c; see include/b200_ggml_ops.h.
 #include "b200_common.cuh"
 
 #include <cuda_bf16.h>

@@ -1,6 +1,6 @@
 // quantize.cu -- (a2) bit-exact block dequantisation and (a3) f32 -> q8_1 activation quantisation.
 //
-// Reference semantics (paths under /root/reference/ggml/src/):
+// Reference semantics (paths under ggml/src/):
 //   dequantize_row_{q4_0,q8_0,q4_K,q5_K,q6_K}   ggml-quants.c:1523, 1617, 2556, 2764, 2978
 //   quantize_row_q8_1_ref                       ggml-quants.c:1160-1193
 // The reference C is compiled without FMA contraction (-std=c11), so every multiply / subtract is its own

@@ -1,7 +1,7 @@
 """Python mirror of include/b200_llama.h: the llama / mixtral decoder that drives the B200 backend through the
 ggml_backend vtables, plus synthetic (random-init) GGUF-shaped models for the configurations BASELINE.json names.
 
-The type mix per tensor follows llama_tensor_get_type for Q4_0 / Q4_K_M / Q5_K_M (/root/reference/src/llama.cpp:17979-18200).
+The type mix per tensor follows llama_tensor_get_type for Q4_0 / Q4_K_M / Q5_K_M (src/llama.cpp:17979-18200).
 """
 from __future__ import annotations
 
@@ -103,7 +103,7 @@ class ModelShape:
 
 
 SHAPES = {
-    # SURVEY.md section 8 table (standard public hyper-parameters)
+    # standard public hyper-parameters
     "tinyllama-1.1b-q4_0": ModelShape("tinyllama-1.1b-q4_0", 2048, 22, 32, 4, 5632, 32000, "Q4_0"),
     "llama2-7b-q4_k_m": ModelShape("llama2-7b-q4_k_m", 4096, 32, 32, 32, 11008, 32000, "Q4_K_M"),
     "llama2-13b-q5_k_m": ModelShape("llama2-13b-q5_k_m", 5120, 40, 40, 40, 13824, 32000, "Q5_K_M"),
@@ -177,7 +177,7 @@ def tensor_shape(s: ModelShape, name: str) -> tuple[int, int, int]:
 
 
 def weight_bytes_per_token(s: ModelShape) -> int:
-    """Bytes of weights one decoded token must stream (SURVEY.md 8d): every matrix once, experts: n_expert_used of n_expert;
+    """Bytes of weights one decoded token must stream: every matrix once, experts: n_expert_used of n_expert;
     the token_embd row and the f32 norm vectors are not counted."""
     total = 0
     for name, ty in tensor_types(s).items():
@@ -316,7 +316,7 @@ class LlamaModel:
             seen[key] = name
 
     def kv_fill_random(self, n_cells: int, seed: int = 7) -> None:
-        """Fill KV cells [0, n_cells) of every layer with N(0,1) values stored in the cache type (SURVEY.md 8d)."""
+        """Fill KV cells [0, n_cells) of every layer with N(0,1) values stored in the cache type."""
         rng = np.random.default_rng(seed)
         s = self.shape
         width = s.head_dim * s.n_head_kv

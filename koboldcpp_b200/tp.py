@@ -1,7 +1,7 @@
 """Tensor-parallel sharding of a llama model's tensors, one process per GPU (include/b200_comm.h, b200_llama.h tp_world > 1).
 
 The reference shards every weight matrix by output rows over the devices of one process and moves activations / results
-through the main GPU for every matmul (/root/reference/ggml/src/ggml-cuda.cu:623-953 split buffer type, :1519-1657 matmul
+through the main GPU for every matmul (ggml/src/ggml-cuda.cu:623-953 split buffer type, :1519-1657 matmul
 loop).  Here the rows are cut so that whole heads and whole ffn columns stay on one rank, and the two matrices that close a
 residual branch (attn_output, ffn_down) are cut along K instead, which leaves two all-reduces per layer as the only
 exchange.  Everything in this file is host logic on numpy arrays of raw GGUF block bytes: it runs (and is tested) without a GPU.
