@@ -4,7 +4,7 @@
 // sink_attn_tile_kernel works on tiles of 64 cells that arrive by cp.async.  A CTA serves 64 columns of one kv head, a column being a token and
 // one of the query heads that share the keys, 16 columns a warp.  sink_attn_mma_kernel, which needs no workspace, converts every tile for every query head
 // and block of 64 tokens, with its loads in front of its products: 214 us for 512 tokens behind 512, 32 heads over 8 of 128; both launches here
-// take 70.  Bound by instruction issue (scores, exponentials), as fattn_mma_prefill_kernel, whose tile step this is.
+// take 63.  Bound by instruction issue (scores, exponentials), as fattn_mma_prefill_kernel, whose tile step this is.
 // Whether half a tile is seen wholly, partly or not at all follows from the positions of the warp's tokens (their smallest and largest) when they
 // belong to one sequence, else token by token; only partly seen halves, and those with a soft cap or a distance bias, go value by value.
 // A softmax step is 32 cells, half a tile: the running maximum and with it the bf16 roundings of the weights are those of sink_attn_mma_kernel,
