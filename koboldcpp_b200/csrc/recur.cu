@@ -72,17 +72,34 @@ __global__ void __launch_bounds__(128) short_conv_kernel(const b200_short_conv_a
 
 // ------------------------------------------------------------------------------------------------ gated delta rule
 // The columns of the state never interact: column j of S [dim, vdim] sees  S_j <- g S_j + k u_j  with  u_j = beta (v_j - g k.S_j),
-// and the read-out is  o_j = q.S_j(new) = g q.S_j(old) + (q.k) u_j,  so one pass over the old column gives both sums a token
-// needs.  8 lanes share DR_CPL columns, lane r of them keeping the rows 4 (r + 8 i) .. + 3 of each in registers over the whole token loop, so a sum
-// over a column is three exchanges among 8 lanes, and two rows are worked on at a time (packed f32: one issue slot for both).
-// What bounds it: the chain S -> sums -> u -> S of a token, and the shared-memory pipe (a 16-byte load of a warp takes four of its cycles however
-// few addresses differ).  So every q and k piece that is loaded serves two columns, the four warps that carry the state do nothing else, and
-// four more warps prepare the next chunk of tokens meanwhile: q and k as unit vectors (q scaled), q.k, the decay and beta once per token.  512
-// tokens, 32 heads of 128 x 128: 183 us with one column a lane, eight warps that staged and scanned in turn, and unpacked arithmetic; 139 us here.
-// CHAN: the decay is one factor per key channel (row of S) instead of one per head.  The old column is multiplied by it first, then
-// ks, qs are sums over the decayed column and  o_j = qs + (q.k) u_j;  the factors of a chunk are staged like q and k.
-constexpr int DR_CW = 4, DR_CPL = 2, DR_WARPS = 4, DR_COLS = DR_CW * DR_CPL * DR_WARPS;
-template <int DQ, bool CHAN> constexpr int dr_chunk() { return DQ * (CHAN ? 3 : 2) <= 8 ? 16 : DQ * (CHAN ? 3 : 2) <= 16 ? 8 : 4; }  // two chunks in 48 KB
+// and the read-out is  o_j = q.S_j(new).  Token by token that is a chain S -> sums over the column -> u -> S of about 500 cycles, most of it latency.
+// So four tokens are taken at once.  With S0 in front of them and G(t, j) = g_(j+1) ... g_t (products: nothing is divided),
+//   u_t = beta_t (v_t - G(t, -1) k_t.S0 - sum_(j < t) G(t, j) (k_t.k_j) u_j),   o_t = G(t, -1) q_t.S0 + sum_(j <= t) G(t, j) (q_t.k_j) u_j,
+//   S <- G(3, -1) S0 + sum_j G(3, j) k_j u_j:
+// the eight sums over a column all read S0 and travel together, the dot products among the tokens do not depend on S and are made ahead, and what is left
+// in a chain is a triangle of four.  The tokens behind the last whole group of four go through the same steps one by one.
+//   * A warp carries 8 columns: LR lanes share CPL of them, lane r of them keeping rows 4 (r + LR i) .. + 3 in registers.  Rows are worked on two
+//     at a time (packed f32).  16 lanes and 4 columns: a 16-byte load of k or q, four cycles of the shared-memory pipe, serves 16 products;
+//     the sums of the four columns are exchanged so that four lanes end up with one column (halving: 16 + 8 values, then 11).  Column c of lane r is
+//     number c ^ (r / 4) of the group: what a lane gives away in that exchange has the same names in all lanes.
+//   * Four warps carry the state and do nothing else; four more prepare the next chunk meanwhile, a group of four tokens each: q and k as unit vectors
+//     (q scaled), their dot products, decays and beta.
+// What bounds it: issue (about 570 instructions a warp for four tokens, 208 of them packed multiply-adds of two to three cycles each) and the latency of
+// the exchanges; with a decay per channel the staging warps' exponentials.  512 tokens, 32 heads of 128 x 128: 136 us token by token, 87 us here;
+// 312 tokens, 22 heads of 64 x 64 with decays per channel 80 -> 53 us with the convolution in front.
+// CHAN: the decay is one factor per key channel (row of S) instead of one per head: G is a vector, and what is staged are G(t, -1) k_t and G(t, -1) q_t for
+// the sums, G(3, j) k_j for the update and G(3, -1) itself; the dot products are taken with G between their factors.
+constexpr int DR_T = 4, DR_WARPS = 4, DR_COLS = 8 * DR_WARPS;
+template <int DQ, bool CHAN> constexpr int dr_chunk() { return DQ * (CHAN ? 2 : 1) <= 8 ? 16 : 8; }  // tokens staged at once: DR_T for each staging warp, if two chunks fit 64 KB
+// coefficients of a group of tokens, in floats from the group's row: beta_t | beta_t G(t, -1) | beta_t G(t, j) k_t.k_j for (1, 0) (2, 0) (2, 1) (3, 0) .. |
+// G(3, j) | G(t, -1) | G(t, j) q_t.k_j, four a token.  Of an incomplete group every token is a group of its own.
+constexpr int DR_BETA = 0, DR_BG = 4, DR_KK = 8, DR_LAST = 16, DR_G = 20, DR_QK = 24, DR_COEF = 40;
+// a sequence shorter than this goes token by token: with a decay per channel the exponentials of a group, which one warp stages, take longer than four steps
+template <bool CHAN> constexpr int dr_grouped() { return CHAN ? 16 : DR_T; }
+template <int DQ, bool CHAN> constexpr int dr_smem() {
+    constexpr int C = dr_chunk<DQ, CHAN>();
+    return 4 * 2 * C * (32 * DQ * (CHAN ? 4 : 2) + DR_COLS + DR_COEF / DR_T);
+}
 __device__ __forceinline__ unsigned long long dr_pack(float lo, float hi) { unsigned long long r; asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi)); return r; }
 __device__ __forceinline__ float2 dr_unpack(unsigned long long x) { float2 r; asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(x)); return r; }
 __device__ __forceinline__ unsigned long long dr_fma(unsigned long long x, unsigned long long y, unsigned long long z) {
@@ -95,24 +112,314 @@ __device__ __forceinline__ unsigned long long dr_mul(unsigned long long x, unsig
     asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(x), "l"(y));
     return r;
 }
+__device__ __forceinline__ unsigned long long dr_add(unsigned long long x, unsigned long long y) {
+    unsigned long long r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(x), "l"(y));
+    return r;
+}
 // the meeting of both roles: all warps of the CTA, from whichever branch they come (__syncthreads() wants one place for all threads)
 __device__ __forceinline__ void dr_meet() { asm volatile("bar.sync 1, %0;" ::"n"(DR_WARPS * 64) : "memory"); }
-template <int DQ, bool CHAN>  // float4 groups per lane: dim <= 32 DQ
-__global__ void __launch_bounds__(DR_WARPS * 64) delta_rule_scan_kernel(const b200_delta_rule_args a) {
-    constexpr int DP = 32 * DQ, DR_CHUNK = dr_chunk<DQ, CHAN>();
-    __shared__ __align__(16) float sq[2][DR_CHUNK][DP], sk[2][DR_CHUNK][DP];
-    __shared__ __align__(16) float sgc[CHAN ? 2 : 1][CHAN ? DR_CHUNK : 1][CHAN ? DP : 4];
-    __shared__ float sv[2][DR_CHUNK][DR_COLS];
-    __shared__ __align__(16) float4 stok[2][DR_CHUNK];  // g, g (1 with CHAN), beta, q.k
+// sums over lanes that differ in bit `off`: N values become N / 2, the lanes with the bit set keep the upper half
+template <int N>
+__device__ __forceinline__ void dr_halve(float *v, bool upper, int off) {
+#pragma unroll
+    for (int i = 0; i < N / 2; i++) {
+        const float send = upper ? v[i] : v[i + N / 2], keep = upper ? v[i + N / 2] : v[i];
+        v[i] = keep + __shfl_xor_sync(0xffffffffu, send, off);
+    }
+}
+template <int DQ, bool CHAN>
+struct DrSmem {  // of one of the two buffers
+    static constexpr int C = dr_chunk<DQ, CHAN>(), DP = 32 * DQ;
+    float *k, *q, *kd, *g, *v, *coef;  // k, q [C][DP] for the sums; CHAN: kd [C][DP] for the update, g [C][DP]; v [C / 4][DR_COLS][4]; coef [C / 4][DR_COEF]
+    __device__ __forceinline__ DrSmem(float *base, int buf) {
+        base += buf * (dr_smem<DQ, CHAN>() / 8);
+        k = base;
+        q = k + C * DP;
+        kd = CHAN ? q + C * DP : k;
+        g = CHAN ? kd + C * DP : q;
+        v = (CHAN ? g : q) + C * DP;
+        coef = v + C * DR_COLS;
+    }
+};
+
+// products of the lane's pieces of a row vector with its columns.  The columns are the inner loop: an instruction that reads the same register pair in the same
+// place as the one before it issues in two cycles, with three new pairs it takes three.
+template <int CPL, int NR>
+__device__ __forceinline__ void dr_dots(const unsigned long long (&x)[NR][2], const unsigned long long (&y)[CPL][NR][2], float *to, int stride) {
+    unsigned long long s[CPL][2];
+#pragma unroll
+    for (int i = 0; i < NR; i++) {
+#pragma unroll
+        for (int e = 0; e < 2; e++) {
+#pragma unroll
+            for (int c = 0; c < CPL; c++) s[c][e] = i == 0 ? dr_mul(x[0][e], y[c][0][e]) : dr_fma(x[i][e], y[c][i][e], s[c][e]);
+        }
+    }
+#pragma unroll
+    for (int c = 0; c < CPL; c++) {
+        const float2 z = dr_unpack(dr_add(s[c][0], s[c][1]));
+        to[c * stride] = z.x + z.y;
+    }
+}
+
+// ===== T tokens of a chunk, tok .. tok + T - 1 (T == DR_T: a whole group), against the columns that the warp carries
+template <int DQ, bool CHAN, int T>
+__device__ __forceinline__ void dr_step(unsigned long long (&S)[DQ == 1 ? 2 : 4][DQ == 1 ? 1 : DQ / 2][2], const DrSmem<DQ, CHAN> &sm, int tok, int warp, int lane, float *out, int64_t out_stride,
+                                        bool col_ok) {
+    constexpr int LR = DQ == 1 ? 8 : 16, CPL = LR / 4, NR = DQ == 1 ? 1 : DQ / 2, DP = 32 * DQ;
+    const int r = lane & (LR - 1), cg = lane / LR;
+    unsigned long long kk[T][NR][2];
+    float ks[CPL * T], qs[CPL * T];  // [column][token]
+    // the k sums travel while the q sums are made, the q sums while S moves on
+#pragma unroll
+    for (int t = 0; t < T; t++) {
+#pragma unroll
+        for (int i = 0; i < NR; i++) {
+            const ulonglong2 kv = *reinterpret_cast<const ulonglong2 *>(sm.k + (tok + t) * DP + 4 * (r + LR * i));
+            kk[t][i][0] = kv.x; kk[t][i][1] = kv.y;
+        }
+        dr_dots<CPL, NR>(kk[t], S, ks + t, T);
+    }
+    // one column for each four lanes: the lane's column 0 (columns are numbered from there: what a lane gives away are always the upper ones)
+#pragma unroll
+    for (int n = CPL / 2; n >= 1; n >>= 1) {
+#pragma unroll
+        for (int i = 0; i < T * n; i++) ks[i] += __shfl_xor_sync(0xffffffffu, ks[i + T * n], 4 * n);
+    }
+#pragma unroll
+    for (int t = 0; t < T; t++) ks[t] += __shfl_xor_sync(0xffffffffu, ks[t], 2);
+#pragma unroll
+    for (int t = 0; t < T; t++) ks[t] += __shfl_xor_sync(0xffffffffu, ks[t], 1);
+#pragma unroll
+    for (int t = 0; t < T; t++) {
+        unsigned long long qq[NR][2];
+#pragma unroll
+        for (int i = 0; i < NR; i++) {
+            const ulonglong2 qv = *reinterpret_cast<const ulonglong2 *>(sm.q + (tok + t) * DP + 4 * (r + LR * i));
+            qq[i][0] = qv.x; qq[i][1] = qv.y;
+        }
+        dr_dots<CPL, NR>(qq, S, qs + t, T);
+    }
+    const int col = warp * 8 + cg * CPL + (r >> 2);
+    const int group = tok / DR_T, i0 = tok % DR_T;
+    const float *co = sm.coef + group * DR_COEF;
+    float u[T], last, o;
+    if constexpr (T == 4) {
+        const float4 v = *reinterpret_cast<const float4 *>(sm.v + (group * DR_COLS + col) * 4), be = *reinterpret_cast<const float4 *>(co + DR_BETA), bg = *reinterpret_cast<const float4 *>(co + DR_BG);
+        const float4 a = *reinterpret_cast<const float4 *>(co + DR_KK), w = *reinterpret_cast<const float4 *>(co + DR_LAST), qk = *reinterpret_cast<const float4 *>(co + DR_QK + 4 * (r & 3));
+        const float2 a2 = *reinterpret_cast<const float2 *>(co + DR_KK + 4);
+        u[0] = be.x * v.x - bg.x * ks[0];
+        u[1] = (be.y * v.y - bg.y * ks[1]) - a.x * u[0];
+        u[2] = ((be.z * v.z - bg.z * ks[2]) - a.y * u[0]) - a.z * u[1];
+        u[3] = (((be.w * v.w - bg.w * ks[3]) - a.w * u[0]) - a2.x * u[1]) - a2.y * u[2];
+        o = qk.x * u[0];  // (of the tokens behind the lane's nothing enters, not even as 0 times it)
+        if ((r & 3) > 0) o += qk.y * u[1];
+        if ((r & 3) > 1) o += qk.z * u[2];
+        if ((r & 3) > 2) o += qk.w * u[3];
+        if (!CHAN) { u[0] *= w.x; u[1] *= w.y; u[2] *= w.z; u[3] *= w.w; }
+        last = co[DR_G + 3];
+    } else {
+        u[0] = co[DR_BETA + i0] * sm.v[(group * DR_COLS + col) * 4 + i0] - co[DR_BG + i0] * ks[0];
+        last = co[DR_G + i0];
+        o = co[DR_QK + 4 * i0] * u[0];
+    }
+    if (CHAN) {
+#pragma unroll
+        for (int t = 0; t < T; t++) {
+#pragma unroll
+            for (int i = 0; i < NR; i++) {
+                const ulonglong2 kv = *reinterpret_cast<const ulonglong2 *>(sm.kd + (tok + t) * DP + 4 * (r + LR * i));
+                kk[t][i][0] = kv.x; kk[t][i][1] = kv.y;
+            }
+        }
+    }
+    unsigned long long gv[NR][2];
+#pragma unroll
+    for (int i = 0; i < NR; i++) {
+        if (CHAN) {
+            const ulonglong2 x = *reinterpret_cast<const ulonglong2 *>(sm.g + tok * DP + 4 * (r + LR * i));
+            gv[i][0] = x.x; gv[i][1] = x.y;
+        } else {
+            gv[i][0] = gv[i][1] = dr_pack(last, last);
+        }
+    }
+    unsigned long long u2[CPL][T];
+#pragma unroll
+    for (int c = 0; c < CPL; c++) {
+#pragma unroll
+        for (int t = 0; t < T; t++) {
+            const float x = c == 0 ? u[t] : __shfl_xor_sync(0xffffffffu, u[t], 4 * c);
+            u2[c][t] = dr_pack(x, x);
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < NR; i++) {
+#pragma unroll
+        for (int e = 0; e < 2; e++) {
+            unsigned long long add[CPL];  // (the small terms k u are the ones that are rounded first)
+#pragma unroll
+            for (int t = 0; t < T; t++) {
+#pragma unroll
+                for (int c = 0; c < CPL; c++) add[c] = t == 0 ? dr_mul(kk[0][i][e], u2[c][0]) : dr_fma(kk[t][i][e], u2[c][t], add[c]);
+            }
+#pragma unroll
+            for (int c = 0; c < CPL; c++) S[c][i][e] = dr_fma(S[c][i][e], gv[i][e], add[c]);
+        }
+    }
+    // the read-out of token r & 3
+#pragma unroll
+    for (int n = CPL / 2; n >= 1; n >>= 1) {
+#pragma unroll
+        for (int i = 0; i < T * n; i++) qs[i] += __shfl_xor_sync(0xffffffffu, qs[i + T * n], 4 * n);
+    }
+    if constexpr (T == 4) {
+#pragma unroll
+        for (int i = 0; i < 2; i++) {
+            const float send = r & 2 ? qs[i] : qs[i + 2], keep = r & 2 ? qs[i + 2] : qs[i];
+            qs[i] = keep + __shfl_xor_sync(0xffffffffu, send, 2);
+        }
+        const float send = r & 1 ? qs[0] : qs[1], keep = r & 1 ? qs[1] : qs[0];
+        qs[0] = keep + __shfl_xor_sync(0xffffffffu, send, 1);
+        if (col_ok) out[(r & 3) * out_stride] = co[DR_G + (r & 3)] * qs[0] + o;
+    } else {
+        qs[0] += __shfl_xor_sync(0xffffffffu, qs[0], 2);
+        qs[0] += __shfl_xor_sync(0xffffffffu, qs[0], 1);
+        if (col_ok && (r & 3) == 0) out[0] = last * qs[0] + o;
+    }
+}
+
+// ===== staging: T tokens (a whole group, or one by itself) from token t0 of the sequence on, tok of the chunk, by one warp; all loads in flight at once
+template <int DQ, bool CHAN, int T>
+__device__ __forceinline__ void dr_stage(const b200_delta_rule_args &a, const DrSmem<DQ, CHAN> &sm, int64_t t0, int tok, int h, int kvh, int cb, int lane, float decay_rate, float dtb,
+                                         const float (&bias)[CHAN ? DQ : 1]) {
+    constexpr int DP = 32 * DQ;
+    const int D = a.dim, V = a.vdim;
+    const int t4 = T == 1 ? 0 : lane & 3;
+    float q[T][DQ], k[T][DQ], z[CHAN ? T : 1][CHAN ? DQ : 1], v[T];
+    const float ga = CHAN ? 0.f : a.a[(t0 + t4) * a.a_stride + h], be = a.b[(t0 + t4) * a.b_stride + h];
+#pragma unroll
+    for (int t = 0; t < T; t++) {
+#pragma unroll
+        for (int j = 0; j < DQ; j++) {
+            const int d = lane + 32 * j;
+            q[t][j] = d < D ? a.q[(t0 + t) * a.q_stride + (int64_t)kvh * D + d] : 0.f;
+            k[t][j] = d < D ? a.k[(t0 + t) * a.k_stride + (int64_t)kvh * D + d] : 0.f;
+            if (CHAN) z[CHAN ? t : 0][CHAN ? j : 0] = d < D ? a.a[(t0 + t) * a.a_stride + (int64_t)h * D + d] : 0.f;
+        }
+        v[t] = cb + lane < V ? a.v[(t0 + t) * a.v_stride + (int64_t)h * V + cb + lane] : 0.f;
+    }
+    // unit vectors.  Of the 2 T sums of squares number i (q of the tokens, then k) ends up in the lanes from 4 i (T = 4) or 16 i (T = 1) on.
+    float len[2 * T];
+#pragma unroll
+    for (int t = 0; t < T; t++) {
+        len[t] = len[T + t] = 0.f;
+#pragma unroll
+        for (int j = 0; j < DQ; j++) { len[t] += q[t][j] * q[t][j]; len[T + t] += k[t][j] * k[t][j]; }
+    }
+    dr_halve<2 * T>(len, (lane & 16) != 0, 16);
+    if constexpr (T == 4) {
+        dr_halve<4>(len, (lane & 8) != 0, 8);
+        dr_halve<2>(len, (lane & 4) != 0, 4);
+    } else {
+        len[0] += __shfl_xor_sync(0xffffffffu, len[0], 8);
+        len[0] += __shfl_xor_sync(0xffffffffu, len[0], 4);
+    }
+    len[0] += __shfl_xor_sync(0xffffffffu, len[0], 2);
+    len[0] += __shfl_xor_sync(0xffffffffu, len[0], 1);
+    const float f = (a.unit_qk ? 1.0f / sqrtf(len[0] + a.unit_eps) : 1.0f) * (lane < 16 ? a.q_scale : 1.0f);
+#pragma unroll
+    for (int t = 0; t < T; t++) {
+        const float fq = __shfl_sync(0xffffffffu, f, 4 * t), fk = __shfl_sync(0xffffffffu, f, 16 + 4 * t);
+#pragma unroll
+        for (int j = 0; j < DQ; j++) { q[t][j] *= fq; k[t][j] *= fk; }
+    }
+    // dot products q_t.k_j, j <= t, then k_t.k_j, j < t, with the channels' decays between them
+    float dot[T == 4 ? 16 : 1];
+#pragma unroll
+    for (int i = 0; i < (T == 4 ? 16 : 1); i++) dot[i] = 0.f;
+    float *row = sm.k + tok * DP + lane;
+    const int64_t to_q = sm.q - sm.k, to_kd = sm.kd - sm.k, to_g = sm.g - sm.k;
+#pragma unroll
+    for (int j = 0; j < DQ; j++) {
+        float gc[T];
+        if (CHAN) {
+#pragma unroll
+            for (int t = 0; t < T; t++) gc[t] = expf(-decay_rate * softplus_f(z[CHAN ? t : 0][CHAN ? j : 0] + bias[CHAN ? j : 0]));
+        }
+#pragma unroll
+        for (int jj = 0; jj < T; jj++) {
+            float x = k[jj][j];
+#pragma unroll
+            for (int t = jj; t < T; t++) {
+                if (CHAN && t > jj) x *= gc[t];
+                dot[t * (t + 1) / 2 + jj] += q[t][j] * x;
+                if (t > jj) dot[10 + t * (t - 1) / 2 + jj] += k[t][j] * x;
+            }
+            if (CHAN) row[to_kd + jj * DP + 32 * j] = x;
+        }
+        float all = 1.0f;
+#pragma unroll
+        for (int t = 0; t < T; t++) {
+            if (CHAN) all *= gc[t];
+            row[t * DP + 32 * j] = CHAN ? k[t][j] * all : k[t][j];
+            row[to_q + t * DP + 32 * j] = CHAN ? q[t][j] * all : q[t][j];
+        }
+        if (CHAN) row[to_g + 32 * j] = all;
+    }
+    const float g_mine = CHAN ? 1.0f : expf(-decay_rate * softplus_f(ga + dtb)), beta = sigmoidf_(be);
+    float *co = sm.coef + tok / DR_T * DR_COEF, *vs = sm.v + (tok / DR_T * DR_COLS + lane) * 4;
+    if constexpr (T == 1) {
+        const int i = tok % DR_T;
+        vs[i] = v[0];
+        const float qk = warp_sum(dot[0]);
+        if (lane == 0) {
+            co[DR_BETA + i] = beta;
+            co[DR_BG + i] = beta * g_mine;
+            co[DR_G + i] = g_mine;
+            co[DR_QK + 4 * i] = qk;
+        }
+    } else {
+        *reinterpret_cast<float4 *>(vs) = make_float4(v[0], v[1], v[2], v[3]);
+        // value i ends up in lanes 2 i and 2 i + 1
+        dr_halve<16>(dot, (lane & 16) != 0, 16);
+        dr_halve<8>(dot, (lane & 8) != 0, 8);
+        dr_halve<4>(dot, (lane & 4) != 0, 4);
+        dr_halve<2>(dot, (lane & 2) != 0, 2);
+        dot[0] += __shfl_xor_sync(0xffffffffu, dot[0], 1);
+        const int i = lane >> 1, t = (int)(0xFE9FFA94u >> (2 * i)) & 3, j = (int)(0x910E4910u >> (2 * i)) & 3;  // its t and j, two bits each
+        float between = 1.0f, upto = 1.0f, after = 1.0f;  // G(t, j); G(t4, -1); G(3, t4)
+#pragma unroll
+        for (int e = 0; e < DR_T; e++) {
+            const float g = CHAN ? 1.0f : __shfl_sync(0xffffffffu, g_mine, e);
+            if (e > j && e <= t) between *= g;
+            if (e <= t4) upto *= g;
+            else after *= g;
+        }
+        const float beta_t = __shfl_sync(0xffffffffu, beta, t);
+        if ((lane & 1) == 0) co[i >= 10 ? DR_KK + t * (t - 1) / 2 + j : DR_QK + 4 * t + j] = (i >= 10 ? beta_t : 1.0f) * (between * dot[0]);
+        if (lane < DR_T) {
+            co[DR_BETA + lane] = beta;
+            co[DR_BG + lane] = beta * upto;
+            co[DR_LAST + lane] = after;
+            co[DR_G + lane] = upto;
+        }
+    }
+}
+
+template <int DQ, bool CHAN, int CTAS>  // dim <= 32 DQ; CTAs that an SM is to hold
+__global__ void __launch_bounds__(DR_WARPS * 64, CTAS) delta_rule_scan_kernel(const b200_delta_rule_args a) {
+    constexpr int DR_CHUNK = dr_chunk<DQ, CHAN>();
+    extern __shared__ __align__(16) float dr_shared[];
     const int h = blockIdx.y, s = blockIdx.z, kvh = h / (a.heads / a.kv_heads);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int D = a.dim, V = a.vdim;
     const int first = a.seq_info[s], count = a.seq_info[a.n_seq + s], slot = a.seq_info[2 * a.n_seq + s], fresh = a.seq_info[3 * a.n_seq + s];
     if (count <= 0) return;
     const int cb = blockIdx.x * DR_COLS, n_chunks = (count + DR_CHUNK - 1) / DR_CHUNK;
+    const int grouped = count >= dr_grouped<CHAN>() ? ~(DR_T - 1) : 0;  // tokens of a chunk in groups: all but the remainder, or none
     if (warp >= DR_WARPS) {
-        // ===== staging: a warp takes the tokens w, w + DR_WARPS, ... of a chunk, all their loads in flight at once
-        constexpr int TPW = (DR_CHUNK + DR_WARPS - 1) / DR_WARPS;
+        // ===== staging: a warp takes a group of tokens of every chunk, or single tokens
         const int w = warp - DR_WARPS;
         const float decay_rate = expf(a.a_log[h]), dtb = !CHAN && a.dt_bias ? a.dt_bias[h] : 0.f;
         float bias[CHAN ? DQ : 1];
@@ -121,140 +428,101 @@ __global__ void __launch_bounds__(DR_WARPS * 64) delta_rule_scan_kernel(const b2
             for (int j = 0; j < DQ; j++) bias[CHAN ? j : 0] = a.dt_bias && lane + 32 * j < D ? a.dt_bias[(int64_t)h * D + lane + 32 * j] : 0.f;
         }
         for (int c = 0; c < n_chunks; c++) {
-            const int buf = c & 1;
-            float q[TPW][DQ], k[TPW][DQ], z[CHAN ? TPW : 1][CHAN ? DQ : 1], v[TPW], ga[TPW], be[TPW];
-#pragma unroll
-            for (int u = 0; u < TPW; u++) {
-                const int t = c * DR_CHUNK + w + u * DR_WARPS;
-                const bool ok = w + u * DR_WARPS < DR_CHUNK && t < count;
-                const int64_t tok = first + t;
-#pragma unroll
-                for (int j = 0; j < DQ; j++) {
-                    const int d = lane + 32 * j;
-                    q[u][j] = ok && d < D ? a.q[tok * a.q_stride + (int64_t)kvh * D + d] : 0.f;
-                    k[u][j] = ok && d < D ? a.k[tok * a.k_stride + (int64_t)kvh * D + d] : 0.f;
-                    if (CHAN) z[CHAN ? u : 0][CHAN ? j : 0] = ok && d < D ? a.a[tok * a.a_stride + (int64_t)h * D + d] : 0.f;
-                }
-                v[u] = ok && cb + lane < V ? a.v[tok * a.v_stride + (int64_t)h * V + cb + lane] : 0.f;
-                ga[u] = !CHAN && ok ? a.a[tok * a.a_stride + h] : 0.f;
-                be[u] = ok ? a.b[tok * a.b_stride + h] : 0.f;
-            }
-#pragma unroll
-            for (int u = 0; u < TPW; u++) {
-                const int tt = w + u * DR_WARPS;
-                if (c * DR_CHUNK + tt >= count) continue;  // (a short sequence does not wait for tokens that do not exist)
-                float qq = 0.f, kk = 0.f, qk = 0.f;
-#pragma unroll
-                for (int j = 0; j < DQ; j++) { qq += q[u][j] * q[u][j]; kk += k[u][j] * k[u][j]; }
-                qq = warp_sum(qq); kk = warp_sum(kk);
-                const float fq = (a.unit_qk ? 1.0f / sqrtf(qq + a.unit_eps) : 1.0f) * a.q_scale, fk = a.unit_qk ? 1.0f / sqrtf(kk + a.unit_eps) : 1.0f;
-#pragma unroll
-                for (int j = 0; j < DQ; j++) { q[u][j] *= fq; k[u][j] *= fk; qk += q[u][j] * k[u][j]; }
-                qk = warp_sum(qk);
-                if (tt < DR_CHUNK) {
-#pragma unroll
-                    for (int j = 0; j < DQ; j++) {
-                        sq[buf][tt][lane + 32 * j] = q[u][j];
-                        sk[buf][tt][lane + 32 * j] = k[u][j];
-                        if (CHAN) sgc[CHAN ? buf : 0][CHAN ? tt : 0][CHAN ? lane + 32 * j : 0] = expf(-decay_rate * softplus_f(z[CHAN ? u : 0][CHAN ? j : 0] + bias[CHAN ? j : 0]));
-                    }
-                    sv[buf][tt][lane] = v[u];
-                    if (lane == 0) {
-                        const float g = CHAN ? 1.0f : expf(-decay_rate * softplus_f(ga[u] + dtb));
-                        stok[buf][tt] = make_float4(g, g, sigmoidf_(be[u]), qk);
-                    }
-                }
-            }
+            const DrSmem<DQ, CHAN> sm(dr_shared, c & 1);
+            const int nt = min(DR_CHUNK, count - c * DR_CHUNK), in_groups = nt & grouped;
+            const int64_t t0 = first + c * DR_CHUNK;
+            if (DR_T * w < in_groups) dr_stage<DQ, CHAN, DR_T>(a, sm, t0 + DR_T * w, DR_T * w, h, kvh, cb, lane, decay_rate, dtb, bias);
+#pragma unroll 1
+            for (int tok = in_groups + ((w - in_groups / DR_T) & (DR_WARPS - 1)); tok < nt; tok += DR_WARPS)
+                dr_stage<DQ, CHAN, 1>(a, sm, t0 + tok, tok, h, kvh, cb, lane, decay_rate, dtb, bias);
             dr_meet();  // chunk c is ready; chunk c - 1, whose room the next one takes, has been read
         }
         return;
     }
-    // ===== the state: columns cb + lc + DR_CW c of the lane
-    const int r = lane & 7, lc = warp * DR_CW * DR_CPL + (lane >> 3);
-    float *Sp = a.state + (int64_t)slot * a.slot_stride + ((int64_t)h * V + cb + lc) * D;  // column c at Sp + DR_CW c D
-    unsigned long long S[DR_CPL][DQ][2];
+    // ===== the state
+    constexpr int LR = DQ == 1 ? 8 : 16, CPL = LR / 4, NR = DQ == 1 ? 1 : DQ / 2;
+    const int r = lane & (LR - 1), c0 = cb + warp * 8 + lane / LR * CPL;  // the lane's columns are c0 + (c ^ (r / 4))
+    float *Sp = a.state + (int64_t)slot * a.slot_stride + ((int64_t)h * V + c0) * D;
+    const bool pieces = ((D | (int)a.slot_stride) & 3) == 0 && ((uintptr_t)a.state & 15) == 0;  // every column starts on 16 bytes
+    unsigned long long S[CPL][NR][2];
 #pragma unroll
-    for (int c = 0; c < DR_CPL; c++) {
+    for (int c = 0; c < CPL; c++) {
 #pragma unroll
-        for (int i = 0; i < DQ; i++) {
-            float x[4];
-#pragma unroll
-            for (int e = 0; e < 4; e++) { const int d = 4 * (r + 8 * i) + e; x[e] = (!fresh && d < D && cb + lc + DR_CW * c < V) ? Sp[(int64_t)DR_CW * c * D + d] : 0.f; }
-            S[c][i][0] = dr_pack(x[0], x[1]);
-            S[c][i][1] = dr_pack(x[2], x[3]);
+        for (int i = 0; i < NR; i++) {
+            const int d = 4 * (r + LR * i), cc = c ^ (r >> 2);
+            float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (!fresh && c0 + cc < V) {
+                const float *p = Sp + (int64_t)cc * D + d;
+                if (pieces) {
+                    if (d < D) x = *reinterpret_cast<const float4 *>(p);
+                } else {
+                    if (d < D) x.x = p[0];
+                    if (d + 1 < D) x.y = p[1];
+                    if (d + 2 < D) x.z = p[2];
+                    if (d + 3 < D) x.w = p[3];
+                }
+            }
+            S[c][i][0] = dr_pack(x.x, x.y);
+            S[c][i][1] = dr_pack(x.z, x.w);
         }
     }
-    float *out = a.dst + (int64_t)first * a.dst_stride + (int64_t)h * V + cb + lc;
+    const int out_col = c0 + (r >> 2);
+    const bool col_ok = out_col < V;
+    float *out = a.dst + (int64_t)first * a.dst_stride + (int64_t)h * V + out_col;
     for (int ch = 0; ch < n_chunks; ch++) {
-        const int nt = min(DR_CHUNK, count - ch * DR_CHUNK), buf = ch & 1;
+        const int nt = min(DR_CHUNK, count - ch * DR_CHUNK);
+        const DrSmem<DQ, CHAN> sm(dr_shared, ch & 1);
         dr_meet();
-        // unrolled so that the shared-memory loads of the following tokens are issued ahead of the chain S -> sums -> u -> S
-#pragma unroll 2
-        for (int tt = 0; tt < nt; tt++) {
-            const float4 tok = stok[buf][tt];
-            ulonglong2 kv[DQ], qv[DQ];
-            float ks[DR_CPL], qs[DR_CPL];
-#pragma unroll
-            for (int i = 0; i < DQ; i++) {
-                kv[i] = *reinterpret_cast<const ulonglong2 *>(&sk[buf][tt][4 * (r + 8 * i)]);
-                qv[i] = *reinterpret_cast<const ulonglong2 *>(&sq[buf][tt][4 * (r + 8 * i)]);
-                if (CHAN) {
-                    const ulonglong2 gv = *reinterpret_cast<const ulonglong2 *>(&sgc[CHAN ? buf : 0][CHAN ? tt : 0][CHAN ? 4 * (r + 8 * i) : 0]);
-#pragma unroll
-                    for (int c = 0; c < DR_CPL; c++) { S[c][i][0] = dr_mul(S[c][i][0], gv.x); S[c][i][1] = dr_mul(S[c][i][1], gv.y); }
-                }
-            }
-#pragma unroll
-            for (int c = 0; c < DR_CPL; c++) {
-                unsigned long long k0 = dr_mul(kv[0].x, S[c][0][0]), k1 = dr_mul(kv[0].y, S[c][0][1]), q0 = dr_mul(qv[0].x, S[c][0][0]), q1 = dr_mul(qv[0].y, S[c][0][1]);
-#pragma unroll
-                for (int i = 1; i < DQ; i++) {
-                    k0 = dr_fma(kv[i].x, S[c][i][0], k0); k1 = dr_fma(kv[i].y, S[c][i][1], k1);
-                    q0 = dr_fma(qv[i].x, S[c][i][0], q0); q1 = dr_fma(qv[i].y, S[c][i][1], q1);
-                }
-                const float2 ka = dr_unpack(k0), kb = dr_unpack(k1), qa = dr_unpack(q0), qb = dr_unpack(q1);
-                ks[c] = (ka.x + kb.x) + (ka.y + kb.y);
-                qs[c] = (qa.x + qb.x) + (qa.y + qb.y);
-            }
-#pragma unroll
-            for (int off = 4; off >= 1; off >>= 1) {
-#pragma unroll
-                for (int c = 0; c < DR_CPL; c++) { ks[c] += __shfl_xor_sync(0xffffffffu, ks[c], off); qs[c] += __shfl_xor_sync(0xffffffffu, qs[c], off); }
-            }
-            const unsigned long long g2 = dr_pack(tok.x, tok.y);
-#pragma unroll
-            for (int c = 0; c < DR_CPL; c++) {
-                const float u = tok.z * (sv[buf][tt][lc + DR_CW * c] - tok.x * ks[c]);
-                const unsigned long long u2 = dr_pack(u, u);
-#pragma unroll
-                for (int i = 0; i < DQ; i++) {
-                    // (the small term k u is the one that is rounded first)
-                    S[c][i][0] = CHAN ? dr_fma(kv[i].x, u2, S[c][i][0]) : dr_fma(S[c][i][0], g2, dr_mul(kv[i].x, u2));
-                    S[c][i][1] = CHAN ? dr_fma(kv[i].y, u2, S[c][i][1]) : dr_fma(S[c][i][1], g2, dr_mul(kv[i].y, u2));
-                }
-                if (r == 0 && cb + lc + DR_CW * c < V) out[DR_CW * c] = tok.x * qs[c] + tok.w * u;
-            }
-            out += a.dst_stride;
-        }
+        const int in_groups = nt & grouped;
+#pragma unroll 1
+        for (int tt = 0; tt < in_groups; tt += DR_T, out += DR_T * a.dst_stride) dr_step<DQ, CHAN, DR_T>(S, sm, tt, warp, lane, out, a.dst_stride, col_ok);
+#pragma unroll 1
+        for (int tt = in_groups; tt < nt; tt++, out += a.dst_stride) dr_step<DQ, CHAN, 1>(S, sm, tt, warp, lane, out, a.dst_stride, col_ok);
     }
 #pragma unroll
-    for (int c = 0; c < DR_CPL; c++) {
+    for (int c = 0; c < CPL; c++) {
 #pragma unroll
-        for (int i = 0; i < DQ; i++) {
+        for (int i = 0; i < NR; i++) {
+            const int d = 4 * (r + LR * i), cc = c ^ (r >> 2);
             const float2 x = dr_unpack(S[c][i][0]), y = dr_unpack(S[c][i][1]);
-            const float z[4] = {x.x, x.y, y.x, y.y};
-#pragma unroll
-            for (int e = 0; e < 4; e++) { const int d = 4 * (r + 8 * i) + e; if (d < D && cb + lc + DR_CW * c < V) Sp[(int64_t)DR_CW * c * D + d] = z[e]; }
+            if (c0 + cc < V) {
+                float *p = Sp + (int64_t)cc * D + d;
+                if (pieces) {
+                    if (d < D) *reinterpret_cast<float4 *>(p) = make_float4(x.x, x.y, y.x, y.y);
+                } else {
+                    if (d < D) p[0] = x.x;
+                    if (d + 1 < D) p[1] = x.y;
+                    if (d + 2 < D) p[2] = y.x;
+                    if (d + 3 < D) p[3] = y.y;
+                }
+            }
         }
     }
 }
 
+template <int DQ, bool CHAN, int CTAS>
+static int launch_delta_rule3(const b200_delta_rule_args *a, dim3 grid, cudaStream_t st) {
+    constexpr int SMEM = dr_smem<DQ, CHAN>();
+    const auto kern = delta_rule_scan_kernel<DQ, CHAN, CTAS>;
+    if (SMEM > 48 * 1024) {
+        static bool attr_set_dev[16] = {};  // cudaFuncSetAttribute is per device
+        int dev = 0;
+        B200_CUDA_TRY(cudaGetDevice(&dev));
+        if (!attr_set_dev[dev & 15]) {
+            B200_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM));
+            attr_set_dev[dev & 15] = true;
+        }
+    }
+    kern<<<grid, DR_WARPS * 64, SMEM, st>>>(*a);
+    B200_CUDA_TRY(cudaGetLastError());
+    return B200_OK;
+}
+// Up to a CTA an SM: all the registers it wants (512 tokens, 32 heads of 128 x 128: 87 us, 97 with the registers of two).  More CTAs than that:
+// two an SM, whose waiting the other fills.
 template <int DQ, bool CHAN>
 static int launch_delta_rule2(const b200_delta_rule_args *a, cudaStream_t st) {
     const dim3 grid((unsigned)((a->vdim + DR_COLS - 1) / DR_COLS), (unsigned)a->heads, (unsigned)a->n_seq);
-    delta_rule_scan_kernel<DQ, CHAN><<<grid, DR_WARPS * 64, 0, st>>>(*a);
-    B200_CUDA_TRY(cudaGetLastError());
-    return B200_OK;
+    return (int64_t)grid.x * grid.y * grid.z <= 148 ? launch_delta_rule3<DQ, CHAN, 1>(a, grid, st) : launch_delta_rule3<DQ, CHAN, 2>(a, grid, st);
 }
 
 template <int DQ>
