@@ -65,8 +65,9 @@ enum b200_type {
 
 B200_API const char *b200_last_error(void);
 B200_API const char *b200_version(void);
-/* Launch the kernels with the programmatic-dependent-launch attribute (griddepcontrol): a kernel's weight
- * prefetch then overlaps the tail of its producer.  Off by default; the ggml backend turns it on for its graphs. */
+/* Read weights ahead: a GEMV's weights are then fetched while the kernels in front of it in the stream still run, so nothing in the stream may
+ * write them.  Off by default; the ggml backend turns it on for its graphs.  Either way the main kernels carry the programmatic-dependent-launch
+ * attribute: their CTAs may be placed while the kernel in front drains, and (off) touch no global memory before it is done. */
 B200_API void b200_set_pdl(int enabled);
 
 /* ---- device plumbing (so ctypes / cgo / JNI hosts need no CUDA binding of their own) ------------

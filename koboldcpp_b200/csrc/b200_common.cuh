@@ -10,6 +10,7 @@
 #include <cuda_runtime.h>
 #include <cuda_fp16.h>
 #include <stdint.h>
+#include <initializer_list>
 
 #include "../../include/b200_ggml.h"
 
@@ -153,6 +154,31 @@ __device__ __forceinline__ void fence_proxy_async_smem() { asm volatile("fence.p
 // programmatic dependent launch: wait for the producer grid / allow the consumer grid to start
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+// First statement of a kernel that launch_chained() starts: nothing is read or written before the kernels in front of it are done, and no thread leaves
+// without having waited (a grid that ended early would let its own successor start too soon).  p: const __restrict__ pointers, whose loads a compiler may
+// otherwise move in front of the wait.
+template <typename... P>
+__device__ __forceinline__ void pdl_enter(P &...p) {
+    pdl_wait();
+    (void)std::initializer_list<int>{((void)([](P &q) { asm volatile("" : "+l"(q)); }(p)), 0)...};
+    pdl_trigger();
+}
+// Launch that keeps the stream's order but need not wait for the kernel in front to have left the device before its CTAs are placed: the kernel itself
+// waits (pdl_enter).  Saves about 1.5 us a launch in a row of short kernels (two GEMV launches of 2048 x 2048: 12.3 -> 9.4 us).
+template <typename... P, typename... A>
+static inline cudaError_t launch_chained(void (*kern)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, const A &...args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...);
+}
 
 // ---------------------------------------------------------------- cp.async (LDGSTS)
 __device__ __forceinline__ void cp_async16(void *dst, const void *src) {

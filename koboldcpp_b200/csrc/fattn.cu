@@ -563,7 +563,7 @@ static FaPlan fa_plan(const b200_fattn_args *a) {
 }
 
 template <int TYPE, int D, int C>
-static int fa_launch(const FaParams &p, const FaPlan &pl, cudaStream_t st, bool pdl) {
+static int fa_launch(const FaParams &p, const FaPlan &pl, cudaStream_t st) {
     using G = KvGeo<TYPE, D>;
     size_t smem = (size_t)FA_NW * FA_NBUF * 2 * G::TILE_BYTES;
     const size_t red = (size_t)FA_NW * C * (D + FA_RS_PAD) * sizeof(float);
@@ -585,13 +585,13 @@ static int fa_launch(const FaParams &p, const FaPlan &pl, cudaStream_t st, bool 
     at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = at;
-    cfg.numAttrs = pdl ? 1 : 0;
+    cfg.numAttrs = 1;
     B200_CUDA_TRY(cudaLaunchKernelEx(&cfg, fattn_kernel<TYPE, D, C>, p));
     return B200_OK;
 }
 
 template <int TYPE, int D, bool WIDE>
-static int fa_launch_mma_cols(const FaParams &p, const FaPlan &pl, cudaStream_t st, bool pdl) {
+static int fa_launch_mma_cols(const FaParams &p, const FaPlan &pl, cudaStream_t st) {
     using G = MmaGeo<TYPE, D>;
     size_t smem = (size_t)FM_NW * G::WARP_BYTES;
     const size_t merge = ((size_t)(FM_NW + 1) * FM_MAXC * (D + FA_RS_PAD) + 2 * FM_MAXC * FM_MAX_CLUSTER + 2 * FM_MAXC * FA_MAX_SPLITS) * sizeof(float);
@@ -611,12 +611,9 @@ static int fa_launch_mma_cols(const FaParams &p, const FaPlan &pl, cudaStream_t 
     cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
     cudaLaunchAttribute at[2];
-    int na = 0;
-    if (pdl) {
-        at[na].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-        at[na].val.programmaticStreamSerializationAllowed = 1;
-        na++;
-    }
+    int na = 1;
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
     if (pl.cluster) {
         at[na].id = cudaLaunchAttributeClusterDimension;
         at[na].val.clusterDim.x = (unsigned)pl.n_splits;
@@ -633,22 +630,22 @@ static int fa_launch_mma_cols(const FaParams &p, const FaPlan &pl, cudaStream_t 
         FaParams q = p;
         q.cluster_merge = 0;
         q.dyn_tiles = 0;
-        cfg.numAttrs = pdl ? 1 : 0;
+        cfg.numAttrs = 1;
         e = cudaLaunchKernelEx(&cfg, fattn_mma_kernel<TYPE, D, WIDE>, q);
     }
     if (e != cudaSuccess) return cuda_fail(e, "cudaLaunchKernelEx(fattn_mma_kernel)");
     return B200_OK;
 }
 template <int TYPE, int D>
-static int fa_launch_mma(const FaParams &p, const FaPlan &pl, cudaStream_t st, bool pdl) {
+static int fa_launch_mma(const FaParams &p, const FaPlan &pl, cudaStream_t st) {
     // up to 8 columns: half the softmax (f16, 32 heads @ 32k 101 -> 93 us); not with q4_0 and 128 dims, whose unpacking is what bounds a tile (32/8 @ 8k
     // 19.1 us wide, 20.1 narrow)
-    if constexpr (TYPE == B200_TYPE_Q4_0 && D == 128) return fa_launch_mma_cols<TYPE, D, true>(p, pl, st, pdl);
-    else return pl.C > 8 ? fa_launch_mma_cols<TYPE, D, true>(p, pl, st, pdl) : fa_launch_mma_cols<TYPE, D, false>(p, pl, st, pdl);
+    if constexpr (TYPE == B200_TYPE_Q4_0 && D == 128) return fa_launch_mma_cols<TYPE, D, true>(p, pl, st);
+    else return pl.C > 8 ? fa_launch_mma_cols<TYPE, D, true>(p, pl, st) : fa_launch_mma_cols<TYPE, D, false>(p, pl, st);
 }
 
 template <int D>
-static int fa_launch_prefill(const FaParams &p, const FaPlan &pl, cudaStream_t st, bool pdl) {
+static int fa_launch_prefill(const FaParams &p, const FaPlan &pl, cudaStream_t st) {
     const size_t smem = (size_t)FP_NBUF * fp_stage_bytes<D>();
     static bool attr_set_dev[16] = {};  // cudaFuncSetAttribute is per device
     int cur_dev = 0;
@@ -667,23 +664,22 @@ static int fa_launch_prefill(const FaParams &p, const FaPlan &pl, cudaStream_t s
     at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = at;
-    cfg.numAttrs = pdl ? 1 : 0;
+    cfg.numAttrs = 1;
     B200_CUDA_TRY(cudaLaunchKernelEx(&cfg, fattn_mma_prefill_kernel<D>, p));
     return B200_OK;
 }
 
 template <int TYPE, int D>
-static int fa_dispatch_c(const FaParams &p, const FaPlan &pl, cudaStream_t st, bool pdl) {
+static int fa_dispatch_c(const FaParams &p, const FaPlan &pl, cudaStream_t st) {
     switch (pl.C) {
-        case 1: return fa_launch<TYPE, D, 1>(p, pl, st, pdl);
-        case 2: return fa_launch<TYPE, D, 2>(p, pl, st, pdl);
-        case 4: return fa_launch<TYPE, D, 4>(p, pl, st, pdl);
-        case 8: return fa_launch<TYPE, D, 8>(p, pl, st, pdl);
+        case 1: return fa_launch<TYPE, D, 1>(p, pl, st);
+        case 2: return fa_launch<TYPE, D, 2>(p, pl, st);
+        case 4: return fa_launch<TYPE, D, 4>(p, pl, st);
+        case 8: return fa_launch<TYPE, D, 8>(p, pl, st);
     }
     return B200_ERR_INVALID;
 }
 
-extern bool g_mmvq_pdl;
 
 static int fa_check(const b200_fattn_args *a) {
     if (!a || !a->q || !a->k || !a->v || !a->dst) { set_error("b200_flash_attn_ext: NULL argument"); return B200_ERR_INVALID; }
@@ -768,33 +764,32 @@ extern "C" int b200_flash_attn_ext(const b200_fattn_args *a, void *workspace, si
     p.m0 = powf(2.0f, -(a->max_bias) / p.n_head_log2);
     p.m1 = powf(2.0f, -(a->max_bias / 2.0f) / p.n_head_log2);
     const cudaStream_t st = (cudaStream_t)stream;
-    const bool pdl = g_mmvq_pdl;
     if (pl.prefill) {
         if (((uintptr_t)a->q | a->q_nb1 | a->q_nb2) & 7) { set_error("b200_flash_attn_ext: Q must be 8-byte aligned"); return B200_ERR_UNSUPPORTED; }
         switch (a->D) {
-            case 64: return fa_launch_prefill<64>(p, pl, st, pdl);
-            case 80: return fa_launch_prefill<80>(p, pl, st, pdl);
-            case 96: return fa_launch_prefill<96>(p, pl, st, pdl);
-            case 112: return fa_launch_prefill<112>(p, pl, st, pdl);
-            case 256: return fa_launch_prefill<256>(p, pl, st, pdl);
-            default: return fa_launch_prefill<128>(p, pl, st, pdl);
+            case 64: return fa_launch_prefill<64>(p, pl, st);
+            case 80: return fa_launch_prefill<80>(p, pl, st);
+            case 96: return fa_launch_prefill<96>(p, pl, st);
+            case 112: return fa_launch_prefill<112>(p, pl, st);
+            case 256: return fa_launch_prefill<256>(p, pl, st);
+            default: return fa_launch_prefill<128>(p, pl, st);
         }
     }
     if (fa_use_mma(a)) {
         if (((uintptr_t)a->q | a->q_nb1 | a->q_nb2) & 7) { set_error("b200_flash_attn_ext: Q must be 8-byte aligned"); return B200_ERR_UNSUPPORTED; }
-        if (a->type_k == B200_TYPE_Q8_0) return a->D == 128 ? fa_launch_mma<B200_TYPE_Q8_0, 128>(p, pl, st, pdl) : fa_launch_mma<B200_TYPE_Q8_0, 64>(p, pl, st, pdl);
-        if (a->type_k == B200_TYPE_Q4_0) return a->D == 128 ? fa_launch_mma<B200_TYPE_Q4_0, 128>(p, pl, st, pdl) : fa_launch_mma<B200_TYPE_Q4_0, 64>(p, pl, st, pdl);
+        if (a->type_k == B200_TYPE_Q8_0) return a->D == 128 ? fa_launch_mma<B200_TYPE_Q8_0, 128>(p, pl, st) : fa_launch_mma<B200_TYPE_Q8_0, 64>(p, pl, st);
+        if (a->type_k == B200_TYPE_Q4_0) return a->D == 128 ? fa_launch_mma<B200_TYPE_Q4_0, 128>(p, pl, st) : fa_launch_mma<B200_TYPE_Q4_0, 64>(p, pl, st);
         switch (a->D) {
-            case 64: return fa_launch_mma<B200_TYPE_F16, 64>(p, pl, st, pdl);
-            case 80: return fa_launch_mma<B200_TYPE_F16, 80>(p, pl, st, pdl);
-            case 96: return fa_launch_mma<B200_TYPE_F16, 96>(p, pl, st, pdl);
-            case 112: return fa_launch_mma<B200_TYPE_F16, 112>(p, pl, st, pdl);
-            case 256: return fa_launch_mma<B200_TYPE_F16, 256>(p, pl, st, pdl);
-            default: return fa_launch_mma<B200_TYPE_F16, 128>(p, pl, st, pdl);
+            case 64: return fa_launch_mma<B200_TYPE_F16, 64>(p, pl, st);
+            case 80: return fa_launch_mma<B200_TYPE_F16, 80>(p, pl, st);
+            case 96: return fa_launch_mma<B200_TYPE_F16, 96>(p, pl, st);
+            case 112: return fa_launch_mma<B200_TYPE_F16, 112>(p, pl, st);
+            case 256: return fa_launch_mma<B200_TYPE_F16, 256>(p, pl, st);
+            default: return fa_launch_mma<B200_TYPE_F16, 128>(p, pl, st);
         }
     }
     if (a->type_k == B200_TYPE_F16) {
-        return a->D == 128 ? fa_dispatch_c<B200_TYPE_F16, 128>(p, pl, st, pdl) : fa_dispatch_c<B200_TYPE_F16, 64>(p, pl, st, pdl);
+        return a->D == 128 ? fa_dispatch_c<B200_TYPE_F16, 128>(p, pl, st) : fa_dispatch_c<B200_TYPE_F16, 64>(p, pl, st);
     }
-    return a->D == 128 ? fa_dispatch_c<B200_TYPE_Q8_0, 128>(p, pl, st, pdl) : fa_dispatch_c<B200_TYPE_Q8_0, 64>(p, pl, st, pdl);
+    return a->D == 128 ? fa_dispatch_c<B200_TYPE_Q8_0, 128>(p, pl, st) : fa_dispatch_c<B200_TYPE_Q8_0, 64>(p, pl, st);
 }

@@ -16,6 +16,7 @@ using namespace opx;
 // head by itself (a warp per head, the scales parked in shared memory; with qk_unit_rms without a weight); q is rewritten in place, k and v go to the token's cache
 // rows.  A rotated pair is (2i, 2i + 1) or, with rope_halves, (i, i + n_dims / 2).
 __global__ void __launch_bounds__(1024) qkv_store_kernel(const b200_qkv_store_args a) {
+    pdl_enter();
     __shared__ float sh[32];
     extern __shared__ float head_scale[];  // norm_per_head: [n_head + n_head_kv]
     const int t = blockIdx.x;
@@ -134,6 +135,7 @@ constexpr int SA_UNROLL = 4;
 // accumulator) in `part`; sink_attn_merge_kernel joins the stretches and the sink.
 template <int ND, int NV, int WARPS>
 __global__ void __launch_bounds__(WARPS * 32) sink_attn_kernel(const b200_sink_attn_args a, float *__restrict__ part, int n_split) {
+    pdl_enter();
     extern __shared__ float smem[];  // [WARPS][vdim] accumulators, then m[WARPS], l[WARPS]
     const int t = blockIdx.x, h = blockIdx.y;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -249,6 +251,7 @@ __global__ void __launch_bounds__(WARPS * 32) sink_attn_kernel(const b200_sink_a
 
 // one CTA per (token, head), a thread per output column: the stretches' (maximum, sum, accumulator) and the sink become the output row
 __global__ void __launch_bounds__(128) sink_attn_merge_kernel(const b200_sink_attn_args a, const float *__restrict__ part, int n_split) {
+    pdl_enter(part);
     const int64_t pair = blockIdx.x;
     const int V = a.vdim, h = (int)(pair % a.n_head);
     const int64_t t = pair / a.n_head;
@@ -284,12 +287,8 @@ template <int ND, int NV, int WARPS>
 static int launch_sink_attn3(const b200_sink_attn_args *a, float *part, int n_split, cudaStream_t st) {
     const dim3 grid((unsigned)a->n_tokens, (unsigned)a->n_head, (unsigned)n_split);
     const size_t smem = ((size_t)WARPS * a->vdim + 2 * WARPS) * 4;
-    sink_attn_kernel<ND, NV, WARPS><<<grid, WARPS * 32, smem, st>>>(*a, part, n_split);
-    B200_CUDA_TRY(cudaGetLastError());
-    if (n_split > 1) {
-        sink_attn_merge_kernel<<<(unsigned)(a->n_tokens * a->n_head), 128, 0, st>>>(*a, part, n_split);
-        B200_CUDA_TRY(cudaGetLastError());
-    }
+    B200_CUDA_TRY(launch_chained(sink_attn_kernel<ND, NV, WARPS>, grid, WARPS * 32, smem, st, *a, part, n_split));
+    if (n_split > 1) B200_CUDA_TRY(launch_chained(sink_attn_merge_kernel, (unsigned)(a->n_tokens * a->n_head), 128, 0, st, *a, part, n_split));
     return B200_OK;
 }
 template <int ND, int NV>
@@ -362,6 +361,7 @@ __device__ __forceinline__ void gm_stage(unsigned char *dst, int stride, int wid
 
 template <int KS, int VS>
 __global__ void __launch_bounds__(GM_WARPS * 32) sink_attn_mma_kernel(const b200_sink_attn_args a) {
+    pdl_enter();
     constexpr int QSTRIDE = KS * 32 + 16, VSTRIDE = VS * 32 + 16;  // bytes per bf16 row: 8 consecutive rows start in 8 different 16-byte bank groups
     __shared__ __align__(16) unsigned char qs[GM_TOK * QSTRIDE];
     __shared__ __align__(16) unsigned char ks[GM_CELLS * QSTRIDE];
@@ -531,8 +531,7 @@ __global__ void __launch_bounds__(GM_WARPS * 32) sink_attn_mma_kernel(const b200
 template <int KS, int VS>
 static int launch_sink_attn_mma2(const b200_sink_attn_args *a, cudaStream_t st) {
     const dim3 grid((unsigned)((a->n_tokens + GM_TOK - 1) / GM_TOK), (unsigned)a->n_head);
-    sink_attn_mma_kernel<KS, VS><<<grid, GM_WARPS * 32, 0, st>>>(*a);
-    B200_CUDA_TRY(cudaGetLastError());
+    B200_CUDA_TRY(launch_chained(sink_attn_mma_kernel<KS, VS>, grid, GM_WARPS * 32, 0, st, *a));
     return B200_OK;
 }
 template <int KS>
@@ -712,8 +711,7 @@ extern "C" int b200_op_qkv_store(const b200_qkv_store_args *args, b200_stream_t 
     const int threads = a->n_tokens <= 64 ? 1024 : 256;
     const size_t smem = (a->norm_per_head || a->qk_unit_rms) ? (size_t)(a->n_head + a->n_head_kv) * sizeof(float) : 0;
     OPX_REQUIRE(smem <= 32 * 1024, B200_ERR_UNSUPPORTED, "b200_op_qkv_store: per-head norms over at most 8192 heads");
-    qkv_store_kernel<<<(unsigned)a->n_tokens, threads, smem, (cudaStream_t)stream>>>(*a);
-    B200_CUDA_TRY(cudaGetLastError());
+    B200_CUDA_TRY(launch_chained(qkv_store_kernel, (unsigned)a->n_tokens, threads, smem, (cudaStream_t)stream, *a));
     return B200_OK;
 }
 

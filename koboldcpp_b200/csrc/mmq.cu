@@ -236,7 +236,8 @@ struct Dequant64<B200_TYPE_Q8_0> {
 
 // ---------------------------------------------------------------- activation pre-pass: f32 [N][K] -> bf16 [N_pad][K] (pad rows zero)
 __global__ void mmq_x_to_bf16_kernel(const float *__restrict__ x, int64_t x_stride, int64_t K, int64_t N, int64_t n_pad, __nv_bfloat16 *__restrict__ out,
-                                     int64_t x_batch = 0) {
+                                     int64_t x_batch) {
+    pdl_enter(x);
     const int64_t i4 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;  // float4 index within a row
     const int64_t n = blockIdx.y;
     x += (int64_t)blockIdx.z * x_batch;            // a batch of independent products: blockIdx.z
@@ -650,6 +651,7 @@ __global__ void __launch_bounds__(1024, 1) mid_group_kernel(const int32_t *__res
                                                             int64_t b_stride_row, int64_t b_stride_tok, int64_t d_stride_row, int64_t d_stride_tok, int BN,
                                                             MidTables t) {
     __shared__ int count[MID_MAX_EXPERTS], off[MID_MAX_EXPERTS + 1], cursor[MID_MAX_EXPERTS];
+    pdl_enter(ids);
     for (int e = threadIdx.x; e < n_expert; e += blockDim.x) { count[e] = 0; cursor[e] = 0; }
     __syncthreads();
     const int n = n_used * T;
@@ -688,6 +690,7 @@ __global__ void __launch_bounds__(1024, 1) mid_group_kernel(const int32_t *__res
 }
 // gather + convert: sorted row i <- bf16(b[row_src[i]]), K values
 __global__ void mid_gather_bf16_kernel(const float *__restrict__ b, const int *__restrict__ row_src, int64_t K, __nv_bfloat16 *__restrict__ out) {
+    pdl_enter(b, row_src);
     const int64_t i4 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     const int64_t n = blockIdx.y;
     if (i4 * 4 >= K) return;
@@ -774,8 +777,7 @@ extern "C" int b200_mul_mat_q_wait(int type, const void *W, size_t w_row_bytes, 
     __nv_bfloat16 *xb = (__nv_bfloat16 *)workspace;
     if (X) {  // (X == NULL: the workspace holds the bf16 activations of the previous call with this K and N)
         dim3 g1((unsigned)((K / 4 + 255) / 256), (unsigned)n_pad);
-        mmq_x_to_bf16_kernel<<<g1, 256, 0, st>>>(X, x_stride, K, N, n_pad, xb);
-        B200_CUDA_TRY(cudaGetLastError());
+        B200_CUDA_TRY(launch_chained(mmq_x_to_bf16_kernel, g1, 256, 0, st, X, x_stride, K, N, n_pad, xb, (int64_t)0));
     }
     MmqParams p;
     p.W = (const unsigned char *)W; p.w_row_bytes = w_row_bytes; p.Xb = xb; p.dst = dst; p.dst_stride = dst_stride; p.K = K; p.M = M; p.N = N;
@@ -817,8 +819,7 @@ extern "C" int b200_mul_mat_bf16_batched(const void *W, size_t w_row_bytes, size
     const cudaStream_t st = (cudaStream_t)stream;
     __nv_bfloat16 *xb = (__nv_bfloat16 *)workspace;
     dim3 g1((unsigned)((K / 4 + 255) / 256), (unsigned)n_pad, (unsigned)n_batch);
-    mmq_x_to_bf16_kernel<<<g1, 256, 0, st>>>(X, x_stride, K, N, n_pad, xb, x_batch);
-    B200_CUDA_TRY(cudaGetLastError());
+    B200_CUDA_TRY(launch_chained(mmq_x_to_bf16_kernel, g1, 256, 0, st, X, x_stride, K, N, n_pad, xb, x_batch));
     MmqParams p;
     p.W = (const unsigned char *)W; p.w_row_bytes = w_row_bytes; p.Xb = xb; p.dst = dst; p.dst_stride = dst_stride; p.K = K; p.M = M; p.N = N;
     p.tile_tab = nullptr; p.row_dst = nullptr; p.expert_bytes = 0;
@@ -874,12 +875,10 @@ extern "C" int b200_mul_mat_id_q(int type, const void *as, size_t w_row_bytes, s
     t.tile_tab = (int *)((unsigned char *)workspace + mid_xb_bytes(n_rows, K));
     t.row_src = t.tile_tab + 1 + 3 * max_tiles;
     t.row_dst = t.row_src + n_rows;
-    mid_group_kernel<<<1, 1024, 0, st>>>(ids, ids_stride, (int)n_used, (int)T, (int)n_expert, (int)n_b_rows, b_stride_row, b_stride_tok, dst_stride_row,
-                                         dst_stride_tok, (int)bn, t);
-    B200_CUDA_TRY(cudaGetLastError());
+    B200_CUDA_TRY(launch_chained(mid_group_kernel, 1, 1024, 0, st, ids, ids_stride, (int)n_used, (int)T, (int)n_expert, (int)n_b_rows, b_stride_row, b_stride_tok, dst_stride_row,
+                                 dst_stride_tok, (int)bn, t));
     dim3 g1((unsigned)((K / 4 + 255) / 256), (unsigned)n_rows);
-    mid_gather_bf16_kernel<<<g1, 256, 0, st>>>(b, t.row_src, K, xb);
-    B200_CUDA_TRY(cudaGetLastError());
+    B200_CUDA_TRY(launch_chained(mid_gather_bf16_kernel, g1, 256, 0, st, b, t.row_src, K, xb));
     MmqParams p;
     p.W = (const unsigned char *)as; p.w_row_bytes = w_row_bytes; p.Xb = xb; p.dst = dst; p.dst_stride = 0; p.K = K; p.M = M; p.N = n_rows;
     p.tile_tab = t.tile_tab; p.row_dst = t.row_dst; p.expert_bytes = expert_bytes;

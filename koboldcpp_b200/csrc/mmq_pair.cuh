@@ -391,8 +391,6 @@ __global__ void __launch_bounds__(pair_threads<TYPE>(), 1) mmq_pair_kernel(const
     const int rank = (int)cluster_rank(), pair = (int)(blockIdx.x >> 1), n_pairs = (int)(gridDim.x >> 1);
     const long long limit = p.q.wait_limit;
     const int S = p.stages, stage_bytes = A_BYTES + p.bn * MQ_BK;  // (bn / 2 activation rows of 128 bytes)
-    const int nt = GROUPED ? __ldg(p.q.tile_tab) : p.n_tiles_n;
-    const int n_tiles = nt * p.n_tiles_m * (GROUPED ? 1 : p.q.n_batch > 1 ? p.q.n_batch : p.q.ksplit);
     const unsigned full0 = smem_u32(full_bar), peer0 = smem_u32(peer_bar), empty0 = smem_u32(empty_bar), acc_full0 = smem_u32(acc_full), acc_empty0 = smem_u32(acc_empty);
 
     if (tid == 0) {
@@ -413,6 +411,9 @@ __global__ void __launch_bounds__(pair_threads<TYPE>(), 1) mmq_pair_kernel(const
     if (warp == NP || warp >= NP + 2) pair_await();
     tc_fence_after();
     const unsigned tmem_base = tmem_base_s;
+    pdl_enter();
+    const int nt = GROUPED ? p.q.tile_tab[0] : p.n_tiles_n;
+    const int n_tiles = nt * p.n_tiles_m * (GROUPED ? 1 : p.q.n_batch > 1 ? p.q.n_batch : p.q.ksplit);
 
     if (warp < NP) {
         // ===== producers: rows 8 * warp .. 8 * warp + 7 of this CTA's 128
@@ -743,13 +744,15 @@ static int mmq_pair_launch(const MmqParams &q, int64_t n_pad, int64_t w_rows_per
     cfg.blockDim = dim3(pair_threads<TYPE>());
     cfg.dynamicSmemBytes = PAIR_SMEM;
     cfg.stream = st;
-    cudaLaunchAttribute at[1];
+    cudaLaunchAttribute at[2];  // (as launch_chained, in pairs)
     at[0].id = cudaLaunchAttributeClusterDimension;
     at[0].val.clusterDim.x = 2;
     at[0].val.clusterDim.y = 1;
     at[0].val.clusterDim.z = 1;
+    at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = at;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = 2;
     B200_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, tmA, tmB, p));
     return B200_OK;
 }

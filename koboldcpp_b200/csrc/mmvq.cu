@@ -149,6 +149,7 @@ __global__ void __launch_bounds__(MMVQ_THREADS, 1) mmvq_kernel(const __grid_cons
     // when the producer's CTA there has retired, so little overlap is lost.
     const bool acts_first = NCOLS == 1 && p.K <= ACT_RR_MAX && nrows > 0;
     ActRegs aregs;
+    if (p.in_order) pdl_wait();
     // p.prefill stages of the ring are filled BEFORE the wait for the producer kernel (weights do not depend on it)
     int s_fill = 0;
     if (!MULTI || p.ids == nullptr)
@@ -319,6 +320,7 @@ static int launch_mmvq(MmvqParams &p, cudaStream_t st, bool pdl) {
     p.n_stage = (int)ns;
     static const int prefill_pct = getenv("B200_MMVQ_PREFILL") ? atoi(getenv("B200_MMVQ_PREFILL")) : 0;
     p.prefill = pdl ? (int)(ns * prefill_pct / 100) : 0;
+    p.in_order = !pdl;
     static const int dbg = getenv("B200_MMVQ_DBG") ? atoi(getenv("B200_MMVQ_DBG")) : 0;
     p.dbg = dbg;
     TRACE_SLOT(p);
@@ -343,7 +345,7 @@ static int launch_mmvq(MmvqParams &p, cudaStream_t st, bool pdl) {
     at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = at;
-    cfg.numAttrs = pdl ? 1 : 0;
+    cfg.numAttrs = 1;
     B200_CUDA_TRY(cudaLaunchKernelEx(&cfg, mmvq_kernel<TYPE, NCOLS, MULTI>, p));
     return B200_OK;
 }
@@ -406,7 +408,7 @@ static int launch_mmvq3(MmvqParams &p, cudaStream_t st, bool pdl) {
     at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = at;
-    cfg.numAttrs = pdl ? 1 : 0;
+    cfg.numAttrs = 1;
     B200_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, p));
     return B200_OK;
 }
@@ -484,7 +486,7 @@ static int dispatch_cols(MmvqParams &p, int N, cudaStream_t st, bool pdl) {
     return B200_ERR_INVALID;
 }
 
-bool g_mmvq_pdl = false;  // set by the backend when it launches chains of dependent kernels
+bool g_mmvq_pdl = false;  // weights are read ahead of the kernels in front: set by the backend, whose chains write no weights
 
 int mmvq_launch(int type, const b200_gemv_job *jobs, int n_jobs, size_t w_row_bytes, int64_t x_stride, int64_t dst_stride,
                 int64_t K, int64_t N, const int32_t *ids, size_t expert_bytes, int32_t n_expert, cudaStream_t st,

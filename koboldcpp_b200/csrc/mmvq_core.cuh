@@ -16,6 +16,7 @@ struct MmvqParams {
     int            n_stage;
     int            dbg;
     int            prefill;       // ring stages filled before griddepcontrol.wait
+    int            in_order;      // nothing is read before griddepcontrol.wait, weights included (b200_set_pdl is off)
     int            n_it;          // ceil(K / 4096): steps per row
     int            n_expert;
     int            rows_q, rows_rem;   // rows per CTA = rows_q (+1 for the first rows_rem CTAs)

@@ -201,6 +201,7 @@ __global__ void __launch_bounds__(MV_NW * 32, 1) mmvq_mma_kernel(const __grid_co
         cp_async_commit();
         slot_in = slot_in + 1 == SLOTS ? 0 : slot_in + 1;
     };
+    if (p.m.in_order) pdl_wait();
     for (int i = 0; i < SLOTS - 1; i++) copy_block();
     pdl_wait();
     pdl_trigger();
@@ -314,6 +315,7 @@ template <int TYPE>
 static int launch_mmvq_mma(const MmvqParams &m, int N, cudaStream_t st, bool pdl) {
     MvParams p;
     p.m = m;
+    p.m.in_order = !pdl;
     p.n = N;
     p.div_n8 = (unsigned)(((1ull << 32) + m.K / 8 - 1) / (m.K / 8));
     int64_t tiles = 0;
@@ -352,7 +354,7 @@ static int launch_mmvq_mma(const MmvqParams &m, int N, cudaStream_t st, bool pdl
     at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = at;
-    cfg.numAttrs = pdl ? 1 : 0;
+    cfg.numAttrs = 1;
     B200_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, p));
     return B200_OK;
 }

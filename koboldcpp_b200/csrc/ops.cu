@@ -39,24 +39,6 @@ static bool same_shape(const b200_tensor *a, const b200_tensor *b) {
         }                                         \
     } while (0)
 
-// Launch with the programmatic-dependent-launch attribute when the backend asked for it: the kernel may be scheduled while
-// its producer drains (it begins with griddepcontrol.wait) and lets its consumer's prologue start at once.
-extern bool g_mmvq_pdl;
-#define LAUNCH_PDL(kernel, grid, block, st, ...)                                       \
-    do {                                                                               \
-        cudaLaunchConfig_t cfg__ = {};                                                 \
-        cfg__.gridDim = dim3(grid);                                                    \
-        cfg__.blockDim = dim3(block);                                                  \
-        cfg__.stream = (st);                                                           \
-        cudaLaunchAttribute at__[1];                                                   \
-        at__[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;               \
-        at__[0].val.programmaticStreamSerializationAllowed = 1;                        \
-        cfg__.attrs = at__;                                                            \
-        cfg__.numAttrs = g_mmvq_pdl ? 1 : 0;                                           \
-        B200_CUDA_TRY(cudaLaunchKernelEx(&cfg__, kernel, __VA_ARGS__));                \
-    } while (0)
-__device__ __forceinline__ void pdl_enter() { pdl_wait(); pdl_trigger(); }
-
 __device__ __forceinline__ float block_sum(float v, float *sh) {
     v = warp_sum(v);
     const int w = threadIdx.x >> 5, l = threadIdx.x & 31, nw = blockDim.x >> 5;
@@ -80,6 +62,7 @@ __device__ __forceinline__ float block_max(float v, float *sh) {
 
 // ------------------------------------------------------------------------------------------------ RMS_NORM (+MUL)
 __global__ void rms_norm_kernel(TD x, const float *__restrict__ w, TD dst, float eps, float *__restrict__ norm_out) {
+    pdl_enter(w);
     __shared__ float sh[32];
     const int64_t r = blockIdx.x;
     const int64_t i1 = r % x.ne[1], i2 = (r / x.ne[1]) % x.ne[2], i3 = r / (x.ne[1] * x.ne[2]);
@@ -123,6 +106,7 @@ __global__ void rms_norm_kernel(TD x, const float *__restrict__ w, TD dst, float
 // is read once.  Bound by HBM; 512 rows of 4096: 10.8 us in two passes of one piece a thread and trip, 5.9 here (cold).
 template <int NV>
 __global__ void rms_norm_row_kernel(TD x, const float4 *__restrict__ w, TD dst, float eps, float *__restrict__ norm_out) {
+    pdl_enter(w);
     __shared__ float sh[32];
     const int64_t r = blockIdx.x;
     const int64_t i1 = r % x.ne[1], i2 = (r / x.ne[1]) % x.ne[2], i3 = r / (x.ne[1] * x.ne[2]);
@@ -739,6 +723,7 @@ template <int NC, int RPW>
 __global__ void __launch_bounds__(128) gemv_bf16_kernel(const unsigned char *__restrict__ W, int64_t w_row_bytes, int64_t w_batch_bytes, const float *__restrict__ X,
                                                         int64_t x_stride, int64_t x_batch, float *__restrict__ dst, int64_t dst_stride, int64_t dst_batch, int64_t K,
                                                         int64_t M) {
+    pdl_enter(W, X);
     const int64_t m0 = ((int64_t)blockIdx.x * 4 + (threadIdx.x >> 5)) * RPW;
     const int lane = threadIdx.x & 31;
     if (m0 >= M) return;
@@ -787,6 +772,7 @@ template <int NC>
 __global__ void __launch_bounds__(GW_WARPS * 32) gemv_bf16_wide_kernel(const unsigned char *__restrict__ W, int64_t w_row_bytes, int64_t w_batch_bytes, const float *__restrict__ X,
                                                                        int64_t x_stride, int64_t x_batch, float *__restrict__ dst, int64_t dst_stride, int64_t dst_batch,
                                                                        int64_t K, int64_t M) {
+    pdl_enter(W, X);
     __shared__ float part[GW_WARPS][GW_ROWS * NC];
     const int64_t m0 = (int64_t)blockIdx.x * GW_ROWS;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -853,6 +839,7 @@ __device__ __forceinline__ void gm_mma_bf16(float (&c)[4], unsigned a0, unsigned
 __global__ void __launch_bounds__(GM_WARPS * 32) gemv_bf16_mma_kernel(const unsigned char *__restrict__ W, int64_t w_row_bytes, int64_t w_batch_bytes, const float *__restrict__ X,
                                                                       int64_t x_stride, int64_t x_batch, float *__restrict__ dst, int64_t dst_stride, int64_t dst_batch,
                                                                       int64_t K, int64_t M, int nc) {
+    pdl_enter(W, X);
     __shared__ float part[GM_WARPS][GM_ROWS * 8];
     const int64_t m0 = (int64_t)blockIdx.x * GM_ROWS;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t4 = lane & 3;
@@ -911,24 +898,22 @@ __global__ void __launch_bounds__(GM_WARPS * 32) gemv_bf16_mma_kernel(const unsi
 }
 
 template <int NC>
-static void launch_gemv_bf16(const b200_tensor *w, const b200_tensor *x, const b200_tensor *dst, cudaStream_t st) {
+static cudaError_t launch_gemv_bf16(const b200_tensor *w, const b200_tensor *x, const b200_tensor *dst, cudaStream_t st) {
     const int64_t M = w->ne[1], nb = x->ne[2];
     const int64_t wb = w->ne[2] > 1 ? (int64_t)w->nb[2] : 0;
     if constexpr (NC >= 3) {
         if (w->ne[0] % 32 == 0) {
             const dim3 grid((unsigned)((M + GM_ROWS - 1) / GM_ROWS), (unsigned)nb);
-            gemv_bf16_mma_kernel<<<grid, GM_WARPS * 32, 0, st>>>((const unsigned char *)w->data, (int64_t)w->nb[1], wb, (const float *)x->data, (int64_t)(x->nb[1] / 4),
+            return launch_chained(gemv_bf16_mma_kernel, grid, GM_WARPS * 32, 0, st, (const unsigned char *)w->data, (int64_t)w->nb[1], wb, (const float *)x->data, (int64_t)(x->nb[1] / 4),
                                                                  (int64_t)(x->nb[2] / 4), (float *)dst->data, (int64_t)(dst->nb[1] / 4), (int64_t)(dst->nb[2] / 4), w->ne[0], M, NC);
-            return;
         }
         const dim3 grid((unsigned)((M + GW_ROWS - 1) / GW_ROWS), (unsigned)nb);
-        gemv_bf16_wide_kernel<NC><<<grid, GW_WARPS * 32, 0, st>>>((const unsigned char *)w->data, (int64_t)w->nb[1], wb, (const float *)x->data, (int64_t)(x->nb[1] / 4),
+        return launch_chained(gemv_bf16_wide_kernel<NC>, grid, GW_WARPS * 32, 0, st, (const unsigned char *)w->data, (int64_t)w->nb[1], wb, (const float *)x->data, (int64_t)(x->nb[1] / 4),
                                                                   (int64_t)(x->nb[2] / 4), (float *)dst->data, (int64_t)(dst->nb[1] / 4), (int64_t)(dst->nb[2] / 4), w->ne[0], M);
-        return;
     }
     constexpr int RPW = 1;
     const dim3 grid((unsigned)((M + 4 * RPW - 1) / (4 * RPW)), (unsigned)nb);
-    gemv_bf16_kernel<NC, RPW><<<grid, 128, 0, st>>>((const unsigned char *)w->data, (int64_t)w->nb[1], wb, (const float *)x->data, (int64_t)(x->nb[1] / 4),
+    return launch_chained(gemv_bf16_kernel<NC, RPW>, grid, 128, 0, st, (const unsigned char *)w->data, (int64_t)w->nb[1], wb, (const float *)x->data, (int64_t)(x->nb[1] / 4),
                                                     (int64_t)(x->nb[2] / 4), (float *)dst->data, (int64_t)(dst->nb[1] / 4), (int64_t)(dst->nb[2] / 4), w->ne[0], M);
 }
 
@@ -946,12 +931,10 @@ static int rms_norm_launch(const b200_tensor *x, const float *w, const b200_tens
     const int64_t n4 = x->ne[0] / 4;
     if ((bits & 15) == 0 && n4 >= 64 && n4 <= 2048) {
         const int nv = n4 <= 256 ? 1 : 4, threads = (int)(((n4 + nv - 1) / nv + 31) / 32 * 32);
-        if (nv == 1) rms_norm_row_kernel<1><<<(unsigned)rows, threads, 0, st>>>(td(x), (const float4 *)w, td(dst), eps, norm_out);
-        else rms_norm_row_kernel<4><<<(unsigned)rows, threads, 0, st>>>(td(x), (const float4 *)w, td(dst), eps, norm_out);
+        B200_CUDA_TRY(launch_chained(nv == 1 ? rms_norm_row_kernel<1> : rms_norm_row_kernel<4>, (unsigned)rows, threads, 0, st, td(x), (const float4 *)w, td(dst), eps, norm_out));
     } else {
-        rms_norm_kernel<<<(unsigned)rows, block, 0, st>>>(td(x), w, td(dst), eps, norm_out);
+        B200_CUDA_TRY(launch_chained(rms_norm_kernel, (unsigned)rows, block, 0, st, td(x), w, td(dst), eps, norm_out));
     }
-    B200_CUDA_TRY(cudaGetLastError());
     return B200_OK;
 }
 extern "C" int b200_op_rms_norm(const b200_tensor *x, const float *w, const b200_tensor *dst, float eps, b200_stream_t stream) {
@@ -980,9 +963,9 @@ extern "C" int b200_op_silu_mul(const float *gate, const float *up, float *act_o
     // few values: one a thread fills more SMs (14336 of them are 7 CTAs of the vector form, whose thread works through eight exponentials: 1 us more in
     // a chain of launches, 38.4 us for a routed feed-forward of one token against 39.4)
     if (n >= 262144 && (n & 3) == 0 && (((uintptr_t)gate | (uintptr_t)up | (uintptr_t)act_out | (uintptr_t)dst) & 15) == 0)
-        LAUNCH_PDL(silu_mul_vec_kernel, grid1d((n / 4 + 1) / 2, 256), 256, (cudaStream_t)stream, (const float4 *)gate, (const float4 *)up, (float4 *)act_out, (float4 *)dst, n / 4);
+        B200_CUDA_TRY(launch_chained(silu_mul_vec_kernel, grid1d((n / 4 + 1) / 2, 256), 256, 0, (cudaStream_t)stream, (const float4 *)gate, (const float4 *)up, (float4 *)act_out, (float4 *)dst, n / 4));
     else
-        LAUNCH_PDL(silu_mul_kernel, grid1d(n, 256), 256, (cudaStream_t)stream, gate, up, act_out, dst, n);
+        B200_CUDA_TRY(launch_chained(silu_mul_kernel, grid1d(n, 256), 256, 0, (cudaStream_t)stream, gate, up, act_out, dst, n));
     return B200_OK;
 }
 
@@ -1104,7 +1087,7 @@ extern "C" int b200_op_rope_kv_store(const b200_tensor *q, const b200_tensor *q_
     if (nq + nk == 0) return B200_OK;
     const int64_t total = (nq + 31) / 32 * 32 + 2 * ((nk + 31) / 32 * 32);
     const RopeDev rd = rope_dev(rp);
-    LAUNCH_PDL(rope_kv_store_kernel, grid1d(total, 256), 256, (cudaStream_t)stream, a, pos, freq_factors, rd);
+    B200_CUDA_TRY(launch_chained(rope_kv_store_kernel, grid1d(total, 256), 256, 0, (cudaStream_t)stream, a, pos, freq_factors, rd));
     return B200_OK;
 }
 
@@ -1209,8 +1192,8 @@ extern "C" int b200_op_moe_router(const float *logits, int64_t ld_logits, float 
     REQUIRE(n_expert >= 1 && n_expert <= ROUTER_MAX_EXPERT && n_used >= 1 && n_used <= 32 && n_used <= n_expert && n_tok >= 0, B200_ERR_UNSUPPORTED,
             "b200_op_moe_router: up to %d experts, up to 32 used", ROUTER_MAX_EXPERT);
     if (n_tok == 0) return B200_OK;
-    LAUNCH_PDL(moe_router_kernel, (unsigned)((n_tok + ROUTER_WARPS - 1) / ROUTER_WARPS), ROUTER_WARPS * 32, (cudaStream_t)stream, logits, ld_logits, probs, ld_probs, ids,
-               ld_ids, w_gather, wsum, w_out, (int)n_expert, (int)n_used, n_tok);
+    B200_CUDA_TRY(launch_chained(moe_router_kernel, (unsigned)((n_tok + ROUTER_WARPS - 1) / ROUTER_WARPS), ROUTER_WARPS * 32, 0, (cudaStream_t)stream, logits, ld_logits, probs, ld_probs, ids,
+               ld_ids, w_gather, wsum, w_out, (int)n_expert, (int)n_used, n_tok));
     return B200_OK;
 }
 
@@ -1255,16 +1238,15 @@ extern "C" int b200_op_mul_mat_float(const b200_tensor *w, const b200_tensor *x,
         w->ne[0] % 8 == 0 && (((uintptr_t)w->data | w->nb[1] | w->nb[2] | (uintptr_t)x->data | x->nb[1] | x->nb[2]) & 15) == 0 && ((dst->nb[1] | dst->nb[2]) & 3) == 0) {
         const cudaStream_t st = (cudaStream_t)stream;
         switch (x->ne[1]) {
-            case 1: launch_gemv_bf16<1>(w, x, dst, st); break;
-            case 2: launch_gemv_bf16<2>(w, x, dst, st); break;
-            case 3: launch_gemv_bf16<3>(w, x, dst, st); break;
-            case 4: launch_gemv_bf16<4>(w, x, dst, st); break;
-            case 5: launch_gemv_bf16<5>(w, x, dst, st); break;
-            case 6: launch_gemv_bf16<6>(w, x, dst, st); break;
-            case 7: launch_gemv_bf16<7>(w, x, dst, st); break;
-            default: launch_gemv_bf16<8>(w, x, dst, st); break;
+            case 1: B200_CUDA_TRY(launch_gemv_bf16<1>(w, x, dst, st)); break;
+            case 2: B200_CUDA_TRY(launch_gemv_bf16<2>(w, x, dst, st)); break;
+            case 3: B200_CUDA_TRY(launch_gemv_bf16<3>(w, x, dst, st)); break;
+            case 4: B200_CUDA_TRY(launch_gemv_bf16<4>(w, x, dst, st)); break;
+            case 5: B200_CUDA_TRY(launch_gemv_bf16<5>(w, x, dst, st)); break;
+            case 6: B200_CUDA_TRY(launch_gemv_bf16<6>(w, x, dst, st)); break;
+            case 7: B200_CUDA_TRY(launch_gemv_bf16<7>(w, x, dst, st)); break;
+            default: B200_CUDA_TRY(launch_gemv_bf16<8>(w, x, dst, st)); break;
         }
-        B200_CUDA_TRY(cudaGetLastError());
         return B200_OK;
     }
     if (w->type == B200_TYPE_F32 && w->ne[2] == 1 && w->ne[3] == 1 && x->ne[2] == 1 && x->ne[3] == 1 && w->ne[0] >= 512 && w->ne[1] <= 256 && x->ne[1] <= 65535 && dst->nb[0] == 4) {

@@ -21,6 +21,7 @@ __device__ __forceinline__ float softplus_f(float x) { return fmaxf(x, 0.f) + lo
 constexpr int SC_TOK = 16, SC_MAX_TAPS = SC_TOK + 1;
 template <int KMAX>
 __global__ void __launch_bounds__(128) short_conv_kernel(const b200_short_conv_args a) {
+    pdl_enter();
     const int c = blockIdx.x * 128 + threadIdx.x, s = blockIdx.z;
     const int first = a.seq_info[s], count = a.seq_info[a.n_seq + s], slot = a.seq_info[2 * a.n_seq + s], fresh = a.seq_info[3 * a.n_seq + s];
     const int t0 = blockIdx.y * SC_TOK;
@@ -411,6 +412,7 @@ template <int DQ, bool CHAN, int CTAS>  // dim <= 32 DQ; CTAs that an SM is to h
 __global__ void __launch_bounds__(DR_WARPS * 64, CTAS) delta_rule_scan_kernel(const b200_delta_rule_args a) {
     constexpr int DR_CHUNK = dr_chunk<DQ, CHAN>();
     extern __shared__ __align__(16) float dr_shared[];
+    pdl_enter();
     const int h = blockIdx.y, s = blockIdx.z, kvh = h / (a.heads / a.kv_heads);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int D = a.dim, V = a.vdim;
@@ -513,8 +515,7 @@ static int launch_delta_rule3(const b200_delta_rule_args *a, dim3 grid, cudaStre
             attr_set_dev[dev & 15] = true;
         }
     }
-    kern<<<grid, DR_WARPS * 64, SMEM, st>>>(*a);
-    B200_CUDA_TRY(cudaGetLastError());
+    B200_CUDA_TRY(launch_chained(kern, grid, DR_WARPS * 64, SMEM, st, *a));
     return B200_OK;
 }
 // Up to a CTA an SM: all the registers it wants (512 tokens, 32 heads of 128 x 128: 87 us, 97 with the registers of two).  More CTAs than that:
@@ -751,10 +752,7 @@ extern "C" int b200_op_short_conv(const b200_short_conv_args *a, b200_stream_t s
     if (a->n_seq == 0 || a->n_tokens == 0) return B200_OK;
     const dim3 grid((unsigned)((a->channels + 127) / 128), (unsigned)((a->n_tokens + SC_TOK - 1) / SC_TOK), (unsigned)a->n_seq);
     OPX_REQUIRE(grid.y <= 65535, B200_ERR_UNSUPPORTED, "b200_op_short_conv: at most %d tokens in a batch", 65535 * SC_TOK);
-    if (a->taps <= 4) short_conv_kernel<4><<<grid, 128, 0, (cudaStream_t)stream>>>(*a);
-    else if (a->taps <= 8) short_conv_kernel<8><<<grid, 128, 0, (cudaStream_t)stream>>>(*a);
-    else short_conv_kernel<0><<<grid, 128, 0, (cudaStream_t)stream>>>(*a);
-    B200_CUDA_TRY(cudaGetLastError());
+    B200_CUDA_TRY(launch_chained(a->taps <= 4 ? short_conv_kernel<4> : a->taps <= 8 ? short_conv_kernel<8> : short_conv_kernel<0>, grid, 128, 0, (cudaStream_t)stream, *a));
     return B200_OK;
 }
 

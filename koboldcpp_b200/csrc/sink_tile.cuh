@@ -24,6 +24,7 @@ static inline size_t st_workspace(const b200_sink_attn_args *a) { return (size_t
 
 // one CTA a cell: all kv heads' rows, four values a thread and step
 __global__ void __launch_bounds__(256) sink_rows_bf16_kernel(const b200_sink_attn_args a, int ks, int vs, int64_t cells, uint2 *__restrict__ kd, uint2 *__restrict__ vd) {
+    pdl_enter();
     const int64_t c = blockIdx.x;
     const bool used = c < a.n_kv && a.cell_seq[c] >= 0;
     const bool k4 = a.dim % 4 == 0 && a.k_cache_stride % 4 == 0 && ((uintptr_t)a.k_cache & 15) == 0, v4 = a.vdim % 4 == 0 && a.v_cache_stride % 4 == 0 && ((uintptr_t)a.v_cache & 15) == 0;
@@ -49,6 +50,7 @@ __global__ void __launch_bounds__(256) sink_rows_bf16_kernel(const b200_sink_att
 
 template <int KS, int VS>
 __global__ void __launch_bounds__(ST_WARPS * 32, 2) sink_attn_tile_kernel(const b200_sink_attn_args a, const unsigned char *__restrict__ kd, const unsigned char *__restrict__ vd, int64_t cells) {
+    pdl_enter(kd, vd);
     constexpr int KROW = KS * 32, VROW = VS * 32, KSTRIDE = KROW + 16, VSTRIDE = VROW + 16, KTILE = ST_CELLS * KSTRIDE, STAGE = KTILE + ST_CELLS * VSTRIDE, NB = ST_STEP / 8;
     constexpr float LOG2E = 1.4426950408889634f;
     extern __shared__ __align__(128) unsigned char st_smem[];
@@ -290,8 +292,7 @@ template <int KS, int VS>
 static int st_launch2(const b200_sink_attn_args *a, unsigned char *ws, cudaStream_t st) {
     const int64_t cells = st_cells(a);
     unsigned char *kd = ws, *vd = ws + (size_t)a->n_head_kv * cells * KS * 32;
-    sink_rows_bf16_kernel<<<(unsigned)cells, 256, 0, st>>>(*a, KS, VS, cells, (uint2 *)kd, (uint2 *)vd);
-    B200_CUDA_TRY(cudaGetLastError());
+    B200_CUDA_TRY(launch_chained(sink_rows_bf16_kernel, (unsigned)cells, 256, 0, st, *a, KS, VS, cells, (uint2 *)kd, (uint2 *)vd));
     constexpr int smem = ST_NBUF * ST_CELLS * ((KS + VS) * 32 + 32);
     static bool attr_set_dev[16] = {};  // cudaFuncSetAttribute is per device
     int cur_dev = 0;
@@ -302,8 +303,7 @@ static int st_launch2(const b200_sink_attn_args *a, unsigned char *ws, cudaStrea
         attr_set = true;
     }
     const dim3 grid((unsigned)(((int64_t)a->n_tokens * (a->n_head / a->n_head_kv) + ST_COLS - 1) / ST_COLS), (unsigned)a->n_head_kv);
-    sink_attn_tile_kernel<KS, VS><<<grid, ST_WARPS * 32, smem, st>>>(*a, kd, vd, cells);
-    B200_CUDA_TRY(cudaGetLastError());
+    B200_CUDA_TRY(launch_chained(sink_attn_tile_kernel<KS, VS>, grid, ST_WARPS * 32, smem, st, *a, kd, vd, cells));
     return B200_OK;
 }
 template <int KS>
