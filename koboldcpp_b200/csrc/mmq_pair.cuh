@@ -10,6 +10,9 @@
 //   * 16 producer warps a CTA, 8 weight rows each: a warp copies the raw blocks of its rows (256 values of each, contiguous 16-byte cp.async) into
 //     a ring of its own, one or two groups ahead, and unpacks them with packed f32 arithmetic, lane = (K step, half, row), two K
 //     steps at a time into the 128-byte-swizzled operand tiles.  No barrier among the warps.
+//   * a stage holds those two K steps (dense weights: one).  Waiting, passing on and committing cost each warp about 60 instructions among 20 warps, per
+//     stage: with a stage of one step q4_K took 0.324 us a step of 64 values at 64 columns and 0.331 at 128, with two 0.288 and 0.295; a
+//     launch's start and end went from 10.6 .. 16 to 8.3 .. 11 us.
 //   * the MMA warp walks through its loop as a whole and elects a lane for the tcgen05 instructions only: loop counters and descriptors then
 //     live in uniform registers.  (With one lane in the loop every MMA needed a dozen vector instructions, each of which waits its turn
 //     among the producers: 190 cycles an MMA whatever its width.)
@@ -374,13 +377,14 @@ __device__ __forceinline__ PairTile pair_tile(const PairParams &p, int t, int nt
     return r;
 }
 
+template <int TYPE> __host__ __device__ constexpr int pair_steps() { return TYPE == B200_TYPE_BF16 ? 1 : 2; }  // K steps of 64 a stage
 template <int TYPE>
 __host__ __device__ constexpr int pair_threads() { return 32 * ((TYPE == B200_TYPE_BF16 ? 0 : PAIR_PRODUCERS) + 6); }
 
 template <int TYPE, bool GROUPED>
 __global__ void __launch_bounds__(pair_threads<TYPE>(), 1) mmq_pair_kernel(const __grid_constant__ TmapBytes tmA, const __grid_constant__ TmapBytes tmB, const __grid_constant__ PairParams p) {
     constexpr bool DENSE = TYPE == B200_TYPE_BF16;
-    constexpr int NP = DENSE ? 0 : PAIR_PRODUCERS, A_BYTES = MQ_BM * MQ_BK * 2, UNIT = DENSE ? 1 : 4;
+    constexpr int NP = DENSE ? 0 : PAIR_PRODUCERS, SK = pair_steps<TYPE>(), A_STEP = MQ_BM * MQ_BK * 2, A_BYTES = SK * A_STEP, UNIT = DENSE ? 1 : 4;
     constexpr int G256 = DENSE ? 0 : group256_bytes(TYPE);
     extern __shared__ unsigned char smem_raw[];
     unsigned char *smem = reinterpret_cast<unsigned char *>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
@@ -390,7 +394,7 @@ __global__ void __launch_bounds__(pair_threads<TYPE>(), 1) mmq_pair_kernel(const
     const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31, tid = threadIdx.x;
     const int rank = (int)cluster_rank(), pair = (int)(blockIdx.x >> 1), n_pairs = (int)(gridDim.x >> 1);
     const long long limit = p.q.wait_limit;
-    const int S = p.stages, stage_bytes = A_BYTES + p.bn * MQ_BK;  // (bn / 2 activation rows of 128 bytes)
+    const int S = p.stages, b_step = p.bn * MQ_BK, stage_bytes = A_BYTES + SK * b_step;  // (a step: bn / 2 activation rows of 128 bytes)
     const unsigned full0 = smem_u32(full_bar), peer0 = smem_u32(peer_bar), empty0 = smem_u32(empty_bar), acc_full0 = smem_u32(acc_full), acc_empty0 = smem_u32(acc_empty);
 
     if (tid == 0) {
@@ -463,11 +467,11 @@ __global__ void __launch_bounds__(pair_threads<TYPE>(), 1) mmq_pair_kernel(const
             for (int i = 0; i < SLOTS - 1; i++) copy_group();
             const int cc = lane >> 4, h = (lane >> 3) & 1, r = lane & 7;  // chunk of a pair of K steps, half of its bytes, row
             // the lane's four 16-byte pieces of row r, swizzled
-            const unsigned a_row = smem_u32(smem) + (unsigned)(warp * 1024 + r * 128);
+            const unsigned a_row = smem_u32(smem) + (unsigned)(cc * A_STEP + warp * 1024 + r * 128);
             const int f0 = unpack_first(TYPE, h) / 8, f1 = unpack_second(TYPE, h) / 8;
             const unsigned p0 = a_row + (unsigned)((f0 ^ r) << 4), p1 = a_row + (unsigned)(((f0 + 1) ^ r) << 4), p2 = a_row + (unsigned)((f1 ^ r) << 4), p3 = a_row + (unsigned)(((f1 + 1) ^ r) << 4);
-            int s = 0, slot = 0;        // stage of the first K step of the pair
-            unsigned ph = 1;            // parity of its empty barrier: the first pass finds it free
+            int s = 0, slot = 0;
+            unsigned ph = 1;            // parity of the stage's empty barrier: the first pass finds it free
             bool ok = true;  // (the same in all lanes)
             for (int t = pair; t < n_tiles && ok; t += n_pairs) {
                 const PairTile ti = pair_tile<GROUPED>(p, t, nt, UNIT);
@@ -484,24 +488,17 @@ __global__ void __launch_bounds__(pair_threads<TYPE>(), 1) mmq_pair_kernel(const
                     for (int c2 = 0; c2 < 4; c2 += 2) {
                         unsigned o[16];
                         Unpack32<TYPE>::run(row, c2 + cc, h, o);
-                        // stages are freed in order: the second of the two stands for both
-                        const bool wrap = s + 1 >= S;
-                        const int s1 = wrap ? s + 1 - S : s + 1;
-                        const unsigned ph1 = wrap ? ph ^ 1u : ph;
-                        ok = __all_sync(0xffffffffu, pair_wait<20>(empty0 + 8u * s1, ph1, &failed, limit));
+                        ok = __all_sync(0xffffffffu, pair_wait<20>(empty0 + 8u * s, ph, &failed, limit));
                         if (!ok) break;
-                        const int mine = cc ? s1 : s;
-                        const unsigned d = (unsigned)(mine * stage_bytes);
+                        const unsigned d = (unsigned)(s * stage_bytes);
                         asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(p0 + d), "r"(o[0]), "r"(o[1]), "r"(o[2]), "r"(o[3]) : "memory");
                         asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(p1 + d), "r"(o[4]), "r"(o[5]), "r"(o[6]), "r"(o[7]) : "memory");
                         asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(p2 + d), "r"(o[8]), "r"(o[9]), "r"(o[10]), "r"(o[11]) : "memory");
                         asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(p3 + d), "r"(o[12]), "r"(o[13]), "r"(o[14]), "r"(o[15]) : "memory");
                         fence_proxy_async_smem();
                         __syncwarp();
-                        if ((lane & 15) == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(full0 + 8u * mine) : "memory");
-                        s = s1 + 1;
-                        ph = ph1;
-                        if (s == S) { s = 0; ph ^= 1u; }
+                        if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(full0 + 8u * s) : "memory");
+                        if (++s == S) { s = 0; ph ^= 1u; }
                     }
                 }
             }
@@ -518,7 +515,7 @@ __global__ void __launch_bounds__(pair_threads<TYPE>(), 1) mmq_pair_kernel(const
         for (int t = pair; t < n_tiles && ok; t += n_pairs) {
             const PairTile ti = pair_tile<GROUPED>(p, t, nt, UNIT);
             if (rank != 0) {
-                for (int kb = 0; kb < ti.nkb; kb++) {
+                for (int kb = 0; kb < ti.nkb; kb += SK) {
                     ok = __all_sync(0xffffffffu, pair_wait<0>(full0 + 8u * s, ph, &failed, limit));
                     if (!ok) break;
                     if (elected) mbar_arrive_remote(peer_remote + 8u * s);
@@ -533,7 +530,7 @@ __global__ void __launch_bounds__(pair_threads<TYPE>(), 1) mmq_pair_kernel(const
             tc_fence_after();
             unsigned accumulate = 0;
 #pragma unroll 1
-            for (int kb = 0; kb < ti.nkb; kb++) {
+            for (int kb = 0; kb < ti.nkb; kb += SK) {
                 const bool here = pair_wait<0>(full0 + 8u * s, ph, &failed, limit), there = pair_wait<0>(peer0 + 8u * s, ph, &failed, limit);
                 ok = __all_sync(0xffffffffu, here && there);
                 if (!ok) break;
@@ -541,9 +538,12 @@ __global__ void __launch_bounds__(pair_threads<TYPE>(), 1) mmq_pair_kernel(const
                 const unsigned long long ad = desc0 + (unsigned)(s * (stage_bytes >> 4)), bd = ad + (A_BYTES >> 4);
                 if (elected) {
                     // 16 bf16 = 32 bytes further along K inside the swizzle atom: +2 in the (address >> 4) field
-                    tc_mma2_bf16(acc, ad, bd, idesc, accumulate);
 #pragma unroll
-                    for (int k = 1; k < MQ_BK / 16; k++) tc_mma2_bf16(acc, ad + 2u * k, bd + 2u * k, idesc, 1u);
+                    for (int j = 0; j < SK; j++) {
+                        const unsigned long long aj = ad + (unsigned)(j * (A_STEP >> 4)), bj = bd + (unsigned)(j * (b_step >> 4));
+#pragma unroll
+                        for (int k = 0; k < MQ_BK / 16; k++) tc_mma2_bf16(acc, aj + 2u * k, bj + 2u * k, idesc, j + k ? 1u : accumulate);
+                    }
                     tc_commit2(empty0 + 8u * s);
                 }
                 __syncwarp();
@@ -567,19 +567,23 @@ __global__ void __launch_bounds__(pair_threads<TYPE>(), 1) mmq_pair_kernel(const
             const PairTile ti = pair_tile<GROUPED>(p, t, nt, UNIT);
             const int half = ti.n / 2, row = (int)(ti.n0 + rank * half + (GROUPED ? 0 : ti.product * p.q.n_pad));
             const int a_row = DENSE ? (int)(ti.product * p.w_rows_per_product + ti.m0 + rank * MQ_BM) : 0;
-            const unsigned tx = (unsigned)(half * MQ_BK * 2 + (DENSE ? A_BYTES : 0));
+            const unsigned tx = (unsigned)(SK * half * MQ_BK * 2 + (DENSE ? A_BYTES : 0));
             int k = ti.kb0 * MQ_BK;
 #pragma unroll 1
-            for (int kb = 0; kb < ti.nkb; kb++, k += MQ_BK) {
+            for (int kb = 0; kb < ti.nkb; kb += SK, k += SK * MQ_BK) {
                 if (!dead && !pair_wait<20>(empty0 + 8u * s, ph, &failed, limit)) dead = true;
                 if (elected && !dead) {  // no copy without a free stage
                     unsigned char *st = smem + (size_t)(s * stage_bytes);
                     mbar_expect_tx(&full_bar[s], tx);
                     if constexpr (DENSE) tma_load_2d(st, &tmA, k, a_row, &full_bar[s]);
-                    if constexpr (GROUPED) {
-                        for (int r = 0; r < half; r += 16) tma_load_2d(st + A_BYTES + r * MQ_BK * 2, &tmB, k, row + r, &full_bar[s]);
-                    } else {
-                        tma_load_2d(st + A_BYTES, &tmB, k, row, &full_bar[s]);
+#pragma unroll
+                    for (int j = 0; j < SK; j++) {
+                        unsigned char *sb = st + A_BYTES + j * b_step;
+                        if constexpr (GROUPED) {
+                            for (int r = 0; r < half; r += 16) tma_load_2d(sb + r * MQ_BK * 2, &tmB, k + j * MQ_BK, row + r, &full_bar[s]);
+                        } else {
+                            tma_load_2d(sb, &tmB, k + j * MQ_BK, row, &full_bar[s]);
+                        }
                     }
                 }
                 __syncwarp();
@@ -641,12 +645,14 @@ __global__ void __launch_bounds__(pair_threads<TYPE>(), 1) mmq_pair_kernel(const
 }
 
 // ---------------------------------------------------------------- host side
-// Tile width and K split by the time of the longest pair's work, in microseconds.  A K step of 64 costs `unpack` plus 0.6 ns a column while the
-// producers are the slower ones (measured with one tile a pair, see pair_unpack_us), dense weights take 1.25 ns a column but 0.2 at least; a tile
-// more costs about 1.  The last tile's values are stored with nothing behind them to hide it: 30 ns a column (dense 64 x 64 weights: 8.4 us for 64
+// Tile width and K split by the time of the longest pair's work, in microseconds.  A K step of 64 costs what the slower of producers and tensor cores
+// takes, `unpack` or 1.83 ns a column, and a little more where they are level (sixth powers added: within 4 % of q4_K and q6_K at 64 .. 256
+// columns); dense weights take 1.25 ns a column but 0.2 at least; a tile more costs about 1.  The last tile's values are stored with nothing
+// behind them to hide it: 30 ns a column (dense 64 x 64 weights: 8.4 us for 64
 // columns, 12.6 for 512 in tiles of 256; dense 1024 x 1024 over 128 columns 14.5 us as 4 tiles of 128, 11.7 for a kernel with narrower ones).  Two halves of K
 // add into a zeroed dst: that much more traffic, at 1.5 TB/s, and a launch more.  Widths are N / 1, N / 2, ... rounded up to 16.
 struct PairPlan { int bn, ksplit, n_tiles_n; };
+static inline double pair_step_us(double a, double b) { const double a3 = a * a * a, b3 = b * b * b; return sqrt(cbrt(a3 * a3 + b3 * b3)); }
 static inline PairPlan mmq_pair_plan(int64_t M, int64_t N, int64_t K, int n_batch, int pairs, double unpack) {
     PairPlan best = {256, 1, 1};
     double best_cost = -1;
@@ -655,7 +661,7 @@ static inline PairPlan mmq_pair_plan(int64_t M, int64_t N, int64_t K, int n_batc
     const int ks_max = n_batch > 1 || K < 2048 ? 1 : 2;
     for (unsigned parts = (n + 255) / 256, last = (n + 31) / 32; parts <= last; parts++) {
         const unsigned even = ((n + parts - 1) / parts + 15) / 16 * 16, bn = even < 32 ? 32 : even, nt = (n + bn - 1) / bn;
-        const double dense = 1.25e-3 * bn < 0.2 ? 0.2 : 1.25e-3 * bn, step = unpack > 0 ? unpack + 0.6e-3 * bn : dense;
+        const double dense = 1.25e-3 * bn < 0.2 ? 0.2 : 1.25e-3 * bn, step = unpack > 0 ? pair_step_us(unpack, 1.83e-3 * bn) : dense;
         for (int ks = 1; ks <= ks_max; ks++) {
             const uint64_t tiles = (uint64_t)mt * nt * n_batch * ks;
             const double waves = tiles <= np ? 1.0 : (double)((tiles + np - 1) / np);
@@ -677,18 +683,18 @@ static int mmq_pairs() {
     return pairs;
 }
 
-// microseconds a K step of 64 takes while unpacking is the slower side, less 0.6 ns a column: one tile of 256 rows on each of 74 pairs, 64 columns, from the
-// difference between 8192 and 4096 values a row
+// microseconds a K step of 64 takes while unpacking is the slower side: one tile of 256 rows on each of 74 pairs, 64 columns, from the difference
+// between 8192 and 4096 values a row
 template <int TYPE> constexpr double pair_unpack_us() {
     switch (TYPE) {
         case B200_TYPE_BF16: return 0;
-        case B200_TYPE_Q4_0: return 0.29;
-        case B200_TYPE_Q4_K: return 0.30;
-        case B200_TYPE_Q2_K: return 0.32;
-        case B200_TYPE_Q4_1: case B200_TYPE_Q5_K: return 0.34;
-        case B200_TYPE_Q5_0: case B200_TYPE_Q8_0: return 0.38;
-        case B200_TYPE_Q5_1: case B200_TYPE_IQ4_NL: return 0.41;
-        default: return 0.44;  // q6_K, q3_K, iq4_XS
+        case B200_TYPE_Q4_0: case B200_TYPE_Q4_1: case B200_TYPE_Q4_K: return 0.30;
+        case B200_TYPE_Q5_K: return 0.32;
+        case B200_TYPE_Q2_K: return 0.35;
+        case B200_TYPE_Q8_0: return 0.37;
+        case B200_TYPE_Q5_0: case B200_TYPE_Q5_1: return 0.38;
+        case B200_TYPE_IQ4_NL: case B200_TYPE_IQ4_XS: return 0.47;
+        default: return 0.44;  // q6_K, q3_K
     }
 }
 
@@ -722,7 +728,7 @@ static int mmq_pair_launch(const MmqParams &q, int64_t n_pad, int64_t w_rows_per
         p.n_tiles_n = pl.n_tiles_n;
         p.q.ksplit = pl.ksplit;
     }
-    const int stage = MQ_BM * MQ_BK * 2 + p.bn * MQ_BK;
+    const int stage = pair_steps<TYPE>() * (MQ_BM * MQ_BK * 2 + p.bn * MQ_BK);
     p.stages = (PAIR_SMEM - 1024 - raw_bytes(TYPE)) / stage;
     if (p.stages > PAIR_MAX_STAGES) p.stages = PAIR_MAX_STAGES;
     TmapBytes tmA = {}, tmB;
