@@ -206,8 +206,8 @@ B200_API int b200_mul_mat_id_q(int type, const void *as, size_t w_row_bytes, siz
  * of the previous call with the same K and N (sibling matmuls over one activation: Q / K / V, gate / up) and they are used as is. */
 B200_API size_t b200_mul_mat_q_workspace_bytes(int type, int64_t K, int64_t M, int64_t N);
 /* 0, or 1 once a product on the paired-SM kernel (quantised or dense weights, b200_mul_mat_q, b200_mul_mat_id_q, b200_mul_mat_bf16_batched) has given
- * up waiting for its own pipeline in this process: its results are then incomplete, although the call that launched it returned B200_OK.
- * Meaningful after a synchronisation of the stream. */
+ * up waiting for its own pipeline in this process, or a prompt's b200_flash_attn_ext has: its results are then incomplete, although the call that
+ * launched it returned B200_OK.  Meaningful after a synchronisation of the stream. */
 B200_API int b200_gemm_status(void);
 B200_API int b200_mul_mat_q(int type, const void *W, size_t w_row_bytes, const float *X, int64_t x_stride,
                             float *dst, int64_t dst_stride, int64_t K, int64_t M, int64_t N,
@@ -243,6 +243,7 @@ typedef struct {
     size_t      q_nb1, q_nb2, k_nb1, k_nb2, v_nb1, v_nb2, mask_nb1;
     float       scale, max_bias, logit_softcap;
 } b200_fattn_args;
+/* The workspace of a prompt batch (f16 cache, D 64 or 128) is optional: it lets the mask be read once instead of once a kv-head. */
 B200_API size_t b200_flash_attn_workspace_bytes(const b200_fattn_args *a);
 B200_API int b200_flash_attn_ext(const b200_fattn_args *a, void *workspace, size_t workspace_bytes, b200_stream_t stream);
 

@@ -421,6 +421,7 @@ static int g_fa_trace_slot = 0;
 #endif
 }  // namespace b200
 #include "fattn_mma.cuh"
+#include "fattn_tc.cuh"
 namespace b200 {
 
 // ------------------------------------------------------------------------------------------------ host side
@@ -458,6 +459,10 @@ static bool fa_use_mma(const b200_fattn_args *a) {
     return a->type_k == B200_TYPE_F16;
 }
 
+// scratch that the prompt form has a use for: a constant, so that a growing cache or another batch asks for no more.  It is not needed: a call with less works
+// without it.
+static size_t fa_prefill_table(const b200_fattn_args *a) { return (a->D == 64 || a->D == 128) && ft_table_bytes(a) <= FT_TABLE_BYTES ? FT_TABLE_BYTES : 0; }
+
 static FaPlan fa_plan(const b200_fattn_args *a) {
     FaPlan pl;
     const int64_t n_cols = a->N * (a->n_head / a->n_head_kv);
@@ -472,7 +477,7 @@ static FaPlan fa_plan(const b200_fattn_args *a) {
         pl.n_splits = 1;
         pl.tiles_per_split = (int)((a->n_kv + FM_TP - 1) / FM_TP);
         pl.ticket_bytes = 256;
-        pl.part_bytes = 0;
+        pl.part_bytes = fa_prefill_table(a);
         return pl;
     }
     if (fa_use_mma(a)) {
@@ -703,6 +708,8 @@ static int fa_check(const b200_fattn_args *a) {
     return B200_OK;
 }
 
+// bytes of the workspace that a launch may use where another stream's call uses the same memory: what prompts can do without is left out
+size_t fa_shared_bytes(const b200_fattn_args *a, size_t have) { return fa_check(a) == B200_OK && fa_plan(a).prefill ? 0 : have; }
 // bytes of split arrival counters at the front of the workspace (fattn_static.cu clears exactly these before a launch)
 size_t fa_ticket_bytes(const b200_fattn_args *a) { return fa_check(a) == B200_OK ? fa_plan(a).ticket_bytes : 0; }
 
@@ -766,6 +773,12 @@ extern "C" int b200_flash_attn_ext(const b200_fattn_args *a, void *workspace, si
     const cudaStream_t st = (cudaStream_t)stream;
     if (pl.prefill) {
         if (((uintptr_t)a->q | a->q_nb1 | a->q_nb2) & 7) { set_error("b200_flash_attn_ext: Q must be 8-byte aligned"); return B200_ERR_UNSUPPORTED; }
+        if (ft_fits(a)) {
+            unsigned char *table = workspace ? (unsigned char *)workspace + pl.ticket_bytes : nullptr;
+            const size_t room = workspace && workspace_bytes > pl.ticket_bytes ? workspace_bytes - pl.ticket_bytes : 0;
+            const int tc = a->D == 64 ? ft_launch<64>(a, p, table, room, st) : ft_launch<128>(a, p, table, room, st);
+            if (tc != -1000) return tc;
+        }
         switch (a->D) {
             case 64: return fa_launch_prefill<64>(p, pl, st);
             case 80: return fa_launch_prefill<80>(p, pl, st);

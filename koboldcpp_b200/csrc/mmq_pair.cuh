@@ -53,11 +53,6 @@ struct PairParams {
 __device__ __forceinline__ unsigned cluster_rank() { unsigned r; asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r)); return r; }
 __device__ __forceinline__ void pair_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
 __device__ __forceinline__ void pair_await() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
-__device__ __forceinline__ bool elect_lane() {
-    unsigned e;
-    asm volatile("{\n.reg .pred p;\nelect.sync _|p, 0xffffffff;\nselp.u32 %0, 1, 0, p;\n}\n" : "=r"(e));
-    return e != 0;
-}
 __device__ __forceinline__ void tmem_alloc2(unsigned *smem_dst, unsigned ncols) {
     asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(smem_dst)), "r"(ncols) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
@@ -88,33 +83,6 @@ __device__ __forceinline__ unsigned leader_addr(unsigned local) {
     return r;
 }
 __device__ __forceinline__ void mbar_arrive_remote(unsigned bar) { asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory"); }
-__device__ __forceinline__ bool mbar_try(unsigned bar, unsigned parity) {
-    unsigned done;
-    asm volatile(
-        "{\n"
-        ".reg .pred p;\n"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
-        "selp.u32 %0, 1, 0, p;\n"
-        "}\n"
-        : "=r"(done)
-        : "r"(bar), "r"(parity)
-        : "memory");
-    return done != 0;
-}
-// wait with the limit; false, at once, when a role of the CTA has given up.  SLEEP: nanoseconds between two looks (a failing try_wait comes back within
-// some 50 cycles whatever time it is offered, and a dozen polling warps take the issue slots of the others).
-template <int SLEEP>
-__device__ __forceinline__ bool pair_wait(unsigned bar, unsigned parity, volatile int *failed, long long limit) {
-    if (mbar_try(bar, parity)) return true;
-    const long long t0 = clock64();
-    while (!mbar_try(bar, parity)) {
-        if (SLEEP > 0) __nanosleep(SLEEP);
-        if (*failed) return false;
-        if (clock64() - t0 > limit) { *failed = 1; return false; }
-    }
-    return true;
-}
-
 // ---------------------------------------------------------------- 32 values of a row out of shared memory -> 16 packed bf16 pairs
 // Two values at a time (packed f32: one issue slot for both): four small unsigned integers, one per byte of x, become d * q + c as two bf16
 // pairs.  Integers below 128 take the upper mantissa bits of 128 (0x43qq0000 = 128 + q), so that PRMT alone makes the float and the 128
