@@ -57,10 +57,6 @@ __device__ __forceinline__ unsigned pack_h2(float lo, float hi) {
     return *reinterpret_cast<const unsigned *>(&h);
 }
 
-// thread-block cluster: the splits of one (kv-head, column tile) exchange their partial results through distributed shared memory
-__device__ __forceinline__ void cluster_sync_all() {
-    asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
 __device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
 __device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
 // fetch-and-increment of a counter in the shared memory of CTA `rank` of the cluster
@@ -70,16 +66,6 @@ __device__ __forceinline__ unsigned atom_inc_cluster(unsigned *local, unsigned r
     asm volatile("atom.shared::cluster.add.u32 %0, [%1], 1;" : "=r"(v) : "r"(ra) : "memory");
     return v;
 }
-__device__ __forceinline__ float ld_cluster_f32(const float *local, unsigned rank) {
-    unsigned ra;
-    float v;
-    // (not volatile, no memory clobber: the loads of a merge are independent and must overlap -- ordering comes from the
-    // cluster barriers around them)
-    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(ra) : "r"(smem_u32(local)), "r"(rank));
-    asm("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(ra));
-    return v;
-}
-
 // copy rows [row0, row0+16) of one head (f16, D values) into a padded tile; rows >= n_kv are zero-filled
 template <int D>
 __device__ __forceinline__ void mma_load_tile(unsigned char *dst, const unsigned char *base, size_t nb1, int row0, int n_kv, int lane) {
