@@ -509,8 +509,8 @@ static bool fa_use_mma(const b200_fattn_args *a) {
     // group, prompt batch): 32/8 heads @ 32k 67 us in the scalar kernel, 37 here.  One column per kv-head stays with the scalar kernel, whose
     // probabilities and values are f32 (17.8 us for 32 heads @ 2k, 12.3 here in f16)
     if (a->type_k == B200_TYPE_Q8_0) return a->N * (a->n_head / a->n_head_kv) >= 2;
-    // a tiny cache with one or two kv-heads (a rank's share under 8-way tensor parallelism: 8 q-heads on 1 kv-head, 2 MB) is
-    // pure latency: the scalar kernel spreads the q-heads over 8x more CTAs and finishes in 10.6 us against 12.6 us here
+    // a tiny cache (a rank's share under 8-way tensor parallelism, a small model's context) is pure latency: the scalar kernel spreads the q-heads over more
+    // CTAs and keeps f32 probabilities (8 heads on one kv-head of 128, 1024 cells: 6.7 us, 7.9 here; 32 over 4 of 64: 7.1 and 6.8)
     if (a->N == 1 && a->n_head / a->n_head_kv <= 8 && (int64_t)a->n_head_kv * a->n_kv * a->D * 4 < (6 << 20)) return false;
     return a->type_k == B200_TYPE_F16;
 }
