@@ -243,7 +243,9 @@ typedef struct {
     size_t      q_nb1, q_nb2, k_nb1, k_nb2, v_nb1, v_nb2, mask_nb1;
     float       scale, max_bias, logit_softcap;
 } b200_fattn_args;
-/* The workspace of a prompt batch (f16 cache, D 64 or 128) is optional: it lets the mask be read once instead of once a kv-head. */
+/* A workspace starts zeroed.  After that it serves calls of any shape that it is large enough for, one after the other on one stream: the counters at its front are
+ * zero again behind each call, and the scratch of all shapes lies behind them.  Calls that may run at the same time have one each.  The workspace of a
+ * prompt batch (f16 cache, D 64 or 128) is optional: it lets the mask be read once instead of once a kv-head. */
 B200_API size_t b200_flash_attn_workspace_bytes(const b200_fattn_args *a);
 B200_API int b200_flash_attn_ext(const b200_fattn_args *a, void *workspace, size_t workspace_bytes, b200_stream_t stream);
 
@@ -252,7 +254,7 @@ B200_API int b200_flash_attn_ext(const b200_fattn_args *a, void *workspace, size
  * No counterpart in the reference; added at the request of the run's operators.
  * The split partials and arrival counters live in one static device array of B200_FATTN_STATIC_WS_BYTES (8 MiB) that every
  * GPU that loads the library holds until the process exits.  Same kernels, plan and results as b200_flash_attn_ext.
- * Shapes whose b200_flash_attn_workspace_bytes() exceeds the array return B200_ERR_UNSUPPORTED (b200_last_error names both
+ * Shapes whose scratch exceeds the array return B200_ERR_UNSUPPORTED (b200_last_error names both
  * sizes).  ALL calls on a device share the array: calls that overlap on the GPU (different streams, or graph branches that
  * run concurrently) race -- serialise them or use b200_flash_attn_ext with separate workspaces. */
 #define B200_FATTN_STATIC_WS_BYTES (8u << 20)

@@ -28,6 +28,11 @@ constexpr int FA_MAXC  = 8;   // query columns per CTA
 constexpr int FA_MAX_SPLITS = 32;
 constexpr int FA_MAX_CLUSTER = 8;  // splits merged on chip
 constexpr int FA_RS_PAD = 4;   // floats behind the D accumulators of a partial result: m, l, 2 pad
+// A workspace begins with arrival counters, one for each (kv-head, column tile), zero between launches; the scratch of every plan lies behind them, at the same place
+// for all shapes: one workspace serves prompts and decoding in turn, and what one plan leaves in its scratch is never another one's counters.
+// Splits pay below 32.4 waves of unsplit CTAs (one wave saved of more than that is less than the 3 % that fa_plan asks for): 9570 pairs on 148 SMs.
+constexpr int FA_PAIRS = 10240;
+constexpr size_t FA_FRONT = FA_PAIRS * sizeof(int);
 
 struct FaParams {
     const unsigned char *q, *k, *v, *mask;
@@ -485,9 +490,10 @@ struct FaPlan {
     bool prefill;  // tensor-core kernel, prompt form: 64 columns per CTA, tiles shared by its warps, no splits
     bool cluster;  // tensor-core kernel: splits merged through distributed shared memory
     int C, n_ct, n_splits, tiles_per_split;
-    size_t part_bytes, ticket_bytes;
+    size_t part_bytes, ticket_bytes;  // scratch; the counters that this plan uses
 };
 
+int fa_run(const b200_fattn_args *a, void *workspace, size_t front, size_t workspace_bytes, b200_stream_t stream);
 static int fa_sm_count() {
     static int sm = 0;
     if (!sm) {
@@ -573,6 +579,7 @@ static FaPlan fa_plan(const b200_fattn_args *a, bool chip = true) {
             // HBM-bound, a CTA streams a (K, V) tile in ~0.37 us (8 KB at 1/296 of 6.5 TB/s): 16 tiles ~ the 6 us saved
             if (bestc > 0 && costc - best_cost < 16) best = bestc;
         }
+        if (pairs > FA_PAIRS) best = 1;
         pl.n_splits = best;
         pl.cluster = best > 1 && best <= FM_MAX_CLUSTER && (best & (best - 1)) == 0 && !no_cluster;
         pl.tiles_per_split = (n_tiles + best - 1) / best;
@@ -620,7 +627,8 @@ static FaPlan fa_plan(const b200_fattn_args *a, bool chip = true) {
     // Splits that are one cluster merge for less than a microsecond instead of three: where there would be a few splits, as many as fit a cluster, down to one
     // tile a warp, unless more splits shorten the longest warp by more than a tile (8 heads on one kv-head of 128, 2048 cells: 9.2 us as a cluster of 8, 8.3 by tickets)
     static const bool no_cluster = getenv("B200_FA_NO_CLUSTER") != nullptr;
-    if (chip && !no_cluster && best <= 2 * FA_MAX_CLUSTER) {
+    if (pairs > FA_PAIRS) best = 1;
+    else if (chip && !no_cluster && best <= 2 * FA_MAX_CLUSTER) {
         int bestc = 0;
         int64_t costc = -1;
         for (int s = 2; s <= FA_MAX_CLUSTER; s *= 2) {
@@ -795,8 +803,13 @@ static int fa_check(const b200_fattn_args *a) {
 
 // bytes of the workspace that a launch may use where another stream's call uses the same memory: what prompts can do without is left out
 size_t fa_shared_bytes(const b200_fattn_args *a, size_t have) { return fa_check(a) == B200_OK && fa_plan(a).prefill ? 0 : have; }
-// bytes of split arrival counters at the front of the workspace (fattn_static.cu clears exactly these before a launch)
+// For a workspace whose counters are cleared before each launch (fattn_static.cu): bytes of the counters, with the scratch right behind them, and of both
 size_t fa_ticket_bytes(const b200_fattn_args *a) { return fa_check(a) == B200_OK ? fa_plan(a).ticket_bytes : 0; }
+size_t fa_cleared_bytes(const b200_fattn_args *a) {
+    if (fa_check(a) != B200_OK) return 0;
+    const FaPlan pl = fa_plan(a);
+    return pl.ticket_bytes + pl.part_bytes;
+}
 
 }  // namespace b200
 
@@ -813,23 +826,27 @@ extern "C" __attribute__((visibility("default"))) int b200_fattn_trace(unsigned 
 extern "C" size_t b200_flash_attn_workspace_bytes(const b200_fattn_args *a) {
     if (fa_check(a) != B200_OK) return 0;
     const FaPlan pl = fa_plan(a);
-    return pl.ticket_bytes + pl.part_bytes;
+    return pl.part_bytes ? FA_FRONT + pl.part_bytes : pl.ticket_bytes;
 }
 
-// The first ticket_bytes of the workspace are split-K arrival counters: they must be zero on entry and are left
-// zero on exit (the backend zeroes its workspace once, at allocation).
 extern "C" int b200_flash_attn_ext(const b200_fattn_args *a, void *workspace, size_t workspace_bytes, b200_stream_t stream) {
+    return b200::fa_run(a, workspace, FA_FRONT, workspace_bytes, stream);
+}
+
+// The counters at the front of the workspace must be zero on entry and are left zero on exit (the backend zeroes its workspace once, at allocation).
+// front: where the scratch begins
+int b200::fa_run(const b200_fattn_args *a, void *workspace, size_t front, size_t workspace_bytes, b200_stream_t stream) {
     int rc = fa_check(a);
     if (rc) return rc;
     FaPlan pl = fa_plan(a);
     // (short caches need neither workspace nor alignment: a call without them stays one CTA a pair)
-    if (pl.n_splits > 1 && (!workspace || workspace_bytes < pl.ticket_bytes + pl.part_bytes || ((((uintptr_t)workspace) | (uintptr_t)a->dst) & 15))) pl = fa_plan(a, false);
+    if (pl.n_splits > 1 && (!workspace || workspace_bytes < front + pl.part_bytes || ((((uintptr_t)workspace) | (uintptr_t)a->dst) & 15))) pl = fa_plan(a, false);
     if (pl.n_splits > 1 && ((((uintptr_t)workspace) | (uintptr_t)a->dst) & 15)) {
         set_error("b200_flash_attn_ext: dst and workspace must be 16-byte aligned");
         return B200_ERR_UNSUPPORTED;
     }
-    if (pl.n_splits > 1 && (!workspace || workspace_bytes < pl.ticket_bytes + pl.part_bytes)) {
-        set_error("b200_flash_attn_ext: workspace too small (%zu < %zu)", workspace_bytes, pl.ticket_bytes + pl.part_bytes);
+    if (pl.n_splits > 1 && (!workspace || workspace_bytes < front + pl.part_bytes)) {
+        set_error("b200_flash_attn_ext: workspace too small (%zu < %zu)", workspace_bytes, front + pl.part_bytes);
         return B200_ERR_INVALID;
     }
     FaParams p = {};
@@ -837,7 +854,7 @@ extern "C" int b200_flash_attn_ext(const b200_fattn_args *a, void *workspace, si
     p.mask = (const unsigned char *)a->mask;
     p.dst = a->dst;
     p.tickets = (int *)workspace;
-    p.part = workspace ? (float *)((unsigned char *)workspace + pl.ticket_bytes) : nullptr;
+    p.part = workspace ? (float *)((unsigned char *)workspace + front) : nullptr;
     p.D = (int)a->D; p.N = (int)a->N; p.n_head = (int)a->n_head; p.n_head_kv = (int)a->n_head_kv; p.n_kv = (int)a->n_kv;
     p.gqa = (int)(a->n_head / a->n_head_kv);
     p.n_cols = p.N * p.gqa;
@@ -861,8 +878,8 @@ extern "C" int b200_flash_attn_ext(const b200_fattn_args *a, void *workspace, si
     if (pl.prefill) {
         if (((uintptr_t)a->q | a->q_nb1 | a->q_nb2) & 7) { set_error("b200_flash_attn_ext: Q must be 8-byte aligned"); return B200_ERR_UNSUPPORTED; }
         if (ft_fits(a)) {
-            unsigned char *table = workspace ? (unsigned char *)workspace + pl.ticket_bytes : nullptr;
-            const size_t room = workspace && workspace_bytes > pl.ticket_bytes ? workspace_bytes - pl.ticket_bytes : 0;
+            unsigned char *table = workspace ? (unsigned char *)workspace + front : nullptr;
+            const size_t room = workspace && workspace_bytes > front ? workspace_bytes - front : 0;
             const int tc = a->D == 64 ? ft_launch<64>(a, p, table, room, st) : ft_launch<128>(a, p, table, room, st);
             if (tc != -1000) return tc;
         }

@@ -13,7 +13,9 @@
 
 namespace b200 {
 size_t fa_ticket_bytes(const b200_fattn_args *a);  // fattn.cu
+size_t fa_cleared_bytes(const b200_fattn_args *a);
 size_t fa_shared_bytes(const b200_fattn_args *a, size_t have);
+int fa_run(const b200_fattn_args *a, void *workspace, size_t front, size_t workspace_bytes, b200_stream_t stream);
 }
 using namespace b200;
 
@@ -52,7 +54,7 @@ extern "C" size_t b200_flash_attn_static_workspace_max(void) { return B200_FATTN
 
 extern "C" int b200_flash_attn_ext_static(const b200_fattn_args *a, b200_stream_t stream) {
     if (!a) { set_error("b200_flash_attn_ext_static: NULL arguments"); return B200_ERR_INVALID; }
-    const size_t need = b200_flash_attn_workspace_bytes(a);  // 0 for arguments b200_flash_attn_ext will refuse: it reports them
+    const size_t need = fa_cleared_bytes(a);  // 0 for arguments b200_flash_attn_ext will refuse: it reports them
     if (need > B200_FATTN_STATIC_WS_BYTES) {
         set_error("b200_flash_attn_ext_static: this shape needs %zu bytes of scratch, the static array holds %zu "
                   "(use b200_flash_attn_ext with a caller-owned workspace)", need, (size_t)B200_FATTN_STATIC_WS_BYTES);
@@ -65,5 +67,5 @@ extern "C" int b200_flash_attn_ext_static(const b200_fattn_args *a, b200_stream_
     // must start at zero (a finished launch leaves them zero, an aborted one may not): clear them in stream order.
     const size_t tickets = fa_ticket_bytes(a);
     if (need && tickets) B200_CUDA_TRY(cudaMemsetAsync(ws, 0, tickets, (cudaStream_t)stream));
-    return b200_flash_attn_ext(a, ws, fa_shared_bytes(a, B200_FATTN_STATIC_WS_BYTES), stream);
+    return fa_run(a, ws, tickets, fa_shared_bytes(a, B200_FATTN_STATIC_WS_BYTES), stream);
 }
