@@ -154,13 +154,33 @@ __device__ __forceinline__ void fence_proxy_async_smem() { asm volatile("fence.p
 // programmatic dependent launch: wait for the producer grid / allow the consumer grid to start
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+// p, for loads that have to stay behind the wait, barrier or fence in front of this line.  A memory clobber holds ordinary loads only: what a const __restrict__
+// pointer reads, __ldcg and asm without volatile may be moved across it, unless their address is made behind it.
+template <typename T>
+__device__ __forceinline__ T *behind(T *p) {
+    asm volatile("" : "+l"(p));
+    return p;
+}
+// What a kernel in front may have written, through a pointer from behind(): loads that a compiler may gather like __ldg's, but coherent ones (the contract of
+// ld.global.nc, memory that nobody writes while the kernel is there, does not hold for a kernel that is placed early).
+__device__ __forceinline__ int ld_behind(const int *p) { int v; asm("ld.global.b32 %0, [%1];" : "=r"(v) : "l"(p)); return v; }
+__device__ __forceinline__ unsigned short ld_behind(const unsigned short *p) { unsigned short v; asm("ld.global.b16 %0, [%1];" : "=h"(v) : "l"(p)); return v; }
+__device__ __forceinline__ uint4 ld_behind(const uint4 *p) {
+    uint4 v;
+    asm("ld.global.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ float4 ld_behind(const float4 *p) {
+    float4 v;
+    asm("ld.global.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p));
+    return v;
+}
 // First statement of a kernel that launch_chained() starts: nothing is read or written before the kernels in front of it are done, and no thread leaves
-// without having waited (a grid that ended early would let its own successor start too soon).  p: const __restrict__ pointers, whose loads a compiler may
-// otherwise move in front of the wait.
+// without having waited (a grid that ended early would let its own successor start too soon).  p: the kernel's const __restrict__ pointers (see behind()).
 template <typename... P>
 __device__ __forceinline__ void pdl_enter(P &...p) {
     pdl_wait();
-    (void)std::initializer_list<int>{((void)([](P &q) { asm volatile("" : "+l"(q)); }(p)), 0)...};
+    (void)std::initializer_list<int>{((void)(p = behind(p)), 0)...};
     pdl_trigger();
 }
 // Launch that keeps the stream's order but need not wait for the kernel in front to have left the device before its CTAs are placed: the kernel itself

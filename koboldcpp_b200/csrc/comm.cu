@@ -156,8 +156,7 @@ __global__ void __launch_bounds__(PW_THREADS) all_reduce_push_kernel(const PeerW
     const int b = blockIdx.x, t = threadIdx.x;
     const int i = (b * PW_THREADS + t) * 4;
     const bool active = i < n;            // n % 4 == 0 (checked by the host)
-    pdl_wait();                           // src, and the call counter of the previous exchange, are written by kernels in front of us
-    pdl_trigger();
+    pdl_enter(src, residual);             // src, and the call counter of the previous exchange, are written by kernels in front of us
     const unsigned epoch = w.ctr[b] + 1;  // the number of this call: identical on every rank (same graph, same order)
     const int slot = (int)(epoch & 1u);
     if (active) {

@@ -426,7 +426,7 @@ __global__ void __launch_bounds__(FA_NW * 32, 2) fattn_kernel(const __grid_const
     // The merging CTA is alone on the critical path: keep its loads independent and wide.  Phase 1 fetches the (m, l) pairs of
     // all splits in one round trip and turns them into normalised weights in shared memory; phase 2 streams the partial
     // accumulators with 16 independent 16-byte loads in flight per thread.
-    const float *all = p.part + (size_t)pair * p.n_splits * C * RS;
+    const float *all = behind(p.part) + (size_t)pair * p.n_splits * C * RS;
     float *wts = reinterpret_cast<float *>(smem);            // [C][FA_MAX_SPLITS]: exp(m_s - M) / L
     float *lss = wts + C * FA_MAX_SPLITS;                     // [C][FA_MAX_SPLITS]: l_s
     const int ns = p.n_splits;

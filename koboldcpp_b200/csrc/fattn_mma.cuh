@@ -353,6 +353,7 @@ __global__ void __launch_bounds__(FM_NW * 32, 2) fattn_mma_kernel(const __grid_c
 
     // ---- Q: this lane holds columns g and g + 8 (rows of the M side); columns >= ncol are zero.  The loads go out BEFORE the
     // first K/V tiles: behind 128 KB of cp.async per SM they came back 3.5 us later (profiles/r02_fattn_trace_timeline.log)
+    const unsigned char *q_at = behind(p.q);
     float2 qraw[2][KS][2];
     float slope[2];
     const unsigned char *mrow[2];
@@ -366,7 +367,7 @@ __global__ void __launch_bounds__(FM_NW * 32, 2) fattn_mma_kernel(const __grid_c
         if (p.max_bias > 0.0f)  // ALiBi, ggml.c:15743-15766
             slope[hh] = h < p.n_head_log2 ? powf(p.m0, (float)(h + 1)) : powf(p.m1, (float)(2 * (h - p.n_head_log2) + 1));
         mrow[hh] = p.mask != nullptr ? p.mask + (size_t)n * p.mask_nb1 : nullptr;
-        const float *qrow = reinterpret_cast<const float *>(p.q + (size_t)n * p.q_nb1 + (size_t)h * p.q_nb2);
+        const float *qrow = reinterpret_cast<const float *>(q_at + (size_t)n * p.q_nb1 + (size_t)h * p.q_nb2);
 #pragma unroll
         for (int s = 0; s < KS; s++) {
             qraw[hh][s][0] = qraw[hh][s][1] = make_float2(0.f, 0.f);
@@ -391,6 +392,7 @@ __global__ void __launch_bounds__(FM_NW * 32, 2) fattn_mma_kernel(const __grid_c
     unsigned long long skip = 0;
     if (p.N > 1 && p.mask != nullptr) {
         const bool al16 = (((uintptr_t)p.mask | p.mask_nb1) & 15) == 0;
+        const unsigned char *mask = behind(p.mask);
 #pragma unroll 1
         for (int pass = 0; pass < 2; pass++) {
             const int tt = t_first + t_step * (pass * 32 + lane);
@@ -399,9 +401,9 @@ __global__ void __launch_bounds__(FM_NW * 32, 2) fattn_mma_kernel(const __grid_c
                 masked = true;
                 const int key = tt * FM_TP;
                 for (int c = 0; c < ncol; c++) {
-                    const unsigned char *mr = p.mask + (size_t)((col0 + c) / p.gqa) * p.mask_nb1 + 2 * (size_t)key;
+                    const unsigned char *mr = mask + (size_t)((col0 + c) / p.gqa) * p.mask_nb1 + 2 * (size_t)key;
                     if (al16 && key + FM_TP <= p.n_kv) {
-                        const uint4 u0 = __ldg(reinterpret_cast<const uint4 *>(mr)), u1 = __ldg(reinterpret_cast<const uint4 *>(mr) + 1);
+                        const uint4 u0 = ld_behind(reinterpret_cast<const uint4 *>(mr)), u1 = ld_behind(reinterpret_cast<const uint4 *>(mr) + 1);
                         masked = masked && (u0.x & u0.y & u0.z & u0.w & u1.x & u1.y & u1.z & u1.w) == 0xfc00fc00u &&
                                  (u0.x | u0.y | u0.z | u0.w | u1.x | u1.y | u1.z | u1.w) == 0xfc00fc00u;
                     } else {
@@ -652,7 +654,7 @@ __global__ void __launch_bounds__(FM_NW * 32, 2) fattn_mma_kernel(const __grid_c
     FTRACE(6);
     if (!is_last) return;
     __threadfence();
-    const float *all = p.part + (size_t)pair * p.n_splits * C * RS;
+    const float *all = behind(p.part) + (size_t)pair * p.n_splits * C * RS;
     float *wts = reinterpret_cast<float *>(smem);            // [C][FA_MAX_SPLITS]: exp(m_s - M)
     float *lss = wts + FM_MAXC * FA_MAX_SPLITS;               // [C][FA_MAX_SPLITS]: l_s
     const int ns = p.n_splits;
@@ -721,7 +723,7 @@ __device__ __noinline__ unsigned mask_kind_any(const unsigned char *mask, size_t
         unsigned seen = 0;
 #pragma unroll 4
         for (int c = 0; c < ncol; c++) {
-            const unsigned h = key < n_kv ? __ldg(reinterpret_cast<const unsigned short *>(mask + (size_t)((col0 + c) / gqa) * nb1 + 2 * (size_t)key)) : 0xfc00u;
+            const unsigned h = key < n_kv ? ld_behind(reinterpret_cast<const unsigned short *>(mask + (size_t)((col0 + c) / gqa) * nb1 + 2 * (size_t)key)) : 0xfc00u;
             any |= h;
             seen |= h ^ 0xfc00u;
         }
@@ -757,13 +759,14 @@ __global__ void __launch_bounds__(FM_NW * 32, 2) fattn_mma_prefill_kernel(const 
     constexpr int CH = KT / 8, RP = 32 / CH;               // 16-byte pieces of a mask row in a tile; rows per pass
     const bool m16 = (((uintptr_t)p.mask | p.mask_nb1) & 15) == 0;
     enum { ZERO = 0, MIXED = 1, HIDDEN = 2 };
+    const unsigned char *mask = behind(p.mask);
     auto mask_load = [&](int t, uint4 (&u)[16 / RP]) {
         const int key = t * KT + (lane % CH) * 8;
 #pragma unroll
         for (int i = 0; i < 16 / RP; i++) {
             const int c = min(lane / CH + i * RP, ncol - 1);
             u[i] = make_uint4(0u, 0u, 0u, 0u);
-            if (key + 8 <= p.n_kv) u[i] = __ldg(reinterpret_cast<const uint4 *>(p.mask + (size_t)((col0 + c) / p.gqa) * p.mask_nb1 + 2 * (size_t)key));
+            if (key + 8 <= p.n_kv) u[i] = ld_behind(reinterpret_cast<const uint4 *>(mask + (size_t)((col0 + c) / p.gqa) * p.mask_nb1 + 2 * (size_t)key));
         }
     };
     // groups: bit i of a tile that is mixed: some column sees one of its keys 16 i .. 16 i + 15
@@ -786,7 +789,7 @@ __global__ void __launch_bounds__(FM_NW * 32, 2) fattn_mma_prefill_kernel(const 
     };
     auto fast = [&](int t) { return m16 && (t + 1) * KT <= p.n_kv; };
     auto mask_kind_slow = [&](int t, unsigned &groups) {
-        const unsigned r = mask_kind_any<KT>(p.mask, p.mask_nb1, col0, ncol, p.gqa, p.n_kv, t, lane);
+        const unsigned r = mask_kind_any<KT>(mask, p.mask_nb1, col0, ncol, p.gqa, p.n_kv, t, lane);
         groups = r >> 2;
         return (int)(r & 3u);
     };
@@ -835,6 +838,7 @@ __global__ void __launch_bounds__(FM_NW * 32, 2) fattn_mma_prefill_kernel(const 
     for (int st = 0; st < FP_NBUF - 1; st++) load_stage(st, st);
 
     // ---- Q fragments, mask rows, slopes of this warp's columns
+    const unsigned char *q_at = behind(p.q);
     unsigned qa[KS][4];
     float slope[2];
     const unsigned char *mrow[2];
@@ -847,7 +851,7 @@ __global__ void __launch_bounds__(FM_NW * 32, 2) fattn_mma_prefill_kernel(const 
         slope[hh] = 1.0f;
         if (p.max_bias > 0.0f) slope[hh] = h < p.n_head_log2 ? powf(p.m0, (float)(h + 1)) : powf(p.m1, (float)(2 * (h - p.n_head_log2) + 1));
         mrow[hh] = p.mask != nullptr ? p.mask + (size_t)n * p.mask_nb1 : nullptr;
-        const float *qrow = reinterpret_cast<const float *>(p.q + (size_t)n * p.q_nb1 + (size_t)h * p.q_nb2);
+        const float *qrow = reinterpret_cast<const float *>(q_at + (size_t)n * p.q_nb1 + (size_t)h * p.q_nb2);
 #pragma unroll
         for (int s = 0; s < KS; s++) {
             float2 lo = make_float2(0.f, 0.f), hi = make_float2(0.f, 0.f);

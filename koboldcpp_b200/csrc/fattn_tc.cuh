@@ -136,7 +136,7 @@ __device__ __forceinline__ void ft_scores(float (&v)[64], const FaParams &p, con
 #pragma unroll
     for (int i = 0; i < 8; i++) {  // (a mask's keys come in eights)
         mu[i] = make_uint4(0u, 0u, 0u, 0u);
-        if (masked && key0 + 8 * i + 8 <= p.n_kv) mu[i] = __ldg(reinterpret_cast<const uint4 *>(mrow + 2 * (size_t)(key0 + 8 * i)));
+        if (masked && key0 + 8 * i + 8 <= p.n_kv) mu[i] = ld_behind(reinterpret_cast<const uint4 *>(mrow + 2 * (size_t)(key0 + 8 * i)));
     }
 #pragma unroll
     for (int i = 0; i < 64; i++) v[i] *= scale;
@@ -275,10 +275,11 @@ __global__ void __launch_bounds__(FT_WARPS * 32, 1) fattn_tc_kernel(const __grid
     if (warp < FT_SOFTMAX) {
         // ===== Q as f16, swizzled; then every second tile, a thread a column
         const int w = warp >> 2, quarter = warp & 3, row = quarter * 32 + lane;
+        const unsigned char *q_at = behind(p.q);
 #pragma unroll
         for (int i = tid; i < FT_COLS * (D / 8); i += FT_SOFTMAX * 32) {
             const int r = i / (D / 8), c = i % (D / 8), qc = min(col0 + r, p.n_cols - 1), n = token(qc), h = hk * p.gqa + qc - n * p.gqa;  // (columns behind the last: not stored)
-            const float4 *src = reinterpret_cast<const float4 *>(p.q + (size_t)n * p.q_nb1 + (size_t)h * p.q_nb2) + 2 * c;
+            const float4 *src = reinterpret_cast<const float4 *>(q_at + (size_t)n * p.q_nb1 + (size_t)h * p.q_nb2) + 2 * c;
             const float4 a = __ldcg(src), b = __ldcg(src + 1);
             unsigned char *to = sq + r * 128 + ((c % 8) ^ (r & 7)) * 16;
             const uint4 u = make_uint4(pack_h2(a.x, a.y), pack_h2(a.z, a.w), pack_h2(b.x, b.y), pack_h2(b.z, b.w));
@@ -291,7 +292,7 @@ __global__ void __launch_bounds__(FT_WARPS * 32, 1) fattn_tc_kernel(const __grid
 
         const int col = min(col0 + row, p.n_cols - 1), tok = token(col);
         const float slope = ft_slope(p, hk * p.gqa + col - tok * p.gqa), scale = p.softcap != 0.0f ? p.scale / p.softcap : p.scale;
-        const unsigned char *mrow = p.mask != nullptr ? p.mask + (size_t)tok * p.mask_nb1 : nullptr;
+        const unsigned char *mrow = p.mask != nullptr ? behind(p.mask) + (size_t)tok * p.mask_nb1 : nullptr;
         const unsigned lanes = (unsigned)(quarter * 32) << 16, o_at = tmem_o + (unsigned)(w * D) + lanes;
         float m = -INFINITY, l = 0.f;  // what the exponent subtracts (times log2 e), the sum
         bool ok = true;
@@ -529,7 +530,7 @@ __global__ void __launch_bounds__(FT_WARPS * 32, 1) fattn_tc_kernel(const __grid
             }
         };
         if (table != nullptr) {  // a byte of every token's (ft_mask_kernel)
-            const unsigned char *mine = table + token(min(col0 + r0 + lane, p.n_cols - 1));
+            const unsigned char *mine = behind(table) + token(min(col0 + r0 + lane, p.n_cols - 1));
             const bool none = r1 < r0;
 #pragma unroll 1
             for (int t = 0; t < n_tiles; t += 4) {
@@ -544,13 +545,13 @@ __global__ void __launch_bounds__(FT_WARPS * 32, 1) fattn_tc_kernel(const __grid
             }
         } else {  // 8 lanes take a token's 64 keys
             const int n0 = token(min(col0 + r0, p.n_cols - 1)), n1 = r1 < r0 ? n0 : token(col0 + r1), fours = r1 < r0 ? 0 : (n1 - n0) / 4 + 1;
-            const unsigned char *at = p.mask + (size_t)(lane & 7) * 16;
+            const unsigned char *at = behind(p.mask) + (size_t)(lane & 7) * 16;
             for (int t = 0; t < n_tiles; t++) {
                 unsigned any = 0, inf = 0, all = 0xffffffffu;
                 if (t * FT_KEYS + (lane & 7) * 8 + 8 <= p.n_kv) {
 #pragma unroll 8
                     for (int i = 0; i < fours; i++) {
-                        const uint4 u = __ldg(reinterpret_cast<const uint4 *>(at + (size_t)min(n0 + 4 * i + (lane >> 3), n1) * p.mask_nb1 + (size_t)t * FT_KEYS * 2));
+                        const uint4 u = ld_behind(reinterpret_cast<const uint4 *>(at + (size_t)min(n0 + 4 * i + (lane >> 3), n1) * p.mask_nb1 + (size_t)t * FT_KEYS * 2));
                         const unsigned o = u.x | u.y | u.z | u.w;
                         any |= o;
                         inf |= o ^ 0xfc00fc00u;

@@ -183,7 +183,7 @@ __global__ void mmq_x_to_bf16_kernel(const float *__restrict__ x, int64_t x_stri
     out += (int64_t)blockIdx.z * n_pad * K;
     if (i4 * 4 >= K) return;
     float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (n < N) v = __ldg(reinterpret_cast<const float4 *>(x + n * x_stride) + i4);
+    if (n < N) v = ld_behind(reinterpret_cast<const float4 *>(x + n * x_stride) + i4);
     uint2 pk;
     pk.x = pack_bf16(v.x, v.y);
     pk.y = pack_bf16(v.z, v.w);
@@ -618,7 +618,7 @@ __global__ void mid_gather_bf16_kernel(const float *__restrict__ b, const int *_
     const int64_t i4 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     const int64_t n = blockIdx.y;
     if (i4 * 4 >= K) return;
-    const float4 v = __ldg(reinterpret_cast<const float4 *>(b + (int64_t)__ldg(row_src + n)) + i4);
+    const float4 v = ld_behind(reinterpret_cast<const float4 *>(b + (int64_t)ld_behind(row_src + n)) + i4);
     uint2 pk;
     pk.x = pack_bf16(v.x, v.y);
     pk.y = pack_bf16(v.z, v.w);

@@ -323,10 +323,10 @@ __device__ __forceinline__ PairTile pair_tile(const PairParams &p, int t, int nt
     r.kb0 = 0;
     r.nkb = (int)(p.q.K / MQ_BK);
     if constexpr (GROUPED) {
-        const int *te = p.q.tile_tab + 1 + 3 * ni;
-        r.product = __ldg(te);
-        r.n0 = __ldg(te + 1);
-        const int64_t end = __ldg(te + 2);
+        const int *te = behind(p.q.tile_tab) + 1 + 3 * ni;
+        r.product = ld_behind(te);
+        r.n0 = ld_behind(te + 1);
+        const int64_t end = ld_behind(te + 2);
         r.n_end = end < r.n0 + p.bn ? end : r.n0 + p.bn;
         r.n = ((int)(r.n_end - r.n0) + 31) / 32 * 32;
     } else {
@@ -565,6 +565,7 @@ __global__ void __launch_bounds__(pair_threads<TYPE>(), 1) mmq_pair_kernel(const
         unsigned ph = 0;
         const int quarter = warp & 3;
         const unsigned acc_remote = leader_addr(acc_empty0);
+        const int *row_dst = behind(p.q.row_dst);
         for (int t = pair; t < n_tiles; t += n_pairs) {
             const PairTile ti = pair_tile<GROUPED>(p, t, nt, UNIT);
             ok = ok && pair_wait<200>(acc_full0 + 8u * buf, ph, &failed, limit);
@@ -576,15 +577,22 @@ __global__ void __launch_bounds__(pair_threads<TYPE>(), 1) mmq_pair_kernel(const
 #pragma unroll 1
             for (int c0 = 0; c0 < cols; c0 += 32) {
                 float v[32];
+                // scatter: sorted row -> (token, slot).  A lane asks for one of the 32 columns' places: in front of each store a load would wait for its turn
+                const int place = GROUPED && c0 + lane < cols ? ld_behind(row_dst + ti.n0 + c0 + lane) : 0;
                 __syncwarp();
                 tmem_ld32(tmem_base + (unsigned)buf * 256u + ((unsigned)(quarter * 32) << 16) + (unsigned)c0, v);
-                if (row_ok) {
+                if constexpr (GROUPED) {
+#pragma unroll
+                    for (int j = 0; j < 32; j++) {
+                        const int to = __shfl_sync(0xffffffffu, place, j);
+                        if (row_ok && c0 + j < cols) drow[(int64_t)to] = v[j];
+                    }
+                } else if (row_ok) {
 #pragma unroll
                     for (int j = 0; j < 32; j++) {
                         if (c0 + j >= cols) continue;
                         const int64_t n = ti.n0 + c0 + j;
-                        if constexpr (GROUPED) drow[(int64_t)__ldg(p.q.row_dst + n)] = v[j];    // scatter: sorted row -> (token, slot)
-                        else if (p.q.ksplit > 1) atomicAdd(drow + n * p.q.dst_stride, v[j]);    // (result unused: RED.ADD.F32)
+                        if (p.q.ksplit > 1) atomicAdd(drow + n * p.q.dst_stride, v[j]);    // (result unused: RED.ADD.F32)
                         else drow[n * p.q.dst_stride] = v[j];
                     }
                 }

@@ -78,6 +78,7 @@ __device__ __forceinline__ void cta_sync() {
 template <int BAR = 0, int NT = MMVQ_THREADS>
 __device__ __forceinline__ float rms_scale(const float *__restrict__ xs, int64_t K, float norm_eps, float *red) {
     const int n4 = (int)(K / 4);
+    xs = behind(xs);
     float ss = 0.f;
     for (int i4 = threadIdx.x; i4 < n4; i4 += NT) {
         const float4 v = __ldcg(reinterpret_cast<const float4 *>(xs) + i4);
@@ -99,6 +100,8 @@ __device__ __forceinline__ void quantize_activation_row(unsigned char *p, const 
                                                         const float *__restrict__ norm_w, float nscale,
                                                         float *__restrict__ norm_out = nullptr, float *__restrict__ norm_mul_out = nullptr) {
     const int n4 = (int)(K / 4);
+    x = behind(x);
+    norm_w = behind(norm_w);
     int   *aq = (int *)p;
     float *ad = (float *)(p + (size_t)n_it * 4096);
     float *as = (float *)(p + (size_t)n_it * (4096 + 512));
@@ -112,7 +115,7 @@ __device__ __forceinline__ void quantize_activation_row(unsigned char *p, const 
             const int i4 = base + u * NT + threadIdx.x;
             v[u] = i4 < n4 ? __ldcg(reinterpret_cast<const float4 *>(x) + i4) : make_float4(0.f, 0.f, 0.f, 0.f);
             if (norm_w != nullptr && i4 < n4) {
-                const float4 ww = __ldg(reinterpret_cast<const float4 *>(norm_w) + i4);
+                const float4 ww = ld_behind(reinterpret_cast<const float4 *>(norm_w) + i4);
                 v[u].x = v[u].x * nscale; v[u].y = v[u].y * nscale; v[u].z = v[u].z * nscale; v[u].w = v[u].w * nscale;
                 if (norm_out) reinterpret_cast<float4 *>(norm_out)[i4] = v[u];
                 v[u].x = v[u].x * ww.x; v[u].y = v[u].y * ww.y; v[u].z = v[u].z * ww.z; v[u].w = v[u].w * ww.w;
@@ -180,6 +183,8 @@ __device__ __forceinline__ void act_issue(ActRegsT<RR> &r, const float *__restri
     static_assert(RR % 2 == 0, "a thread owns pairs of float4");
     constexpr int NT = MMVQ_THREADS;
     const int n4 = (int)(K / 4);  // K is a multiple of 32
+    x = behind(x);
+    norm_w = behind(norm_w);
 #pragma unroll
     for (int u = 0; u < RR / 2; u++) {
         const int i4 = 2 * (u * NT + threadIdx.x);
@@ -195,8 +200,8 @@ __device__ __forceinline__ void act_issue(ActRegsT<RR> &r, const float *__restri
         for (int u = 0; u < RR / 2; u++) {
             const int i4 = 2 * (u * NT + threadIdx.x);
             if (2 * u * NT < n4) {
-                r.w[2 * u]     = i4 < n4 ? __ldg(reinterpret_cast<const float4 *>(norm_w) + i4) : make_float4(0.f, 0.f, 0.f, 0.f);
-                r.w[2 * u + 1] = i4 < n4 ? __ldg(reinterpret_cast<const float4 *>(norm_w) + i4 + 1) : make_float4(0.f, 0.f, 0.f, 0.f);
+                r.w[2 * u]     = i4 < n4 ? ld_behind(reinterpret_cast<const float4 *>(norm_w) + i4) : make_float4(0.f, 0.f, 0.f, 0.f);
+                r.w[2 * u + 1] = i4 < n4 ? ld_behind(reinterpret_cast<const float4 *>(norm_w) + i4 + 1) : make_float4(0.f, 0.f, 0.f, 0.f);
             }
         }
     }

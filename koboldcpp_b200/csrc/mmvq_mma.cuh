@@ -208,7 +208,7 @@ __global__ void __launch_bounds__(MV_NW * 32, 1) mmvq_mma_kernel(const __grid_co
 
     // ---- the columns as q8_1, once per CTA: word w (4 values) of a block lies at 2 (w & 3) + (w >> 2), so that a lane's two words are neighbours
     {
-        const float *X = p.m.jobs[0].X;
+        const float *X = behind(p.m.jobs[0].X), *norm_w = behind(p.m.norm_w);
         const int n8 = (int)(p.m.K / 8), items = N * n8;  // 8 values each; 4 neighbouring lanes hold a block (n8 is a multiple of 32)
         __shared__ float nscale[8];
         if (p.m.norm_w != nullptr) {
@@ -237,7 +237,7 @@ __global__ void __launch_bounds__(MV_NW * 32, 1) mmvq_mma_kernel(const __grid_co
                     const float s = nscale[n];
 #pragma unroll
                     for (int h = 0; h < 2; h++) {
-                        const float4 w = __ldg(reinterpret_cast<const float4 *>(p.m.norm_w) + 2 * i8 + h);
+                        const float4 w = ld_behind(reinterpret_cast<const float4 *>(norm_w) + 2 * i8 + h);
                         float4 &x = v[u][h];
                         x.x = x.x * s; x.y = x.y * s; x.z = x.z * s; x.w = x.w * s;
                         if (keep && p.m.norm_out) reinterpret_cast<float4 *>(p.m.norm_out + (int64_t)n * p.m.K)[2 * i8 + h] = x;

@@ -122,7 +122,7 @@ __global__ void rms_norm_row_kernel(TD x, const float4 *__restrict__ w, TD dst, 
 #pragma unroll
     for (int k = 0; k < NV; k++) {
         const int i = threadIdx.x + k * blockDim.x;
-        ww[k] = w && i < n4 ? __ldg(w + i) : make_float4(1.f, 1.f, 1.f, 1.f);
+        ww[k] = w && i < n4 ? ld_behind(w + i) : make_float4(1.f, 1.f, 1.f, 1.f);
     }
     float s = 0.f;
 #pragma unroll
@@ -286,7 +286,7 @@ __global__ void rope_kernel(TD x, const int32_t *__restrict__ pos, const float *
 }
 
 __global__ void rope_kv_store_kernel(RopeKvDev a, const int32_t *__restrict__ pos, const float *__restrict__ ff, RopeDev rp) {
-    pdl_enter();
+    pdl_enter(pos, ff);
     rope_kv_store_item(a, pos, ff, rp, (int64_t)blockIdx.x * blockDim.x + threadIdx.x);
 }
 
@@ -567,7 +567,7 @@ __global__ void __launch_bounds__(ROUTER_WARPS * 32) moe_router_kernel(const flo
                                                                        int64_t ld_probs, int32_t *__restrict__ ids, int64_t ld_ids, float *__restrict__ w_gather,
                                                                        float *__restrict__ wsum, float *__restrict__ w_out, int n_expert, int n_used,
                                                                        int64_t n_tok) {
-    pdl_enter();
+    pdl_enter(logits);
     const int lane = threadIdx.x & 31;
     const int64_t tok = (int64_t)blockIdx.x * ROUTER_WARPS + (threadIdx.x >> 5);
     if (tok >= n_tok) return;
@@ -716,7 +716,7 @@ __global__ void __launch_bounds__(128) mul_mat_f32_block_kernel(const float *__r
 // blockIdx.y walks a batch of independent products (the per-head matrices of an attention layer).
 __device__ __forceinline__ uint4 ld_stream16(const uint4 *p) {
     uint4 v;
-    asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+    asm volatile("ld.global.L1::no_allocate.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
     return v;
 }
 template <int NC, int RPW>

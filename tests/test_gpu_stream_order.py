@@ -3,7 +3,7 @@ import ctypes as C
 
 import pytest
 
-from koboldcpp_b200.lib import F32, Q4_0, Q4_K, Q6_K, Tensor, check, lib
+from koboldcpp_b200.lib import F16, F32, Q4_0, Q4_K, Q6_K, FattnArgs, RopeParams, Tensor, check, lib
 
 pytestmark = pytest.mark.gpu
 torch = pytest.importorskip("torch")
@@ -46,6 +46,55 @@ def test_a_product_reads_what_the_launch_in_front_wrote(kind, k, rows, n):
         step(i, torch.cuda.synchronize)
     want = dst.clone()
     assert (want.abs().sum((1, 2)) > 0).all()
+    for _ in range(5):
+        dst.zero_()
+        for i in range(6):
+            step(i, lambda: None)
+        torch.cuda.synchronize()
+        assert torch.equal(dst, want)
+
+
+@pytest.mark.parametrize("D,n", [(64, 64), (96, 64), (128, 4), (64, 1)])
+def test_a_row_of_launches_that_read_one_another(D, n):
+    """Gate -> router logits -> expert ids as positions -> rotation and cache store -> the stored rows as the mask of an attention: prompts on both kernels,
+    a few tokens, one token.  Each launch's input changes from step to step and is written by the launch in front."""
+    heads, experts = 8, 256
+    n_kv = D * heads
+    g = torch.Generator(device="cuda").manual_seed(D + n)
+    rand = lambda *s: torch.randn(*s, generator=g, device="cuda")
+    gates, qs, masks = [rand(n, experts) * 4 for _ in range(6)], [rand(n, heads, D) for _ in range(6)], []
+    for i in range(6):
+        m = torch.where(torch.rand(n, n_kv, generator=g, device="cuda") < 0.5, 0.0, -torch.inf)
+        m[:, 100 * i // 2:][:, :5] = 0
+        masks.append(m)
+    up, gate, logits, q, qo, k, ko = torch.ones(n, experts, device="cuda"), rand(n, experts), rand(n, experts), rand(n, heads, D), rand(n, heads, D), rand(n, heads, D), rand(n, heads, D)
+    probs, ids, w3 = torch.zeros(n, experts, device="cuda"), torch.zeros(n, dtype=torch.int32, device="cuda"), [torch.zeros(n, device="cuda") for _ in range(3)]
+    rows, krows, v = torch.zeros(32 * ((n + 31) // 32), n_kv, dtype=torch.float16, device="cuda"), torch.zeros(n, n_kv, dtype=torch.float16, device="cuda"), torch.zeros(n, n_kv, device="cuda")
+    kc, vc = rand(heads, n_kv, D).half(), rand(heads, n_kv, D).half()
+    dst = torch.zeros(6, n, heads, D, device="cuda")
+    rp = RopeParams(D, 0, 4096, 10000.0, 1.0, 0.0, 1.0, 32.0, 1.0)
+    t = lambda x, *s: C.byref(Tensor.contiguous(x.data_ptr(), F32, s))
+
+    def step(i, wait):
+        gate.copy_(gates[i])
+        q.copy_(qs[i])
+        v.copy_(masks[i])
+        for call in (lambda: lib().b200_op_silu_mul(gate.data_ptr(), up.data_ptr(), None, logits.data_ptr(), n * experts, None),
+                     lambda: lib().b200_op_moe_router(logits.data_ptr(), experts, probs.data_ptr(), experts, ids.data_ptr(), 1, w3[0].data_ptr(), w3[1].data_ptr(), w3[2].data_ptr(), experts, 1, n, None),
+                     lambda: lib().b200_op_rope_kv_store(t(q, D, heads, n), t(qo, D, heads, n), t(k, D, heads, n), t(ko, D, heads, n), t(v, n_kv, n), ids.data_ptr(), None, C.byref(rp), F16,
+                                                         krows.data_ptr(), rows.data_ptr(), None, None, None),
+                     lambda: lib().b200_flash_attn_ext(C.byref(args[i]), ws.data_ptr(), ws.numel(), None)):
+            wait()
+            check(call())
+
+    args = [FattnArgs(qo.data_ptr(), kc.data_ptr(), vc.data_ptr(), rows.data_ptr(), dst[i].data_ptr(), D, n, heads, heads, n_kv, F16, F16, 4 * D * heads, 4 * D, 2 * D, 2 * D * n_kv, 2 * D,
+                      2 * D * n_kv, 2 * n_kv, D ** -0.5, 0.0, 0.0) for i in range(6)]
+    ws = torch.zeros(max(int(lib().b200_flash_attn_workspace_bytes(C.byref(args[0]))), 256), dtype=torch.uint8, device="cuda")
+    for i in range(6):
+        step(i, torch.cuda.synchronize)
+    torch.cuda.synchronize()
+    want = dst.clone()
+    assert torch.isfinite(want).all() and all((want[i] != want[i - 1]).any() for i in range(6))
     for _ in range(5):
         dst.zero_()
         for i in range(6):
