@@ -248,6 +248,9 @@ typedef struct {
  * prompt batch (f16 cache, D 64 or 128) is optional: it lets the mask be read once instead of once a kv-head. */
 B200_API size_t b200_flash_attn_workspace_bytes(const b200_fattn_args *a);
 B200_API int b200_flash_attn_ext(const b200_fattn_args *a, void *workspace, size_t workspace_bytes, b200_stream_t stream);
+/* The same with the limit of each of the kernel's own waits in clock cycles (b200_flash_attn_ext: about two seconds' worth), where a prompt runs on tcgen05 (f16 cache, D 64
+ * or 128).  When one runs out the call ends early: rows of dst that were stored are right, the others are as they were, and b200_gemm_status() becomes 1. */
+B200_API int b200_flash_attn_ext_wait(const b200_fattn_args *a, void *workspace, size_t workspace_bytes, int64_t wait_cycles, b200_stream_t stream);
 
 /* b200_flash_attn_ext without a caller-owned workspace and without any allocation (no cudaMalloc / cudaFree, directly or
  * through a library): for callers under CUDA graph capture, serving loops and harnesses that forbid allocating.

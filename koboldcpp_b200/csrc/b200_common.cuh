@@ -151,6 +151,7 @@ __device__ __forceinline__ void bulk_g2s(void *dst, const void *src, unsigned by
 // order prior generic-proxy accesses to shared memory before subsequent async-proxy (bulk copy) writes
 __device__ __forceinline__ void fence_proxy_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 
+constexpr long long PAIR_WAIT_LIMIT = 4000000000LL;  // clock cycles that the waits of kernels on tcgen05 take at most: about two seconds
 // programmatic dependent launch: wait for the producer grid / allow the consumer grid to start
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }

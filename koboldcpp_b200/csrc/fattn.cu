@@ -493,7 +493,7 @@ struct FaPlan {
     size_t part_bytes, ticket_bytes;  // scratch; the counters that this plan uses
 };
 
-int fa_run(const b200_fattn_args *a, void *workspace, size_t front, size_t workspace_bytes, b200_stream_t stream);
+int fa_run(const b200_fattn_args *a, void *workspace, size_t front, size_t workspace_bytes, int64_t wait_cycles, b200_stream_t stream);
 static int fa_sm_count() {
     static int sm = 0;
     if (!sm) {
@@ -830,12 +830,17 @@ extern "C" size_t b200_flash_attn_workspace_bytes(const b200_fattn_args *a) {
 }
 
 extern "C" int b200_flash_attn_ext(const b200_fattn_args *a, void *workspace, size_t workspace_bytes, b200_stream_t stream) {
-    return b200::fa_run(a, workspace, FA_FRONT, workspace_bytes, stream);
+    return b200_flash_attn_ext_wait(a, workspace, workspace_bytes, PAIR_WAIT_LIMIT, stream);
+}
+
+extern "C" int b200_flash_attn_ext_wait(const b200_fattn_args *a, void *workspace, size_t workspace_bytes, int64_t wait_cycles, b200_stream_t stream) {
+    if (wait_cycles < 0) { set_error("b200_flash_attn_ext_wait: limit below zero"); return B200_ERR_INVALID; }
+    return b200::fa_run(a, workspace, FA_FRONT, workspace_bytes, wait_cycles, stream);
 }
 
 // The counters at the front of the workspace must be zero on entry and are left zero on exit (the backend zeroes its workspace once, at allocation).
 // front: where the scratch begins
-int b200::fa_run(const b200_fattn_args *a, void *workspace, size_t front, size_t workspace_bytes, b200_stream_t stream) {
+int b200::fa_run(const b200_fattn_args *a, void *workspace, size_t front, size_t workspace_bytes, int64_t wait_cycles, b200_stream_t stream) {
     int rc = fa_check(a);
     if (rc) return rc;
     FaPlan pl = fa_plan(a);
@@ -880,7 +885,7 @@ int b200::fa_run(const b200_fattn_args *a, void *workspace, size_t front, size_t
         if (ft_fits(a)) {
             unsigned char *table = workspace ? (unsigned char *)workspace + front : nullptr;
             const size_t room = workspace && workspace_bytes > front ? workspace_bytes - front : 0;
-            const int tc = a->D == 64 ? ft_launch<64>(a, p, table, room, st) : ft_launch<128>(a, p, table, room, st);
+            const int tc = a->D == 64 ? ft_launch<64>(a, p, table, room, wait_cycles, st) : ft_launch<128>(a, p, table, room, wait_cycles, st);
             if (tc != -1000) return tc;
         }
         switch (a->D) {

@@ -15,7 +15,7 @@ namespace b200 {
 size_t fa_ticket_bytes(const b200_fattn_args *a);  // fattn.cu
 size_t fa_cleared_bytes(const b200_fattn_args *a);
 size_t fa_shared_bytes(const b200_fattn_args *a, size_t have);
-int fa_run(const b200_fattn_args *a, void *workspace, size_t front, size_t workspace_bytes, b200_stream_t stream);
+int fa_run(const b200_fattn_args *a, void *workspace, size_t front, size_t workspace_bytes, int64_t wait_cycles, b200_stream_t stream);
 }
 using namespace b200;
 
@@ -67,5 +67,5 @@ extern "C" int b200_flash_attn_ext_static(const b200_fattn_args *a, b200_stream_
     // must start at zero (a finished launch leaves them zero, an aborted one may not): clear them in stream order.
     const size_t tickets = fa_ticket_bytes(a);
     if (need && tickets) B200_CUDA_TRY(cudaMemsetAsync(ws, 0, tickets, (cudaStream_t)stream));
-    return fa_run(a, ws, tickets, fa_shared_bytes(a, B200_FATTN_STATIC_WS_BYTES), stream);
+    return fa_run(a, ws, tickets, fa_shared_bytes(a, B200_FATTN_STATIC_WS_BYTES), PAIR_WAIT_LIMIT, stream);
 }

@@ -20,7 +20,8 @@
 // cycle and SM), and start and end of a CTA.  32 heads of 128, 512 tokens behind 1536: 82 us with mma.sync (fattn_mma_prefill_kernel, which keeps the
 // other head sizes and masks at odd places); 41.5 with tiles of 128 keys and one S a group (a group then waits for its own products: 4700 cycles for two
 // tiles), 38 with tiles of 64, 34.3 with the mask read once (ft_mask_kernel).
-// Waits have a limit, as in the prompt GEMM: a role that gives up sets `failed`, the others follow, and the status word is set.
+// Waits have a limit, as in the prompt GEMM: a role that gives up sets `failed`, the others follow, and the status word is set.  Rows are stored only where no softmax
+// warp had given up when the sums met.
 #pragma once
 #include "tcgen05.cuh"
 
@@ -235,7 +236,7 @@ __device__ __forceinline__ bool ft_wait_last(const volatile int *act, unsigned l
 
 template <int D>
 __global__ void __launch_bounds__(FT_WARPS * 32, 1) fattn_tc_kernel(const __grid_constant__ TmapBytes tmK, const __grid_constant__ TmapBytes tmV, const __grid_constant__ FaParams p, unsigned gqa_div,
-                                                                  const unsigned char *table, int *timeout) {
+                                                                  const unsigned char *table, long long limit, int *timeout) {
     constexpr int TILE = ft_tile_bytes<D>();
     constexpr float LOG2E = 1.4426950408889634f;
     enum { ZERO = 0, MIXED = 1, HIDDEN = 2 };
@@ -252,7 +253,6 @@ __global__ void __launch_bounds__(FT_WARPS * 32, 1) fattn_tc_kernel(const __grid
     unsigned char *sq = smem, *sk = sq + (D / 64 + 1) * FT_Q_PANEL, *sv = sk + FT_NB * TILE;
     volatile unsigned char *kinds = sv + FT_NB * TILE;                                         // [tile][32 columns]: kind | groups of 16 keys << 2
     volatile int *act = reinterpret_cast<int *>(sv + FT_NB * TILE + (size_t)n_tiles * 4);       // the tiles that are worked on: tile << 4 | groups of any column; then -1 -1, and -2 as long as that is not known
-    const long long limit = PAIR_WAIT_LIMIT;
 
     if (tid == 0) {
         for (int i = 0; i < FT_NB; i++) { mbar_init(&k_full[i], 1); mbar_init(&v_full[i], 1); mbar_init(&s_full[i], 1); mbar_init(&p_full[i], 4); mbar_init(&o_done[i], 1); }
@@ -358,6 +358,7 @@ __global__ void __launch_bounds__(FT_WARPS * 32, 1) fattn_tc_kernel(const __grid
         ok = ok && __all_sync(0xffffffffu, ft_wait_last(act, o_done, count, &failed, limit));
         tc_fence_after();
         asm volatile("bar.sync 3, %0;" ::"n"(FT_SOFTMAX * 32) : "memory");
+        ok = __all_sync(0xffffffffu, ok && !failed);  // (whoever of the eight warps gave up had set it by now; a role that gives up later takes rows with it that were right)
         constexpr int OROW = D + 4;
         float *so = reinterpret_cast<float *>(sk);
         static_assert(FT_COLS * OROW * 4 <= 2 * FT_NB * TILE, "results lie where K and V were");
@@ -390,6 +391,7 @@ __global__ void __launch_bounds__(FT_WARPS * 32, 1) fattn_tc_kernel(const __grid
         }
         tc_fence_before();
         asm volatile("bar.sync 3, %0;" ::"n"(FT_SOFTMAX * 32) : "memory");
+        ok = __all_sync(0xffffffffu, ok && !failed);  // (all of a row has been put down, or nothing of it is stored)
         if (ok) {
 #pragma unroll 4
             for (int i = tid; i < ncol * (D / 4); i += FT_SOFTMAX * 32) {
@@ -610,7 +612,7 @@ constexpr size_t FT_TABLE_BYTES = 512 * 1024;
 static size_t ft_table_bytes(const b200_fattn_args *a) { return (size_t)a->N * (size_t)((a->n_kv + FT_KEYS - 1) / FT_KEYS); }
 // -1000: the other kernel's
 template <int D>
-static int ft_launch(const b200_fattn_args *a, const FaParams &p, unsigned char *ws, size_t ws_bytes, cudaStream_t st) {
+static int ft_launch(const b200_fattn_args *a, const FaParams &p, unsigned char *ws, size_t ws_bytes, long long limit, cudaStream_t st) {
     TmapBytes tk, tv;
     if (!ft_encode(tk, a->k, D, a->n_kv, a->n_head_kv, a->k_nb1, a->k_nb2) || !ft_encode(tv, a->v, D, a->n_kv, a->n_head_kv, a->v_nb1, a->v_nb2)) return -1000;
     int *status = nullptr;
@@ -631,7 +633,7 @@ static int ft_launch(const b200_fattn_args *a, const FaParams &p, unsigned char 
         B200_CUDA_TRY(launch_chained(ft_mask_kernel, dim3((unsigned)((p.N + 7) / 8), (unsigned)((n_tiles + FT_MASK_TILES - 1) / FT_MASK_TILES)), 256, 0, st, p.mask, p.mask_nb1, p.N, p.n_kv, n_tiles, table));
     }
     const dim3 grid((unsigned)((p.n_cols + FT_COLS - 1) / FT_COLS), (unsigned)p.n_head_kv);
-    B200_CUDA_TRY(launch_chained(fattn_tc_kernel<D>, grid, FT_WARPS * 32, ft_smem<D>(n_tiles), st, tk, tv, p, div, (const unsigned char *)table, status));
+    B200_CUDA_TRY(launch_chained(fattn_tc_kernel<D>, grid, FT_WARPS * 32, ft_smem<D>(n_tiles), st, tk, tv, p, div, (const unsigned char *)table, limit, status));
     return B200_OK;
 }
 

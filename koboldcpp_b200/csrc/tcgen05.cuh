@@ -74,7 +74,6 @@ __device__ __forceinline__ void tma_load_2d(void *dst, const void *tmap, int c0,
 
 struct alignas(64) TmapBytes { unsigned char b[128]; };  // CUtensorMap without pulling <cuda.h> into device code
 
-constexpr long long PAIR_WAIT_LIMIT = 4000000000LL;  // clock cycles: about two seconds
 __device__ __forceinline__ bool elect_lane() {
     unsigned e;
     asm volatile("{\n.reg .pred p;\nelect.sync _|p, 0xffffffff;\nselp.u32 %0, 1, 0, p;\n}\n" : "=r"(e));

@@ -201,6 +201,7 @@ _SIGS = {
                                             C.c_int64, C.c_int32, C.c_void_p, C.c_size_t, C.c_void_p]),
     "b200_flash_attn_workspace_bytes": (C.c_size_t, [C.POINTER(FattnArgs)]),
     "b200_flash_attn_ext": (C.c_int, [C.POINTER(FattnArgs), C.c_void_p, C.c_size_t, C.c_void_p]),
+    "b200_flash_attn_ext_wait": (C.c_int, [C.POINTER(FattnArgs), C.c_void_p, C.c_size_t, C.c_int64, C.c_void_p]),
     "b200_flash_attn_static_workspace_max": (C.c_size_t, []),
     "b200_flash_attn_ext_static": (C.c_int, [C.POINTER(FattnArgs), C.c_void_p]),
 }
