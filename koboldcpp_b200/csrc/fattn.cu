@@ -124,10 +124,9 @@ __device__ __forceinline__ void cluster_sync_all() {
 __device__ __forceinline__ float ld_cluster_f32(const float *local, unsigned rank) {
     unsigned ra;
     float v;
-    // (not volatile, no memory clobber: the loads of a merge are independent and must overlap -- ordering comes from the
-    // cluster barriers around them)
     asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(ra) : "r"(smem_u32(local)), "r"(rank));
-    asm("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(ra));
+    // (volatile: stays between the cluster barriers around it; no memory clobber: nothing else has to wait for it, and the loads of a merge overlap all the same)
+    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(ra));
     return v;
 }
 

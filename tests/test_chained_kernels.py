@@ -34,3 +34,13 @@ def test_no_load_of_constant_memory():
     for name in HELPERS:
         text = re.sub(r"//.*", "", (CSRC / name).read_text())
         assert "__ldg(" not in text and "ld.global.nc" not in text, name
+
+
+def test_loads_from_a_peers_shared_memory_stay_between_the_cluster_barriers():
+    """A compiler may move an asm without volatile across a barrier, whose clobber holds ordinary loads and volatile ones."""
+    found = 0
+    for path in sorted(CSRC.glob("*.cu*")):
+        for keyword in re.findall(r"(asm(?: volatile)?)\s*\(\s*\"ld\.shared::cluster", path.read_text()):
+            found += 1
+            assert keyword == "asm volatile", path.name
+    assert found
