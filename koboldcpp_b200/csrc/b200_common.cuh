@@ -151,6 +151,19 @@ __device__ __forceinline__ void bulk_g2s(void *dst, const void *src, unsigned by
 // order prior generic-proxy accesses to shared memory before subsequent async-proxy (bulk copy) writes
 __device__ __forceinline__ void fence_proxy_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 
+// SMs of the device, for plans of launches; without a device (sizes of workspaces can be asked for there too) those of a B200
+static inline int sm_count() {
+    static int sm = 0;
+    if (!sm) {
+        int dev = 0, n = 0;
+        if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) {
+            cudaGetLastError();
+            n = 148;
+        }
+        sm = n;
+    }
+    return sm;
+}
 constexpr long long PAIR_WAIT_LIMIT = 4000000000LL;  // clock cycles that the waits of kernels on tcgen05 take at most: about two seconds
 // programmatic dependent launch: wait for the producer grid / allow the consumer grid to start
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }

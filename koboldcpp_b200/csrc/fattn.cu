@@ -493,18 +493,6 @@ struct FaPlan {
 };
 
 int fa_run(const b200_fattn_args *a, void *workspace, size_t front, size_t workspace_bytes, int64_t wait_cycles, b200_stream_t stream);
-static int fa_sm_count() {
-    static int sm = 0;
-    if (!sm) {
-        int dev = 0;
-        if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) {
-            cudaGetLastError();
-            sm = 148;
-        }
-    }
-    return sm;
-}
-
 static bool fa_use_mma(const b200_fattn_args *a) {
     static const bool off = getenv("B200_FA_NO_MMA") != nullptr;  // developer switch: the scalar kernel
     if (a->D != 64 && a->D != 128) return true;  // head sizes 80 / 96 / 112 / 256 exist on the tensor-core kernels only
@@ -548,7 +536,7 @@ static FaPlan fa_plan(const b200_fattn_args *a, bool chip = true) {
         pl.n_ct = (int)((n_cols + pl.C - 1) / pl.C);
         const int n_tiles = (int)((a->n_kv + FM_TP - 1) / FM_TP);
         const int64_t pairs = (int64_t)pl.n_ct * a->n_head_kv;
-        const int slots = 2 * fa_sm_count();
+        const int slots = 2 * sm_count();
         int best = 1;
         int64_t best_cost = -1;
         for (int s = 1; s <= FA_MAX_SPLITS; s++) {
@@ -598,7 +586,7 @@ static FaPlan fa_plan(const b200_fattn_args *a, bool chip = true) {
     // tiles-per-warp bound.
     {
         const int n_tiles0 = (int)((a->n_kv + FA_TP - 1) / FA_TP);
-        const int slots0 = 2 * fa_sm_count();
+        const int slots0 = 2 * sm_count();
         while (pl.C > 1 && n_tiles0 <= 4 * FA_MAX_SPLITS * FA_NW &&
                ((n_cols + pl.C - 1) / pl.C) * a->n_head_kv * FA_MAX_SPLITS < slots0) pl.C /= 2;
     }
@@ -609,7 +597,7 @@ static FaPlan fa_plan(const b200_fattn_args *a, bool chip = true) {
     pl.n_ct = (int)((n_cols + pl.C - 1) / pl.C);
     const int n_tiles = (int)((a->n_kv + FA_TP - 1) / FA_TP);
     const int64_t pairs = (int64_t)pl.n_ct * a->n_head_kv;
-    const int slots = 2 * fa_sm_count();
+    const int slots = 2 * sm_count();
     // choose the split count that minimises (waves x tiles per split), i.e. the length of the critical path;
     // every warp should still see >= 2 tiles; ties go to fewer splits (less merge traffic)
     int best = 1;

@@ -276,8 +276,8 @@ static int sink_attn_splits(const b200_sink_attn_args *a) {
     const int64_t pairs = (int64_t)a->n_tokens * a->n_head;
     // a batch of several sequences fills the device by itself, and its stretches would be unequal; below a few thousand cells a
     // pair's CTA is bound by its fixed costs, not by the cells, and the merge would only add a launch
-    if (pairs * 2 > 148 || a->n_kv < 2048) return 1;
-    int s = (int)((2 * 148 + pairs - 1) / pairs);
+    if (pairs * 2 > sm_count() || a->n_kv < 2048) return 1;
+    int s = (int)((2 * sm_count() + pairs - 1) / pairs);
     const int most = a->n_kv / 128;  // at least 128 cells per stretch
     if (s > most) s = most;
     if (s > 64) s = 64;
@@ -293,7 +293,7 @@ static int launch_sink_attn3(const b200_sink_attn_args *a, float *part, int n_sp
 }
 template <int ND, int NV>
 static int launch_sink_attn2(const b200_sink_attn_args *a, float *part, int n_split, cudaStream_t st) {
-    if ((int64_t)a->n_tokens * a->n_head < 2 * 148 && a->n_kv > 64) return launch_sink_attn3<ND, NV, 16>(a, part, n_split, st);
+    if ((int64_t)a->n_tokens * a->n_head < 2 * sm_count() && a->n_kv > 64) return launch_sink_attn3<ND, NV, 16>(a, part, n_split, st);
     return launch_sink_attn3<ND, NV, 4>(a, part, 1, st);
 }
 template <int ND>

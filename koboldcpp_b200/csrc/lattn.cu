@@ -502,7 +502,7 @@ static int launch_latent_attn3(const b200_latent_attn_args *a, cudaStream_t st) 
 template <int NL, int NR>
 static int launch_latent_attn2(const b200_latent_attn_args *a, cudaStream_t st) {
     // few (token, head) pairs: 16 warps share the cells of a pair
-    if ((int64_t)a->n_tokens * a->n_head < 2 * 148 && a->n_kv > 64) return launch_latent_attn3<NL, NR, 16>(a, st);
+    if ((int64_t)a->n_tokens * a->n_head < 2 * sm_count() && a->n_kv > 64) return launch_latent_attn3<NL, NR, 16>(a, st);
     // prompt batches: heads of a token share the staged rows (16-byte copies: rows and the cache base must allow them)
     if (a->n_head >= 2 && (a->kv_rank + a->rot_dim) % 4 == 0 && a->cache_stride % 4 == 0 && ((uintptr_t)a->cache & 15) == 0 &&
         (size_t)LT_CELLS * (a->kv_rank + a->rot_dim) * 4 <= 160 * 1024)

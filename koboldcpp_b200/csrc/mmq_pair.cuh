@@ -649,15 +649,7 @@ static inline PairPlan mmq_pair_plan(int64_t M, int64_t N, int64_t K, int n_batc
 }
 
 // pairs of CTAs that the device can hold at once (the same for every instantiation: one CTA an SM by its shared memory)
-static int mmq_pairs() {
-    static int pairs = 0;
-    if (!pairs) {
-        int dev = 0, sms = 0;
-        if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) { cudaGetLastError(); sms = 148; }
-        pairs = sms / 2;
-    }
-    return pairs;
-}
+static int mmq_pairs() { return sm_count() / 2; }
 
 // microseconds a K step of 64 takes while unpacking is the slower side: one tile of 256 rows on each of 74 pairs, 64 columns, from the difference
 // between 8192 and 4096 values a row

@@ -523,7 +523,7 @@ static int launch_delta_rule3(const b200_delta_rule_args *a, dim3 grid, cudaStre
 template <int DQ, bool CHAN>
 static int launch_delta_rule2(const b200_delta_rule_args *a, cudaStream_t st) {
     const dim3 grid((unsigned)((a->vdim + DR_COLS - 1) / DR_COLS), (unsigned)a->heads, (unsigned)a->n_seq);
-    return (int64_t)grid.x * grid.y * grid.z <= 148 ? launch_delta_rule3<DQ, CHAN, 1>(a, grid, st) : launch_delta_rule3<DQ, CHAN, 2>(a, grid, st);
+    return (int64_t)grid.x * grid.y * grid.z <= sm_count() ? launch_delta_rule3<DQ, CHAN, 1>(a, grid, st) : launch_delta_rule3<DQ, CHAN, 2>(a, grid, st);
 }
 
 template <int DQ>
