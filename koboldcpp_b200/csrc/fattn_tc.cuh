@@ -12,8 +12,10 @@
 //     none sees stay out of P . V whatever they hold.
 //   * the maximum that the exponent subtracts follows the true one only when that has grown by 8 (a factor of 256, which f16 and the f32 sums hold
 //     without loss), so O is hardly ever rescaled (at every growth: 40 us below instead of 33).  The largest weight is then no power of two and is rounded
-//     like the others, 4 % of the error against 64 bits (2.83e-4 -> 2.94e-4).  So the first quarter of Q's dims also brings what its f16 leaves over, two
-//     more MMAs a tile: 2.73e-4.  For all dims it would be 2.04e-4, for 42 us.
+//     like the others, 4 % of the error against 64 bits (2.83e-4 -> 2.94e-4).  So a quarter of Q's dims also brings what its f16 leaves over, two more MMAs
+//     a tile: those blocks of 16 dims, of all the CTA's columns, that leave over most (a fixed quarter does nothing for queries that lie in the others: 2.84e-4 -> 2.96e-4).
+//     White queries 2.73e-4, queries in three of four dims 2.6e-4; a column's last bits thus depend on the columns beside it.  For all dims it would be 2.04e-4,
+//     for 42 us; the weights as two f16 each 2.1e-4, for 38.
 //   * a key that is hidden from one column and visible to another of the CTA takes part with weight 0.  If its values are not finite, that column's
 //     result is not either: such columns are computed again, key by key over what they see (ft_column_alone).
 // What bounds it: K, V and mask on their way from L2 (32 KB a tile and CTA, 1150 cycles) and the softmax (940 cycles a tile for both groups: exponentials at 16 a
@@ -90,10 +92,25 @@ __host__ __device__ constexpr unsigned ft_idesc(int n, bool b_mn) { return (1u <
 __device__ __forceinline__ float ft_slope(const FaParams &p, int h) {
     return p.max_bias > 0.0f ? (h < p.n_head_log2 ? powf(p.m0, (float)(h + 1)) : powf(p.m1, (float)(2 * (h - p.n_head_log2) + 1))) : 1.0f;
 }
-// what two f16 leave over of two floats
-__device__ __forceinline__ unsigned ft_rest(float x, float y, unsigned h2) {
+// two f32 at a time: one issue slot for both
+__device__ __forceinline__ float2 ft_fma2(float2 x, float2 y, float2 z) {
+    float2 r;
+    asm("{\n.reg .b64 a, b, c;\nmov.b64 a, {%2, %3};\nmov.b64 b, {%4, %5};\nmov.b64 c, {%6, %7};\nfma.rn.f32x2 a, a, b, c;\nmov.b64 {%0, %1}, a;\n}\n"
+        : "=f"(r.x), "=f"(r.y) : "f"(x.x), "f"(x.y), "f"(y.x), "f"(y.y), "f"(z.x), "f"(z.y));
+    return r;
+}
+__device__ __forceinline__ float2 ft_add2(float2 x, float2 y) {
+    float2 r;
+    asm("{\n.reg .b64 a, b;\nmov.b64 a, {%2, %3};\nmov.b64 b, {%4, %5};\nadd.rn.f32x2 a, a, b;\nmov.b64 {%0, %1}, a;\n}\n" : "=f"(r.x), "=f"(r.y) : "f"(x.x), "f"(x.y), "f"(y.x), "f"(y.y));
+    return r;
+}
+// what two f16 leave over of two floats; its square is added to energy
+__device__ __forceinline__ unsigned ft_rest(float x, float y, unsigned h2, float &energy) {
     const float2 h = __half22float2(*reinterpret_cast<const __half2 *>(&h2));
-    return pack_h2(x - h.x, y - h.y);
+    x -= h.x;
+    y -= h.y;
+    energy = fmaf(x, x, fmaf(y, y, energy));
+    return pack_h2(x, y);
 }
 
 // one column by one warp, touching the keys that it sees and no others
@@ -247,6 +264,7 @@ __global__ void __launch_bounds__(FT_WARPS * 32, 1) fattn_tc_kernel(const __grid
     __shared__ unsigned tmem_base_s, again[4];
     __shared__ volatile int failed, scanned[FT_MASK];
     __shared__ float top[2][FT_COLS], total[2][FT_COLS];
+    __shared__ int rest_of[2];  // blocks of 16 dims whose remainder the last panel of Q holds
     const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31, tid = threadIdx.x;
     const int hk = blockIdx.y, col0 = (int)(gridDim.x - 1 - blockIdx.x) * FT_COLS, ncol = min(FT_COLS, p.n_cols - col0);  // (long causal walks first)
     const int n_tiles = (p.n_kv + FT_KEYS - 1) / FT_KEYS;
@@ -276,16 +294,44 @@ __global__ void __launch_bounds__(FT_WARPS * 32, 1) fattn_tc_kernel(const __grid
         // ===== Q as f16, swizzled; then every second tile, a thread a column
         const int w = warp >> 2, quarter = warp & 3, row = quarter * 32 + lane;
         const unsigned char *q_at = behind(p.q);
+        constexpr int CH = D / 8, ROWS = FT_SOFTMAX * 32 / CH;  // a thread takes 8 dims, number c of a row, of every ROWS-th column
+        const int c = tid % CH;
+        float energy = 0.f;
+        uint4 rest[FT_COLS / ROWS];
 #pragma unroll
-        for (int i = tid; i < FT_COLS * (D / 8); i += FT_SOFTMAX * 32) {
-            const int r = i / (D / 8), c = i % (D / 8), qc = min(col0 + r, p.n_cols - 1), n = token(qc), h = hk * p.gqa + qc - n * p.gqa;  // (columns behind the last: not stored)
+        for (int i = 0; i < FT_COLS / ROWS; i++) {
+            const int r = tid / CH + i * ROWS, qc = min(col0 + r, p.n_cols - 1), n = token(qc), h = hk * p.gqa + qc - n * p.gqa;  // (columns behind the last: not stored)
             const float4 *src = reinterpret_cast<const float4 *>(q_at + (size_t)n * p.q_nb1 + (size_t)h * p.q_nb2) + 2 * c;
             const float4 a = __ldcg(src), b = __ldcg(src + 1);
             unsigned char *to = sq + r * 128 + ((c % 8) ^ (r & 7)) * 16;
             const uint4 u = make_uint4(pack_h2(a.x, a.y), pack_h2(a.z, a.w), pack_h2(b.x, b.y), pack_h2(b.z, b.w));
             *reinterpret_cast<uint4 *>(to + c / 8 * FT_Q_PANEL) = u;
-            if (c < D / 32)  // the last panel: what f16 leaves over of the first D / 4 dims
-                *reinterpret_cast<uint4 *>(to + D / 64 * FT_Q_PANEL) = make_uint4(ft_rest(a.x, a.y, u.x), ft_rest(a.z, a.w, u.y), ft_rest(b.x, b.y, u.z), ft_rest(b.z, b.w, u.w));
+            rest[i] = make_uint4(ft_rest(a.x, a.y, u.x, energy), ft_rest(a.z, a.w, u.y, energy), ft_rest(b.x, b.y, u.z, energy), ft_rest(b.z, b.w, u.w, energy));
+        }
+        // the D / 64 blocks that leave over most go to the last panel (sums in a fixed order, equal ones by number: the same choice every time)
+        float *sums = reinterpret_cast<float *>(top);  // (not in use yet)
+        sums[tid] = energy;
+        asm volatile("bar.sync 3, %0;" ::"n"(FT_SOFTMAX * 32) : "memory");
+        energy = 0.f;
+#pragma unroll
+        for (int i = 0; i < FT_SOFTMAX; i++) energy += sums[32 * i + lane];
+#pragma unroll
+        for (int off = CH; off < 32; off *= 2) energy += __shfl_xor_sync(0xffffffffu, energy, off);
+        energy += __shfl_xor_sync(0xffffffffu, energy, 1);
+        energy = energy < 1e30f ? energy : 1e30f;  // (also what is not a number)
+        int rank = 0;
+#pragma unroll
+        for (int b = 0; b < D / 16; b++) {
+            const float e = __shfl_sync(0xffffffffu, energy, 2 * b);
+            rank += e > energy || (e == energy && b < c / 2) ? 1 : 0;
+        }
+        if (rank < D / 64) {
+            if (tid < CH) rest_of[rank] = c / 2;  // (the two threads of a block write the same)
+#pragma unroll
+            for (int i = 0; i < FT_COLS / ROWS; i++) {
+                const int r = tid / CH + i * ROWS;
+                *reinterpret_cast<uint4 *>(sq + D / 64 * FT_Q_PANEL + r * 128 + ((2 * rank + (c & 1)) ^ (r & 7)) * 16) = rest[i];
+            }
         }
         fence_proxy_async_smem();
         asm volatile("bar.sync 2, %0;" ::"n"(FT_SOFTMAX * 32 + 32) : "memory");
@@ -336,14 +382,19 @@ __global__ void __launch_bounds__(FT_WARPS * 32, 1) fattn_tc_kernel(const __grid
                     }
                 }
                 const float mb = m == -INFINITY ? 0.f : m;  // (nothing seen yet: 2^-inf = 0 throughout)
-                float sum[4] = {0.f, 0.f, 0.f, 0.f};
+                const float2 c2 = make_float2(c, c), mb2 = make_float2(-mb, -mb);
+                float2 sum[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
 #pragma unroll
-                for (int i = 0; i < 64; i++) v[i] = ex2(fmaf(v[i], c, -mb));
+                for (int i = 0; i < 64; i += 2) {
+                    const float2 e = ft_fma2(make_float2(v[i], v[i + 1]), c2, mb2);
+                    v[i] = ex2(e.x);
+                    v[i + 1] = ex2(e.y);
+                }
 #pragma unroll
-                for (int i = 0; i < 64; i++) sum[i & 3] += v[i];
+                for (int i = 0; i < 64; i += 2) sum[i / 2 & 1] = ft_add2(sum[i / 2 & 1], make_float2(v[i], v[i + 1]));
 #pragma unroll
                 for (int i = 0; i < 32; i++) x[i] = pack_h2(v[2 * i], v[2 * i + 1]);
-                l += (sum[0] + sum[1]) + (sum[2] + sum[3]);
+                l += (sum[0].x + sum[0].y) + (sum[1].x + sum[1].y);
             }
             tmem_st32(s_at, x);  // (over scores that have been read)
             tmem_wait_st();
@@ -409,6 +460,12 @@ __global__ void __launch_bounds__(FT_WARPS * 32, 1) fattn_tc_kernel(const __grid
         const bool elected = elect_lane();
         const unsigned long long qd = umma_desc_sw128(smem_u32(sq)), kd0 = umma_desc_sw128(smem_u32(sk));
         const unsigned kf = smem_u32(k_full), od = smem_u32(o_done);
+        unsigned rest_at[D / 64];
+#pragma unroll
+        for (int j = 0; j < D / 64; j++) {
+            const int kk = __shfl_sync(0xffffffffu, rest_of[j], 0);
+            rest_at[j] = (unsigned)(kk / 4 * (FT_PANEL >> 4) + 2 * (kk % 4));
+        }
         bool ok = true;
         for (int i = 0;; i++) {
             const unsigned b = i % FT_NB, ph = (i / FT_NB) & 1;
@@ -426,9 +483,9 @@ __global__ void __launch_bounds__(FT_WARPS * 32, 1) fattn_tc_kernel(const __grid
                 const unsigned long long kd = kd0 + b * (TILE >> 4);
                 const unsigned sd = tmem + b * FT_KEYS;
 #pragma unroll
-                for (int k = 0; k < D / 16 + D / 64; k++) {  // all of Q, then the rest of its first quarter (the panel behind the others)
-                    const int kk = k < D / 16 ? k : k - D / 16;
-                    tc_mma_bf16(sd, qd + (unsigned)(k / 4 * (FT_Q_PANEL >> 4) + 2 * (k % 4)), kd + (unsigned)(kk / 4 * (FT_PANEL >> 4) + 2 * (kk % 4)), ft_idesc(FT_KEYS, false), k != 0);
+                for (int k = 0; k < D / 16 + D / 64; k++) {  // all of Q, then what it leaves over of two blocks (one with 64 dims; the panel behind the others)
+                    const unsigned at = k < D / 16 ? (unsigned)(k / 4 * (FT_PANEL >> 4) + 2 * (k % 4)) : rest_at[k < D / 16 ? 0 : k - D / 16];
+                    tc_mma_bf16(sd, qd + (unsigned)(k / 4 * (FT_Q_PANEL >> 4) + 2 * (k % 4)), kd + at, ft_idesc(FT_KEYS, false), k != 0);
                 }
                 tc_commit(&s_full[b]);
             }
