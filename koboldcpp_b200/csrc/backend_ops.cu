@@ -712,6 +712,7 @@ static void run_mul_mat_id(ExecCtx &x, const ggml_tensor *n) {
     x.launches++;
 }
 
+int fa_launches(const b200_fattn_args *a, size_t workspace_bytes);  // fattn.cu
 static void run_flash_attn(ExecCtx &x, const ggml_tensor *n) {
     const ggml_tensor *q = n->src[0], *k = n->src[1], *v = n->src[2], *m = n->src[3];
     b200_fattn_args a;
@@ -727,7 +728,7 @@ static void run_flash_attn(ExecCtx &x, const ggml_tensor *n) {
     const size_t need = b200_flash_attn_workspace_bytes(&a);
     if (need > x.fa_ws_bytes) backend_abort("flash_attn workspace", "workspace smaller than planned");
     B200_CHECK_RC(b200_flash_attn_ext(&a, x.fa_ws, x.fa_ws_bytes, x.stream));
-    x.launches++;
+    x.launches += fa_launches(&a, x.fa_ws_bytes);
 }
 
 size_t node_fa_workspace(const ggml_tensor *n) {

@@ -798,6 +798,11 @@ size_t fa_cleared_bytes(const b200_fattn_args *a) {
     return pl.ticket_bytes + pl.part_bytes;
 }
 
+// kernels that b200_flash_attn_ext launches for these arguments
+int fa_launches(const b200_fattn_args *a, size_t workspace_bytes) {
+    return fa_check(a) == B200_OK && fa_plan(a).prefill && ft_fits(a) && workspace_bytes > FA_FRONT && ft_mask_once(a, workspace_bytes - FA_FRONT) ? 2 : 1;
+}
+
 }  // namespace b200
 
 using namespace b200;

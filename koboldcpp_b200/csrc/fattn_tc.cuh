@@ -667,6 +667,9 @@ static bool ft_encode(TmapBytes &tm, const void *base, int64_t D, int64_t rows, 
 // 26.4 -> 16.6 us, 16 heads, 213 tokens alone 12.9 -> 10.7; over 8 tiles with 8 heads a kv-head 8.9 -> 10.1, and still 22.5 -> 24.8 over 31.
 constexpr size_t FT_TABLE_BYTES = 512 * 1024;
 static size_t ft_table_bytes(const b200_fattn_args *a) { return (size_t)a->N * (size_t)((a->n_kv + FT_KEYS - 1) / FT_KEYS); }
+static bool ft_mask_once(const b200_fattn_args *a, size_t room) {
+    return a->mask && room >= ft_table_bytes(a) && (a->n_kv + FT_KEYS - 1) / FT_KEYS >= 6 * (a->n_head / a->n_head_kv);
+}
 // -1000: the other kernel's
 template <int D>
 static int ft_launch(const b200_fattn_args *a, const FaParams &p, unsigned char *ws, size_t ws_bytes, long long limit, cudaStream_t st) {
@@ -685,7 +688,7 @@ static int ft_launch(const b200_fattn_args *a, const FaParams &p, unsigned char 
     const unsigned div = (unsigned)(((1ull << 32) + p.gqa - 1) / p.gqa);  // (exact while columns x gqa < 2^32: ft_fits)
     const int n_tiles = (p.n_kv + FT_KEYS - 1) / FT_KEYS;
     unsigned char *table = nullptr;
-    if (p.mask != nullptr && ws != nullptr && ws_bytes >= ft_table_bytes(a) && n_tiles >= 6 * p.gqa) {
+    if (ws != nullptr && ft_mask_once(a, ws_bytes)) {
         table = ws;
         B200_CUDA_TRY(launch_chained(ft_mask_kernel, dim3((unsigned)((p.N + 7) / 8), (unsigned)((n_tiles + FT_MASK_TILES - 1) / FT_MASK_TILES)), 256, 0, st, p.mask, p.mask_nb1, p.N, p.n_kv, n_tiles, table));
     }
