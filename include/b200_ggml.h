@@ -245,7 +245,9 @@ typedef struct {
 } b200_fattn_args;
 /* A workspace starts zeroed.  After that it serves calls of any shape that it is large enough for, one after the other on one stream: the counters at its front are
  * zero again behind each call, and the scratch of all shapes lies behind them.  Calls that may run at the same time have one each.  The workspace of a
- * prompt batch (f16 cache, D 64 or 128) is optional: it lets the mask be read once instead of once a kv-head. */
+ * prompt batch (f16 cache, D 64 or 128) is optional: it lets the mask be read once instead of once a kv-head.
+ * Such a batch gives a query whose result is not finite, because values that it sees or that its neighbours see are not, a second pass over what it sees, cell by cell by
+ * one warp: right, but slow (milliseconds where 32k cells are seen and many queries are concerned). */
 B200_API size_t b200_flash_attn_workspace_bytes(const b200_fattn_args *a);
 B200_API int b200_flash_attn_ext(const b200_fattn_args *a, void *workspace, size_t workspace_bytes, b200_stream_t stream);
 /* The same with the limit of each of the kernel's own waits in clock cycles (b200_flash_attn_ext: about two seconds' worth), where a prompt runs on tcgen05 (f16 cache, D 64

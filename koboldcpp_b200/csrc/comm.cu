@@ -289,7 +289,7 @@ extern "C" int b200_all_reduce_sum_add_f32(const float *src, const float *residu
     // The exchange kernel uses no shared memory but ASKS for 150 KB: its CTAs then never share an SM with a CTA of the GEMVs around
     // it.  Under programmatic dependent launch its 16 small CTAs otherwise become resident next to the (register-lean) decode GEMV
     // CTAs and poll for their peers' data there while the next GEMV's prologue runs on the same SM: Llama-3-70B over 8 GPUs 186 ->
-    // 241 tok/s (profiles/r02_tp70_variants_n8.log).  B200_AR_SMEM overrides (0: none).
+    // 241 tok/s (profiles/tp70_variants_n8.log).  B200_AR_SMEM overrides (0: none).
     static const int ar_smem = getenv("B200_AR_SMEM") ? atoi(getenv("B200_AR_SMEM")) : 150000;
     if (ar_smem > 0) {
         static bool attr_set_dev[16] = {};

@@ -2,7 +2,7 @@
 //
 // The scalar flash-decode kernel (fattn_kernel) spent 782 warp instructions per (16 keys x K+V) tile -- 128 FFMA plus 128
 // f16->f32 conversions for one query column, ~70 shared loads, a 27-shuffle butterfly -- and ran out of issue slots at 3.0 TB/s with
-// two warps per scheduler (ncu: profiles/r02_ncu_fattn_f16_scalar.txt).  Here a warp keeps up to 16 query columns (all q-heads of a
+// two warps per scheduler (ncu: profiles/ncu_fattn_f16_scalar.txt).  Here a warp keeps up to 16 query columns (all q-heads of a
 // GQA group x the tokens of a small batch) as the M side of mma.sync.m16n8k16 tiles:
 //   S (16 q x 16 keys) = Q (16 x D, f16 A fragments resident in registers) . K^T   -- K rows come out of shared memory with
 //                                                                                     ldmatrix (B fragments, keys = n)
@@ -352,7 +352,7 @@ __global__ void __launch_bounds__(FM_NW * 32, 2) fattn_mma_kernel(const __grid_c
     FTRACE(1);
 
     // ---- Q: this lane holds columns g and g + 8 (rows of the M side); columns >= ncol are zero.  The loads go out BEFORE the
-    // first K/V tiles: behind 128 KB of cp.async per SM they came back 3.5 us later (profiles/r02_fattn_trace_timeline.log)
+    // first K/V tiles: behind 128 KB of cp.async per SM they came back 3.5 us later
     const unsigned char *q_at = behind(p.q);
     float2 qraw[2][KS][2];
     float slope[2];
@@ -419,7 +419,7 @@ __global__ void __launch_bounds__(FM_NW * 32, 2) fattn_mma_kernel(const __grid_c
     // ---- decode inside a cluster, opt-in (p.dyn_tiles): the KV tiles of the (kv-head, column tile) are handed out DYNAMICALLY
     // to the warps of all its CTAs (a counter in the shared memory of CTA 0, fetched one iteration ahead): with fixed ranges the
     // CTAs of a launch finish up to 4 us apart (they do not get equal shares of the HBM bandwidth) and the merge waits for the
-    // last one (profiles/r02_fattn_trace_timeline.log).  Not the default: see fattn.cu.
+    // last one.  Not the default: see fattn.cu.
     const bool dyn = p.dyn_tiles != 0;
     __shared__ unsigned tile_ctr;
     if (dyn) {
@@ -582,7 +582,7 @@ __global__ void __launch_bounds__(FM_NW * 32, 2) fattn_mma_kernel(const __grid_c
     if (p.cluster_merge) {
         // ---- the splits of this (kv-head, column tile) are one thread-block cluster (cluster rank == split): every CTA merges a
         // slice of the head dims of all columns straight out of its peers' shared memory -- no global round trip, no ticket
-        // (the global-memory merge below took 7 us of a 20 us launch at 7B @ 4k, profiles/r02_fattn_trace_timeline.log)
+        // (the global-memory merge below took 7 us of a 20 us launch at 7B @ 4k)
         cluster_sync_all();
         FTRACE(5);
         const int ns = p.n_splits;

@@ -381,7 +381,7 @@ static int launch_mmvq3(MmvqParams &p, cudaStream_t st, bool pdl) {
     p.part_rows = (int)part_rows;
     // row segments per warp that go out before griddepcontrol.wait: the activation loads queue behind them on the SM's ingest
     // path, so small launches (whose critical path is the activation phase) send one, large ones two (measured,
-    // profiles/r02_gemv_prefill_sweep.log)
+    // profiles/gemv_prefill_sweep.log)
     static const int prefill = getenv("B200_MMVQ_PREFILL") ? atoi(getenv("B200_MMVQ_PREFILL")) : -1;
     p.prefill = !pdl ? 0 : prefill >= 0 ? prefill : (nit1 && steps >= 2 ? 2 : 1);
     static const int dbg = getenv("B200_MMVQ_DBG") ? atoi(getenv("B200_MMVQ_DBG")) : 0;  // developer knobs: 1 no activation phase, 2 no dot

@@ -1,6 +1,6 @@
 // mmvq3.cuh -- the decode (one activation column) GEMV: lean skeleton around the per-type row dots of mmvq_core.cuh.
 //
-// Why a third skeleton (measured on B200, profiles/r02_gemv_chain_hot_cold_dbg.log): a
+// Why a third skeleton (measured on B200): a
 // chain of decode GEMVs ran as fast from L2 as from HBM -- the launches were bound by their own instruction stream, not by memory:
 // ~1030 warp instructions of prologue per warp (a per-CTA row table, ring fills issued serially by lane 0 at ~67 instructions
 // per copy pair, eight predicated activation loads whatever K is) and ~400 per (two rows x 4096 weights) step, of which 128 are

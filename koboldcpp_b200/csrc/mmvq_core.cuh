@@ -168,7 +168,7 @@ __device__ void load_activations(unsigned char *act_base, const float *__restric
 // trip and the quantisation overlaps the arrival of the weights.
 // A thread owns 8 consecutive values (two float4), four lanes one q8_1 block: the per-block work (two IEEE divisions, the
 // reductions, the fp16 roundings) is paid once per 8 values -- the quantisation is replicated in every CTA and sits on the critical
-// path of every launch (1.4 us of a 3.9 us 4096 x 4096 launch when a thread owned 4 values, profiles/r02_gemv_trace_timeline.log).
+// path of every launch (1.4 us of a 3.9 us 4096 x 4096 launch when a thread owned 4 values).
 constexpr int ACT_RR     = 8;                               // float4 per thread
 constexpr int ACT_RR_MAX = ACT_RR * 4 * MMVQ_THREADS;       // 16384 values
 template <int RR>

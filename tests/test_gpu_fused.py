@@ -125,7 +125,7 @@ def test_rope_kv_store_equals_separate_nodes(kv_type, D, NH, HK, T):
 
 def test_folded_nodes_keep_their_values():
     """The graph executor folds RMS_NORM->MUL into the GEMV prologue, ADD into its epilogue and SILU*up into the pair epilogue.
-    The folded nodes are still graph nodes another ggml_backend_sched split may read (ADVICE r1): with the optional outputs of
+    The folded nodes are still graph nodes another ggml_backend_sched split may read: with the optional outputs of
     b200_gemv_fuse the launch must store exactly what the unfused kernels would have stored."""
     L = lib()
     K, M = 4096, 1000

@@ -48,7 +48,7 @@ def test_other_weight_types_stay_on_the_backend(ftype):
 @pytest.mark.parametrize("type_kv", ["f16", "q8_0"])
 def test_k_shift_graph_stays_on_the_backend(dense, type_kv):
     """koboldcpp's ContextShift: llama_kv_cache_seq_rm + seq_add -> build_k_shift (src/llama.cpp:10144-10192): ROPE in place on the
-    f16 cache, or CPY(q8_0 -> f32) -> ROPE -> CPY(f32 -> q8_0) pinned to the KV backend (ADVICE r1: used to abort / fall to the CPU)."""
+    f16 cache, or CPY(q8_0 -> f32) -> ROPE -> CPY(f32 -> q8_0) pinned to the KV backend (used to abort / fall to the CPU)."""
     o = LC.run(dense, "b200", n_prompt=40, n_gen=8, sched_debug=True, dry_devices=1, type_kv=type_kv, shift_at=4, shift_by=8)
     assert o["sched"]["cpu_nodes"] == ONLY_EMBD, o["sched"]
 

@@ -1,6 +1,6 @@
 """Summarise an `ncu --metrics gpu__time_duration.sum --csv` launch list into per-kernel shares of ONE decoded token.
 
-    python tools/summarise_launches.py gpurun_out/launches.csv <launches_per_token> [token_index] > profiles/rNN_launches_*.txt
+    python tools/summarise_launches.py launches.csv <launches_per_token> [token_index] > launches.txt
 
 The capture covers several tokens of `bench.py --steps 2 --warmup 3`; the token_index-th complete token (default: the last one
 that fits) is cut out by position.  ncu times are cold-cache and serialised: compare SHARES, not absolutes."""
