@@ -11,7 +11,7 @@
 //     throughout, mixed, or hidden (-inf throughout), and which groups of 16 keys anybody sees.  Tiles that no column sees are not loaded, groups that
 //     none sees stay out of P . V whatever they hold.
 //   * the maximum that the exponent subtracts follows the true one only when that has grown by 8 (a factor of 256, which f16 and the f32 sums hold
-//     without loss), so O is hardly ever rescaled (at every growth: 40 us below instead of 33).  The largest weight is then no power of two and is rounded
+//     without loss), so O is hardly ever rescaled (at every growth: 41 us below instead of 34).  The largest weight is then no power of two and is rounded
 //     like the others, 4 % of the error against 64 bits (2.83e-4 -> 2.94e-4).  So a quarter of Q's dims also brings what its f16 leaves over, two more MMAs
 //     a tile: those blocks of 16 dims, of all the CTA's columns, that leave over most (a fixed quarter does nothing for queries that lie in the others: 2.84e-4 -> 2.96e-4).
 //     White queries 2.73e-4, queries in three of four dims 2.6e-4; a column's last bits thus depend on the columns beside it.  For all dims it would be 2.04e-4,
@@ -21,7 +21,7 @@
 // What bounds it: K, V and mask on their way from L2 (32 KB a tile and CTA, 1150 cycles) and the softmax (940 cycles a tile for both groups: exponentials at 16 a
 // cycle and SM), and start and end of a CTA.  32 heads of 128, 512 tokens behind 1536: 82 us with mma.sync (fattn_mma_prefill_kernel, which keeps the
 // other head sizes and masks at odd places); 41.5 with tiles of 128 keys and one S a group (a group then waits for its own products: 4700 cycles for two
-// tiles), 38 with tiles of 64, 34.3 with the mask read once (ft_mask_kernel).
+// tiles), 38 with tiles of 64, 34.3 with the mask read once (ft_mask_kernel), 32.1 .. 32.8 with all of Q asked for at once.
 // Waits have a limit, as in the prompt GEMM: a role that gives up sets `failed`, the others follow, and the status word is set.  Rows are stored only where no softmax
 // warp had given up when the sums met.
 #pragma once
@@ -104,13 +104,13 @@ __device__ __forceinline__ float2 ft_add2(float2 x, float2 y) {
     asm("{\n.reg .b64 a, b;\nmov.b64 a, {%2, %3};\nmov.b64 b, {%4, %5};\nadd.rn.f32x2 a, a, b;\nmov.b64 {%0, %1}, a;\n}\n" : "=f"(r.x), "=f"(r.y) : "f"(x.x), "f"(x.y), "f"(y.x), "f"(y.y));
     return r;
 }
-// what two f16 leave over of two floats; its square is added to energy
-__device__ __forceinline__ unsigned ft_rest(float x, float y, unsigned h2, float &energy) {
-    const float2 h = __half22float2(*reinterpret_cast<const __half2 *>(&h2));
-    x -= h.x;
-    y -= h.y;
-    energy = fmaf(x, x, fmaf(y, y, energy));
-    return pack_h2(x, y);
+// what two pairs of f16 leave over of four floats; its square is added to energy
+__device__ __forceinline__ void ft_rest(float4 &x, unsigned h0, unsigned h1, float2 &energy) {
+    const float2 minus = make_float2(-1.0f, -1.0f);
+    const float2 a = ft_fma2(__half22float2(*reinterpret_cast<const __half2 *>(&h0)), minus, make_float2(x.x, x.y));
+    const float2 b = ft_fma2(__half22float2(*reinterpret_cast<const __half2 *>(&h1)), minus, make_float2(x.z, x.w));
+    energy = ft_fma2(a, a, ft_fma2(b, b, energy));
+    x = make_float4(a.x, a.y, b.x, b.y);
 }
 
 // one column by one warp, touching the keys that it sees and no others
@@ -296,19 +296,32 @@ __global__ void __launch_bounds__(FT_WARPS * 32, 1) fattn_tc_kernel(const __grid
         const unsigned char *q_at = behind(p.q);
         constexpr int CH = D / 8, ROWS = FT_SOFTMAX * 32 / CH;  // a thread takes 8 dims, number c of a row, of every ROWS-th column
         const int c = tid % CH;
-        float energy = 0.f;
-        uint4 rest[FT_COLS / ROWS];
+        float4 qv[FT_COLS / ROWS][2];
+        uint4 qh[FT_COLS / ROWS];
 #pragma unroll
         for (int i = 0; i < FT_COLS / ROWS; i++) {
             const int r = tid / CH + i * ROWS, qc = min(col0 + r, p.n_cols - 1), n = token(qc), h = hk * p.gqa + qc - n * p.gqa;  // (columns behind the last: not stored)
             const float4 *src = reinterpret_cast<const float4 *>(q_at + (size_t)n * p.q_nb1 + (size_t)h * p.q_nb2) + 2 * c;
-            const float4 a = __ldcg(src), b = __ldcg(src + 1);
-            unsigned char *to = sq + r * 128 + ((c % 8) ^ (r & 7)) * 16;
-            const uint4 u = make_uint4(pack_h2(a.x, a.y), pack_h2(a.z, a.w), pack_h2(b.x, b.y), pack_h2(b.z, b.w));
-            *reinterpret_cast<uint4 *>(to + c / 8 * FT_Q_PANEL) = u;
-            rest[i] = make_uint4(ft_rest(a.x, a.y, u.x, energy), ft_rest(a.z, a.w, u.y, energy), ft_rest(b.x, b.y, u.z, energy), ft_rest(b.z, b.w, u.w, energy));
+            qv[i][0] = __ldcg(src);
+            qv[i][1] = __ldcg(src + 1);
         }
-        // the D / 64 blocks that leave over most go to the last panel (sums in a fixed order, equal ones by number: the same choice every time)
+#pragma unroll
+        for (int i = 0; i < FT_COLS / ROWS; i++) {
+            const int r = tid / CH + i * ROWS;
+            const float4 a = qv[i][0], b = qv[i][1];
+            qh[i] = make_uint4(pack_h2(a.x, a.y), pack_h2(a.z, a.w), pack_h2(b.x, b.y), pack_h2(b.z, b.w));
+            *reinterpret_cast<uint4 *>(sq + c / 8 * FT_Q_PANEL + r * 128 + ((c % 8) ^ (r & 7)) * 16) = qh[i];
+        }
+        // the D / 64 blocks that leave over most go to the last panel (sums in a fixed order, equal ones by number: the same choice every time).  It takes 0.1 .. 0.2 us of a
+        // CTA's start (32 heads, 73 tokens alone 9.06 -> 9.27 us, 8 on one kv-head 8.88 -> 8.98); all loads of Q in flight at once give more back
+        // where Q comes from HBM (512 tokens behind 1536: 34.3 -> 32.1 .. 32.8).  A first product that begins without the panel is no faster.
+        float2 energy2 = make_float2(0.f, 0.f);
+#pragma unroll
+        for (int i = 0; i < FT_COLS / ROWS; i++) {
+            ft_rest(qv[i][0], qh[i].x, qh[i].y, energy2);
+            ft_rest(qv[i][1], qh[i].z, qh[i].w, energy2);
+        }
+        float energy = energy2.x + energy2.y;
         float *sums = reinterpret_cast<float *>(top);  // (not in use yet)
         sums[tid] = energy;
         asm volatile("bar.sync 3, %0;" ::"n"(FT_SOFTMAX * 32) : "memory");
@@ -330,11 +343,11 @@ __global__ void __launch_bounds__(FT_WARPS * 32, 1) fattn_tc_kernel(const __grid
 #pragma unroll
             for (int i = 0; i < FT_COLS / ROWS; i++) {
                 const int r = tid / CH + i * ROWS;
-                *reinterpret_cast<uint4 *>(sq + D / 64 * FT_Q_PANEL + r * 128 + ((2 * rank + (c & 1)) ^ (r & 7)) * 16) = rest[i];
+                *reinterpret_cast<uint4 *>(sq + D / 64 * FT_Q_PANEL + r * 128 + ((2 * rank + (c & 1)) ^ (r & 7)) * 16) = make_uint4(pack_h2(qv[i][0].x, qv[i][0].y), pack_h2(qv[i][0].z, qv[i][0].w), pack_h2(qv[i][1].x, qv[i][1].y), pack_h2(qv[i][1].z, qv[i][1].w));
             }
         }
         fence_proxy_async_smem();
-        asm volatile("bar.sync 2, %0;" ::"n"(FT_SOFTMAX * 32 + 32) : "memory");
+        asm volatile("bar.arrive 2, %0;" ::"n"(FT_SOFTMAX * 32 + 32) : "memory");
 
         const int col = min(col0 + row, p.n_cols - 1), tok = token(col);
         const float slope = ft_slope(p, hk * p.gqa + col - tok * p.gqa), scale = p.softcap != 0.0f ? p.scale / p.softcap : p.scale;
@@ -460,10 +473,10 @@ __global__ void __launch_bounds__(FT_WARPS * 32, 1) fattn_tc_kernel(const __grid
         const bool elected = elect_lane();
         const unsigned long long qd = umma_desc_sw128(smem_u32(sq)), kd0 = umma_desc_sw128(smem_u32(sk));
         const unsigned kf = smem_u32(k_full), od = smem_u32(o_done);
-        unsigned rest_at[D / 64];
+        unsigned rest_at[D / 64];  // (a reduction over the warp leaves it where the descriptors want it, the same in all lanes: through a shuffle every tile paid for it)
 #pragma unroll
         for (int j = 0; j < D / 64; j++) {
-            const int kk = __shfl_sync(0xffffffffu, rest_of[j], 0);
+            const int kk = (int)__reduce_or_sync(0xffffffffu, (unsigned)rest_of[j]);
             rest_at[j] = (unsigned)(kk / 4 * (FT_PANEL >> 4) + 2 * (kk % 4));
         }
         bool ok = true;
@@ -479,9 +492,9 @@ __global__ void __launch_bounds__(FT_WARPS * 32, 1) fattn_tc_kernel(const __grid
                 break;
             }
             tc_fence_after();
+            const unsigned long long kd = kd0 + b * (TILE >> 4);
+            const unsigned sd = tmem + b * FT_KEYS;
             if (elected) {
-                const unsigned long long kd = kd0 + b * (TILE >> 4);
-                const unsigned sd = tmem + b * FT_KEYS;
 #pragma unroll
                 for (int k = 0; k < D / 16 + D / 64; k++) {  // all of Q, then what it leaves over of two blocks (one with 64 dims; the panel behind the others)
                     const unsigned at = k < D / 16 ? (unsigned)(k / 4 * (FT_PANEL >> 4) + 2 * (k % 4)) : rest_at[k < D / 16 ? 0 : k - D / 16];
