@@ -201,10 +201,8 @@ struct MmqParams {
     const int *tile_tab;
     const int *row_dst;
     size_t expert_bytes;
-    // split-K (mmq_pair_kernel, one product): a tile owns a contiguous share of K and ADDS its sums into a zeroed dst (red.global.add.f32).  Only 1
-    // or 2: the sum of two partials does not depend on their arrival order.
-    int ksplit;
-    // batch of independent products of one shape (not grouped, no split-K): W advances by w_batch_bytes, dst by dst_batch floats, the
+    int ksplit;  // parts of K that the pairs of a cluster take (mmq_pair_kernel, not grouped)
+    // batch of independent products of one shape (not grouped): W advances by w_batch_bytes, dst by dst_batch floats, the
     // bf16 activations by n_pad rows
     int n_batch;
     size_t w_batch_bytes;

@@ -16,13 +16,18 @@
 //   * the MMA warp walks through its loop as a whole and elects a lane for the tcgen05 instructions only: loop counters and descriptors then
 //     live in uniform registers.  (With one lane in the loop every MMA needed a dozen vector instructions, each of which waits its turn
 //     among the producers: 190 cycles an MMA whatever its width.)
-//   * the accumulators are double-buffered in TMEM (2 x 256 columns): four epilogue warps store tile i while tile i + 1 is computed.
+//   * the accumulators are double-buffered in TMEM (2 x 256 columns): four epilogue warps store tile i while tile i + 1 is computed.  The last tile, with
+//     nothing behind it, is stored by all that are left, twenty warps (dense weights: twelve): 6144 x 4096 bf16 over 512 columns 28 -> 22 us,
+//     11008 x 4096 q4_K 55.5 -> 49.1.
+//   * where the tiles leave pairs idle, a cluster of up to eight pairs takes one tile, each a part of K; the parts meet in distributed shared memory and are
+//     added in the order of K (pair_merge).  5120 x 5120 over 199 columns, 20 tiles in three parts: q5_K 32.4 -> 21.9 us, q6_K 43 -> 24; 1024 x 4096 q4_K over
+//     300 columns, 12 in four, 19.4 -> 13.6; 256 x 5120 q6_K over 400, 5 in seven, 24.7 -> 13.5.
 //   * BN is chosen on the host so that the tiles fill the pairs evenly (mmq_pair_plan): 512 columns are 2 x 256 or 3 x 176, whichever leaves
 //     the last wave fuller.  In the grouped form (routed experts) the width of every tile follows its rows.
 // Every wait has a limit (MmqParams::wait_limit).  A role whose wait runs out sets `failed` of its CTA and leaves its loop: no store, copy or MMA, and no
 // arrival (an arrival that no wait stands before could find a phase whose arrivals are all there, waiting for bytes only).  Whoever
 // waits for it, in either CTA, gives up in turn.  An accumulator is announced when the operands of all its K steps had arrived, so what is
-// stored is right (of two halves of K: what is added); the rest of the result stays as it was, *timeout is set, and the CTA stays until
+// stored is right (of several parts of K nothing is stored unless all of them are there); the rest of the result stays as it was, *timeout is set, and the CTA stays until
 // copies and MMAs in flight have ended.
 #pragma once
 
@@ -30,6 +35,7 @@ namespace b200 {
 
 constexpr int PAIR_PRODUCERS = 16;                   // warps that unpack, 8 rows of the CTA's 128 each
 constexpr int PAIR_MAX_STAGES = 8;
+constexpr int PAIR_MAX_SPLIT = 8;                    // parts of K: a cluster of 16 CTAs at most
 constexpr int PAIR_SMEM = 232448 - 1024 - 1024;      // dynamic shared memory: what a CTA can have, less static data and alignment
 
 // 256-value groups of 128 rows as they lie in memory: 16-byte pieces a row (a 2-byte aligned row starts up to 14 bytes into its first one)
@@ -70,17 +76,24 @@ __device__ __forceinline__ void tc_mma2_bf16(unsigned tmem_d, unsigned long long
         "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
         : "memory");
 }
-// arrives on `bar` of both CTAs when the MMAs issued so far have retired
-__device__ __forceinline__ void tc_commit2(unsigned bar) {
-    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(bar), "h"((unsigned short)3) : "memory");
+// arrives on `bar` of both CTAs (a bit each in `both`) when the MMAs issued so far have retired
+__device__ __forceinline__ void tc_commit2(unsigned bar, unsigned short both) {
+    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(bar), "h"(both) : "memory");
 }
-// the pair's first CTA's copy of a shared variable, and an arrival there.  (The default semantics: what the barrier guards is in shared memory or TMEM
+// CTA `rank`'s copy of a shared variable, and an arrival there.  (The default semantics: what the barrier guards is in shared memory or TMEM
 // and complete when the arrival is issued; a release at cluster scope would wait for the thread's outstanding memory operations, about 1000
 // cycles a K step.)
-__device__ __forceinline__ unsigned leader_addr(unsigned local) {
+__device__ __forceinline__ unsigned cluster_addr(unsigned local, int rank) {
     unsigned r;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(r) : "r"(local));
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(local), "r"(rank));
     return r;
+}
+// what another CTA has written before the cluster barrier in front of the load
+__device__ __forceinline__ int ld_cluster(unsigned at) { int v; asm volatile("ld.shared::cluster.b32 %0, [%1];" : "=r"(v) : "r"(at) : "memory"); return v; }
+__device__ __forceinline__ float4 ld_cluster4(unsigned at) {
+    float4 v;
+    asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(at) : "memory");
+    return v;
 }
 __device__ __forceinline__ void mbar_arrive_remote(unsigned bar) { asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory"); }
 // ---------------------------------------------------------------- 32 values of a row out of shared memory -> 16 packed bf16 pairs
@@ -314,7 +327,7 @@ struct PairTile {
     int kb0, nkb;        // K steps of 64
 };
 template <bool GROUPED>
-__device__ __forceinline__ PairTile pair_tile(const PairParams &p, int t, int nt, int ksteps_unit) {
+__device__ __forceinline__ PairTile pair_tile(const PairParams &p, int t, int nt, int ksteps_unit, int split) {
     PairTile r;
     const int ni = t % nt;
     int rest = t / nt;
@@ -333,21 +346,75 @@ __device__ __forceinline__ PairTile pair_tile(const PairParams &p, int t, int nt
         r.n0 = (int64_t)ni * p.bn;
         r.n_end = r.n0 + p.bn < p.q.N ? r.n0 + p.bn : p.q.N;
         r.n = p.bn;
-        if (p.q.n_batch > 1) {
-            r.product = rest;
-        } else {
-            r.product = 0;
-            const int units = r.nkb / ksteps_unit, u0 = rest * units / p.q.ksplit, u1 = (rest + 1) * units / p.q.ksplit;
-            r.kb0 = u0 * ksteps_unit;
-            r.nkb = (u1 - u0) * ksteps_unit;
-        }
+        r.product = rest;
+        const int units = r.nkb / ksteps_unit, u0 = split * units / p.q.ksplit, u1 = (split + 1) * units / p.q.ksplit;
+        r.kb0 = u0 * ksteps_unit;
+        r.nkb = (u1 - u0) * ksteps_unit;
     }
     return r;
 }
 
 template <int TYPE> __host__ __device__ constexpr int pair_steps() { return TYPE == B200_TYPE_BF16 ? 1 : 2; }  // K steps of 64 a stage
+// warps: producers, MMAs, copies, four that store; of dense weights, which have no producers, eight more for the meeting of a tile's parts
 template <int TYPE>
-__host__ __device__ constexpr int pair_threads() { return 32 * ((TYPE == B200_TYPE_BF16 ? 0 : PAIR_PRODUCERS) + 6); }
+__host__ __device__ constexpr int pair_threads() { return 32 * (6 + (TYPE == B200_TYPE_BF16 ? 8 : PAIR_PRODUCERS)); }
+
+// ===== the parts of a tile meet.  Each CTA lays its accumulators, [column][128 rows], over its operand ring, which its MMAs have left; behind the
+// cluster's barrier CTA (split, rank) reads columns split / ksplit of them from every CTA with its rows and adds them in the order of K.
+// All threads of the cluster come here.
+template <int TYPE>
+__device__ __forceinline__ void pair_merge(const PairParams &p, const PairTile &ti, unsigned char *smem, unsigned tmem_base, unsigned acc_full0, int rank, int split, volatile int *failed,
+                                           volatile int *part_there) {
+    constexpr int MW = pair_threads<TYPE>() / 128 * 4;  // warps that read TMEM: whole sets of its four quarters
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, ks = p.q.ksplit, cols = (int)(ti.n_end - ti.n0);
+    const bool ok = __all_sync(0xffffffffu, pair_wait<20>(acc_full0, 0, failed, p.q.wait_limit));
+    tc_fence_after();
+    if (ok && warp < MW) {
+        const int quarter = warp & 3;
+        float *mine = reinterpret_cast<float *>(smem) + quarter * 32 + lane;
+#pragma unroll 1
+        for (int c0 = 32 * (warp >> 2); c0 < cols; c0 += 8 * MW) {
+            float v[32];
+            tmem_ld32(tmem_base + ((unsigned)(quarter * 32) << 16) + (unsigned)c0, v);
+#pragma unroll
+            for (int j = 0; j < 32; j++) if (c0 + j < cols) mine[(c0 + j) * MQ_BM] = v[j];
+        }
+    }
+    const int all = __syncthreads_and(ok);
+    if (threadIdx.x == 0) *part_there = all;
+    __syncwarp();
+    pair_arrive();
+    pair_await();
+    bool there = true;
+#pragma unroll 1
+    for (int s = 0; s < ks; s++) there = there && ld_cluster(cluster_addr(smem_u32(const_cast<int *>(part_there)), 2 * s + rank)) != 0;
+    if (!there) return;
+    const int per = (cols + ks - 1) / ks, c1 = min(cols, (split + 1) * per);
+    const int64_t m = ti.m0 + rank * MQ_BM + 4 * lane;
+    float *drow = p.q.dst + m + ti.product * p.q.dst_batch + ti.n0 * p.q.dst_stride;
+    const bool whole = m + 3 < p.q.M && ((uintptr_t)p.q.dst & 15) == 0 && ((p.q.dst_stride | p.q.dst_batch) & 3) == 0;
+    const unsigned here = smem_u32(smem) + 16u * lane;
+#pragma unroll 1
+    for (int c = split * per + warp; c < c1; c += pair_threads<TYPE>() / 32) {
+        float4 v[4], sum = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 1
+        for (int s0 = 0; s0 < ks; s0 += 4) {
+#pragma unroll
+            for (int s = 0; s < 4; s++) if (s0 + s < ks) v[s] = ld_cluster4(cluster_addr(here, 2 * (s0 + s) + rank) + (unsigned)c * (MQ_BM * 4));
+#pragma unroll
+            for (int s = 0; s < 4; s++) if (s0 + s < ks) { sum.x += v[s].x; sum.y += v[s].y; sum.z += v[s].z; sum.w += v[s].w; }
+        }
+        float *d = drow + c * p.q.dst_stride;
+        if (whole) {
+            *reinterpret_cast<float4 *>(d) = sum;
+        } else {
+            if (m < p.q.M) d[0] = sum.x;
+            if (m + 1 < p.q.M) d[1] = sum.y;
+            if (m + 2 < p.q.M) d[2] = sum.z;
+            if (m + 3 < p.q.M) d[3] = sum.w;
+        }
+    }
+}
 
 template <int TYPE, bool GROUPED>
 __global__ void __launch_bounds__(pair_threads<TYPE>(), 1) mmq_pair_kernel(const __grid_constant__ TmapBytes tmA, const __grid_constant__ TmapBytes tmB, const __grid_constant__ PairParams p) {
@@ -358,9 +425,12 @@ __global__ void __launch_bounds__(pair_threads<TYPE>(), 1) mmq_pair_kernel(const
     unsigned char *smem = reinterpret_cast<unsigned char *>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     __shared__ __align__(8) unsigned long long full_bar[PAIR_MAX_STAGES], peer_bar[PAIR_MAX_STAGES], empty_bar[PAIR_MAX_STAGES], acc_full[2], acc_empty[2];
     __shared__ unsigned tmem_base_s;
-    __shared__ volatile int failed;
+    __shared__ volatile int failed, part_there;
     const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31, tid = threadIdx.x;
-    const int rank = (int)cluster_rank(), pair = (int)(blockIdx.x >> 1), n_pairs = (int)(gridDim.x >> 1);
+    // a cluster is ksplit pairs: its pairs take parts of K of the same tile
+    const int in_cluster = (int)cluster_rank(), rank = in_cluster & 1, leader = in_cluster & ~1, split = in_cluster >> 1, ksplit = GROUPED ? 1 : p.q.ksplit;
+    const int pair = (int)blockIdx.x / (2 * ksplit), n_pairs = (int)gridDim.x / (2 * ksplit);
+    const unsigned short both = (unsigned short)(3u << leader);
     const long long limit = p.q.wait_limit;
     const int S = p.stages, b_step = p.bn * MQ_BK, stage_bytes = A_BYTES + SK * b_step;  // (a step: bn / 2 activation rows of 128 bytes)
     const unsigned full0 = smem_u32(full_bar), peer0 = smem_u32(peer_bar), empty0 = smem_u32(empty_bar), acc_full0 = smem_u32(acc_full), acc_empty0 = smem_u32(acc_empty);
@@ -373,6 +443,7 @@ __global__ void __launch_bounds__(pair_threads<TYPE>(), 1) mmq_pair_kernel(const
         }
         for (int b = 0; b < 2; b++) { mbar_init(&acc_full[b], 1); mbar_init(&acc_empty[b], 8); }
         failed = 0;
+        part_there = 1;
         mbar_fence_init();
     }
     if (warp == NP) tmem_alloc2(&tmem_base_s, 512);
@@ -385,7 +456,7 @@ __global__ void __launch_bounds__(pair_threads<TYPE>(), 1) mmq_pair_kernel(const
     const unsigned tmem_base = tmem_base_s;
     pdl_enter();
     const int nt = GROUPED ? p.q.tile_tab[0] : p.n_tiles_n;
-    const int n_tiles = nt * p.n_tiles_m * (GROUPED ? 1 : p.q.n_batch > 1 ? p.q.n_batch : p.q.ksplit);
+    const int n_tiles = nt * p.n_tiles_m * (GROUPED ? 1 : p.q.n_batch);
 
     if (warp < NP) {
         // ===== producers: rows 8 * warp .. 8 * warp + 7 of this CTA's 128
@@ -405,7 +476,7 @@ __global__ void __launch_bounds__(pair_threads<TYPE>(), 1) mmq_pair_kernel(const
             for (int j = 0; j < PER; j++) to[j] = smem_u32(raw) + (unsigned)((lane + 32 * j) / PIECES * ROW + (lane + 32 * j) % PIECES * 16);
             auto copy_group = [&]() {
                 if (left == 0 && ct < n_tiles) {
-                    const PairTile ti = pair_tile<GROUPED>(p, ct, nt, UNIT);
+                    const PairTile ti = pair_tile<GROUPED>(p, ct, nt, UNIT, split);
                     left = ti.nkb / 4;
                     ct += n_pairs;
 #pragma unroll
@@ -442,7 +513,7 @@ __global__ void __launch_bounds__(pair_threads<TYPE>(), 1) mmq_pair_kernel(const
             unsigned ph = 1;            // parity of the stage's empty barrier: the first pass finds it free
             bool ok = true;  // (the same in all lanes)
             for (int t = pair; t < n_tiles && ok; t += n_pairs) {
-                const PairTile ti = pair_tile<GROUPED>(p, t, nt, UNIT);
+                const PairTile ti = pair_tile<GROUPED>(p, t, nt, UNIT, split);
                 unsigned at = raw_aligned(TYPE) ? 0u : (unsigned)(uintptr_t)row_base(ti, r) & 15u;  // where in its first piece the row's group starts
 #pragma unroll 1
                 for (int g = ti.nkb / 4; g > 0 && ok; g--) {
@@ -476,12 +547,12 @@ __global__ void __launch_bounds__(pair_threads<TYPE>(), 1) mmq_pair_kernel(const
         // ===== the pair's MMAs (first CTA); the second CTA passes on that its half of a stage is ready
         const unsigned long long desc0 = umma_desc_sw128(smem_u32(smem));
         const bool elected = elect_lane();
-        const unsigned peer_remote = leader_addr(peer0);
+        const unsigned peer_remote = cluster_addr(peer0, leader);
         int s = 0, buf = 0;
         unsigned ph = 0, aph = 1;
         bool ok = true;  // (the same in all lanes)
         for (int t = pair; t < n_tiles && ok; t += n_pairs) {
-            const PairTile ti = pair_tile<GROUPED>(p, t, nt, UNIT);
+            const PairTile ti = pair_tile<GROUPED>(p, t, nt, UNIT, split);
             if (rank != 0) {
                 for (int kb = 0; kb < ti.nkb; kb += SK) {
                     ok = __all_sync(0xffffffffu, pair_wait<0>(full0 + 8u * s, ph, &failed, limit));
@@ -512,14 +583,14 @@ __global__ void __launch_bounds__(pair_threads<TYPE>(), 1) mmq_pair_kernel(const
 #pragma unroll
                         for (int k = 0; k < MQ_BK / 16; k++) tc_mma2_bf16(acc, aj + 2u * k, bj + 2u * k, idesc, j + k ? 1u : accumulate);
                     }
-                    tc_commit2(empty0 + 8u * s);
+                    tc_commit2(empty0 + 8u * s, both);
                 }
                 __syncwarp();
                 accumulate = 1;
                 if (++s == S) { s = 0; ph ^= 1u; }
             }
             if (!ok) break;
-            if (elected) tc_commit2(acc_full0 + 8u * buf);
+            if (elected) tc_commit2(acc_full0 + 8u * buf, both);
             __syncwarp();
             buf ^= 1;
             if (buf == 0) aph ^= 1u;
@@ -532,7 +603,7 @@ __global__ void __launch_bounds__(pair_threads<TYPE>(), 1) mmq_pair_kernel(const
         int s = 0;
         unsigned ph = 1;
         for (int t = pair; t < n_tiles; t += n_pairs) {
-            const PairTile ti = pair_tile<GROUPED>(p, t, nt, UNIT);
+            const PairTile ti = pair_tile<GROUPED>(p, t, nt, UNIT, split);
             const int half = ti.n / 2, row = (int)(ti.n0 + rank * half + (GROUPED ? 0 : ti.product * p.q.n_pad));
             const int a_row = DENSE ? (int)(ti.product * p.w_rows_per_product + ti.m0 + rank * MQ_BM) : 0;
             const unsigned tx = (unsigned)(SK * half * MQ_BK * 2 + (DENSE ? A_BYTES : 0));
@@ -558,24 +629,39 @@ __global__ void __launch_bounds__(pair_threads<TYPE>(), 1) mmq_pair_kernel(const
                 if (++s == S) { s = 0; ph ^= 1u; }
             }
         }
-    } else {
-        // ===== epilogue: TMEM lanes 32 * (warp % 4) .. of this CTA's 128 rows
+    }
+    // ===== epilogue: four warps, one for each 32 of this CTA's 128 rows (TMEM lanes 32 * (warp % 4) ..); of the last tile, behind which nothing is left to
+    // do, the producers (dense weights: the warps without another role) store their share of the columns
+    if (ksplit == 1 && warp != NP && warp != NP + 1) {
+        constexpr int SETS = (pair_threads<TYPE>() / 32 - 2) / 4;
+        const bool always = warp >= NP + 2 && warp < NP + 6;
+        const int set = always ? 0 : DENSE ? (warp - 2) / 4 : 1 + warp / 4;
         bool ok = true;
         int buf = 0;
         unsigned ph = 0;
         const int quarter = warp & 3;
-        const unsigned acc_remote = leader_addr(acc_empty0);
+        const unsigned acc_remote = cluster_addr(acc_empty0, leader);
         const int *row_dst = behind(p.q.row_dst);
-        for (int t = pair; t < n_tiles; t += n_pairs) {
-            const PairTile ti = pair_tile<GROUPED>(p, t, nt, UNIT);
-            ok = ok && pair_wait<200>(acc_full0 + 8u * buf, ph, &failed, limit);
+        for (int t = always || pair >= n_tiles ? pair : pair + (n_tiles - 1 - pair) / n_pairs * n_pairs; t < n_tiles; t += n_pairs) {
+            const PairTile ti = pair_tile<GROUPED>(p, t, nt, UNIT, split);
+            const bool last = t + n_pairs >= n_tiles;
+            if (always) {
+                ok = __all_sync(0xffffffffu, ok && pair_wait<20>(acc_full0 + 8u * buf, ph, &failed, limit));
+                if (last && !ok) part_there = 0;
+            } else {
+                buf = (t - pair) / n_pairs & 1;
+            }
+            if (last) {
+                asm volatile("bar.sync 1, %0;" ::"n"(SETS * 128) : "memory");
+                if (!always) ok = part_there != 0;
+            }
             tc_fence_after();
             const int64_t m = ti.m0 + rank * MQ_BM + quarter * 32 + lane;
             const bool row_ok = m < p.q.M && ok;
-            float *drow = p.q.dst + m + (!GROUPED && p.q.n_batch > 1 ? ti.product * p.q.dst_batch : 0);
+            float *drow = p.q.dst + m + (GROUPED ? 0 : ti.product * p.q.dst_batch);
             const int cols = (int)(ti.n_end - ti.n0);
 #pragma unroll 1
-            for (int c0 = 0; c0 < cols; c0 += 32) {
+            for (int c0 = last ? 32 * set : 0; c0 < cols; c0 += last ? 32 * SETS : 32) {
                 float v[32];
                 // scatter: sorted row -> (token, slot).  A lane asks for one of the 32 columns' places: in front of each store a load would wait for its turn
                 const int place = GROUPED && c0 + lane < cols ? ld_behind(row_dst + ti.n0 + c0 + lane) : 0;
@@ -591,21 +677,20 @@ __global__ void __launch_bounds__(pair_threads<TYPE>(), 1) mmq_pair_kernel(const
 #pragma unroll
                     for (int j = 0; j < 32; j++) {
                         if (c0 + j >= cols) continue;
-                        const int64_t n = ti.n0 + c0 + j;
-                        if (p.q.ksplit > 1) atomicAdd(drow + n * p.q.dst_stride, v[j]);    // (result unused: RED.ADD.F32)
-                        else drow[n * p.q.dst_stride] = v[j];
+                        drow[(ti.n0 + c0 + j) * p.q.dst_stride] = v[j];
                     }
                 }
             }
             tc_fence_before();
             __syncwarp();
-            if (lane == 0 && ok) mbar_arrive_remote(acc_remote + 8u * buf);
+            if (always && lane == 0 && ok) mbar_arrive_remote(acc_remote + 8u * buf);
             buf ^= 1;
             if (buf == 0) ph ^= 1u;
         }
     }
     __syncwarp();
     if (warp < NP || warp == NP + 1) pair_await();
+    if (!GROUPED && ksplit > 1) pair_merge<TYPE>(p, pair_tile<GROUPED>(p, pair, nt, UNIT, split), smem, tmem_base, acc_full0, rank, split, &failed, &part_there);
     __syncthreads();
     if (failed) {  // copies and MMAs that were requested end within this time
         if (tid == 0) atomicExch(p.timeout, 1);
@@ -621,35 +706,43 @@ __global__ void __launch_bounds__(pair_threads<TYPE>(), 1) mmq_pair_kernel(const
 }
 
 // ---------------------------------------------------------------- host side
-// Tile width and K split by the time of the longest pair's work, in microseconds.  A K step of 64 costs what the slower of producers and tensor cores
+// Tile width and parts of K by the time of the longest pair's work, in microseconds.  A K step of 64 costs what the slower of producers and tensor cores
 // takes, `unpack` or 1.83 ns a column, and a little more where they are level (sixth powers added: within 4 % of q4_K and q6_K at 64 .. 256
 // columns); dense weights take 1.25 ns a column but 0.2 at least; a tile more costs about 1.  The last tile's values are stored with nothing
-// behind them to hide it: 30 ns a column (dense 64 x 64 weights: 8.4 us for 64
-// columns, 12.6 for 512 in tiles of 256; dense 1024 x 1024 over 128 columns 14.5 us as 4 tiles of 128, 11.7 for a kernel with narrower ones).  Two halves of K
-// add into a zeroed dst: that much more traffic, at 1.5 TB/s, and a launch more.  Widths are N / 1, N / 2, ... rounded up to 16.
+// behind them to hide it: 12 ns a column.  Parts of K meet for 1.6 + 0.2 a part + 8 ns a column (1024 x 4096 q4_K over 20 columns: 22.5 us in one part, 15.3, 13.0,
+// 11.0, 10.8, 10.1, 10.2, 9.3 in two .. eight), and a cluster takes one tile, so that there are no more tiles than clusters.  Widths are N / 1, N / 2, ...
+// rounded up to 16.
+
 struct PairPlan { int bn, ksplit, n_tiles_n; };
 static inline double pair_step_us(double a, double b) { const double a3 = a * a * a, b3 = b * b * b; return sqrt(cbrt(a3 * a3 + b3 * b3)); }
-static inline PairPlan mmq_pair_plan(int64_t M, int64_t N, int64_t K, int n_batch, int pairs, double unpack) {
+// stages of the ring beside `raw` bytes; a tile's parts lie in them when they meet
+static inline int pair_stages(int bn, int steps, int raw) {
+    const int n = (PAIR_SMEM - 1024 - raw) / (steps * (MQ_BM * MQ_BK * 2 + bn * MQ_BK));
+    return n > PAIR_MAX_STAGES ? PAIR_MAX_STAGES : n;
+}
+static inline bool pair_parts_fit(int bn, int steps, int raw) { return pair_stages(bn, steps, raw) * steps * (MQ_BM * MQ_BK * 2 + bn * MQ_BK) >= bn * MQ_BM * 4; }
+// clusters[ks]: clusters of ks pairs that the device holds at once
+static inline PairPlan mmq_pair_plan(int64_t M, int64_t N, int64_t K, int n_batch, const int *clusters, double unpack, int unit, int steps_stage, int raw) {
     PairPlan best = {256, 1, 1};
     double best_cost = -1;
-    const unsigned mt = (unsigned)((M + 255) / 256), n = (unsigned)N, np = (unsigned)pairs;  // (32-bit: the divisions of up to 30 candidates are host time of each call)
-    const double steps = (double)(K / MQ_BK), halves = 2.0 + (double)M * N * 4 / 1.5e6;
-    const int ks_max = n_batch > 1 || K < 2048 ? 1 : 2;
+    const unsigned mt = (unsigned)((M + 255) / 256), n = (unsigned)N, np = (unsigned)clusters[1];  // (32-bit: the divisions of up to 30 candidates are host time of each call)
+    const int units = (int)(K / MQ_BK / unit);
     for (unsigned parts = (n + 255) / 256, last = (n + 31) / 32; parts <= last; parts++) {
         const unsigned even = ((n + parts - 1) / parts + 15) / 16 * 16, bn = even < 32 ? 32 : even, nt = (n + bn - 1) / bn;
         const double dense = 1.25e-3 * bn < 0.2 ? 0.2 : 1.25e-3 * bn, step = unpack > 0 ? pair_step_us(unpack, 1.83e-3 * bn) : dense;
-        for (int ks = 1; ks <= ks_max; ks++) {
-            const uint64_t tiles = (uint64_t)mt * nt * n_batch * ks;
+        const uint64_t tiles = (uint64_t)mt * nt * n_batch;
+        for (int ks = 1; ks <= PAIR_MAX_SPLIT && ks <= units; ks++) {
+            if (ks > 1 && (tiles > (uint64_t)clusters[ks] || !pair_parts_fit((int)bn, steps_stage, raw))) continue;
             const double waves = tiles <= np ? 1.0 : (double)((tiles + np - 1) / np);
-            const double cost = waves * (steps / ks * step + 1.0) + 0.03 * bn + (ks == 2 ? halves : 0.0);
+            const double cost = waves * ((units + ks - 1) / ks * unit * step + 1.0) + (ks == 1 ? 0.012 * bn : 1.6 + 0.2 * ks + 0.008 * bn);
             if (best_cost < 0 || cost < 0.98 * best_cost) { best_cost = cost; best = {(int)bn, ks, (int)nt}; }
         }
     }
     return best;
 }
 
-// pairs of CTAs that the device can hold at once (the same for every instantiation: one CTA an SM by its shared memory)
-static int mmq_pairs() { return sm_count() / 2; }
+// what the device holds at once, one CTA an SM: clusters of 1 .. PAIR_MAX_SPLIT pairs
+struct PairDevice { std::atomic<bool> known{false}; int clusters[PAIR_MAX_SPLIT + 1]; };
 
 // microseconds a K step of 64 takes while unpacking is the slower side: one tile of 256 rows on each of 74 pairs, 64 columns, from the difference
 // between 8192 and 4096 values a row
@@ -669,13 +762,32 @@ template <int TYPE> constexpr double pair_unpack_us() {
 template <int TYPE, bool GROUPED>
 static int mmq_pair_launch(const MmqParams &q, int64_t n_pad, int64_t w_rows_per_product, int64_t max_tiles_n, int64_t grouped_bn, cudaStream_t st) {
     const auto kern = mmq_pair_kernel<TYPE, GROUPED>;
-    static bool attr_set_dev[16] = {};  // cudaFuncSetAttribute is per device
+    cudaLaunchConfig_t cfg = {};
+    cfg.blockDim = dim3(pair_threads<TYPE>());
+    cfg.dynamicSmemBytes = PAIR_SMEM;
+    cfg.stream = st;
+    cudaLaunchAttribute at[2];  // (as launch_chained, in clusters)
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.y = 1;
+    at[0].val.clusterDim.z = 1;
+    at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    static PairDevice devices[16];  // (attributes and what fits are a device's; two threads that come first find the same)
     int cur_dev = 0;
     B200_CUDA_TRY(cudaGetDevice(&cur_dev));
-    bool &attr_set = attr_set_dev[cur_dev & 15];
-    if (!attr_set) {
+    PairDevice &dev = devices[cur_dev & 15];
+    if (!dev.known.load(std::memory_order_acquire)) {
         B200_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, PAIR_SMEM));
-        attr_set = true;
+        B200_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+        dev.clusters[1] = sm_count() / 2;
+        for (int ks = 2; ks <= PAIR_MAX_SPLIT; ks++) {
+            cfg.gridDim = dim3((unsigned)(2 * ks));
+            at[0].val.clusterDim.x = (unsigned)(2 * ks);
+            cfg.numAttrs = 1;
+            if (cudaOccupancyMaxActiveClusters(&dev.clusters[ks], kern, &cfg) != cudaSuccess) { dev.clusters[ks] = 0; cudaGetLastError(); }
+        }
+        dev.known.store(true, std::memory_order_release);
     }
     PairParams p;
     p.q = q;
@@ -690,15 +802,13 @@ static int mmq_pair_launch(const MmqParams &q, int64_t n_pad, int64_t w_rows_per
         p.n_tiles_n = 0;
         p.q.ksplit = 1;
     } else {
-        const PairPlan pl = mmq_pair_plan(q.M, q.N, q.K, q.n_batch, mmq_pairs(), pair_unpack_us<TYPE>());
+        const PairPlan pl = mmq_pair_plan(q.M, q.N, q.K, q.n_batch, dev.clusters, pair_unpack_us<TYPE>(), TYPE == B200_TYPE_BF16 ? 1 : 4, pair_steps<TYPE>(), raw_bytes(TYPE));
         p.bn = pl.bn;
         p.box = pl.bn / 2;
         p.n_tiles_n = pl.n_tiles_n;
         p.q.ksplit = pl.ksplit;
     }
-    const int stage = pair_steps<TYPE>() * (MQ_BM * MQ_BK * 2 + p.bn * MQ_BK);
-    p.stages = (PAIR_SMEM - 1024 - raw_bytes(TYPE)) / stage;
-    if (p.stages > PAIR_MAX_STAGES) p.stages = PAIR_MAX_STAGES;
+    p.stages = pair_stages(p.bn, pair_steps<TYPE>(), raw_bytes(TYPE));
     TmapBytes tmA = {}, tmB;
     if (TYPE == B200_TYPE_BF16) {
         const int64_t products = GROUPED ? q.n_expert : q.n_batch;
@@ -707,25 +817,11 @@ static int mmq_pair_launch(const MmqParams &q, int64_t n_pad, int64_t w_rows_per
     }
     const int rc = encode_rows(tmB, q.Xb, q.K, n_pad * (q.n_batch > 1 ? q.n_batch : 1), (size_t)q.K * 2, p.box);
     if (rc != B200_OK) return rc;
-    if (p.q.ksplit > 1) {
-        if (q.dst_stride == q.M) B200_CUDA_TRY(cudaMemsetAsync(q.dst, 0, (size_t)q.M * q.N * sizeof(float), st));
-        else B200_CUDA_TRY(cudaMemset2DAsync(q.dst, (size_t)q.dst_stride * sizeof(float), 0, (size_t)q.M * sizeof(float), (size_t)q.N, st));
-    }
-    const int64_t tiles = (int64_t)p.n_tiles_m * (GROUPED ? max_tiles_n : p.n_tiles_n) * (GROUPED ? 1 : q.n_batch > 1 ? q.n_batch : p.q.ksplit);
+    const int64_t tiles = (int64_t)p.n_tiles_m * (GROUPED ? max_tiles_n : p.n_tiles_n * (int64_t)q.n_batch);
     if (tiles > 0x3fffffff) { set_error("b200_mul_mat_q: too many tiles"); return B200_ERR_UNSUPPORTED; }
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)(2 * (tiles < mmq_pairs() ? tiles : mmq_pairs())));
-    cfg.blockDim = dim3(pair_threads<TYPE>());
-    cfg.dynamicSmemBytes = PAIR_SMEM;
-    cfg.stream = st;
-    cudaLaunchAttribute at[2];  // (as launch_chained, in pairs)
-    at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = 2;
-    at[0].val.clusterDim.y = 1;
-    at[0].val.clusterDim.z = 1;
-    at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[1].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = at;
+    const int clusters = dev.clusters[p.q.ksplit];
+    cfg.gridDim = dim3((unsigned)(2 * p.q.ksplit * (tiles < clusters ? tiles : clusters)));
+    at[0].val.clusterDim.x = (unsigned)(2 * p.q.ksplit);
     cfg.numAttrs = 2;
     B200_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, tmA, tmB, p));
     return B200_OK;

@@ -49,6 +49,37 @@ def test_edges_of_tiles(t, K, M, N):
     assert rel(got[:, :M], expected(t, w, x, K)) < 4e-3
 
 
+@pytest.mark.parametrize("t", [Q4_K, Q6_K, Q4_0, BF16])
+@pytest.mark.parametrize("K,M,N", [(2048, 1, 9), (2560, 257, 70), (1280, 515, 31), (5120, 1000, 199), (11008, 300, 17), (4096, 4096, 40), (4096, 2048, 300)])
+def test_parts_of_k(t, K, M, N):
+    """Few tiles and many K steps: a tile's parts, of unequal size, are added in one order whatever the run; ragged rows, and a result whose rows start at odd places."""
+    rng = np.random.default_rng(K + M + N + t)
+    x = rng.standard_normal((N, K)).astype(np.float32)
+    if t == BF16:
+        bits = (rng.standard_normal((M, K)).astype(np.float32).view(np.uint32) >> 16).astype(np.uint16)
+        w, want = bits.view(np.uint8), x.astype(np.float64) @ (bits.astype(np.uint32) << 16).view(np.float32).astype(np.float64).T
+    else:
+        w = random_blocks(rng, t, M, K)
+        want = expected(t, w, x, K)
+    got = product(t, w, x, K, M, dst_stride=M + 5)
+    assert np.isnan(got[:, M:]).all()
+    assert rel(got[:, :M], want) < 4e-3
+    for _ in range(3):
+        assert np.array_equal(product(t, w, x, K, M), got[:, :M])
+
+
+def test_experts_without_a_valid_pair():
+    """No tile at all: nothing is stored, and the launch ends."""
+    K, M, used, n_expert, T = 512, 300, 2, 4, 40
+    rng = np.random.default_rng(1)
+    w, b = random_blocks(rng, Q4_K, n_expert * M, K), rng.standard_normal((T, 1, K)).astype(np.float32)
+    need = lib().b200_mul_mat_id_q_workspace_bytes(Q4_K, K, M, used, T, n_expert)
+    dw, db, di = H.DeviceBuffer.from_numpy(w.reshape(-1)), H.DeviceBuffer.from_numpy(b), H.DeviceBuffer.from_numpy(np.full((T, used), -1, np.int32))
+    dd, ws, rs = H.DeviceBuffer.from_numpy(np.full((T, used, M), 7.0, np.float32)), H.DeviceBuffer(need + 512), row_size(Q4_K, K)
+    check(lib().b200_mul_mat_id_q(Q4_K, dw.ptr, rs, rs * M, n_expert, di.ptr, used, db.ptr, K, K, dd.ptr, M, used * M, K, M, used, 1, T, (ws.ptr + 255) // 256 * 256, need, None))
+    assert (dd.to_numpy(np.float32, (T, used, M)) == 7.0).all()
+
+
 @pytest.mark.parametrize("t", [Q6_K, Q8_0, Q4_0, Q2_K, Q3_K, Q5_0, Q5_1, IQ4_XS])
 @pytest.mark.parametrize("offset,pad", [(0, 0), (2, 0), (6, 2), (14, 10), (4, 6), (8, 12)])
 def test_rows_at_any_even_byte(t, offset, pad):
@@ -95,7 +126,7 @@ sys.path[:0] = [{root!r}, {tests!r}]
 import koboldcpp_b200.host as H, orc as O
 from koboldcpp_b200.lib import Q4_K, check, lib, row_size
 from koboldcpp_b200.llama import random_blocks
-K, M, N = 1792, 19500, 200
+K, M, N = {shape}
 rng = np.random.default_rng(0)
 w, x = random_blocks(rng, Q4_K, M, K), rng.standard_normal((N, K)).astype(np.float32)
 want = x.astype(np.float64) @ np.stack([O.dequantize(Q4_K, r, K) for r in w]).astype(np.float64).T
@@ -119,10 +150,10 @@ assert not stored.all()
 """
 
 
-def give_up(more="", limits=(0,)):
+def give_up(more="", limits=(0,), shape=(1792, 19500, 200)):
     """The statements above in a process of their own (that a product gave up is remembered for the life of a process), then `more`."""
     tests = Path(__file__).resolve().parent
-    r = subprocess.run([sys.executable, "-c", GIVE_UP.format(root=str(tests.parent), tests=str(tests), more=more, limits=limits)], capture_output=True, text=True, timeout=300)
+    r = subprocess.run([sys.executable, "-c", GIVE_UP.format(root=str(tests.parent), tests=str(tests), more=more, limits=limits, shape=shape)], capture_output=True, text=True, timeout=300)
     assert r.returncode == 0, r.stdout[-2000:] + r.stderr[-2000:]
 
 
@@ -130,6 +161,11 @@ def test_what_is_stored_is_right_when_waits_run_out():
     """With a limit of some cycles the pipeline gives up at its start, in its middle or not at all, in either CTA of a pair: every value is the right one, to
     the bit, or was never written."""
     give_up(limits=(100_000, 20_000, 6_000, 2_000, 700, 200, 0))
+
+
+def test_parts_of_k_are_stored_together_or_not_at_all():
+    """The same where the pairs of a cluster take parts of K: two tiles of 256 rows, long rows (the wait for an accumulator is one of 20 us)."""
+    give_up(limits=(100_000, 50_000, 20_000, 9_000, 6_000, 2_000, 200, 0), shape=(32768, 300, 100))
 
 
 def test_status_is_set_for_a_caller_without_a_backend():
