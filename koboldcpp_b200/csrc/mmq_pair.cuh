@@ -51,6 +51,7 @@ struct PairParams {
     int bn;                      // columns of a tile (grouped: at most), a multiple of 16; grouped: of 32
     int box;                     // activation rows of one TMA box: all of the CTA's, grouped: 16
     int stages;
+    int share;                   // the last tile of a pair is stored by all warps (of tiles of up to 32 columns, one step of a warp, there is nothing to share; a part of K meets the others)
     int n_tiles_n, n_tiles_m;    // n_tiles_n of the grouped form: read from the tile table
     int *timeout;
 };
@@ -359,6 +360,37 @@ template <int TYPE> __host__ __device__ constexpr int pair_steps() { return TYPE
 template <int TYPE>
 __host__ __device__ constexpr int pair_threads() { return 32 * (6 + (TYPE == B200_TYPE_BF16 ? 8 : PAIR_PRODUCERS)); }
 
+// ===== 32 columns of an accumulator, and every `step`-th after them, to the result: a warp's 32 rows
+template <bool GROUPED>
+__device__ __forceinline__ void pair_store(const PairParams &p, const PairTile &ti, unsigned acc, int rank, int c0, int step, bool ok) {
+    const int quarter = (int)(threadIdx.x >> 5) & 3, lane = threadIdx.x & 31, cols = (int)(ti.n_end - ti.n0);
+    const int64_t m = ti.m0 + rank * MQ_BM + quarter * 32 + lane;
+    const bool row_ok = m < p.q.M && ok;
+    float *drow = p.q.dst + m + (GROUPED ? 0 : ti.product * p.q.dst_batch);
+    const int *row_dst = behind(p.q.row_dst);
+#pragma unroll 1
+    for (; c0 < cols; c0 += step) {
+        float v[32];
+        // scatter: sorted row -> (token, slot).  A lane asks for one of the 32 columns' places: in front of each store a load would wait for its turn
+        const int place = GROUPED && c0 + lane < cols ? ld_behind(row_dst + ti.n0 + c0 + lane) : 0;
+        __syncwarp();
+        tmem_ld32(acc + ((unsigned)(quarter * 32) << 16) + (unsigned)c0, v);
+        if constexpr (GROUPED) {
+#pragma unroll
+            for (int j = 0; j < 32; j++) {
+                const int to = __shfl_sync(0xffffffffu, place, j);
+                if (row_ok && c0 + j < cols) drow[(int64_t)to] = v[j];
+            }
+        } else if (row_ok) {
+#pragma unroll
+            for (int j = 0; j < 32; j++) {
+                if (c0 + j >= cols) continue;
+                drow[(ti.n0 + c0 + j) * p.q.dst_stride] = v[j];
+            }
+        }
+    }
+}
+
 // ===== the parts of a tile meet.  Each CTA lays its accumulators, [column][128 rows], over its operand ring, which its MMAs have left; behind the
 // cluster's barrier CTA (split, rank) reads columns split / ksplit of them from every CTA with its rows and adds them in the order of K.
 // All threads of the cluster come here.
@@ -416,7 +448,8 @@ __device__ __forceinline__ void pair_merge(const PairParams &p, const PairTile &
     }
 }
 
-template <int TYPE, bool GROUPED>
+// SHARE: p.share may be set.  (Experts of a few rows have a kernel without that code, in whose loops it cost 2 %: 10 tokens, 3 of 8 experts of 2048 x 7936 q4_K, 140.6 -> 143.6 us.)
+template <int TYPE, bool GROUPED, bool SHARE>
 __global__ void __launch_bounds__(pair_threads<TYPE>(), 1) mmq_pair_kernel(const __grid_constant__ TmapBytes tmA, const __grid_constant__ TmapBytes tmB, const __grid_constant__ PairParams p) {
     constexpr bool DENSE = TYPE == B200_TYPE_BF16;
     constexpr int NP = DENSE ? 0 : PAIR_PRODUCERS, SK = pair_steps<TYPE>(), A_STEP = MQ_BM * MQ_BK * 2, A_BYTES = SK * A_STEP, UNIT = DENSE ? 1 : 4;
@@ -428,7 +461,8 @@ __global__ void __launch_bounds__(pair_threads<TYPE>(), 1) mmq_pair_kernel(const
     __shared__ volatile int failed, part_there;
     const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31, tid = threadIdx.x;
     // a cluster is ksplit pairs: its pairs take parts of K of the same tile
-    const int in_cluster = (int)cluster_rank(), rank = in_cluster & 1, leader = in_cluster & ~1, split = in_cluster >> 1, ksplit = GROUPED ? 1 : p.q.ksplit;
+    const int in_cluster = (int)cluster_rank(), rank = GROUPED ? in_cluster : in_cluster & 1, leader = GROUPED ? 0 : in_cluster & ~1, split = GROUPED ? 0 : in_cluster >> 1,
+              ksplit = GROUPED ? 1 : p.q.ksplit;
     const int pair = (int)blockIdx.x / (2 * ksplit), n_pairs = (int)gridDim.x / (2 * ksplit);
     const unsigned short both = (unsigned short)(3u << leader);
     const long long limit = p.q.wait_limit;
@@ -629,64 +663,38 @@ __global__ void __launch_bounds__(pair_threads<TYPE>(), 1) mmq_pair_kernel(const
                 if (++s == S) { s = 0; ph ^= 1u; }
             }
         }
-    }
-    // ===== epilogue: four warps, one for each 32 of this CTA's 128 rows (TMEM lanes 32 * (warp % 4) ..); of the last tile, behind which nothing is left to
-    // do, the producers (dense weights: the warps without another role) store their share of the columns
-    if (ksplit == 1 && warp != NP && warp != NP + 1) {
-        constexpr int SETS = (pair_threads<TYPE>() / 32 - 2) / 4;
-        const bool always = warp >= NP + 2 && warp < NP + 6;
-        const int set = always ? 0 : DENSE ? (warp - 2) / 4 : 1 + warp / 4;
+    } else if (warp < NP + 6 && ksplit == 1) {
+        // ===== epilogue: TMEM lanes 32 * (warp % 4) .. of this CTA's 128 rows; of the last tile only the wait for it, if all share it
         bool ok = true;
         int buf = 0;
         unsigned ph = 0;
-        const int quarter = warp & 3;
         const unsigned acc_remote = cluster_addr(acc_empty0, leader);
-        const int *row_dst = behind(p.q.row_dst);
-        for (int t = always || pair >= n_tiles ? pair : pair + (n_tiles - 1 - pair) / n_pairs * n_pairs; t < n_tiles; t += n_pairs) {
+        for (int t = pair; t < n_tiles; t += n_pairs) {
             const PairTile ti = pair_tile<GROUPED>(p, t, nt, UNIT, split);
-            const bool last = t + n_pairs >= n_tiles;
-            if (always) {
-                ok = __all_sync(0xffffffffu, ok && pair_wait<20>(acc_full0 + 8u * buf, ph, &failed, limit));
-                if (last && !ok) part_there = 0;
-            } else {
-                buf = (t - pair) / n_pairs & 1;
-            }
-            if (last) {
-                asm volatile("bar.sync 1, %0;" ::"n"(SETS * 128) : "memory");
-                if (!always) ok = part_there != 0;
-            }
+            ok = __all_sync(0xffffffffu, ok && pair_wait<200>(acc_full0 + 8u * buf, ph, &failed, limit));
             tc_fence_after();
-            const int64_t m = ti.m0 + rank * MQ_BM + quarter * 32 + lane;
-            const bool row_ok = m < p.q.M && ok;
-            float *drow = p.q.dst + m + (GROUPED ? 0 : ti.product * p.q.dst_batch);
-            const int cols = (int)(ti.n_end - ti.n0);
-#pragma unroll 1
-            for (int c0 = last ? 32 * set : 0; c0 < cols; c0 += last ? 32 * SETS : 32) {
-                float v[32];
-                // scatter: sorted row -> (token, slot).  A lane asks for one of the 32 columns' places: in front of each store a load would wait for its turn
-                const int place = GROUPED && c0 + lane < cols ? ld_behind(row_dst + ti.n0 + c0 + lane) : 0;
-                __syncwarp();
-                tmem_ld32(tmem_base + (unsigned)buf * 256u + ((unsigned)(quarter * 32) << 16) + (unsigned)c0, v);
-                if constexpr (GROUPED) {
-#pragma unroll
-                    for (int j = 0; j < 32; j++) {
-                        const int to = __shfl_sync(0xffffffffu, place, j);
-                        if (row_ok && c0 + j < cols) drow[(int64_t)to] = v[j];
-                    }
-                } else if (row_ok) {
-#pragma unroll
-                    for (int j = 0; j < 32; j++) {
-                        if (c0 + j >= cols) continue;
-                        drow[(ti.n0 + c0 + j) * p.q.dst_stride] = v[j];
-                    }
-                }
+            if (SHARE && p.share && t + n_pairs >= n_tiles) {
+                if (!ok) part_there = 0;
+                break;
             }
+            pair_store<GROUPED>(p, ti, tmem_base + (unsigned)buf * 256u, rank, 0, 32, ok);
             tc_fence_before();
             __syncwarp();
-            if (always && lane == 0 && ok) mbar_arrive_remote(acc_remote + 8u * buf);
+            if (lane == 0 && ok) mbar_arrive_remote(acc_remote + 8u * buf);
             buf ^= 1;
             if (buf == 0) ph ^= 1u;
         }
+    }
+    // ===== the last tile, behind which nothing is left to do: its columns are shared by the epilogue and the producers (dense weights: the warps without another role)
+    if (SHARE && p.share && warp != NP && warp != NP + 1 && pair < n_tiles) {
+        constexpr int SETS = (pair_threads<TYPE>() / 32 - 2) / 4;
+        const int before = (n_tiles - 1 - pair) / n_pairs;  // tiles of this pair in front of it
+        const PairTile ti = pair_tile<GROUPED>(p, pair + before * n_pairs, nt, UNIT, split);
+        __syncwarp();
+        asm volatile("bar.sync 1, %0;" ::"n"(SETS * 128) : "memory");
+        tc_fence_after();
+        const int set = warp < NP ? 1 + warp / 4 : (warp - NP - 2) / 4;
+        pair_store<GROUPED>(p, ti, *const_cast<volatile unsigned *>(&tmem_base_s) + (unsigned)(before & 1) * 256u, rank, 32 * set, 32 * SETS, part_there != 0);
     }
     __syncwarp();
     if (warp < NP || warp == NP + 1) pair_await();
@@ -759,9 +767,12 @@ template <int TYPE> constexpr double pair_unpack_us() {
     }
 }
 
-template <int TYPE, bool GROUPED>
+template <int TYPE, bool GROUPED, bool SHARE = true>
 static int mmq_pair_launch(const MmqParams &q, int64_t n_pad, int64_t w_rows_per_product, int64_t max_tiles_n, int64_t grouped_bn, cudaStream_t st) {
-    const auto kern = mmq_pair_kernel<TYPE, GROUPED>;
+    if constexpr (GROUPED && SHARE) {
+        if (q.N <= 32 * (int64_t)q.n_expert) return mmq_pair_launch<TYPE, GROUPED, false>(q, n_pad, w_rows_per_product, max_tiles_n, grouped_bn, st);
+    }
+    const auto kern = mmq_pair_kernel<TYPE, GROUPED, SHARE>;
     cudaLaunchConfig_t cfg = {};
     cfg.blockDim = dim3(pair_threads<TYPE>());
     cfg.dynamicSmemBytes = PAIR_SMEM;
@@ -801,12 +812,14 @@ static int mmq_pair_launch(const MmqParams &q, int64_t n_pad, int64_t w_rows_per
         p.box = 16;
         p.n_tiles_n = 0;
         p.q.ksplit = 1;
+        p.share = SHARE;
     } else {
         const PairPlan pl = mmq_pair_plan(q.M, q.N, q.K, q.n_batch, dev.clusters, pair_unpack_us<TYPE>(), TYPE == B200_TYPE_BF16 ? 1 : 4, pair_steps<TYPE>(), raw_bytes(TYPE));
         p.bn = pl.bn;
         p.box = pl.bn / 2;
         p.n_tiles_n = pl.n_tiles_n;
         p.q.ksplit = pl.ksplit;
+        p.share = pl.ksplit == 1 && pl.bn > 32;
     }
     p.stages = pair_stages(p.bn, pair_steps<TYPE>(), raw_bytes(TYPE));
     TmapBytes tmA = {}, tmB;
