@@ -429,22 +429,21 @@ static int dispatch_cols(MmvqParams &p, int N, cudaStream_t st, bool pdl) {
             if (rc != -1000) return rc;
         }
     }
-    // Several columns of one activation matrix: the integer tensor cores, whose cost hardly grows with the columns.  The line lies where the dp4a form
-    // begins to lose over all measured shapes (K 512 .. 14336, M 64 .. 32000), dp4a -> tensor: q4_K 4096 x 14336 at 4 columns 24.2 -> 17.7 us, at 8
-    // 40.5 -> 19.9; q5_K 24.5 -> 20.1 and 41.4 -> 22.4; q6_K, whose rows lie at any even byte, 27.0 -> 27.6 at 4, 35.1 -> 28.4 at 6.  Few rows leave
-    // each warp one block: below 512 rows dp4a is ahead at 4 columns (q4_K 2048 x 256 7.3 -> 8.3, q5_K 8.0 -> 8.3), level at 5 and 6 (q4_K 2048 x 64 8.5 -> 8.4,
-    // q6_K 9.6 -> 10.5) and behind at 7 and 8 (q4_K 10.5 -> 8.5, q5_K 10.5 -> 8.5).  How K is cut, and with it the last bits, follows from the
-    // launch's rows.
-    if constexpr (TYPE == B200_TYPE_Q4_K || TYPE == B200_TYPE_Q5_K || TYPE == B200_TYPE_Q6_K) {
-        bool same_x = p.ids == nullptr;
+    // Several columns of one activation matrix: the integer tensor cores, whose cost hardly grows with the columns; dp4a spends 8 instructions a column and 32 weights.
+    // dp4a -> tensor, us, at 2 / 4 / 8 columns: 22016 x 4096 q4_0 25.6 -> 18.8 / 39.1 -> 20.4 / - ; 32000 x 2048 q8_0 25.6 -> 17.5 / 37.2 -> 18.9 / 64.7 -> 21.3;
+    // 32000 x 2048 q4_K 22.8 -> 14.1 at 2; 5120 x 13824 q6_K 36.9 -> 26.9 at 4; 2048 x 2048 q4_0 4.5 -> 4.1 / 6.7 -> 4.7 / 12.1 -> 5.8; 256 x 256 3.7 -> 3.5 / 5.5 -> 3.6 /
+    // 9.5 -> 3.9.  Where it loses are two columns of few and long rows, which leave most warps without a tile: 256 x 2048 3.7 -> 3.8 (q6_K 4.3), 1024 x 4096 q4_0 4.8 -> 5.2,
+    // q4_K 4.7 -> 5.4, q8_0 5.1 -> 6.9.  The choice does not look at the rows all the same, so that a row's bits do not depend on the launch it is part of.
+    if constexpr (TYPE == B200_TYPE_Q4_0 || TYPE == B200_TYPE_Q8_0 || TYPE == B200_TYPE_Q4_K || TYPE == B200_TYPE_Q5_K || TYPE == B200_TYPE_Q6_K) {
+        bool same_x = p.ids == nullptr && p.K % 256 == 0;
         for (int j = 1; j < p.n_jobs; j++) same_x = same_x && p.jobs[j].X == p.jobs[0].X;
-        if (N >= (TYPE == B200_TYPE_Q6_K ? 6 : 4) && (p.total_rows >= 512 || N >= 7) && same_x && (!multi || N <= 4)) {
+        if (N >= 2 && same_x && (!multi || N <= 4)) {
             int rc = B200_OK;
             if (multi) {  // (several jobs have a limit of rows, whichever kernel serves them)
                 MmvqPlan pl;
                 rc = mmvq_plan<TYPE>(p, N, multi, pl);
             }
-            if (!rc) rc = launch_mmvq_mma<TYPE>(p, N, st, pdl);
+            if (!rc) rc = N <= 2 ? launch_mmvq_mma<TYPE, 2>(p, N, st, pdl) : N <= 4 ? launch_mmvq_mma<TYPE, 4>(p, N, st, pdl) : launch_mmvq_mma<TYPE, 8>(p, N, st, pdl);
             if (rc != -1000) return rc;
         }
     }

@@ -26,9 +26,30 @@ def test_columns(t, K, M, N):
     assert close(H.mul_mat_vec_q(t, w, x, K, M), O.mul_mat_q8_1(t, w, x, K, M))
 
 
+@pytest.mark.parametrize("t", [Q4_0, Q8_0, Q4_K, Q5_K, Q6_K])
+@pytest.mark.parametrize("K,M", [(256, 1), (256, 17), (512, 640), (1280, 33), (2304, 527), (4096, 300), (8192, 64), (13824, 130)])
+@pytest.mark.parametrize("N", [2, 3, 4, 5, 6, 7, 8])
+def test_packed_columns(t, K, M, N):
+    """Two, four or eight columns to a tile; columns of very different size, one of zeros, and one with a single value that is not."""
+    rng = np.random.default_rng(K + M + N + t)
+    w, x = random_blocks(rng, t, M, K), rng.standard_normal((N, K)).astype(np.float32)
+    x *= np.float32(10.0) ** rng.integers(-3, 4, (N, 1))
+    x[N // 2] = 0
+    if N > 3:
+        x[1] = 0
+        x[1, K - 1] = 3
+    got, want = H.mul_mat_vec_q(t, w, x, K, M), O.mul_mat_q8_1(t, w, x, K, M)
+    for n in range(N):
+        if not want[n].any():
+            assert (got[n] == 0).all()
+        else:
+            assert close(got[n], want[n]), n
+
+
+@pytest.mark.parametrize("t,N", [(Q6_K, 6), (Q6_K, 2), (Q6_K, 3), (Q4_0, 2), (Q4_0, 4), (Q4_0, 7), (Q8_0, 2), (Q8_0, 3), (Q8_0, 8)])
 @pytest.mark.parametrize("offset,pad", [(2, 0), (6, 2), (14, 10), (8, 4)])
-def test_rows_at_any_even_byte(offset, pad):
-    t, K, M, N = Q6_K, 1024, 515, 6
+def test_rows_at_any_even_byte(t, N, offset, pad):
+    K, M = 1024, 515
     rng = np.random.default_rng(offset)
     w, x = random_blocks(rng, t, M, K), rng.standard_normal((N, K)).astype(np.float32)
     rs = row_size(t, K)
@@ -40,9 +61,10 @@ def test_rows_at_any_even_byte(offset, pad):
     assert close(dd.to_numpy(np.float32, (N, M)), O.mul_mat_q8_1(t, w, x, K, M))
 
 
-@pytest.mark.parametrize("t", [Q4_K, Q5_K])
-def test_jobs_with_norm_and_residual(t):
-    K, N, Ms, eps = 1280, 4, [100, 16, 433], 1e-5
+@pytest.mark.parametrize("t", [Q4_0, Q8_0, Q4_K, Q5_K, Q6_K])
+@pytest.mark.parametrize("K,N", [(1280, 4), (1280, 3), (1280, 2), (11008, 3)])
+def test_jobs_with_norm_and_residual(t, K, N):
+    Ms, eps = [100, 16, 433], 1e-5
     rng = np.random.default_rng(N + t)
     ws = [random_blocks(rng, t, M, K) for M in Ms]
     x, nw = rng.standard_normal((N, K)).astype(np.float32), rng.standard_normal(K).astype(np.float32)
