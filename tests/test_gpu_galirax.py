@@ -87,6 +87,22 @@ def test_qkv_store_bias_norm_rotation_cells(Hh, G, D, V, dims, extra):
     assert (kc[untouched] == 7.0).all() and (vc[untouched] == 7.0).all() and (kc[:, G * D:] == 7.0).all() and (vc[:, G * V:] == 7.0).all()
 
 
+@pytest.mark.parametrize("Hh,G,D,V,dims,extra", [(4, 2, 16, 24, 8, True), (5, 5, 10, 6, 10, False), (2, 1, 64, 64, 64, True), (6, 2, 96, 40, 0, True), (1, 1, 7, 5, 2, False)])
+def test_qkv_store_of_a_long_batch(Hh, G, D, V, dims, extra):
+    """More than 64 tokens share a table of sines and cosines among the heads: the values of the same tokens in smaller batches, but for the order of a norm's sum and the
+    rounding of two products (2^-24 each)."""
+    rng = np.random.default_rng(Hh * D + V)
+    T, eps = 70, 1e-5
+    q, k, v = rng.standard_normal((T, Hh, D)), rng.standard_normal((T, G, D)), rng.standard_normal((T, G, V))
+    pos, cells = rng.integers(0, 5000, T), rng.permutation(T)
+    rot = {"base": 3000.0, "dims": dims, "scaling": {"factor": 8.0, "low": 1.0, "high": 4.0, "original": 64}}
+    vecs = {"q.b": rng.standard_normal(Hh * D), "k.norm": 1 + 0.3 * rng.standard_normal(G * D)} if extra else {}
+    whole = run_qkv_store(q, k, v, vecs, pos, cells, rot, T, eps)
+    for part in (slice(0, 64), slice(64, T)):
+        gq, kc, vc = run_qkv_store(q[part], k[part], v[part], vecs, pos[part], cells[part], rot, T, eps)
+        assert rel(whole[0][part], gq) < 3e-7 and rel(whole[1][cells[part]], kc[cells[part]]) < 3e-7 and np.array_equal(vc[cells[part]], whole[2][cells[part]])
+
+
 def run_sink_attn(q, kc, vc, cell_seq, cell_pos, tok_seq, tok_pos, sink, scale, G, window=0, keep_first=0, bf16=0):
     T, Hh, D = q.shape
     V = vc.shape[1] // G
