@@ -79,6 +79,32 @@ def test_short_convolution_whole_and_in_portions(Cn, taps, portions, act):
     assert rel(run_short_conv(u, w, bias, [T], taps, act), want) < 3e-6
 
 
+@pytest.mark.parametrize("Cn,taps,act", [(4096, 4, 1), (4098, 3, 0), (3584, 7, 1), (5000, 2, 0)])
+def test_short_convolution_of_a_large_batch(Cn, taps, act):
+    """Two channels a thread where the rows allow it: the values, to the bit, of rows that do not (an odd stride); a fresh sequence, one that goes on, and one token."""
+    rng = np.random.default_rng(Cn)
+    counts, slots, fresh = [337, 1, 450], [2, 0, 1], [1, 0, 0]
+    T = sum(counts)
+    u, w, bias = rng.standard_normal((T, Cn)).astype(np.float32), rng.standard_normal((Cn, taps)).astype(np.float32), rng.standard_normal(Cn).astype(np.float32)
+    before = rng.standard_normal((3, (taps - 1) * Cn)).astype(np.float32)
+    info = dev(seq_info([(sum(counts[:i]), counts[i], slots[i], fresh[i]) for i in range(3)]), np.int32)
+    dw, db, got, tails = dev(w), dev(bias), [], []
+    for pad in (2, 1):
+        dx, dy, tail = dev(np.pad(u, ((0, 0), (0, pad)))), H.DeviceBuffer(4 * T * (Cn + pad) + 256), dev(before)
+        a = ShortConvArgs(x=dx.ptr, x_stride=Cn + pad, bias=db.ptr, w=dw.ptr, seq_info=info.ptr, n_seq=3, tail=tail.ptr, slot_stride=(taps - 1) * Cn, dst=dy.ptr, dst_stride=Cn + pad,
+                          channels=Cn, taps=taps, act=act, n_tokens=T)
+        check(lib().b200_op_short_conv(C.byref(a), None))
+        got.append(dy.to_numpy(np.float32, (T, Cn + pad))[:, :Cn])
+        tails.append(tail.to_numpy(np.float32, (3, (taps - 1) * Cn)))
+    assert np.array_equal(*got) and np.array_equal(*tails)
+    at = 0
+    for n, slot, new in zip(counts, slots, fresh):
+        want, last = R.short_conv(u[at:at + n].astype(np.float64) + bias, w.astype(np.float64), np.zeros((taps - 1, Cn)) if new else before[slot].reshape(taps - 1, Cn).astype(np.float64))
+        assert rel(got[0][at:at + n], R.silu(want) if act else want) < 3e-6
+        assert rel(tails[0][slot].reshape(taps - 1, Cn), last) < 3e-7
+        at += n
+
+
 def run_delta(q, k, v, a, b, a_log, dt_bias, portions, eps=1e-6):
     """q, k [T, G, D]; v [T, H, V]; a, b [T, H]; one sequence in portions in slot 1 of 2, the other slot full of stale values."""
     T, G, D = q.shape
