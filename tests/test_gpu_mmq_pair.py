@@ -68,6 +68,17 @@ def test_parts_of_k(t, K, M, N):
         assert np.array_equal(product(t, w, x, K, M), got[:, :M])
 
 
+@pytest.mark.parametrize("K", [64, 960, 1088, 4032, 4096, 4160, 8256])
+def test_rows_of_activations_of_any_length(K):
+    """The conversion of the activations takes 4096 values of a row at a time."""
+    M, N = 70, 19
+    rng = np.random.default_rng(K)
+    x = rng.standard_normal((N, K)).astype(np.float32)
+    bits = (rng.standard_normal((M, K)).astype(np.float32).view(np.uint32) >> 16).astype(np.uint16)
+    want = x.astype(np.float64) @ (bits.astype(np.uint32) << 16).view(np.float32).astype(np.float64).T
+    assert rel(product(BF16, bits.view(np.uint8), x, K, M), want) < 4e-3
+
+
 def test_experts_without_a_valid_pair():
     """No tile at all: nothing is stored, and the launch ends."""
     K, M, used, n_expert, T = 512, 300, 2, 4, 40
