@@ -4,7 +4,9 @@
 // sink_attn_tile_kernel works on tiles of 64 cells that arrive by cp.async.  A CTA serves 64 columns of one kv head, a column being a token and
 // one of the query heads that share the keys, 16 columns a warp.  sink_attn_mma_kernel, which needs no workspace, converts every tile for every query head
 // and block of 64 tokens, with its loads in front of its products: 214 us for 512 tokens behind 512, 32 heads over 8 of 128; both launches here
-// take 63.  Bound by instruction issue (scores, exponentials), as fattn_mma_prefill_kernel, whose tile step this is.
+// take 56.  Bound by the latency of a tile's steps, of which two warps a scheduler (248 registers a thread) hide little, and by fetching their instructions: an instruction
+// a scheduler every 4.4 cycles.  What a tile's cells are is asked for a tile ahead, and comes to shared memory as the rows do: 58.4 us with both read where they are
+// needed; 32 heads over 4 of 64, 100 tokens behind 1400, 48.7 -> 42.1.
 // Whether half a tile is seen wholly, partly or not at all follows from the positions of the warp's tokens (their smallest and largest) when they
 // belong to one sequence, else token by token; only partly seen halves, and those with a soft cap or a distance bias, go value by value.
 // A softmax step is 32 cells, half a tile: the running maximum and with it the bf16 roundings of the weights are those of sink_attn_mma_kernel,
@@ -76,13 +78,21 @@ __global__ void __launch_bounds__(ST_WARPS * 32, 2) sink_attn_tile_kernel(const 
     const int rs0 = __shfl_sync(0xffffffffu, my_seq, g), rp0 = __shfl_sync(0xffffffffu, my_pos, g), rl0 = sa_chunk_start(rp0, a.chunk);
     const int rs1 = __shfl_sync(0xffffffffu, my_seq, g + 8), rp1 = __shfl_sync(0xffffffffu, my_pos, g + 8), rl1 = sa_chunk_start(rp1, a.chunk);
     enum { WHOLE = 0, PART = 1, HIDDEN = 2, BOTH_HIDDEN = HIDDEN | HIDDEN << 2 };
-    auto tile_kinds = [&](int t) {  // of the tile's halves, two bits each; lane looks at cells lane and lane + 32
-        int kinds = 0;
+    // the cells of the tile to be looked at next, lane and lane + 32 of it: asked for a tile ahead
+    int look_seq[2], look_pos[2];
+    auto look_at = [&](int t) {
 #pragma unroll
         for (int i = 0; i < 2; i++) {
             const int64_t c = (int64_t)t * ST_CELLS + lane + 32 * i;
-            int cs = -1, cp = 0;
-            if (c < a.n_kv) { cs = a.cell_seq[c]; cp = a.cell_pos[c]; }
+            look_seq[i] = -1; look_pos[i] = 0;
+            if (c < a.n_kv) { look_seq[i] = a.cell_seq[c]; look_pos[i] = a.cell_pos[c]; }
+        }
+    };
+    auto tile_kinds = [&]() {  // of that tile's halves, two bits each
+        int kinds = 0;
+#pragma unroll
+        for (int i = 0; i < 2; i++) {
+            const int cs = look_seq[i], cp = look_pos[i];
             bool all, none;
             if (!uniform) {  // token by token: its columns follow one another
                 all = none = true;
@@ -104,9 +114,11 @@ __global__ void __launch_bounds__(ST_WARPS * 32, 2) sink_attn_tile_kernel(const 
 
     // the CTA's next tile that one of its warps sees: the same for all threads; what this warp sees of it
     int next = 0;
+    look_at(0);
     auto advance = [&](int &kinds) {
         for (; next < n_tiles; next++) {
-            kinds = tile_kinds(next);
+            kinds = tile_kinds();
+            look_at(next + 1);
             if (__syncthreads_or(kinds != BOTH_HIDDEN)) return next++;
         }
         return -1;
@@ -121,8 +133,13 @@ __global__ void __launch_bounds__(ST_WARPS * 32, 2) sink_attn_tile_kernel(const 
             for (int i = tid; i < ST_CELLS * (VROW / 16); i += ST_WARPS * 32) cp_async16(base + KTILE + i / (VROW / 16) * VSTRIDE + i % (VROW / 16) * 16, vt + (size_t)i * 16);
             if (tid < ST_CELLS) {
                 const int64_t c = (int64_t)t * ST_CELLS + tid;
-                cseq[st][tid] = c < a.n_kv ? a.cell_seq[c] : -1;
-                cpos[st][tid] = c < a.n_kv ? a.cell_pos[c] : 0;
+                if (c < a.n_kv) {
+                    cp_async4(&cseq[st][tid], a.cell_seq + c);
+                    cp_async4(&cpos[st][tid], a.cell_pos + c);
+                } else {
+                    cseq[st][tid] = -1;
+                    cpos[st][tid] = 0;
+                }
             }
         }
         cp_async_commit();
