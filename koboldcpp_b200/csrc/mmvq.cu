@@ -388,11 +388,12 @@ static int launch_mmvq3(MmvqParams &p, cudaStream_t st, bool pdl) {
     p.dbg = dbg;
     TRACE_SLOT(p);
     const size_t smem = bar_bytes + act_bytes + ns * n_ring * G3::STAGE2 + part_bytes;
-    auto kern = nit1 ? mmvq3_kernel<TYPE, TYPE2, MULTI, true> : mmvq3_kernel<TYPE, TYPE2, MULTI, false>;
-    static bool attr_set_dev[16][2] = {};  // cudaFuncSetAttribute is per device (one table per template instantiation)
+    const bool half = p.K <= 2048;
+    auto kern = half ? mmvq3_kernel<TYPE, TYPE2, MULTI, true, true> : nit1 ? mmvq3_kernel<TYPE, TYPE2, MULTI, true> : mmvq3_kernel<TYPE, TYPE2, MULTI, false>;
+    static bool attr_set_dev[16][3] = {};  // cudaFuncSetAttribute is per device (one table per template instantiation)
     int cur_dev = 0;
     B200_CUDA_TRY(cudaGetDevice(&cur_dev));
-    bool &attr_set = attr_set_dev[cur_dev & 15][nit1 ? 1 : 0];
+    bool &attr_set = attr_set_dev[cur_dev & 15][half ? 2 : nit1 ? 1 : 0];
     if (!attr_set) {
         B200_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cap));
         attr_set = true;

@@ -64,12 +64,15 @@ __device__ __forceinline__ void lane_acts_load2(LaneActs &A, unsigned char *act_
 
 // TYPE2 != TYPE: a multi-job launch whose jobs are of two weight types (attn_q / attn_k Q4_K + attn_v Q6_K of the *_K_M mixes): bit j
 // of p.t2_mask says job j is TYPE2; its rows are contiguous (row stride = row size).
-template <int TYPE, int TYPE2, bool MULTI, bool NIT1>
+// HALF (K <= 2048): a row is at most 16 slices of 128 values, so lanes 0-15 take row A of a pair and lanes 16-31 row B in one pass, where half of the warp had nothing to do.
+// The sums are the same, to the bit.  5632 x 2 rows of 2048: q4_0 8.2 -> 7.0 us, q4_K 7.3 -> 6.4, q6_K 10.0 -> 8.7; 32000 of 2048 q6_K 17.4 -> 12.8; q8_0, which waits for memory, is unchanged (11.0).
+template <int TYPE, int TYPE2, bool MULTI, bool NIT1, bool HALF = false>
 __global__ void __launch_bounds__(MMVQ_THREADS, 1) mmvq3_kernel(const __grid_constant__ MmvqParams p) {
     using G3 = Geo3<TYPE>;
     using G3b = Geo3<TYPE2>;
     constexpr bool MIXED = TYPE != TYPE2;
     static_assert(!MIXED || MULTI, "two weight types need a multi-job launch");
+    static_assert(NIT1 || !HALF, "rows of 2048 values are one step");
     constexpr bool ALIGNED16 = G3::ALIGNED16 && G3b::ALIGNED16;
     constexpr int SEG = G3::SEG, SEGb = G3b::SEG;
     constexpr int STAGE = G3::STAGE > G3b::STAGE ? G3::STAGE : G3b::STAGE, STAGE2 = 2 * STAGE;
@@ -79,6 +82,7 @@ __global__ void __launch_bounds__(MMVQ_THREADS, 1) mmvq3_kernel(const __grid_con
     TRACE(0);
     if (!(p.dbg & 4)) pdl_trigger();  // one CTA per SM: a dependent CTA can only become resident when this one retires
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int ls = HALF ? lane & 15 : lane;  // slice of the row
     const int h = lane >> 4;  // lanes 0-15 work for row A of a pair, lanes 16-31 for row B
     const int n_stage = p.n_stage, n_it = NIT1 ? 1 : p.n_it;
     // K > 4096: the warps form n_it groups of g; a group owns one 4096-weight slice of K for every row of the CTA (so a lane's
@@ -182,7 +186,7 @@ __global__ void __launch_bounds__(MMVQ_THREADS, 1) mmvq3_kernel(const __grid_con
     // lanes past the end of the row in the last slice (and, for q4_0/q8_0, a partial last 128-weight slice)
     int nblk = 4;
     if (wit == n_it - 1) {
-        nblk = (int)(p.K / 32) - 4 * ((n_it - 1) * 32 + lane);
+        nblk = (int)(p.K / 32) - 4 * ((n_it - 1) * 32 + ls);
         nblk = nblk < 0 ? 0 : (nblk > 4 ? 4 : nblk);
     }
 
@@ -202,7 +206,7 @@ __global__ void __launch_bounds__(MMVQ_THREADS, 1) mmvq3_kernel(const __grid_con
         }
         else load_activations<1>(act_base, p.jobs[0].X, p.x_stride, p.K, n_it, p.norm_w, p.norm_eps, red, n_out, nm_out);
         __syncthreads();
-        if (active) lane_acts_load2<TYPE, TYPE2>(A, act_base, n_it, wit, lane);  // once per kernel
+        if (active) lane_acts_load2<TYPE, TYPE2>(A, act_base, n_it, wit, ls);  // once per kernel
         TRACE(4);
     }
 
@@ -235,7 +239,13 @@ __global__ void __launch_bounds__(MMVQ_THREADS, 1) mmvq3_kernel(const __grid_con
         const unsigned char *st = my_ring + (size_t)cstage * STAGE2;
         unsigned tmask = 0;  // mixed-type launch: which of the two rows are of the second type (all lanes vote: nblk is per lane)
         if constexpr (MIXED) tmask = __ballot_sync(0xffffffffu, r.t2 != 0);
-        if (nblk > 0 && !(p.dbg & 2)) {
+        if (HALF) {
+            if (nblk > 0 && r.src != nullptr && !(p.dbg & 2)) {
+                const unsigned char *row = st + (h ? STAGE + misB : misA);
+                if (MIXED && r.t2) RowDot<TYPE2>::run(row, ls, A, nblk, accA);
+                else RowDot<TYPE>::run(row, ls, A, nblk, accA);
+            }
+        } else if (nblk > 0 && !(p.dbg & 2)) {
             if constexpr (!MIXED) {
                 if (vA && vB) {
                     RowDot<TYPE>::run(st + misA, lane, A, nblk, accA);
@@ -271,8 +281,8 @@ __global__ void __launch_bounds__(MMVQ_THREADS, 1) mmvq3_kernel(const __grid_con
         cphase ^= (cstage == 0);
         // both row sums in one butterfly: lanes 0-15 end with sum(accA), lanes 16-31 with sum(accB) (same pairing order as
         // warp_sum)
-        float v = h ? accB : accA;
-        v += __shfl_xor_sync(0xffffffffu, h ? accA : accB, 16);
+        float v = HALF || !h ? accA : accB;
+        if (!HALF) v += __shfl_xor_sync(0xffffffffu, h ? accA : accB, 16);
 #pragma unroll
         for (int o = 8; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
         if constexpr (!NIT1) {
