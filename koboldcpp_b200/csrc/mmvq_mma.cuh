@@ -579,8 +579,10 @@ static int launch_mmvq_mma(const MmvqParams &m, int N, cudaStream_t st, bool pdl
     }
     const int64_t at_once = g_sm_count / p.c, tiles_each = (tiles + at_once - 1) / at_once;
     p.batch = p.c == 1 ? 0 : (int)((tiles_each < 64 ? tiles_each : 64) + MV_NW - 1) / MV_NW * MV_NW;  // (a multiple of the groups: a group's tiles follow one another)
-    const size_t acts = (mv_act_bytes<TYPE>((int64_t)per * 256, N) + 127) / 128 * 128 + (2 * MV_NW * 128 + p.batch * N * MV_ROWS) * sizeof(float), slot = (size_t)MV_NW * MV_ROWS * mv_row<TYPE>(),
-                 cap = g_smem_optin - 2048;
+    const size_t slot = (size_t)MV_NW * MV_ROWS * mv_row<TYPE>(), cap = g_smem_optin - 2048;
+    auto beside = [&]() { return (mv_act_bytes<TYPE>((int64_t)per * 256, N) + 127) / 128 * 128 + (2 * MV_NW * 128 + p.batch * N * MV_ROWS) * sizeof(float); };  // the ring
+    while (p.batch > MV_NW && beside() + 2 * slot > cap) p.batch -= MV_NW;  // (what is refused does not follow from the rows either)
+    const size_t acts = beside();
     p.slots = acts + 4 * slot <= cap ? 4 : acts + 3 * slot <= cap ? 3 : 2;
     if (acts + p.slots * slot > cap) return -1000;
     const size_t smem = acts + p.slots * slot;
