@@ -99,8 +99,9 @@ __global__ void __launch_bounds__(1024) qkv_store_kernel(const b200_qkv_store_ar
                 sn *= a.rope_mscale; cs *= a.rope_mscale;
             }
             const float tq = which ? 1.0f : q_temp;
-            dst[e0] = (u * cs - w * sn) * tq;
-            dst[e1] = (w * cs + u * sn) * tq;
+            // (which of the two products is rounded by itself is written down: left to the compiler, it was another one with a table)
+            dst[e0] = __fmaf_rn(u, cs, -__fmul_rn(w, sn)) * tq;
+            dst[e1] = __fmaf_rn(w, cs, __fmul_rn(u, sn)) * tq;
         }
     }
     if (a.v_unit_rms) {  // a warp per head of v: statistics, then the scaled row

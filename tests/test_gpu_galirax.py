@@ -42,7 +42,7 @@ def test_norm_with_bias_and_output_gate(kind, n, rows):
     assert rel(dout.to_numpy(np.float32, (rows, n)), res + base * R.sigmoid(gate)) < 3e-6
 
 
-def run_qkv_store(q, k, v, vecs, pos, cells, rot, n_cells, eps, lead=3):
+def run_qkv_store(q, k, v, vecs, pos, cells, rot, n_cells, eps, lead=3, **more):
     """q, k, v [T, heads, size] are handed over as column ranges of one wider row, as the fused projection leaves them."""
     T, Hh, D = q.shape
     G, V = k.shape[1], v.shape[2]
@@ -57,7 +57,7 @@ def run_qkv_store(q, k, v, vecs, pos, cells, rot, n_cells, eps, lead=3):
     g = lambda n: dv[n].ptr if n in dv else None
     a = QkvStoreArgs(q=d.ptr + 4 * oq, q_stride=row, k=d.ptr + 4 * ok, k_stride=row, v=d.ptr + 4 * ov, v_stride=row, q_bias=g("q.b"), k_bias=g("k.b"), v_bias=g("v.b"),
                      q_norm=g("q.norm"), k_norm=g("k.norm"), pos=dp.ptr, cells=dc.ptr, freqs=df.ptr, k_cache=kc.ptr, k_cache_stride=G * D + 2, v_cache=vc.ptr,
-                     v_cache_stride=G * V + 1, n_head=Hh, n_head_kv=G, dim=D, vdim=V, n_dims=rot["dims"], n_tokens=T, eps=eps)
+                     v_cache_stride=G * V + 1, n_head=Hh, n_head_kv=G, dim=D, vdim=V, n_dims=rot["dims"], n_tokens=T, eps=eps, **more)
     check(lib().b200_op_qkv_store(C.byref(a), None))
     out = d.to_numpy(np.float32, (T, row))
     assert np.array_equal(out[:, :lead], buf[:, :lead].astype(np.float32)) and np.array_equal(out[:, ok:], buf[:, ok:].astype(np.float32))  # only q is rewritten
@@ -101,6 +101,24 @@ def test_qkv_store_of_a_long_batch(Hh, G, D, V, dims, extra):
     for part in (slice(0, 64), slice(64, T)):
         gq, kc, vc = run_qkv_store(q[part], k[part], v[part], vecs, pos[part], cells[part], rot, T, eps)
         assert rel(whole[0][part], gq) < 3e-7 and rel(whole[1][cells[part]], kc[cells[part]]) < 3e-7 and np.array_equal(vc[cells[part]], whole[2][cells[part]])
+
+
+@pytest.mark.parametrize("Hh,G,D,V,dims", [(8, 2, 64, 64, 64), (5, 5, 10, 6, 10), (4, 2, 96, 40, 32)])
+@pytest.mark.parametrize("form", [{}, {"rope_halves": 1}, {"rope_mscale": 1.25}, {"norm_per_head": 1}, {"qk_unit_rms": 1}, {"q_temp_coef": 0.1, "q_temp_every": 100}])
+def test_a_token_is_rotated_the_same_in_every_batch(Hh, G, D, V, dims, form):
+    """To the bit, with and without the table that more than 64 tokens have.  (Not with a norm over all heads, whose sum is cut by the threads of a CTA.)"""
+    rng = np.random.default_rng(Hh * D + V)
+    T = 130
+    q, k, v = rng.standard_normal((T, Hh, D)), rng.standard_normal((T, G, D)), rng.standard_normal((T, G, V))
+    pos, cells = rng.integers(0, 5000, T), rng.permutation(T)
+    rot = {"base": 3000.0, "dims": dims, "scaling": {"factor": 8.0, "low": 1.0, "high": 4.0, "original": 64}}
+    vecs = {"q.b": rng.standard_normal(Hh * D), "k.b": rng.standard_normal(G * D)}
+    if "norm_per_head" in form:
+        vecs |= {"q.norm": 1 + 0.3 * rng.standard_normal(D), "k.norm": 1 + 0.3 * rng.standard_normal(D)}
+    whole = run_qkv_store(q, k, v, vecs, pos, cells, rot, T, 1e-5, **form)
+    for part in (slice(0, 1), slice(1, 65), slice(65, T)):  # one token, 64 and 65
+        gq, kc, vc = run_qkv_store(q[part], k[part], v[part], vecs, pos[part], cells[part], rot, T, 1e-5, **form)
+        assert np.array_equal(whole[0][part], gq) and np.array_equal(whole[1][cells[part]], kc[cells[part]]) and np.array_equal(whole[2][cells[part]], vc[cells[part]])
 
 
 def run_sink_attn(q, kc, vc, cell_seq, cell_pos, tok_seq, tok_pos, sink, scale, G, window=0, keep_first=0, bf16=0):
