@@ -75,6 +75,7 @@ __device__ __forceinline__ void cta_sync() {
     if constexpr (BAR == 0) __syncthreads();
     else asm volatile("bar.sync %0, %1;" ::"n"(BAR), "n"(NT) : "memory");
 }
+__device__ __forceinline__ float square4(const float4 v) { return __fmaf_rn(v.w, v.w, __fmaf_rn(v.z, v.z, __fmaf_rn(v.x, v.x, __fmul_rn(v.y, v.y)))); }
 template <int BAR = 0, int NT = MMVQ_THREADS>
 __device__ __forceinline__ float rms_scale(const float *__restrict__ xs, int64_t K, float norm_eps, float *red) {
     const int n4 = (int)(K / 4);
@@ -82,7 +83,7 @@ __device__ __forceinline__ float rms_scale(const float *__restrict__ xs, int64_t
     float ss = 0.f;
     for (int i4 = threadIdx.x; i4 < n4; i4 += NT) {
         const float4 v = __ldcg(reinterpret_cast<const float4 *>(xs) + i4);
-        ss += v.x * v.x + v.y * v.y + v.z * v.z + v.w * v.w;
+        ss += square4(v);
     }
     ss = warp_sum(ss);
     cta_sync<BAR, NT>();  // red[] may still be read by a previous call

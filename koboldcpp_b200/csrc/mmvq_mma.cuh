@@ -10,7 +10,7 @@
 //   * a warp takes 16 rows x one 256-value block at a time; their raw bytes (16-byte cp.async pieces, rows may start at any even byte) wait in a
 //     ring of its own, one to three blocks ahead; the ring is filled before the wait for the producer kernel;
 //   * the activations of all columns are quantised once per CTA into shared memory, in the order in which a lane reads its operand.  All loads of
-//     MV_U x 4096 values are in flight at once, and the norm's sums are taken from the same registers;
+//     MV_U x 4096 values are in flight at once, and the norm's squares are taken from the same registers;
 //   * KS warps share a row tile, each a part of K; their sums meet in shared memory in a fixed order.  KS is chosen so that rows and K parts
 //     fill the device evenly.
 #pragma once
@@ -377,7 +377,7 @@ __global__ void __launch_bounds__(MV_NW * 32, 1) mmvq_mma_kernel(const __grid_co
         const float *X = behind(p.m.jobs[0].X) + k0, *norm_w = p.m.norm_w ? behind(p.m.norm_w) + k0 : nullptr;
         // 32 neighbouring lanes take 256 values of a column, 8 each: row w of [column][256-value block]; 4 lanes hold a block of 32
         const int rows = N * nsb, uwarp = __shfl_sync(0xffffffffu, warp, 0);
-        __shared__ float nscale[8], nsum[8];
+        __shared__ float nscale[8];
         const bool keep = cluster == 0;
         const unsigned div_nsb = p.div_nsb[rank];
         const int q_lane = (lane >> 2) * N * 32 + 16 * (lane & 1) + 4 * ((lane >> 1) & 1);  // words 2 q and 2 q + 1 of a block lie at 2 (w & 3) + (w >> 2), q = lane & 3
@@ -398,30 +398,41 @@ __global__ void __launch_bounds__(MV_NW * 32, 1) mmvq_mma_kernel(const __grid_co
         load(0);
         for (int i = p.m.in_order ? 0 : 1; i < SLOTS - 1; i++) copy_block();
         if (norm_w != nullptr) {
-            for (int base = 0;;) {  // sums of squares of each 256 values, in order
+            // The sum of squares in the order of rms_scale, so that a column's norm, and with it its quants, is the same whichever kernel takes it: squares of four values
+            // each, in aq ([column][four values], the quants come later), then thread t adds those of t, t + 512, ...  With two CTAs: of both.
+            float *sq = reinterpret_cast<float *>(aq);
+            for (int base = 0;;) {
 #pragma unroll
                 for (int u = 0; u < MV_U; u++) {
-                    const float4 a = v[u][0], c = v[u][1];
-                    const float s = warp_sum(((a.x * a.x + a.y * a.y) + (a.z * a.z + a.w * a.w)) + ((c.x * c.x + c.y * c.y) + (c.z * c.z + c.w * c.w)));
                     const int w = base + u * MV_NW + uwarp;
-                    if (lane == 0 && w < rows) part[w] = s;
+                    if (w < rows) reinterpret_cast<float2 *>(sq)[w * 32 + lane] = make_float2(square4(v[u][0]), square4(v[u][1]));
                 }
                 base += CHUNK;
                 if (base >= rows) break;
                 load(base);
             }
-            __syncthreads();
-            if (warp < N) {
-                float s = 0.f;
-                for (int w = lane; w < nsb; w += 32) s += part[warp * nsb + w];
-                s = warp_sum(s);
-                if (lane == 0) nsum[warp] = s;
-            }
             if (C > 1) mv_cluster_meet();
             else __syncthreads();
-            if ((int)threadIdx.x < N) {
-                const float s = C > 1 ? mv_cluster_ld(nsum + threadIdx.x, 0) + mv_cluster_ld(nsum + threadIdx.x, 1) : nsum[threadIdx.x];
-                nscale[threadIdx.x] = rsqrtf(s / (float)p.m.K + p.m.norm_eps);
+            float ss[NP];
+#pragma unroll
+            for (int n = 0; n < NP; n++) ss[n] = 0.f;
+            const int n4 = nsb_all * 64, first4 = nsb_all / C * 64;  // (of the second CTA, if there is one: nsb_all / 2 blocks lie in front of it)
+            for (int i4 = threadIdx.x; i4 < n4; i4 += MV_NW * 32) {
+                const int of = C > 1 && i4 >= first4 ? 1 : 0, at = i4 - of * first4, per = of ? n4 - first4 : C > 1 ? first4 : n4;
+#pragma unroll
+                for (int n = 0; n < NP; n++)
+                    if (n < N) ss[n] += C > 1 ? mv_cluster_ld(sq + n * per + at, of) : sq[n * per + at];
+            }
+#pragma unroll
+            for (int n = 0; n < NP; n++) {
+                const float s = warp_sum(ss[n]);
+                if (lane == 0) part[n * MV_NW + warp] = s;
+            }
+            if (C > 1) mv_cluster_meet();  // (and both have read the squares)
+            else __syncthreads();
+            if (warp < N) {
+                const float s = warp_sum(lane < MV_NW ? part[warp * MV_NW + lane] : 0.f);
+                if (lane == 0) nscale[warp] = rsqrtf(s / (float)p.m.K + p.m.norm_eps);
             }
             __syncthreads();
             if (rows > CHUNK) load(0);

@@ -8,7 +8,7 @@ import pytest
 
 import koboldcpp_b200.host as H
 import orc as O
-from koboldcpp_b200.lib import Q4_0, Q4_K, Q5_K, Q6_K, Q8_0, GemvFuse, GemvJob, check, lib, row_size
+from koboldcpp_b200.lib import Q4_0, Q4_1, Q4_K, Q5_K, Q6_K, Q8_0, GemvFuse, GemvJob, check, lib, row_size
 from koboldcpp_b200.llama import random_blocks
 
 pytestmark = pytest.mark.gpu
@@ -145,3 +145,25 @@ def test_many_columns_of_few_rows(t, K, M, N):
     rng = np.random.default_rng(K + M + t)
     w, x = random_blocks(rng, t, M, K), rng.standard_normal((N, K)).astype(np.float32)
     assert close(H.mul_mat_vec_q(t, w, x, K, M), O.mul_mat_q8_1(t, w, x, K, M))
+
+
+@pytest.mark.parametrize("t", [Q4_0, Q8_0, Q4_K, Q5_K, Q6_K])
+@pytest.mark.parametrize("K,N", [(256, 8), (1280, 3), (2048, 2), (5120, 4), (4352, 8), (8192, 4), (11008, 3), (8448, 8)])
+def test_norm_is_that_of_the_other_kernel(t, K, N):
+    """A column's norm to the bit (q4_1 has no tensor form): a last bit of it moves values to another quant."""
+    M, eps = 80, 1e-5
+    rng = np.random.default_rng(K + N)
+    x = (rng.standard_normal((N, K)) * np.exp(rng.standard_normal((N, 1)))).astype(np.float32)
+    nw = (1 + 0.3 * rng.standard_normal(K)).astype(np.float32)
+    dx, dn = H.DeviceBuffer.from_numpy(x), H.DeviceBuffer.from_numpy(nw)
+
+    def norm(kind):
+        dw, dd, dnorm, dmul = H.DeviceBuffer.from_numpy(random_blocks(rng, kind, M, K), pad=16), *(H.DeviceBuffer(4 * N * n) for n in (M, K, K))
+        jobs, fuse = (GemvJob * 1)(), GemvFuse()
+        fuse.norm_weight, fuse.norm_eps, fuse.norm_out, fuse.norm_mul_out = dn.ptr, eps, dnorm.ptr, dmul.ptr
+        jobs[0].W, jobs[0].X, jobs[0].dst, jobs[0].M, jobs[0].id_index = dw.ptr, dx.ptr, dd.ptr, M, -1
+        check(lib().b200_mul_mat_vec_q_fused(kind, jobs, 1, row_size(kind, K), K, M, K, N, C.byref(fuse), None))
+        return dnorm.to_numpy(np.float32, (N, K)), dmul.to_numpy(np.float32, (N, K))
+
+    for got, want in zip(norm(t), norm(Q4_1)):
+        assert np.array_equal(got, want)
