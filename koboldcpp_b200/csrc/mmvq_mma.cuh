@@ -6,7 +6,7 @@
 //     for the others', so that one set of sums, and one scaling, serves two (four) sub-blocks.
 //   * the sums start from the bits of 1.5 * 2^23, which makes floats of them without a conversion; a sub-block's scale is multiplied in by the same FMA that
 //     takes that start away (exact: below 2^24).
-//   * minima of q4_K and q5_K (mins . sums of the activations) are one f16 tile a 256-value block: both factors are f16 values.
+//   * minima of q4_K and q5_K (mins . sums of the activations) are one f16 tile a 256-value block, packed as the columns are: both factors are f16 values.
 //   * a warp takes 16 rows x one 256-value block at a time; their raw bytes (16-byte cp.async pieces, rows may start at any even byte) wait in a
 //     ring of its own, one to three blocks ahead; the ring is filled before the wait for the producer kernel;
 //   * the activations of all columns are quantised once per CTA into shared memory, in the order in which a lane reads its operand.  All loads of
@@ -117,16 +117,15 @@ struct MvLane {
     static constexpr int G = 8 / NP;
     int t4, gb, sub;
     unsigned mask[G];                  // all ones in the tile that takes this lane's operand
-    unsigned bq, sc, su;               // operand of the lane's column in the first block; scales from column col on; (K-quants) f16 sums of column g
+    unsigned bq, sc, su, su_mask;      // operand of the lane's column in the first block; scales from column col on; (K-quants) its f16 sums, and which of the two
     unsigned bq_step, sc_step, ai;     // from a block to the next; ai: q6_K, from the scales to the integer sums
-    bool col;                          // column g exists
 };
 __device__ __forceinline__ int mv_sbyte(unsigned w, int k) { return (int)(signed char)(w >> (8 * k)); }
 
-// one 256-value block of rows g and g + 8: acc[0..1] += row g, columns col and col + 1 of sub-block `sub`; acc[2..3] += row g + 8; low[] (K-quants): what the minima
-// take away, columns 2 t4 and 2 t4 + 1.  r0, r1: the rows' first bytes
+// one 256-value block of rows g and g + 8: acc[0..1] += row g, columns col and col + 1 of sub-block `sub`; acc[2..3] += row g + 8.  r0, r1: the
+// rows' first bytes
 template <int TYPE, int NP>
-__device__ __forceinline__ void mv_block(unsigned r0, unsigned r1, const MvLane<NP> &L, int sb, float (&acc)[4], float (&low)[4]) {
+__device__ __forceinline__ void mv_block(unsigned r0, unsigned r1, const MvLane<NP> &L, int sb, float (&acc)[4]) {
     constexpr int G = MvLane<NP>::G;
     const int t4 = L.t4;
     const int magic[4] = {MV_MAGIC, MV_MAGIC, MV_MAGIC, MV_MAGIC};
@@ -263,15 +262,19 @@ __device__ __forceinline__ void mv_block(unsigned r0, unsigned r1, const MvLane<
             m[i] = *reinterpret_cast<const unsigned *>(&y);
         }
         float sm[4];
-        mv_mma_f16(sm, m[0], m[1], L.col ? mv_ld<unsigned>(L.su + (size_t)sb * (L.bq_step / 2)) : 0u);
+        mv_mma_f16(sm, m[0], m[1], mv_ld<unsigned>(L.su + (size_t)sb * (L.bq_step / 2)) & L.su_mask);
         const float d0 = h2f((unsigned short)(h0.x & 0xffff)), n0 = h2f((unsigned short)(h0.x >> 16)), d1 = h2f((unsigned short)(h1.x & 0xffff)), n1 = h2f((unsigned short)(h1.x >> 16));
-        acc[0] += d0 * sd[0]; acc[1] += d0 * sd[1]; acc[2] += d1 * sd[2]; acc[3] += d1 * sd[3];
-        low[0] += n0 * sm[0]; low[1] += n0 * sm[1]; low[2] += n1 * sm[2]; low[3] += n1 * sm[3];
+        // (here and not behind the row: of activations of one sign two large sums would be left, of whose difference little remains)
+        acc[0] = fmaf(-n0, sm[0], fmaf(d0, sd[0], acc[0])); acc[1] = fmaf(-n0, sm[1], fmaf(d0, sd[1], acc[1]));
+        acc[2] = fmaf(-n1, sm[2], fmaf(d1, sd[2], acc[2])); acc[3] = fmaf(-n1, sm[3], fmaf(d1, sd[3], acc[3]));
     } else {
         constexpr int BB = type_block_bytes(TYPE);
         const MvRun e0(r0 + 2 + 4 * t4), e1(r1 + 2 + 4 * t4), o0(r0 + 2 + BB + 4 * t4), o1(r1 + 2 + BB + 4 * t4);  // quants of even and odd blocks
         uint2 b = make_uint2(0u, 0u);
         int k[4];
+        // A block's sum by itself, so that the chain of roundings is shorter.  (q4_0 of four columns and fewer adds two or four terms a block, and is 4 % slower so.)
+        constexpr bool OWN = TYPE == B200_TYPE_Q8_0 || NP == 8;
+        float own[4] = {0.f, 0.f, 0.f, 0.f}, *sd = OWN ? own : acc;
 #pragma unroll
         for (int blk = 0; blk < 8; blk++) {
             const int j = blk % G, set = blk - j, at = 2 * BB * (blk / 2);
@@ -292,15 +295,16 @@ __device__ __forceinline__ void mv_block(unsigned r0, unsigned r1, const MvLane<
                 const float d0 = h2f(mv_ld<unsigned short>(r0 + BB * mine)), d1 = h2f(mv_ld<unsigned short>(r1 + BB * mine));
                 if constexpr (TYPE == B200_TYPE_Q4_0) {
                     const float4 d = mv_ld<float4>(sc + mine * L.sc_step);  // d, -8 s of both columns
-                    acc[0] += d0 * fmaf(d.x, mv_float(k[0]), d.y); acc[1] += d0 * fmaf(d.z, mv_float(k[1]), d.w);
-                    acc[2] += d1 * fmaf(d.x, mv_float(k[2]), d.y); acc[3] += d1 * fmaf(d.z, mv_float(k[3]), d.w);
+                    sd[0] += d0 * fmaf(d.x, mv_float(k[0]), d.y); sd[1] += d0 * fmaf(d.z, mv_float(k[1]), d.w);
+                    sd[2] += d1 * fmaf(d.x, mv_float(k[2]), d.y); sd[3] += d1 * fmaf(d.z, mv_float(k[3]), d.w);
                 } else {
                     const float2 d = mv_ld<float2>(sc + mine * L.sc_step);
-                    acc[0] += d0 * d.x * mv_float(k[0]); acc[1] += d0 * d.y * mv_float(k[1]);
-                    acc[2] += d1 * d.x * mv_float(k[2]); acc[3] += d1 * d.y * mv_float(k[3]);
+                    sd[0] += d0 * d.x * mv_float(k[0]); sd[1] += d0 * d.y * mv_float(k[1]);
+                    sd[2] += d1 * d.x * mv_float(k[2]); sd[3] += d1 * d.y * mv_float(k[3]);
                 }
             }
         }
+        if constexpr (OWN) { acc[0] += own[0]; acc[1] += own[1]; acc[2] += own[2]; acc[3] += own[3]; }
     }
 }
 
@@ -413,21 +417,24 @@ __global__ void __launch_bounds__(MV_NW * 32, 1) mmvq_mma_kernel(const __grid_co
             }
             if (C > 1) mv_cluster_meet();
             else __syncthreads();
-            float ss[NP];
+            auto add_up = [&](auto square) {
+                float ss[NP];
 #pragma unroll
-            for (int n = 0; n < NP; n++) ss[n] = 0.f;
-            const int n4 = nsb_all * 64, first4 = nsb_all / C * 64;  // (of the second CTA, if there is one: nsb_all / 2 blocks lie in front of it)
-            for (int i4 = threadIdx.x; i4 < n4; i4 += MV_NW * 32) {
-                const int of = C > 1 && i4 >= first4 ? 1 : 0, at = i4 - of * first4, per = of ? n4 - first4 : C > 1 ? first4 : n4;
+                for (int n = 0; n < NP; n++) ss[n] = 0.f;
+#pragma unroll 2
+                for (int i4 = threadIdx.x; i4 < nsb_all * 64; i4 += MV_NW * 32) {
 #pragma unroll
-                for (int n = 0; n < NP; n++)
-                    if (n < N) ss[n] += C > 1 ? mv_cluster_ld(sq + n * per + at, of) : sq[n * per + at];
-            }
+                    for (int n = 0; n < NP; n++) ss[n] += square(n < N ? n : 0, i4);  // (of columns that do not exist: another's, for nobody)
+                }
 #pragma unroll
-            for (int n = 0; n < NP; n++) {
-                const float s = warp_sum(ss[n]);
-                if (lane == 0) part[n * MV_NW + warp] = s;
-            }
+                for (int n = 0; n < NP; n++) {
+                    const float s = warp_sum(ss[n]);
+                    if (lane == 0) part[n * MV_NW + warp] = s;
+                }
+            };
+            const int first4 = nsb_all / 2 * 64;  // where the second CTA's part begins
+            if (C == 1) add_up([&](int n, int i4) { return sq[n * nsb * 64 + i4]; });
+            else add_up([&](int n, int i4) { const bool far = i4 >= first4; return mv_cluster_ld(sq + n * (far ? nsb_all * 64 - first4 : first4) + (far ? i4 - first4 : i4), far); });
             if (C > 1) mv_cluster_meet();  // (and both have read the squares)
             else __syncthreads();
             if (warp < N) {
@@ -492,8 +499,9 @@ __global__ void __launch_bounds__(MV_NW * 32, 1) mmvq_mma_kernel(const __grid_co
     L.sc = (unsigned)(as - smem) + cp2 * (TYPE == B200_TYPE_Q4_0 ? 8 : 4);
     L.sc_step = sc_step;
     L.ai = (unsigned)(ai - as);
-    L.col = g < N;
-    L.su = (unsigned)(ai - smem) + (L.col ? g : 0) * 16 + 4 * t4;
+    L.su = (unsigned)(ai - smem) + (ncol < N ? ncol : 0) * 16 + 4 * t4;
+    // of the sub-blocks 2 t4 and 2 t4 + 1, those whose sums this column of the tile holds
+    L.su_mask = ncol >= N || (NP == 2 && L.gb >> 1 != (t4 & 1)) ? 0u : NP == 8 ? 0xffffffffu : L.gb & 1 ? 0xffff0000u : 0x0000ffffu;
     auto store = [&](const Tile &ti, int r, int n, float v) {
         const int64_t o = (int64_t)n * p.m.dst_stride + ti.row + r;
         if (p.m.raw_dst[ti.job]) p.m.raw_dst[ti.job][o] = v;
@@ -505,7 +513,7 @@ __global__ void __launch_bounds__(MV_NW * 32, 1) mmvq_mma_kernel(const __grid_co
     for (; t < t1; t += step) {
         const Tile ti = tile(t);
         const int64_t M = p.m.jobs[ti.job].M, last = M - 1;
-        float acc[4] = {0.f, 0.f, 0.f, 0.f}, low[4] = {0.f, 0.f, 0.f, 0.f};
+        float acc[4] = {0.f, 0.f, 0.f, 0.f};
         unsigned at0 = 0, at1 = 0;  // where in its slot row the block starts
         if constexpr (!ALIGNED) {
             const uintptr_t base = (uintptr_t)ti.W + (size_t)(sbk + sb0) * BB;
@@ -518,7 +526,7 @@ __global__ void __launch_bounds__(MV_NW * 32, 1) mmvq_mma_kernel(const __grid_co
             copy_block();
             __syncwarp();  // (mma.sync and bar.sync want a warp that is together: nothing but this promises it behind a branch that lanes take differently)
             const unsigned rows = (unsigned)(ring - smem) + slot * MV_ROWS * ROW;
-            mv_block<TYPE, NP>(rows + g * ROW + at0, rows + (g + 8) * ROW + at1, L, sb0 + b, acc, low);
+            mv_block<TYPE, NP>(rows + g * ROW + at0, rows + (g + 8) * ROW + at1, L, sb0 + b, acc);
             if constexpr (!ALIGNED) { at0 = (at0 + BB) & 15u; at1 = (at1 + BB) & 15u; }
             slot = slot + 1 == SLOTS ? 0 : slot + 1;
         }
@@ -530,8 +538,8 @@ __global__ void __launch_bounds__(MV_NW * 32, 1) mmvq_mma_kernel(const __grid_co
         // ---- the group's sums meet in a fixed order: part[buf][warp][row][column]
         float *mine = part + ((size_t)buf * MV_NW + warp) * 128;
         if (2 * t4 < NP) {
-            *reinterpret_cast<float2 *>(mine + g * 8 + 2 * t4) = make_float2(acc[0] - low[0], acc[1] - low[1]);
-            *reinterpret_cast<float2 *>(mine + (g + 8) * 8 + 2 * t4) = make_float2(acc[2] - low[2], acc[3] - low[3]);
+            *reinterpret_cast<float2 *>(mine + g * 8 + 2 * t4) = make_float2(acc[0], acc[1]);
+            *reinterpret_cast<float2 *>(mine + (g + 8) * 8 + 2 * t4) = make_float2(acc[2], acc[3]);
         }
         __syncwarp();
         if (KS > 1) asm volatile("bar.sync %0, %1;" ::"r"(1 + grp), "r"(KS * 32) : "memory");
@@ -539,8 +547,10 @@ __global__ void __launch_bounds__(MV_NW * 32, 1) mmvq_mma_kernel(const __grid_co
         for (int i = kp * 32 + lane; i < 128; i += KS * 32) {
             const int r = i & 15, n = i >> 4;
             if (n >= N || ti.row + r >= M) continue;
-            float v = 0.f;
-            for (int k = 0; k < KS; k++) v += all[k * 128 + r * 8 + n];
+            const float *x = all + r * 8 + n;  // (added in pairs: fewer roundings of a row's whole sum)
+            float v = x[0];
+            if (KS == 2) v += x[128];
+            else if (KS >= 4) { v = (v + x[128]) + (x[256] + x[384]); if (KS == 8) v += (x[512] + x[640]) + (x[768] + x[896]); }
             if (C > 1) sums[((t - t0) / n_clusters * N + n) * MV_ROWS + r] = v;
             else store(ti, r, n, v);
         }

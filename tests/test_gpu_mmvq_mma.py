@@ -167,3 +167,28 @@ def test_norm_is_that_of_the_other_kernel(t, K, N):
 
     for got, want in zip(norm(t), norm(Q4_1)):
         assert np.array_equal(got, want)
+
+
+@pytest.mark.parametrize("t", [Q4_K, Q5_K])
+@pytest.mark.parametrize("K,N", [(7936, 2), (7936, 3), (6144, 4), (5120, 5), (3072, 8), (13824, 4)])
+def test_activations_of_one_sign(t, K, N):
+    """The minima take away most of what the quants add up to, block by block: a row's error is that of its blocks' sums.  A block of 256 rounds 8 partial sums of its
+    quants, of 1/8 .. 8/8 of what they add up to (A), as many of its minima and the difference: about 2^-24 A (0.43 sqrt(2 * 3.2 + 1) = 1.2 for roundings at all places of a
+    binade); bound 2.  (Two sums of whole rows, subtracted at the end, are 2.5 to 4 off.)"""
+    M = 512
+    rng = np.random.default_rng(K + N + t)
+    w = random_blocks(rng, t, M, K)
+    q = rng.integers(1, 33, (N, K // 32, 32))
+    q[:, :, 5] = 127  # scale 2^-7 and sums below 2048: exact in f16, so that quantised activations are the activations
+    x = (q.reshape(N, K) / 128).astype(np.float32)
+    rows = np.stack([O.dequantize(t, r, K) for r in w]).astype(np.float64)
+    blocks = w.reshape(M, K // 256, -1)
+    low = blocks[:, :, 2:4].copy().view(np.float16).astype(np.float64)[:, :, 0]
+    s = blocks[:, :, 4:16].astype(np.int64)
+    mins = np.concatenate([s[:, :, 4:8] & 63, (s[:, :, 8:] >> 4) | (s[:, :, 4:8] >> 6 << 4)], axis=2) * low[:, :, None]  # [row][block][8]
+    quants = rows.reshape(M, K // 256, 8, 32) + mins[..., None]
+    A = np.einsum("mbsi,nbsi->nmb", quants, x.reshape(N, K // 256, 8, 32).astype(np.float64))
+    err = H.mul_mat_vec_q(t, w, x, K, M) - x.astype(np.float64) @ rows.T
+    c = np.sqrt((err ** 2).mean() / (A ** 2).sum(2).mean()) * 2 ** 24
+    print("error", c)
+    assert c < 2
