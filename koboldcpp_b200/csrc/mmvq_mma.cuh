@@ -308,7 +308,8 @@ __device__ __forceinline__ void mv_block(unsigned r0, unsigned r1, const MvLane<
     }
 }
 
-template <int TYPE, int NP>
+// NORM: there is a norm.  (A kernel of its own: in one for both, which needs all registers, its sums made the loop over the blocks 3 to 6 % slower.)
+template <int TYPE, int NP, bool NORM>
 __global__ void __launch_bounds__(MV_NW * 32, 1) mmvq_mma_kernel(const __grid_constant__ MvParams p) {
     constexpr int BB = mv_bytes<TYPE>(), PIECES = mv_pieces<TYPE>(), ROW = mv_row<TYPE>(), PER = (MV_ROWS * PIECES + 31) / 32;
     constexpr bool ALIGNED = mv_aligned(TYPE);
@@ -378,7 +379,7 @@ __global__ void __launch_bounds__(MV_NW * 32, 1) mmvq_mma_kernel(const __grid_co
     // go out in front of the weights: behind some 100 KB of those they would wait for a microsecond.
     {
         const int64_t k0 = (int64_t)sbk * 256;
-        const float *X = behind(p.m.jobs[0].X) + k0, *norm_w = p.m.norm_w ? behind(p.m.norm_w) + k0 : nullptr;
+        const float *X = behind(p.m.jobs[0].X) + k0, *norm_w = NORM ? behind(p.m.norm_w) + k0 : nullptr;
         // 32 neighbouring lanes take 256 values of a column, 8 each: row w of [column][256-value block]; 4 lanes hold a block of 32
         const int rows = N * nsb, uwarp = __shfl_sync(0xffffffffu, warp, 0);
         __shared__ float nscale[8];
@@ -401,7 +402,7 @@ __global__ void __launch_bounds__(MV_NW * 32, 1) mmvq_mma_kernel(const __grid_co
         };
         load(0);
         for (int i = p.m.in_order ? 0 : 1; i < SLOTS - 1; i++) copy_block();
-        if (norm_w != nullptr) {
+        if constexpr (NORM) {
             // The sum of squares in the order of rms_scale, so that a column's norm, and with it its quants, is the same whichever kernel takes it: squares of four values
             // each, in aq ([column][four values], the quants come later), then thread t adds those of t, t + 512, ...  With two CTAs: of both.
             float *sq = reinterpret_cast<float *>(aq);
@@ -450,7 +451,7 @@ __global__ void __launch_bounds__(MV_NW * 32, 1) mmvq_mma_kernel(const __grid_co
             for (int u = 0; u < MV_U; u++) {
                 const int w = base + u * MV_NW + uwarp, n = nsb == 1 ? w : (int)__umulhi((unsigned)w, div_nsb), sb = w - n * nsb;
                 if (w >= rows) continue;
-                if (norm_w != nullptr) {
+                if constexpr (NORM) {
                     const float s = nscale[n];
                     const int i4 = sb * 64 + 2 * lane;
 #pragma unroll
@@ -574,8 +575,11 @@ __global__ void __launch_bounds__(MV_NW * 32, 1) mmvq_mma_kernel(const __grid_co
 }
 
 // -1000: not for this kernel (shared memory)
-template <int TYPE, int NP>
+template <int TYPE, int NP, bool NORM = false>
 static int launch_mmvq_mma(const MmvqParams &m, int N, cudaStream_t st, bool pdl) {
+    if constexpr (!NORM) {
+        if (m.norm_w) return launch_mmvq_mma<TYPE, NP, true>(m, N, st, pdl);
+    }
     MvParams p;
     p.m = m;
     p.m.in_order = !pdl;
@@ -607,7 +611,7 @@ static int launch_mmvq_mma(const MmvqParams &m, int N, cudaStream_t st, bool pdl
     p.slots = acts + 4 * slot <= cap ? 4 : acts + 3 * slot <= cap ? 3 : 2;
     if (acts + p.slots * slot > cap) return -1000;
     const size_t smem = acts + p.slots * slot;
-    const auto kern = mmvq_mma_kernel<TYPE, NP>;
+    const auto kern = mmvq_mma_kernel<TYPE, NP, NORM>;
     static bool attr_set_dev[16] = {};  // cudaFuncSetAttribute is per device
     int cur_dev = 0;
     B200_CUDA_TRY(cudaGetDevice(&cur_dev));
