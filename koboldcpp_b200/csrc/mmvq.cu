@@ -418,6 +418,16 @@ static int launch_mmvq3(MmvqParams &p, cudaStream_t st, bool pdl) {
 #include "mmvq_mma.cuh"
 namespace b200 {
 
+// Two columns of few and long rows, where the tensor form is not ahead yet: what bounds such a launch is the way from the first load of the columns to their quants, which is
+// longer there.  Tensor -> dp4a, us: 1024 rows of 4096 q4_0 5.2 -> 4.9, q8_0 6.6 -> 5.2, q4_K 5.3 -> 4.7, q5_K 5.6 -> 4.8, q6_K 6.0 -> 5.1; 256 x 2048 q4_K 3.9 -> 3.6, q6_K 4.1 -> 3.8; 512 x
+// 5120 q8_0 7.6 -> 6.0; 512 x 8192 q5_K 6.8 -> 6.4.  Level at 1024 values (q8_0 512 rows 3.8, 3.8), 1536 rows (q4_K 2048 values 4.4, 4.3; q6_K 5120 7.6, 7.8) and 11008 (q8_0 512 rows 8.4 -> 9.7).
+template <int TYPE>
+static bool mmvq_few(const MmvqParams &p, int N) {
+    if (N != 2) return false;
+    if (TYPE == B200_TYPE_Q4_0) return p.K == 4096 && p.total_rows <= 1200;
+    return p.K > 1024 && p.K <= 8192 && p.total_rows <= (p.K <= 4096 ? 1536 : 1200);
+}
+
 template <int TYPE>
 static int dispatch_cols(MmvqParams &p, int N, cudaStream_t st, bool pdl) {
     const bool multi = p.n_jobs > 1 || p.ids != nullptr;
@@ -433,12 +443,11 @@ static int dispatch_cols(MmvqParams &p, int N, cudaStream_t st, bool pdl) {
     // Several columns of one activation matrix: the integer tensor cores, whose cost hardly grows with the columns; dp4a spends 8 instructions a column and 32 weights.
     // dp4a -> tensor, us, at 2 / 4 / 8 columns: 22016 x 4096 q4_0 25.6 -> 18.8 / 39.1 -> 20.4 / - ; 32000 x 2048 q8_0 25.6 -> 17.5 / 37.2 -> 18.9 / 64.7 -> 21.3;
     // 32000 x 2048 q4_K 22.8 -> 14.1 at 2; 5120 x 13824 q6_K 36.9 -> 26.9 at 4; 2048 x 2048 q4_0 4.5 -> 4.1 / 6.7 -> 4.7 / 12.1 -> 5.8; 256 x 256 3.7 -> 3.5 / 5.5 -> 3.6 /
-    // 9.5 -> 3.9.  Where it loses are two columns of few and long rows, which leave most warps without a tile: 256 x 2048 3.7 -> 3.8 (q6_K 4.3), 1024 x 4096 q4_0 4.8 -> 5.2,
-    // q4_K 4.7 -> 5.4, q8_0 5.1 -> 6.9.  The choice does not look at the rows all the same, so that a row's bits do not depend on the launch it is part of.
+    // 9.5 -> 3.9.
     if constexpr (TYPE == B200_TYPE_Q4_0 || TYPE == B200_TYPE_Q8_0 || TYPE == B200_TYPE_Q4_K || TYPE == B200_TYPE_Q5_K || TYPE == B200_TYPE_Q6_K) {
         bool same_x = p.ids == nullptr && p.K % 256 == 0;
         for (int j = 1; j < p.n_jobs; j++) same_x = same_x && p.jobs[j].X == p.jobs[0].X;
-        if (N >= 2 && same_x && (!multi || N <= 4)) {
+        if (N >= 2 && same_x && (!multi || N <= 4) && !mmvq_few<TYPE>(p, N)) {
             int rc = B200_OK;
             if (multi) {  // (several jobs have a limit of rows, whichever kernel serves them)
                 MmvqPlan pl;

@@ -11,8 +11,8 @@
 //     ring of its own, one to three blocks ahead; the ring is filled before the wait for the producer kernel;
 //   * the activations of all columns are quantised once per CTA into shared memory, in the order in which a lane reads its operand.  All loads of
 //     MV_U x 4096 values are in flight at once, and the norm's squares are taken from the same registers;
-//   * KS warps share a row tile, each a part of K; their sums meet in shared memory in a fixed order.  KS is chosen so that rows and K parts
-//     fill the device evenly.
+//   * KS warps share a row tile, each a part of K; their sums meet in shared memory in a fixed order; two CTAs share row tiles, half of K each, where the columns
+//     are long or row tiles few.  How K is cut follows from K, the columns and the rows of the launch.
 #pragma once
 
 namespace b200 {
@@ -551,7 +551,10 @@ __global__ void __launch_bounds__(MV_NW * 32, 1) mmvq_mma_kernel(const __grid_co
             const float *x = all + r * 8 + n;  // (added in pairs: fewer roundings of a row's whole sum)
             float v = x[0];
             if (KS == 2) v += x[128];
-            else if (KS >= 4) { v = (v + x[128]) + (x[256] + x[384]); if (KS == 8) v += (x[512] + x[640]) + (x[768] + x[896]); }
+            else if (KS >= 4) {
+                v = (v + x[128]) + (x[256] + x[384]);
+                for (int k = 4; k < KS; k += 4) v += (x[k * 128] + x[k * 128 + 128]) + (x[k * 128 + 256] + x[k * 128 + 384]);
+            }
             if (C > 1) sums[((t - t0) / n_clusters * N + n) * MV_ROWS + r] = v;
             else store(ti, r, n, v);
         }
@@ -590,23 +593,30 @@ static int launch_mmvq_mma(const MmvqParams &m, int N, cudaStream_t st, bool pdl
     const int rc = device_props();
     if (rc) return rc;
     const int nsb = (int)(m.K / 256);
-    // How K is cut, into halves for two CTAs and among warps, follows from K and N alone, so that a row's bits do not depend on the launch it is part of.  Two
-    // CTAs share row tiles, half of K each, where the columns are many enough to quantise that half the work makes up for the meeting (about 1 us): 5120 x 13824
-    // q6_K at 4 columns 32.3 -> 27.8 us, 4096 x 11008 q4_K 17.0 -> 15.8; 4096 x 4096 q4_0 at 4 columns 8.4 -> 8.6, 22016 x 4096 q4_K 21.8 -> 23.4.
-    p.c = nsb >= 2 && m.K * N >= 26000 ? 2 : 1;
+    // How K is cut, into halves for two CTAs and among warps.  Two CTAs share row tiles where the columns are many enough to quantise that half the work makes up for
+    // the meeting (about 1 us): 5120 x 13824 q6_K at 4 columns 32.3 -> 27.8 us, 4096 x 11008 q4_K 17.0 -> 15.8; 4096 x 4096 q4_0 at 4 columns 8.4 -> 8.6, 22016 x 4096
+    // q4_K 21.8 -> 23.4.  Where half of the SMs would have no tile, from fewer values on: 512 rows, one CTA -> two with all warps on a tile, 4096 q8_0 at 3 columns
+    // 7.7 -> 6.5, 5120 q6_K at 4 10.5 -> 8.9, 11008 q5_K at 2 9.9 -> 7.8; 3072 q6_K at 3 (9216 values) 6.2 -> 6.4, 4096 q4_0 at 2 (8192) 5.1 -> 5.4.
+    p.c = nsb >= 2 && m.K * N >= (tiles > g_sm_count / 2 ? 26000 : m.K >= 4096 ? 12000 : 13000) ? 2 : 1;
     const int per = (nsb + p.c - 1) / p.c;
     // (warps a tile: more of them help where rows are few, and meet more often where they are many.  One CTA, 2 columns, with 1, 2, 4, 8 warps: 4096 x 4096 q4_0 9.8,
     // 7.4, 7.1, 7.2 us, 22016 x 4096 q4_K 18.3, 19.3, 19.5, 20.8; two CTAs, 4 columns, 5120 x 13824 q6_K 32.6, 27.8, 29.3, 28.2)
     p.ks = p.c == 2 ? (per >= 24 ? 8 : per >= 16 ? 4 : 2) : per >= 32 ? 8 : per >= 8 ? 4 : per >= 4 ? 2 : 1;
+    // Few tiles leave warps idle that could take a part: with rows of up to 1792 values (1024 x 512 q5_K at 2 / 4 columns 4.8 -> 4.2 / 4.6 -> 4.0), and with two CTAs.  One CTA's
+    // longer rows are level or slower so (512 x 5120 q4_0 at 4 columns 7.3 -> 8.2): what they wait for is the quantisation.
+    const int64_t at_once = g_sm_count / p.c, tiles_each = (tiles + at_once - 1) / at_once;
+    if (per < 8 || p.c == 2) {
+        for (int ks = MV_NW / (tiles_each <= 1 ? 1 : tiles_each <= 2 ? 2 : tiles_each <= 4 ? 4 : MV_NW); ks > p.ks; ks /= 2)
+            if (ks <= per) p.ks = ks;
+    }
     for (int r = 0; r < 2; r++) {
         const unsigned each = (unsigned)((r + 1) * nsb / p.c - r * nsb / p.c);
         p.div_nsb[r] = each > 1 ? (unsigned)(((1ull << 32) + each - 1) / each) : 0;
     }
-    const int64_t at_once = g_sm_count / p.c, tiles_each = (tiles + at_once - 1) / at_once;
     p.batch = p.c == 1 ? 0 : (int)((tiles_each < 64 ? tiles_each : 64) + MV_NW - 1) / MV_NW * MV_NW;  // (a multiple of the groups: a group's tiles follow one another)
     const size_t slot = (size_t)MV_NW * MV_ROWS * mv_row<TYPE>(), cap = g_smem_optin - 2048;
     auto beside = [&]() { return (mv_act_bytes<TYPE>((int64_t)per * 256, N) + 127) / 128 * 128 + (2 * MV_NW * 128 + p.batch * N * MV_ROWS) * sizeof(float); };  // the ring
-    while (p.batch > MV_NW && beside() + 2 * slot > cap) p.batch -= MV_NW;  // (what is refused does not follow from the rows either)
+    while (p.batch > MV_NW && beside() + 2 * slot > cap) p.batch -= MV_NW;
     const size_t acts = beside();
     p.slots = acts + 4 * slot <= cap ? 4 : acts + 3 * slot <= cap ? 3 : 2;
     if (acts + p.slots * slot > cap) return -1000;

@@ -1,4 +1,4 @@
-"""The GEMV of several columns on the integer tensor cores: row tiles of 16 and their remainders, K parts for 1 to 16 warps, odd and even column counts,
+"""The GEMV of several columns on the integer tensor cores: row tiles of 16 and their remainders, K parts for 1 to 16 warps and for two CTAs, odd and even column counts,
 rows at any even byte, jobs of different sizes, norm prologue, residual and raw results.  Against the oracle's q8_1 arithmetic: sums of K / 32 exact
 products in f32, 2^-24 sqrt(K / 32) of their size, bound 3e-5 as for the other GEMV kernels."""
 import ctypes as C
@@ -192,3 +192,43 @@ def test_activations_of_one_sign(t, K, N):
     c = np.sqrt((err ** 2).mean() / (A ** 2).sum(2).mean()) * 2 ** 24
     print("error", c)
     assert c < 2
+
+
+def two_jobs(t, ws, xs, K, N):
+    """Two matrices in one launch, each with the activations at an address of its own."""
+    total = sum(len(w) for w in ws)
+    dws, dxs, dd = [H.DeviceBuffer.from_numpy(w, pad=16) for w in ws], [H.DeviceBuffer.from_numpy(x) for x in xs], H.DeviceBuffer(4 * N * total)
+    jobs, at = (GemvJob * 2)(), 0
+    for i, (w, dw) in enumerate(zip(ws, dws)):
+        jobs[i].W, jobs[i].X, jobs[i].dst, jobs[i].M, jobs[i].id_index = dw.ptr, dxs[i].ptr, dd.ptr + 4 * at, len(w), -1
+        at += len(w)
+    check(lib().b200_mul_mat_vec_q_multi(t, jobs, 2, row_size(t, K), K, total, K, N, None, 0, 0, None))
+    return dd.to_numpy(np.float32, (N, total))
+
+
+@pytest.mark.parametrize("t,K,M", [(Q4_0, 4096, 1024), (Q8_0, 2048, 256), (Q8_0, 4096, 1024), (Q8_0, 8192, 512), (Q4_K, 4096, 1536), (Q5_K, 2048, 1024), (Q6_K, 5120, 512), (Q6_K, 1280, 16)])
+def test_two_columns_of_few_rows_are_the_dp4a_forms(t, K, M):
+    """To the bit: jobs whose activations lie at different places have no other form."""
+    rng = np.random.default_rng(K + M + t)
+    w, x = random_blocks(rng, t, M, K), rng.standard_normal((2, K)).astype(np.float32)
+    want = two_jobs(t, [w[:M // 2], w[M // 2:]], [x, x.copy()], K, 2)
+    assert np.array_equal(H.mul_mat_vec_q(t, w, x, K, M), want)
+    assert close(want, O.mul_mat_q8_1(t, w, x, K, M))
+
+
+@pytest.mark.parametrize("t,K,N,M", [(Q4_K, 4096, 7, 2500), (Q6_K, 4096, 8, 20000), (Q4_0, 4096, 7, 76800), (Q8_0, 8192, 8, 40000), (Q5_K, 13824, 3, 5000), (Q4_K, 2048, 3, 50000),
+                                     (Q6_K, 5120, 4, 1184), (Q8_0, 4096, 3, 1200), (Q5_K, 7168, 2, 1201)])
+def test_many_row_tiles(t, K, N, M):
+    """Several row tiles a cluster and several batches of them (64 and, where shared memory holds no more, fewer), one tile a cluster with all warps: 1000 rows again and again,
+    which are to come out the same wherever they lie, and twice the same."""
+    each = min(M, 1000)
+    rng = np.random.default_rng(K + M + N + t)
+    w, x = random_blocks(rng, t, each, K), rng.standard_normal((N, K)).astype(np.float32)
+    dw, dx, dd = H.DeviceBuffer.from_numpy(np.tile(w, (-(-M // each), 1))[:M], pad=16), H.DeviceBuffer.from_numpy(x), H.DeviceBuffer(4 * N * M)
+    got = []
+    for _ in range(2):
+        check(lib().b200_mul_mat_vec_q(t, dw.ptr, row_size(t, K), dx.ptr, K, dd.ptr, M, K, M, N, None))
+        got.append(dd.to_numpy(np.float32, (N, M)))
+    assert np.array_equal(*got)
+    assert close(got[0][:, :each], O.mul_mat_q8_1(t, w, x, K, each))
+    assert np.array_equal(got[0], np.tile(got[0][:, :each], (1, -(-M // each)))[:, :M])
