@@ -457,7 +457,10 @@ static int dispatch_cols(MmvqParams &p, int N, cudaStream_t st, bool pdl) {
             if (rc != -1000) return rc;
         }
     }
-    if (!multi && N > 1 && !mmvq_fits<TYPE>(p, N)) {  // long rows: the columns' activations fill shared memory (13824 values: 7 or 8): half of them at a time
+    // Long rows, whose columns' activations fill shared memory: half of the columns at a time.  (K-quants, whose rows are whole blocks of 256, come here with three columns or
+    // more only when the tensor form has refused them, which holds more of them than dp4a does.)
+    constexpr bool KQ = TYPE == B200_TYPE_Q4_K || TYPE == B200_TYPE_Q5_K || TYPE == B200_TYPE_Q6_K;
+    if (!multi && N > 1 && ((KQ && N > 2) || !mmvq_fits<TYPE>(p, N))) {
         const int first = N / 2;
         MmvqParams q = p;
         int rc = dispatch_cols<TYPE>(q, first, st, pdl);
@@ -484,12 +487,16 @@ static int dispatch_cols(MmvqParams &p, int N, cudaStream_t st, bool pdl) {
     switch (N) {
         case 1: return launch_mmvq<TYPE, 1, false>(p, st, pdl);
         case 2: return launch_mmvq<TYPE, 2, false>(p, st, pdl);
-        case 3: return launch_mmvq<TYPE, 3, false>(p, st, pdl);
-        case 4: return launch_mmvq<TYPE, 4, false>(p, st, pdl);
-        case 5: return launch_mmvq<TYPE, 5, false>(p, st, pdl);
-        case 6: return launch_mmvq<TYPE, 6, false>(p, st, pdl);
-        case 7: return launch_mmvq<TYPE, 7, false>(p, st, pdl);
-        case 8: return launch_mmvq<TYPE, 8, false>(p, st, pdl);
+    }
+    if constexpr (!KQ) {
+        switch (N) {
+            case 3: return launch_mmvq<TYPE, 3, false>(p, st, pdl);
+            case 4: return launch_mmvq<TYPE, 4, false>(p, st, pdl);
+            case 5: return launch_mmvq<TYPE, 5, false>(p, st, pdl);
+            case 6: return launch_mmvq<TYPE, 6, false>(p, st, pdl);
+            case 7: return launch_mmvq<TYPE, 7, false>(p, st, pdl);
+            case 8: return launch_mmvq<TYPE, 8, false>(p, st, pdl);
+        }
     }
     set_error("b200_mul_mat_vec_q: N=%d out of range 1..8", N);
     return B200_ERR_INVALID;
