@@ -123,8 +123,8 @@ B200_API int b200_quantize_q8_1(const float *x, int64_t x_stride, void *y, int64
  * The activation is quantised to q8_1 inside the kernel (same arithmetic as b200_quantize_q8_1).
  * K must be a multiple of 256 for K-quants and of 32 for Q4_0/Q8_0.  W must be 16-byte aligned and
  * readable up to the next 16-byte boundary past its last row (true for any cudaMalloc'ed tensor). */
-/* q4_0, q8_0, q4_K, q5_K and q6_K with two columns or more: the order of a row's sums, and with it the last bits of the results, may follow from how many rows the launch
- * has (over all its jobs).  The same call gives the same bits. */
+/* q4_0, q8_0, q4_K, q5_K and q6_K with four columns or more: the order of a row's sums, and with it the last bits of the results, may follow from how many rows the launch
+ * has (over all its jobs).  With fewer columns it does not.  The same call gives the same bits. */
 B200_API int b200_mul_mat_vec_q(int type, const void *W, size_t w_row_bytes, const float *X, int64_t x_stride,
                                 float *dst, int64_t dst_stride, int64_t K, int64_t M, int64_t N, b200_stream_t stream);
 

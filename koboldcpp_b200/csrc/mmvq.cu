@@ -418,16 +418,6 @@ static int launch_mmvq3(MmvqParams &p, cudaStream_t st, bool pdl) {
 #include "mmvq_mma.cuh"
 namespace b200 {
 
-// Two columns of few and long rows, where the tensor form is not ahead yet: what bounds such a launch is the way from the first load of the columns to their quants, which is
-// longer there.  Tensor -> dp4a, us: 1024 rows of 4096 q4_0 5.2 -> 4.9, q8_0 6.6 -> 5.2, q4_K 5.3 -> 4.7, q5_K 5.6 -> 4.8, q6_K 6.0 -> 5.1; 256 x 2048 q4_K 3.9 -> 3.6, q6_K 4.1 -> 3.8; 512 x
-// 5120 q8_0 7.6 -> 6.0; 512 x 8192 q5_K 6.8 -> 6.4.  Level at 1024 values (q8_0 512 rows 3.8, 3.8), 1536 rows (q4_K 2048 values 4.4, 4.3; q6_K 5120 7.6, 7.8) and 11008 (q8_0 512 rows 8.4 -> 9.7).
-template <int TYPE>
-static bool mmvq_few(const MmvqParams &p, int N) {
-    if (N != 2) return false;
-    if (TYPE == B200_TYPE_Q4_0) return p.K == 4096 && p.total_rows <= 1200;
-    return p.K > 1024 && p.K <= 8192 && p.total_rows <= (p.K <= 4096 ? 1536 : 1200);
-}
-
 template <int TYPE>
 static int dispatch_cols(MmvqParams &p, int N, cudaStream_t st, bool pdl) {
     const bool multi = p.n_jobs > 1 || p.ids != nullptr;
@@ -443,11 +433,14 @@ static int dispatch_cols(MmvqParams &p, int N, cudaStream_t st, bool pdl) {
     // Several columns of one activation matrix: the integer tensor cores, whose cost hardly grows with the columns; dp4a spends 8 instructions a column and 32 weights.
     // dp4a -> tensor, us, at 2 / 4 / 8 columns: 22016 x 4096 q4_0 25.6 -> 18.8 / 39.1 -> 20.4 / - ; 32000 x 2048 q8_0 25.6 -> 17.5 / 37.2 -> 18.9 / 64.7 -> 21.3;
     // 32000 x 2048 q4_K 22.8 -> 14.1 at 2; 5120 x 13824 q6_K 36.9 -> 26.9 at 4; 2048 x 2048 q4_0 4.5 -> 4.1 / 6.7 -> 4.7 / 12.1 -> 5.8; 256 x 256 3.7 -> 3.5 / 5.5 -> 3.6 /
-    // 9.5 -> 3.9.
+    // 9.5 -> 3.9.  Two and three columns of few rows lose: what bounds such a launch is the way from the first load of the columns to their quants, which is longer here.  Two
+    // columns, 1024 rows of 4096 q4_0 4.9 -> 5.2, q8_0 5.2 -> 6.6, q4_K 4.7 -> 5.3, q5_K 4.8 -> 5.6, q6_K 5.1 -> 6.0; 512 rows of 1536 q5_K 3.6 -> 4.4, 2048 q6_K 3.8 -> 4.2, 5120 q8_0 6.0 -> 7.7,
+    // 6144 6.1 -> 8.7 (0.71, the least of all), 8192 q5_K 6.4 -> 6.8; level at 2048 rows.  Three columns, 512 rows of 4096 q8_0 6.0 -> 7.0, q5_K 5.8 -> 6.3, q6_K 5.8 -> 6.6; level at 1536.  They stay
+    // here, because with fewer than four columns a row's bits do not depend on the rows of its launch: one kernel, cut in one way, has to take few rows and many.
     if constexpr (TYPE == B200_TYPE_Q4_0 || TYPE == B200_TYPE_Q8_0 || TYPE == B200_TYPE_Q4_K || TYPE == B200_TYPE_Q5_K || TYPE == B200_TYPE_Q6_K) {
         bool same_x = p.ids == nullptr && p.K % 256 == 0;
         for (int j = 1; j < p.n_jobs; j++) same_x = same_x && p.jobs[j].X == p.jobs[0].X;
-        if (N >= 2 && same_x && (!multi || N <= 4) && !mmvq_few<TYPE>(p, N)) {
+        if (N >= 2 && same_x && (!multi || N <= 4)) {
             int rc = B200_OK;
             if (multi) {  // (several jobs have a limit of rows, whichever kernel serves them)
                 MmvqPlan pl;
@@ -457,10 +450,10 @@ static int dispatch_cols(MmvqParams &p, int N, cudaStream_t st, bool pdl) {
             if (rc != -1000) return rc;
         }
     }
-    // Long rows, whose columns' activations fill shared memory: half of the columns at a time.  (K-quants, whose rows are whole blocks of 256, come here with three columns or
-    // more only when the tensor form has refused them, which holds more of them than dp4a does.)
+    // Long rows, whose columns' activations fill shared memory: half of the columns at a time.  (K-quants, whose rows are whole blocks of 256, come here only when the tensor
+    // form has refused them, which holds more of them than dp4a does.)
     constexpr bool KQ = TYPE == B200_TYPE_Q4_K || TYPE == B200_TYPE_Q5_K || TYPE == B200_TYPE_Q6_K;
-    if (!multi && N > 1 && ((KQ && N > 2) || !mmvq_fits<TYPE>(p, N))) {
+    if (!multi && N > 1 && (KQ || !mmvq_fits<TYPE>(p, N))) {
         const int first = N / 2;
         MmvqParams q = p;
         int rc = dispatch_cols<TYPE>(q, first, st, pdl);
@@ -486,10 +479,10 @@ static int dispatch_cols(MmvqParams &p, int N, cudaStream_t st, bool pdl) {
     }
     switch (N) {
         case 1: return launch_mmvq<TYPE, 1, false>(p, st, pdl);
-        case 2: return launch_mmvq<TYPE, 2, false>(p, st, pdl);
     }
     if constexpr (!KQ) {
         switch (N) {
+            case 2: return launch_mmvq<TYPE, 2, false>(p, st, pdl);
             case 3: return launch_mmvq<TYPE, 3, false>(p, st, pdl);
             case 4: return launch_mmvq<TYPE, 4, false>(p, st, pdl);
             case 5: return launch_mmvq<TYPE, 5, false>(p, st, pdl);

@@ -12,7 +12,7 @@
 //   * the activations of all columns are quantised once per CTA into shared memory, in the order in which a lane reads its operand.  All loads of
 //     MV_U x 4096 values are in flight at once, and the norm's squares are taken from the same registers;
 //   * KS warps share a row tile, each a part of K; their sums meet in shared memory in a fixed order; two CTAs share row tiles, half of K each, where the columns
-//     are long or row tiles few.  How K is cut follows from K, the columns and the rows of the launch.
+//     are long or, with four columns or more, row tiles few.
 #pragma once
 
 namespace b200 {
@@ -593,19 +593,22 @@ static int launch_mmvq_mma(const MmvqParams &m, int N, cudaStream_t st, bool pdl
     const int rc = device_props();
     if (rc) return rc;
     const int nsb = (int)(m.K / 256);
-    // How K is cut, into halves for two CTAs and among warps.  Two CTAs share row tiles where the columns are many enough to quantise that half the work makes up for
-    // the meeting (about 1 us): 5120 x 13824 q6_K at 4 columns 32.3 -> 27.8 us, 4096 x 11008 q4_K 17.0 -> 15.8; 4096 x 4096 q4_0 at 4 columns 8.4 -> 8.6, 22016 x 4096
-    // q4_K 21.8 -> 23.4.  Where half of the SMs would have no tile, from fewer values on: 512 rows, one CTA -> two with all warps on a tile, 4096 q8_0 at 3 columns
-    // 7.7 -> 6.5, 5120 q6_K at 4 10.5 -> 8.9, 11008 q5_K at 2 9.9 -> 7.8; 3072 q6_K at 3 (9216 values) 6.2 -> 6.4, 4096 q4_0 at 2 (8192) 5.1 -> 5.4.
-    p.c = nsb >= 2 && m.K * N >= (tiles > g_sm_count / 2 ? 26000 : m.K >= 4096 ? 12000 : 13000) ? 2 : 1;
+    // How K is cut, into halves for two CTAs and among warps.  With two and three columns it follows from K and the columns alone, so that a row's bits do not depend on the
+    // launch it is part of; with more, where few rows leave most of the device idle, from the rows too.  Two CTAs share row tiles where the columns are many enough to quantise
+    // that half the work makes up for the meeting (about 1 us): 5120 x 13824 q6_K at 4 columns 32.3 -> 27.8 us, 4096 x 11008 q4_K 17.0 -> 15.8; 4096 x 4096 q4_0 at 4 columns
+    // 8.4 -> 8.6, 22016 x 4096 q4_K 21.8 -> 23.4.  Where half of the SMs would have no tile, from fewer values on: 512 rows, one CTA -> two with all warps on a tile, 4 columns,
+    // 4096 q8_0 8.7 -> 6.6, 5120 q6_K 10.5 -> 8.9; 3072 q4_0 (12288 values) 5.2 -> 5.3.  Two and three columns over 16000 values: level
+    // where rows are many (22016 x 8192 q4_K at 2 columns 1.11 and 1.07 of dp4a's speed), 512 x 8192 q6_K at 2 columns 8.6 -> 7.3, q4_0 at 3 8.5 -> 7.0.
+    const bool by_rows = N >= 4;
+    p.c = nsb >= 2 && m.K * N >= (!by_rows ? 16000 : tiles > g_sm_count / 2 ? 26000 : m.K >= 4096 ? 12000 : 13000) ? 2 : 1;
     const int per = (nsb + p.c - 1) / p.c;
     // (warps a tile: more of them help where rows are few, and meet more often where they are many.  One CTA, 2 columns, with 1, 2, 4, 8 warps: 4096 x 4096 q4_0 9.8,
     // 7.4, 7.1, 7.2 us, 22016 x 4096 q4_K 18.3, 19.3, 19.5, 20.8; two CTAs, 4 columns, 5120 x 13824 q6_K 32.6, 27.8, 29.3, 28.2)
     p.ks = p.c == 2 ? (per >= 24 ? 8 : per >= 16 ? 4 : 2) : per >= 32 ? 8 : per >= 8 ? 4 : per >= 4 ? 2 : 1;
-    // Few tiles leave warps idle that could take a part: with rows of up to 1792 values (1024 x 512 q5_K at 2 / 4 columns 4.8 -> 4.2 / 4.6 -> 4.0), and with two CTAs.  One CTA's
-    // longer rows are level or slower so (512 x 5120 q4_0 at 4 columns 7.3 -> 8.2): what they wait for is the quantisation.
+    // Few tiles leave warps idle that could take a part: with rows of up to 1792 values (1024 x 512 q5_K at 4 columns 4.6 -> 4.0), and with two CTAs.  One CTA's longer rows are
+    // level or slower so (512 x 5120 q4_0 at 4 columns 7.3 -> 8.2): what they wait for is the quantisation.
     const int64_t at_once = g_sm_count / p.c, tiles_each = (tiles + at_once - 1) / at_once;
-    if (per < 8 || p.c == 2) {
+    if (by_rows && (per < 8 || p.c == 2)) {
         for (int ks = MV_NW / (tiles_each <= 1 ? 1 : tiles_each <= 2 ? 2 : tiles_each <= 4 ? 4 : MV_NW); ks > p.ks; ks /= 2)
             if (ks <= per) p.ks = ks;
     }

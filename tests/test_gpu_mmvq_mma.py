@@ -194,26 +194,19 @@ def test_activations_of_one_sign(t, K, N):
     assert c < 2
 
 
-def two_jobs(t, ws, xs, K, N):
-    """Two matrices in one launch, each with the activations at an address of its own."""
-    total = sum(len(w) for w in ws)
-    dws, dxs, dd = [H.DeviceBuffer.from_numpy(w, pad=16) for w in ws], [H.DeviceBuffer.from_numpy(x) for x in xs], H.DeviceBuffer(4 * N * total)
-    jobs, at = (GemvJob * 2)(), 0
-    for i, (w, dw) in enumerate(zip(ws, dws)):
-        jobs[i].W, jobs[i].X, jobs[i].dst, jobs[i].M, jobs[i].id_index = dw.ptr, dxs[i].ptr, dd.ptr + 4 * at, len(w), -1
-        at += len(w)
-    check(lib().b200_mul_mat_vec_q_multi(t, jobs, 2, row_size(t, K), K, total, K, N, None, 0, 0, None))
-    return dd.to_numpy(np.float32, (N, total))
-
-
-@pytest.mark.parametrize("t,K,M", [(Q4_0, 4096, 1024), (Q8_0, 2048, 256), (Q8_0, 4096, 1024), (Q8_0, 8192, 512), (Q4_K, 4096, 1536), (Q5_K, 2048, 1024), (Q6_K, 5120, 512), (Q6_K, 1280, 16)])
-def test_two_columns_of_few_rows_are_the_dp4a_forms(t, K, M):
-    """To the bit: jobs whose activations lie at different places have no other form."""
-    rng = np.random.default_rng(K + M + t)
-    w, x = random_blocks(rng, t, M, K), rng.standard_normal((2, K)).astype(np.float32)
-    want = two_jobs(t, [w[:M // 2], w[M // 2:]], [x, x.copy()], K, 2)
-    assert np.array_equal(H.mul_mat_vec_q(t, w, x, K, M), want)
-    assert close(want, O.mul_mat_q8_1(t, w, x, K, M))
+@pytest.mark.parametrize("t", [Q4_0, Q8_0, Q4_K, Q5_K, Q6_K])
+@pytest.mark.parametrize("K,N", [(512, 2), (2048, 3), (4096, 2), (4096, 3), (13824, 2), (13824, 3)])
+def test_bits_of_two_and_three_columns_do_not_follow_from_the_rows(t, K, N):
+    """One and two CTAs a row tile: rows of a large launch, of a small one, of a single one, and in a launch of several matrices."""
+    M = 5000
+    rng = np.random.default_rng(K + N + t)
+    w, x = random_blocks(rng, t, M, K), rng.standard_normal((N, K)).astype(np.float32)
+    whole = H.mul_mat_vec_q(t, w, x, K, M)
+    for part in (slice(0, 1000), slice(4321, 4322), slice(100, 2500)):
+        assert np.array_equal(H.mul_mat_vec_q(t, w[part], x, K, part.stop - part.start), whole[:, part])
+    parts = [slice(0, 300), slice(300, 301), slice(301, 1400)]
+    for got, part in zip(H.mul_mat_vec_q_multi(t, [w[p] for p in parts], x, K), parts):
+        assert np.array_equal(got, whole[:, part])
 
 
 @pytest.mark.parametrize("t,K,N,M", [(Q4_K, 4096, 7, 2500), (Q6_K, 4096, 8, 20000), (Q4_0, 4096, 7, 76800), (Q8_0, 8192, 8, 40000), (Q5_K, 13824, 3, 5000), (Q4_K, 2048, 3, 50000),
