@@ -729,18 +729,18 @@ static inline int pair_stages(int bn, int steps, int raw) {
     return n > PAIR_MAX_STAGES ? PAIR_MAX_STAGES : n;
 }
 static inline bool pair_parts_fit(int bn, int steps, int raw) { return pair_stages(bn, steps, raw) * steps * (MQ_BM * MQ_BK * 2 + bn * MQ_BK) >= bn * MQ_BM * 4; }
-// clusters[ks]: clusters of ks pairs that the device holds at once
+// clusters[ks]: clusters of ks pairs that the device holds at once, not more for a larger ks
 static inline PairPlan mmq_pair_plan(int64_t M, int64_t N, int64_t K, int n_batch, const int *clusters, double unpack, int unit, int steps_stage, int raw) {
     PairPlan best = {256, 1, 1};
     double best_cost = -1;
-    const unsigned mt = (unsigned)((M + 255) / 256), n = (unsigned)N, np = (unsigned)clusters[1];  // (32-bit: the divisions of up to 30 candidates are host time of each call)
+    const unsigned mt = (unsigned)((M + 255) / 256), n = (unsigned)N, np = (unsigned)clusters[1];  // (32-bit: the divisions of every width, one for each 32 columns, are host time of each call)
     const int units = (int)(K / MQ_BK / unit);
     for (unsigned parts = (n + 255) / 256, last = (n + 31) / 32; parts <= last; parts++) {
         const unsigned even = ((n + parts - 1) / parts + 15) / 16 * 16, bn = even < 32 ? 32 : even, nt = (n + bn - 1) / bn;
         const double dense = 1.25e-3 * bn < 0.2 ? 0.2 : 1.25e-3 * bn, step = unpack > 0 ? pair_step_us(unpack, 1.83e-3 * bn) : dense;
         const uint64_t tiles = (uint64_t)mt * nt * n_batch;
         for (int ks = 1; ks <= PAIR_MAX_SPLIT && ks <= units; ks++) {
-            if (ks > 1 && (tiles > (uint64_t)clusters[ks] || !pair_parts_fit((int)bn, steps_stage, raw))) continue;
+            if (ks > 1 && (tiles > (uint64_t)clusters[ks] || !pair_parts_fit((int)bn, steps_stage, raw))) break;  // (there are no more of the larger clusters)
             const double waves = tiles <= np ? 1.0 : (double)((tiles + np - 1) / np);
             const double cost = waves * ((units + ks - 1) / ks * unit * step + 1.0) + (ks == 1 ? 0.012 * bn : 1.6 + 0.2 * ks + 0.008 * bn);
             if (best_cost < 0 || cost < 0.98 * best_cost) { best_cost = cost; best = {(int)bn, ks, (int)nt}; }
@@ -784,21 +784,27 @@ static int mmq_pair_launch(const MmqParams &q, int64_t n_pad, int64_t w_rows_per
     at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = at;
-    static PairDevice devices[16];  // (attributes and what fits are a device's; two threads that come first find the same)
+    static PairDevice devices[16];  // (attributes and what fits are a device's)
+    static std::mutex first;
     int cur_dev = 0;
     B200_CUDA_TRY(cudaGetDevice(&cur_dev));
     PairDevice &dev = devices[cur_dev & 15];
     if (!dev.known.load(std::memory_order_acquire)) {
-        B200_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, PAIR_SMEM));
-        B200_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-        dev.clusters[1] = sm_count() / 2;
-        for (int ks = 2; ks <= PAIR_MAX_SPLIT; ks++) {
-            cfg.gridDim = dim3((unsigned)(2 * ks));
-            at[0].val.clusterDim.x = (unsigned)(2 * ks);
-            cfg.numAttrs = 1;
-            if (cudaOccupancyMaxActiveClusters(&dev.clusters[ks], kern, &cfg) != cudaSuccess) { dev.clusters[ks] = 0; cudaGetLastError(); }
+        // (one thread finds out and writes it down, once: another that comes meanwhile would plan with what is half written)
+        std::lock_guard<std::mutex> lock(first);
+        if (!dev.known.load(std::memory_order_relaxed)) {
+            B200_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, PAIR_SMEM));
+            B200_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+            dev.clusters[1] = sm_count() / 2;
+            for (int ks = 2; ks <= PAIR_MAX_SPLIT; ks++) {
+                cfg.gridDim = dim3((unsigned)(2 * ks));
+                at[0].val.clusterDim.x = (unsigned)(2 * ks);
+                cfg.numAttrs = 1;
+                if (cudaOccupancyMaxActiveClusters(&dev.clusters[ks], kern, &cfg) != cudaSuccess) { dev.clusters[ks] = 0; cudaGetLastError(); }
+                if (dev.clusters[ks] > dev.clusters[ks - 1]) dev.clusters[ks] = dev.clusters[ks - 1];
+            }
+            dev.known.store(true, std::memory_order_release);
         }
-        dev.known.store(true, std::memory_order_release);
     }
     PairParams p;
     p.q = q;
