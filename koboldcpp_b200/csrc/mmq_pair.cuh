@@ -721,7 +721,8 @@ __global__ void __launch_bounds__(pair_threads<TYPE>(), 1) mmq_pair_kernel(const
 // 11.0, 10.8, 10.1, 10.2, 9.3 in two .. eight), and a cluster takes one tile, so that there are no more tiles than clusters.  Widths are N / 1, N / 2, ...
 // rounded up to 16.
 
-struct PairPlan { int bn, ksplit, n_tiles_n; };
+constexpr double PAIR_NEXT_US = 4;  // a launch behind another: its start, and the end of the one in front that is no longer hidden (3 .. 6 measured)
+struct PairPlan { int bn, ksplit, n_tiles_n; double tile, cost; };  // microseconds of a tile, of all
 static inline double pair_step_us(double a, double b) { const double a3 = a * a * a, b3 = b * b * b; return sqrt(cbrt(a3 * a3 + b3 * b3)); }
 // stages of the ring beside `raw` bytes; a tile's parts lie in them when they meet
 static inline int pair_stages(int bn, int steps, int raw) {
@@ -731,7 +732,7 @@ static inline int pair_stages(int bn, int steps, int raw) {
 static inline bool pair_parts_fit(int bn, int steps, int raw) { return pair_stages(bn, steps, raw) * steps * (MQ_BM * MQ_BK * 2 + bn * MQ_BK) >= bn * MQ_BM * 4; }
 // clusters[ks]: clusters of ks pairs that the device holds at once, not more for a larger ks
 static inline PairPlan mmq_pair_plan(int64_t M, int64_t N, int64_t K, int n_batch, const int *clusters, double unpack, int unit, int steps_stage, int raw) {
-    PairPlan best = {256, 1, 1};
+    PairPlan best = {256, 1, 1, 0, 0};
     double best_cost = -1;
     const unsigned mt = (unsigned)((M + 255) / 256), n = (unsigned)N, np = (unsigned)clusters[1];  // (32-bit: the divisions of every width, one for each 32 columns, are host time of each call)
     const int units = (int)(K / MQ_BK / unit);
@@ -742,11 +743,23 @@ static inline PairPlan mmq_pair_plan(int64_t M, int64_t N, int64_t K, int n_batc
         for (int ks = 1; ks <= PAIR_MAX_SPLIT && ks <= units; ks++) {
             if (ks > 1 && (tiles > (uint64_t)clusters[ks] || !pair_parts_fit((int)bn, steps_stage, raw))) break;  // (there are no more of the larger clusters)
             const double waves = tiles <= np ? 1.0 : (double)((tiles + np - 1) / np);
-            const double cost = waves * ((units + ks - 1) / ks * unit * step + 1.0) + (ks == 1 ? 0.012 * bn : 1.6 + 0.2 * ks + 0.008 * bn);
-            if (best_cost < 0 || cost < 0.98 * best_cost) { best_cost = cost; best = {(int)bn, ks, (int)nt}; }
+            const double tile = (units + ks - 1) / ks * unit * step + 1.0, cost = waves * tile + (ks == 1 ? 0.012 * bn : 1.6 + 0.2 * ks + 0.008 * bn);
+            if (best_cost < 0 || cost < 0.98 * best_cost) { best_cost = cost; best = {(int)bn, ks, (int)nt, tile, cost}; }
         }
     }
     return best;
+}
+
+// Rows whose tiles are whole waves, if the rest is better off in a launch of its own, where its few tiles are taken in parts of K; else 0.  (Two halves of K, added into a zeroed
+// result, once did this for products of a little more than a wave.  One launch -> two, us: 20480 x 2560 over 40 columns q6_K 42.8 -> 35.1, with the halves 39.1, q8_0 38.9 -> 32.9, 37.1;
+// 11008 x 4096 q6_K over 280 69.6 -> 55.0, 65.1; 28672 x 4096 q4_K over 280 90.4 -> 79.8, 96.7.)  A rest of more tiles than there are clusters of two pairs stays: 13824 x 5120 q6_K over 280, 84.
+static inline int64_t mmq_pair_whole_waves(const PairPlan &pl, int64_t M, int64_t N, int64_t K, const int *clusters, double unpack, int unit, int steps_stage, int raw) {
+    const int64_t np = clusters[1], nt = pl.n_tiles_n, tiles = (M + 255) / 256 * nt, mt = tiles / np * np / nt;
+    if (pl.ksplit > 1 || tiles <= np || tiles % np == 0 || mt <= 0 || mt * 256 >= M) return 0;
+    const double whole = (double)((mt * nt + np - 1) / np) * pl.tile + 0.012 * pl.bn;
+    if (whole + PAIR_NEXT_US > 0.93 * pl.cost) return 0;
+    const PairPlan rest = mmq_pair_plan(M - mt * 256, N, K, 1, clusters, unpack, unit, steps_stage, raw);
+    return whole + PAIR_NEXT_US + rest.cost < 0.93 * pl.cost ? mt * 256 : 0;
 }
 
 // what the device holds at once, one CTA an SM: clusters of 1 .. PAIR_MAX_SPLIT pairs
@@ -820,7 +833,19 @@ static int mmq_pair_launch(const MmqParams &q, int64_t n_pad, int64_t w_rows_per
         p.q.ksplit = 1;
         p.share = SHARE;
     } else {
-        const PairPlan pl = mmq_pair_plan(q.M, q.N, q.K, q.n_batch, dev.clusters, pair_unpack_us<TYPE>(), TYPE == B200_TYPE_BF16 ? 1 : 4, pair_steps<TYPE>(), raw_bytes(TYPE));
+        constexpr int UNIT = TYPE == B200_TYPE_BF16 ? 1 : 4;
+        const PairPlan pl = mmq_pair_plan(q.M, q.N, q.K, q.n_batch, dev.clusters, pair_unpack_us<TYPE>(), UNIT, pair_steps<TYPE>(), raw_bytes(TYPE));
+        const int64_t rows = q.n_batch > 1 ? 0 : mmq_pair_whole_waves(pl, q.M, q.N, q.K, dev.clusters, pair_unpack_us<TYPE>(), UNIT, pair_steps<TYPE>(), raw_bytes(TYPE));
+        if (rows) {
+            MmqParams part = q;
+            part.M = rows;
+            const int rc = mmq_pair_launch<TYPE, GROUPED, SHARE>(part, n_pad, w_rows_per_product, max_tiles_n, grouped_bn, st);
+            if (rc != B200_OK) return rc;
+            part.W += (size_t)rows * q.w_row_bytes;
+            part.dst += rows;
+            part.M = q.M - rows;
+            return mmq_pair_launch<TYPE, GROUPED, SHARE>(part, n_pad, w_rows_per_product, max_tiles_n, grouped_bn, st);
+        }
         p.bn = pl.bn;
         p.box = pl.bn / 2;
         p.n_tiles_n = pl.n_tiles_n;

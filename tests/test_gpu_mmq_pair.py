@@ -130,6 +130,27 @@ def test_rows_of_activations_of_any_length(K):
     assert rel(product(BF16, bits.view(np.uint8), x, K, M), want) < 4e-3
 
 
+@pytest.mark.parametrize("t,K,M,N,whole", [(Q6_K, 2560, 20483, 40, 18944), (Q8_0, 2560, 20000, 100, 18944), (Q4_K, 2560, 19300, 200, 18944), (Q6_K, 4096, 11008, 280, 9472), (BF16, 4096, 19300, 40, 18944)])
+def test_rows_behind_whole_waves(t, K, M, N, whole):
+    """A little more than a wave of tiles (74 pairs): the rows behind row `whole` are a launch of their own, in parts of K.  Rows at its edge and a sample of the others, and
+    nothing beyond the last row."""
+    rng = np.random.default_rng(K + M + N + t)
+    each, x = 500, rng.standard_normal((N, K)).astype(np.float32)
+    if t == BF16:
+        bits = (rng.standard_normal((each, K)).astype(np.float32).view(np.uint32) >> 16).astype(np.uint16)
+        w, W = bits.view(np.uint8), (bits.astype(np.uint32) << 16).view(np.float32).astype(np.float64)
+    else:
+        w = random_blocks(rng, t, each, K).reshape(each, -1)
+        W = np.stack([O.dequantize(t, r, K) for r in w]).astype(np.float64)
+    at = rng.integers(0, each, M)  # which of the rows each is
+    got = product(t, w[at], x, K, M, dst_stride=M + 3)
+    assert np.isnan(got[:, M:]).all()
+    want = (x.astype(np.float64) @ W.T)[:, at]
+    for rows in (slice(0, M), slice(whole - 256, whole), slice(whole, whole + 256), slice(M - 30, M)):
+        assert rel(got[:, rows], want[:, rows]) < 6e-3, rows
+    assert np.array_equal(got, product(t, w[at], x, K, M, dst_stride=M + 3), equal_nan=True)
+
+
 @pytest.mark.parametrize("T", [40, 150])
 def test_experts_without_a_valid_pair(T):
     """No tile at all: nothing is stored, and the launch ends.  (Up to 32 pairs an expert on average, and more: a kernel each.)"""
