@@ -225,3 +225,33 @@ def test_many_row_tiles(t, K, N, M):
     assert np.array_equal(*got)
     assert close(got[0][:, :each], O.mul_mat_q8_1(t, w, x, K, each))
     assert np.array_equal(got[0], np.tile(got[0][:, :each], (1, -(-M // each)))[:, :M])
+
+
+@pytest.mark.parametrize("scale", ["any", "halves", "edges"])
+@pytest.mark.parametrize("N", [2, 4, 8])
+def test_quants_of_the_columns(N, scale):
+    """What b200_quantize_q8_1 makes of the columns, seen through q8_0 rows with a single 1: scale times quant, exact in f32.  Values of every size, values halfway between two
+    quants, and blocks whose largest value lies around the limits of the shortcut for its quotient."""
+    K = 1024
+    rng = np.random.default_rng(N)
+    w = np.zeros((K, K // 32, 34), np.uint8)
+    w[:, :, :2] = np.array([1], np.float16).view(np.uint8)
+    w[np.arange(K), np.arange(K) // 32, 2 + np.arange(K) % 32] = 1
+    dw, dd = H.DeviceBuffer.from_numpy(w.reshape(K, -1), pad=16), H.DeviceBuffer(4 * N * K)
+    for _ in range(20):
+        x = rng.standard_normal((N, K // 32, 32)).astype(np.float32)
+        if scale == "any":
+            x *= (np.float32(10) ** rng.uniform(-9, 5, (N, K // 32, 1))).astype(np.float32)
+        elif scale == "halves":
+            x = (rng.integers(-127, 127, x.shape) + np.float32(0.5)).astype(np.float32)
+            x[:, :, 7] = 127
+            x *= np.float32(2) ** rng.integers(-12, 8, (N, K // 32, 1)).astype(np.float32)
+        else:
+            x *= (np.float32(1e-25) * np.float32(2) ** rng.integers(-60, 4, (N, K // 32, 1)).astype(np.float32)).astype(np.float32)
+            x[:, ::5] = 0
+        x = x.reshape(N, K)
+        packed = H.quantize_q8_1(x).reshape(N, K // 32, 36)
+        want = packed[:, :, :2].copy().view(np.float16).astype(np.float32) * packed[:, :, 4:].view(np.int8).astype(np.float32)
+        dx = H.DeviceBuffer.from_numpy(x)
+        check(lib().b200_mul_mat_vec_q(Q8_0, dw.ptr, row_size(Q8_0, K), dx.ptr, K, dd.ptr, K, K, K, N, None))
+        assert np.array_equal(dd.to_numpy(np.float32, (N, K)), want.reshape(N, K))
