@@ -1,5 +1,5 @@
 #!/usr/bin/env python
-"""Round benchmark: batch-1 decode of a Llama-2-7B-shaped Q4_K_M model at 4k context on B200.
+"""Batch-1 decode of a Llama-2-7B-shaped Q4_K_M model at 4k context on B200.
 
 One "step" = one decoded token = one pass of the hot path (all MUL_MATs as decode GEMVs + FLASH_ATTN_EXT over the f16 KV
 cache + the small ops of the graph) through the ggml_backend boundary of libkcpp_b200.so.
@@ -14,7 +14,7 @@ Legs (all printed in ONE JSON line by rank 0):
              libkcpp_b200.so attached by ggml_backend_register, on a GGUF file of the workload (tools/make_gguf.py).
   cpu_baseline  the reference's own llama.cpp + CPU backend (oracle/_ref) decoding the same GGUF on this box's host cores
              (bounded sample: 16 tokens at n_kv = 4096).
-  tp_70b     auxiliary: BASELINE.json configs[4], ONE Llama-3-70B-shaped Q4_K_M model sharded over all N ranks (strong scaling,
+  tp_70b     auxiliary: ONE Llama-3-70B-shaped Q4_K_M model sharded over all N ranks (strong scaling,
              NCCL all-reduce / all-gather in the captured graph); at N = 1 the same model on one GPU, so 1 -> N speed-up is
              the ratio of the tp_70b values of two runs.
 `--impl reference` prints the CPU arm only.   N > 1: the headline legs run one 7B replica per rank (weak scaling, no data-path
@@ -303,7 +303,7 @@ TP_WORKLOAD = "llama3-70b-q4_k_m"
 
 
 def tp_leg(rank: int, world: int, local_rank: int, dist, steps: int, warmup: int) -> dict:
-    """BASELINE.json configs[4]: Llama-3-70B-shaped Q4_K_M, ONE model sharded over all `world` ranks (strong scaling): q/k/v, gate/up
+    """Llama-3-70B-shaped Q4_K_M, ONE model sharded over all `world` ranks (strong scaling): q/k/v, gate/up
     and the head split by rows (whole heads per rank), attn_output / ffn_down split along K with one NCCL all-reduce each, the
     logits all-gathered (koboldcpp_b200/tp.py, csrc/comm.cu).  world == 1 is the same model on one GPU (42 GB of weights).
     Timed like the main legs: resident replay with CUDA events on the backend stream, and the public call with host tokens in /
@@ -1313,7 +1313,7 @@ def main() -> int:
     ap.add_argument("--no-llamacpp", action="store_true", help="skip the e2e_llamacpp leg (reference llama.cpp driving the B200 backend)")
     ap.add_argument("--cpu-budget", type=float, default=18.0)
     ap.add_argument("--no-tp70", action="store_true", default=bool(os.environ.get("B200_BENCH_NO_TP70")),
-                    help="skip the auxiliary 70B tensor-parallel leg (BASELINE.json configs[4])")
+                    help="skip the auxiliary 70B tensor-parallel leg")
     ap.add_argument("--design", default="", choices=["", "genesun", "galirax", "zevopel", "medodra", "mafuzen", "tugezen"],
                     help="instead of the default workload: prefill / decode of this design at real layer shapes beside the closest existing model at equal size")
     ap.add_argument("--design-sizes", default="", help="comma-separated subset of the sizes of the design (genesun: " + ",".join(DESIGN_SIZES) + "; the others: " + ",".join(GALIRAX_SIZES) + ")")

@@ -1,5 +1,5 @@
 """Python mirror of include/b200_llama.h: the llama / mixtral decoder that drives the B200 backend through the
-ggml_backend vtables, plus synthetic (random-init) GGUF-shaped models for the configurations BASELINE.json names.
+ggml_backend vtables, plus synthetic (random-init) GGUF-shaped models of the benchmarks.
 
 The type mix per tensor follows llama_tensor_get_type for Q4_0 / Q4_K_M / Q5_K_M (src/llama.cpp:17979-18200).
 """
@@ -83,7 +83,7 @@ def _l():
 
 @dataclass
 class ModelShape:
-    """Hyper-parameters + quantisation mix of one BASELINE.json configuration."""
+    """Hyper-parameters + quantisation mix of one model shape."""
     name: str
     n_embd: int
     n_layer: int

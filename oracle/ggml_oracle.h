@@ -66,7 +66,7 @@ int orc_quantize_row(int type, const float *src, void *dst, int64_t k);
 float orc_vec_dot(int wtype, int64_t n, const void *w, const void *act);
 
 /* The integer arithmetic the GPU path performs: weights x 32-wide q8_1 activation blocks
- * (Appendix A of SURVEY.md; reference CUDA vecdotq.cuh:23-42,151-163,357-379,413-442,476-496),
+ * (reference CUDA vecdotq.cuh:23-42,151-163,357-379,413-442,476-496),
  * accumulated in double. Used for tight-tolerance kernel checks. */
 double orc_vec_dot_q8_1(int wtype, int64_t n, const void *w, const void *act_q8_1);
 

@@ -107,7 +107,7 @@ int main(int argc, char **argv) {
 
     const int n_vocab = llama_n_vocab(model);
     std::vector<llama_token> prompt((size_t)a.n_prompt);
-    for (int i = 0; i < a.n_prompt; i++) prompt[(size_t)i] = (llama_token)(((int64_t)i * 7919 + 1) % n_vocab);  // SURVEY.md 8(d): fixed ids
+    for (int i = 0; i < a.n_prompt; i++) prompt[(size_t)i] = (llama_token)(((int64_t)i * 7919 + 1) % n_vocab);  // fixed ids
 
     auto argmax2 = [&](const float *lg, float *margin) {
         int best = 0;
@@ -175,7 +175,7 @@ int main(int argc, char **argv) {
     }
 
     if (a.kv_fill > n_past) {
-        // "KV pre-filled to N cells"  without computing an N-token prompt on the CPU: take the session state
+        // KV pre-filled to N cells without computing an N-token prompt on the CPU: take the session state
         // the reference itself serialises (llama_state_get_data, src/llama.cpp:20825-20845: arch, output ids, logits, embeddings, then
         // cell_count, per-cell {pos, n_seq_id, seq_ids}, v_trans, n_layer, per layer {type, row size, rows} for K and for V), repeat
         // the prompt's cell rows cyclically up to N cells with positions 0..N-1, and hand it back through llama_state_set_data.

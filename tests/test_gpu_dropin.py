@@ -4,7 +4,7 @@ B200 backend -- then the reference's ggml_backend_compare_graph_backend (ggml-ba
 both the B200 backend and the reference CPU backend and hands the pair to the checker below.
 
 This is the method of upstream's test-backend-ops: normalised mean squared error per node.  Thresholds: 1e-6 for float ops;
-2e-3 for the quantised matmuls and attention (the CPU path quantises activations to q8_0 / q8_K, ours to q8_1: SURVEY.md 8c)."""
+2e-3 for the quantised matmuls and attention (the CPU path quantises activations to q8_0 / q8_K, ours to q8_1)."""
 from __future__ import annotations
 
 import ctypes as C

@@ -1,8 +1,8 @@
 """GPU parity tests: the CUDA path (through the C ABI, host buffers in/out) against the oracle on identical
-seeded inputs, against the reference's committed golden vectors, and -- at BASELINE.json's full sizes --
+seeded inputs, against the reference's committed golden vectors, and -- at the full sizes of a 7B decoder --
 through size-independent properties (linearity, row permutation, split invariance).
 
-Bars (SURVEY.md 8c): bit-exact for block dequantisation and q8_1 quantisation; for MUL_MAT / MUL_MAT_ID /
+Bars: bit-exact for block dequantisation and q8_1 quantisation; for MUL_MAT / MUL_MAT_ID /
 FLASH_ATTN_EXT a stated tolerance against (1) the integer-exact q8_1 contraction, (2) the CPU backend's result
 and (3) fp64 ground truth.
 """
@@ -17,7 +17,7 @@ pytestmark = pytest.mark.gpu
 WT = R.WEIGHT_TYPES
 NAME = R.TYPE_NAMES
 
-# tolerances (measured headroom: see DESIGN.md "Parity")
+# tolerances
 TOL_Q81 = 3e-5     # |gpu - exact q8_1 contraction| / max|ref|: only fp32 summation order differs
 TOL_CPU_NMSE = 2e-2  # ||gpu - cpu|| / ||cpu||: q8_1 (32-wide) vs q8_0/q8_K (CPU) activation rounding
 TOL_FA = {1: 2.5e-3, 8: 5e-3, 2: 5e-3}  # max abs error of attention outputs vs fp64 (outputs are O(0.3)); q8_0 KV also rounds Q to int8

@@ -1,6 +1,6 @@
 """GPU parity of whole-token decode through the ggml_backend boundary (b200_llama_* -> graph_compute) against the fp64
 restatement in llama_ref.py.  Tolerances: matmuls run on q8_1-quantised activations (like the reference CUDA path), which
-puts ~1e-2 relative noise on each matmul (SURVEY.md 8c row 1); logits of a 2-3 layer model must agree to 4e-2 of their
+puts ~1e-2 relative noise on each matmul; logits of a 2-3 layer model must agree to 4e-2 of their
 RMS and the executor variants (graphs / fusion on or off) must agree with each other far tighter than that."""
 from __future__ import annotations
 

@@ -1,11 +1,10 @@
-"""G1: greedy-token parity through the reference's REAL llama.cpp (north_star: "identical greedy-decoded
-tokens over 128 steps").
+"""Greedy-token parity through the reference's REAL llama.cpp: identical greedy-decoded tokens over 128 steps.
 
 oracle/_ref/llama_harness (the unmodified src/llama.cpp + ggml_backend_sched compiled from /root/reference) decodes a synthetic
 GGUF twice: on the reference CPU backend, and with libkcpp_b200.so attached by ggml_backend_register (Route 2).  Asserted:
   * the two greedy token streams are identical (prompt logits + 128 generated tokens);
   * the logits of every step agree to a stated relative L2 (the CPU path quantises activations to q8_0 / q8_K, the B200 path to
-    q8_1 for decode and bf16 for prompt batches: SURVEY.md 8c puts that noise at ~1e-2);
+    q8_1 for decode and bf16 for prompt batches: noise of ~1e-2);
   * the scheduler left only the token-embedding GET_ROWS on the CPU backend (llama.cpp keeps token_embd in a host buffer).
 The models are random-init with the reference quantiser (tools/make_gguf.py "margin model"; the margin statistics are asserted
 too, so a degenerate fixture cannot make the token check vacuous).
@@ -25,7 +24,7 @@ pytestmark = [pytest.mark.gpu, pytest.mark.skipif(not LC.available(), reason="or
 
 # Relative L2 of a step's logits, B200 vs the reference CPU backend.  Deep random-init models amplify rounding differences: the
 # reference's OWN builds disagree with each other by several percent on the C1 fixture (AVX2 vs AVX-512 build 4.5e-2, flash
-# attention on vs off 5.1e-2, f16 vs q8_0 KV 5.5e-2: measured with tools in this repo, see DESIGN.md).  The bar is therefore stated
+# attention on vs off 5.1e-2, f16 vs q8_0 KV 5.5e-2: measured with tools in this repo).  The bar is therefore stated
 # against that spread, measured in the same test: B200-vs-CPU <= 1.5 x (CPU flash-attention-on vs CPU flash-attention-off), with
 # an absolute floor for the shallow fixtures where the spread is tiny.
 LOGIT_TOL_FLOOR = 2.5e-2
@@ -68,7 +67,7 @@ def check_parity(cpu, gpu, a, b, min_margin_sigma):
 
 
 def test_c1_tinyllama_q4_0_pp128_tg128_identical_tokens():
-    """BASELINE configs[0]: TinyLlama-1.1B-shaped Q4_0 (output Q6_K), pp128 + tg128 greedy, f16 KV, flash attention."""
+    """TinyLlama-1.1B-shaped Q4_0 (output Q6_K), pp128 + tg128 greedy, f16 KV, flash attention."""
     model = G.build_fixture("tinyllama-1.1b-q4_0", layer_gain=3.0)
     cpu, gpu, a, b = both(model, 128, 128)
     assert len(cpu["tokens"]) == 129

@@ -1,6 +1,6 @@
 """GPU parity of the tcgen05 prefill GEMM (b200_mul_mat_q) against fp64 dequant(W).x (oracle dequantisation) and the
 reference CPU backend's MUL_MAT where oracle/_ref is present.  Operands are bf16 on the tensor cores (8 mantissa bits):
-the stated tolerance is 4e-3 relative L2 against fp64 -- tighter than the ~1e-2 of the q8 integer paths (SURVEY.md 8c)."""
+the stated tolerance is 4e-3 relative L2 against fp64 -- tighter than the ~1e-2 of the q8 integer paths."""
 from __future__ import annotations
 
 import numpy as np
@@ -110,7 +110,7 @@ def test_mul_mat_id_batched_invalid_ids_are_skipped():
 
 @pytest.mark.parametrize("K,M,N", [(5120, 13824, 512), (13824, 5120, 512), (5120, 5120, 512)])
 def test_mmq_c3_shapes_sampled_rows(K, M, N):
-    """BASELINE configs[2] (13B pp512) shapes; fp64 check on a sample of output rows (the full fp64 product is 36 G flop)."""
+    """Shapes of a 13B decoder and 512 tokens; fp64 check on a sample of output rows (the full fp64 product is 36 G flop)."""
     t = Q5_K if K != 13824 else Q6_K
     rng = np.random.default_rng(K + M)
     w = random_blocks(rng, t, M, K)

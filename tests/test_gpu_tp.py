@@ -1,4 +1,4 @@
-"""GPU (>= 2 devices) parity of the tensor-parallel decoder (SURVEY 8e, one process per GPU, NCCL): attn_output / ffn_down
+"""GPU (>= 2 devices) parity of the tensor-parallel decoder (one process per GPU, NCCL): attn_output / ffn_down
 split along K + all-reduce, everything else split by rows, logits all-gathered -- against the same model on one GPU."""
 from __future__ import annotations
 

@@ -52,7 +52,7 @@ def test_vec_dot_and_mul_mat_golden(golden, t):
 @pytest.mark.parametrize("t", WT, ids=[NAME[t] for t in WT])
 def test_q8_1_contraction_close_to_cpu_and_fp64(golden, t):
     """The GPU-path arithmetic (q8_1 activations) vs the CPU path (q8_0/q8_K) vs fp64 dequant(W)@x.
-    This measures the tolerance the GPU parity tests use (SURVEY 8c)."""
+    This measures the tolerance the GPU parity tests use."""
     w, x = golden[f"mm_{NAME[t]}_w"], golden["mm_x"]
     K, M = x.shape[1], w.shape[0]
     wd = np.stack([O.dequantize(t, r, K) for r in w]).astype(np.float64)

@@ -1,4 +1,4 @@
-"""Auxiliary measurements of the BASELINE.json configurations that are not the round bench line (bench.py is configs[1]):
+"""Auxiliary measurements of model shapes that bench.py does not measure:
   C3  Llama-2-13B-shaped Q5_K_M (Q6_K mix): pp512 prefill through the tensor-core GEMM + multi-column attention
   C4  Mixtral-8x7B-shaped Q4_K_M: batch-1 decode with MUL_MAT_ID expert GEMVs and a q8_0 KV cache at n_kv = 32768
   C1  TinyLlama-1.1B-shaped Q4_0: pp128 + tg128 (the reference's CPU-runnable case, here on the GPU)

@@ -1,4 +1,4 @@
-"""Synthetic (random-init) GGUF models of the shapes BASELINE.json names.
+"""Synthetic (random-init) GGUF models of the benchmarks' shapes.
 
     python tools/make_gguf.py --shape tinyllama-1.1b-q4_0 --out /tmp/tiny.gguf [--quantizer reference|blocks] [--layers N]
 
