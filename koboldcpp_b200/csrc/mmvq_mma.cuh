@@ -596,7 +596,8 @@ static int launch_mmvq_mma(const MmvqParams &m, int N, cudaStream_t st, bool pdl
     // How K is cut, into halves for two CTAs and among warps.  With two and three columns it follows from K and the columns alone, so that a row's bits do not depend on the
     // launch it is part of; with more, where few rows leave most of the device idle, from the rows too.  Two CTAs share row tiles where the columns are many enough to quantise
     // that half the work makes up for the meeting (about 1 us): 5120 x 13824 q6_K at 4 columns 32.3 -> 27.8 us, 4096 x 11008 q4_K 17.0 -> 15.8; 4096 x 4096 q4_0 at 4 columns
-    // 8.4 -> 8.6, 22016 x 4096 q4_K 21.8 -> 23.4.  Where half of the SMs would have no tile, from fewer values on: 512 rows, one CTA -> two with all warps on a tile, 4 columns,
+    // 8.4 -> 8.6, 22016 x 4096 q4_K 21.8 -> 23.4.  (The line is not sharp: between 20000 and 33000 values two CTAs are 0.94 .. 1.07 times as fast from 4096 rows on, and 0.95 .. 1.23 at
+    // 1536 and 2400 rows; at 16400 values 0.90 .. 0.98 and 0.97 .. 1.09.)  Where half of the SMs would have no tile, from fewer values on: 512 rows, one CTA -> two with all warps on a tile, 4 columns,
     // 4096 q8_0 8.7 -> 6.6, 5120 q6_K 10.5 -> 8.9; 3072 q4_0 (12288 values) 5.2 -> 5.3.  Two and three columns over 16000 values: level
     // where rows are many (22016 x 8192 q4_K at 2 columns 1.11 and 1.07 of dp4a's speed), 512 x 8192 q6_K at 2 columns 8.6 -> 7.3, q4_0 at 3 8.5 -> 7.0.
     const bool by_rows = N >= 4;
