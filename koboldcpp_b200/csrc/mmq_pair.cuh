@@ -21,7 +21,8 @@
 //     11008 x 4096 q4_K 55.5 -> 49.1.
 //   * where the tiles leave pairs idle, a cluster of up to eight pairs takes one tile, each a part of K; the parts meet in distributed shared memory and are
 //     added in the order of K (pair_merge).  5120 x 5120 over 199 columns, 20 tiles in three parts: q5_K 32.4 -> 21.9 us, q6_K 43 -> 24; 1024 x 4096 q4_K over
-//     300 columns, 12 in four, 19.4 -> 13.6; 256 x 5120 q6_K over 400, 5 in seven, 24.7 -> 13.5.
+//     300 columns, 12 in four, 19.4 -> 13.6; 256 x 5120 q6_K over 400, 5 in seven, 24.7 -> 13.5.  Rows whose tiles are left over behind whole waves are a launch of their own
+//     where that is shorter (mmq_pair_whole_waves).
 //   * BN is chosen on the host so that the tiles fill the pairs evenly (mmq_pair_plan): 512 columns are 2 x 256 or 3 x 176, whichever leaves
 //     the last wave fuller.  In the grouped form (routed experts) the width of every tile follows its rows.
 // Every wait has a limit (MmqParams::wait_limit).  A role whose wait runs out sets `failed` of its CTA and leaves its loop: no store, copy or MMA, and no

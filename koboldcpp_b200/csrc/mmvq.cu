@@ -431,12 +431,12 @@ static int dispatch_cols(MmvqParams &p, int N, cudaStream_t st, bool pdl) {
         }
     }
     // Several columns of one activation matrix: the integer tensor cores, whose cost hardly grows with the columns; dp4a spends 8 instructions a column and 32 weights.
-    // dp4a -> tensor, us, at 2 / 4 / 8 columns: 22016 x 4096 q4_0 25.6 -> 18.8 / 39.1 -> 20.4 / - ; 32000 x 2048 q8_0 25.6 -> 17.5 / 37.2 -> 18.9 / 64.7 -> 21.3;
-    // 32000 x 2048 q4_K 22.8 -> 14.1 at 2; 5120 x 13824 q6_K 36.9 -> 26.9 at 4; 2048 x 2048 q4_0 4.5 -> 4.1 / 6.7 -> 4.7 / 12.1 -> 5.8; 256 x 256 3.7 -> 3.5 / 5.5 -> 3.6 /
-    // 9.5 -> 3.9.  Two and three columns of few rows lose: what bounds such a launch is the way from the first load of the columns to their quants, which is longer here.  Two
-    // columns, 1024 rows of 4096 q4_0 4.9 -> 5.2, q8_0 5.2 -> 6.6, q4_K 4.7 -> 5.3, q5_K 4.8 -> 5.6, q6_K 5.1 -> 6.0; 512 rows of 1536 q5_K 3.6 -> 4.4, 2048 q6_K 3.8 -> 4.2, 5120 q8_0 6.0 -> 7.7,
-    // 6144 6.1 -> 8.7 (0.71, the least of all), 8192 q5_K 6.4 -> 6.8; level at 2048 rows.  Three columns, 512 rows of 4096 q8_0 6.0 -> 7.0, q5_K 5.8 -> 6.3, q6_K 5.8 -> 6.6; level at 1536.  They stay
-    // here, because with fewer than four columns a row's bits do not depend on the rows of its launch: one kernel, cut in one way, has to take few rows and many.
+    // dp4a -> tensor, us, at 2 / 4 / 8 columns: 32000 x 2048 q4_0 24.3 -> 14.3 / 37.4 -> 14.9 / 70.4 -> 17.5, q8_0 25.6 -> 17.1 / 37.2 -> 19.0 / 64.7 -> 21.4; q4_K 22.8 -> 14.1 at 2;
+    // 5120 x 13824 q6_K 36.9 -> 26.1 at 4, 74.6 -> 32.7 at 8; 2048 x 2048 q4_0 4.5 -> 4.0 / 6.7 -> 4.5 / 12.1 -> 5.5; 256 x 256 3.7 -> 3.2 / 5.5 -> 3.2 / 9.5 -> 3.5.
+    // Two and three columns of few rows lose: what bounds such a launch is the way from the first load of the columns to their quants, which is longer here.  Two columns, 1024 rows of
+    // 4096 q4_0 4.82 -> 5.08, q8_0 5.17 -> 6.75, q4_K 4.70 -> 5.31, q5_K 4.76 -> 5.58, q6_K 5.07 -> 6.03; 512 rows of 1536 q5_K 3.62 -> 4.42, 2048 q6_K 3.83 -> 4.20,
+    // 6144 q8_0 6.13 -> 8.70 (the most of all), 8192 q5_K 6.44 -> 6.81; level at 2048 rows.  Three columns, 512 rows of 4096 q8_0 5.98 -> 7.06, q5_K 5.79 -> 6.34, q6_K 5.84 -> 6.65; level at 1536.  They stay here, because with fewer than four columns a row's bits do not depend on the rows
+    // of its launch: one kernel, cut in one way, has to take few rows and many.
     if constexpr (TYPE == B200_TYPE_Q4_0 || TYPE == B200_TYPE_Q8_0 || TYPE == B200_TYPE_Q4_K || TYPE == B200_TYPE_Q5_K || TYPE == B200_TYPE_Q6_K) {
         bool same_x = p.ids == nullptr && p.K % 256 == 0;
         for (int j = 1; j < p.n_jobs; j++) same_x = same_x && p.jobs[j].X == p.jobs[0].X;

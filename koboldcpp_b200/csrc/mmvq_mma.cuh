@@ -272,9 +272,7 @@ __device__ __forceinline__ void mv_block(unsigned r0, unsigned r1, const MvLane<
         const MvRun e0(r0 + 2 + 4 * t4), e1(r1 + 2 + 4 * t4), o0(r0 + 2 + BB + 4 * t4), o1(r1 + 2 + BB + 4 * t4);  // quants of even and odd blocks
         uint2 b = make_uint2(0u, 0u);
         int k[4];
-        // A block's sum by itself, so that the chain of roundings is shorter.  (q4_0 of four columns and fewer adds two or four terms a block, and is 4 % slower so.)
-        constexpr bool OWN = TYPE == B200_TYPE_Q8_0 || NP == 8;
-        float own[4] = {0.f, 0.f, 0.f, 0.f}, *sd = OWN ? own : acc;
+        float sd[4] = {0.f, 0.f, 0.f, 0.f};  // a block's sum by itself: chains of roundings are shorter (1.2e-7 off the exact sum of 5120 values at six columns -> 7.9e-8)
 #pragma unroll
         for (int blk = 0; blk < 8; blk++) {
             const int j = blk % G, set = blk - j, at = 2 * BB * (blk / 2);
@@ -304,7 +302,7 @@ __device__ __forceinline__ void mv_block(unsigned r0, unsigned r1, const MvLane<
                 }
             }
         }
-        if constexpr (OWN) { acc[0] += own[0]; acc[1] += own[1]; acc[2] += own[2]; acc[3] += own[3]; }
+        acc[0] += sd[0]; acc[1] += sd[1]; acc[2] += sd[2]; acc[3] += sd[3];
     }
 }
 
@@ -548,12 +546,18 @@ __global__ void __launch_bounds__(MV_NW * 32, 1) mmvq_mma_kernel(const __grid_co
         for (int i = kp * 32 + lane; i < 128; i += KS * 32) {
             const int r = i & 15, n = i >> 4;
             if (n >= N || ti.row + r >= M) continue;
-            const float *x = all + r * 8 + n;  // (added in pairs: fewer roundings of a row's whole sum)
+            // K-quants in pairs, which rounds less.  (For the others a chain: what pairs do to the registers of their kernels makes 32000 x 1024 q8_0 with two to four columns 6 to 8 %
+            // slower; what the chain does to those of K-quants, 32000 x 8192 q4_K with three and four 10 %.)
+            const float *x = all + r * 8 + n;
             float v = x[0];
-            if (KS == 2) v += x[128];
-            else if (KS >= 4) {
-                v = (v + x[128]) + (x[256] + x[384]);
-                for (int k = 4; k < KS; k += 4) v += (x[k * 128] + x[k * 128 + 128]) + (x[k * 128 + 256] + x[k * 128 + 384]);
+            if constexpr (type_block_values(TYPE) == 256) {
+                if (KS == 2) v += x[128];
+                else if (KS >= 4) {
+                    v = (v + x[128]) + (x[256] + x[384]);
+                    for (int k = 4; k < KS; k += 4) v += (x[k * 128] + x[k * 128 + 128]) + (x[k * 128 + 256] + x[k * 128 + 384]);
+                }
+            } else {
+                for (int k = 1; k < KS; k++) v += x[k * 128];
             }
             if (C > 1) sums[((t - t0) / n_clusters * N + n) * MV_ROWS + r] = v;
             else store(ti, r, n, v);

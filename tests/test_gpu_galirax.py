@@ -89,8 +89,7 @@ def test_qkv_store_bias_norm_rotation_cells(Hh, G, D, V, dims, extra):
 
 @pytest.mark.parametrize("Hh,G,D,V,dims,extra", [(4, 2, 16, 24, 8, True), (5, 5, 10, 6, 10, False), (2, 1, 64, 64, 64, True), (6, 2, 96, 40, 0, True), (1, 1, 7, 5, 2, False)])
 def test_qkv_store_of_a_long_batch(Hh, G, D, V, dims, extra):
-    """More than 64 tokens share a table of sines and cosines among the heads: the values of the same tokens in smaller batches, but for the order of a norm's sum and the
-    rounding of two products (2^-24 each)."""
+    """More than 64 tokens share a table of sines and cosines among the heads: the values of the same tokens in smaller batches, but for the order of a norm's sum."""
     rng = np.random.default_rng(Hh * D + V)
     T, eps = 70, 1e-5
     q, k, v = rng.standard_normal((T, Hh, D)), rng.standard_normal((T, G, D)), rng.standard_normal((T, G, V))
