@@ -808,9 +808,9 @@ static int mmq_pair_launch(const MmqParams &q, int64_t n_pad, int64_t w_rows_per
         std::lock_guard<std::mutex> lock(first);
         if (!dev.known.load(std::memory_order_relaxed)) {
             B200_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, PAIR_SMEM));
-            B200_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+            if (!GROUPED) B200_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
             dev.clusters[1] = sm_count() / 2;
-            for (int ks = 2; ks <= PAIR_MAX_SPLIT; ks++) {
+            for (int ks = 2; !GROUPED && ks <= PAIR_MAX_SPLIT; ks++) {  // (experts take no parts of K)
                 cfg.gridDim = dim3((unsigned)(2 * ks));
                 at[0].val.clusterDim.x = (unsigned)(2 * ks);
                 cfg.numAttrs = 1;
